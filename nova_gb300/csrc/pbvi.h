@@ -55,6 +55,11 @@ struct BackupEngine {
     // Per-step scratch:
     unsigned long long *hash = nullptr;  // [r] row hash of the input Gamma
     unsigned *rep = nullptr;             // [r] lowest index with a bitwise-identical row
+    unsigned long long *dedupKeys = nullptr;  // [dedupCap] hash table of the rows (dedup_hash_kernel)
+    unsigned *dedupLow = nullptr;
+    unsigned *dedupDone = nullptr;       // [1] finished blocks of dedup_rep_kernel
+    unsigned dedupCap = 0;
+    bool dedupClean = false;             // the table is free (left so by a finished dedup)
     unsigned *uniqJ = nullptr;           // [r] unique index -> lowest original index
     unsigned *nUniqueDev = nullptr;      // device scalar
     float *Gt = nullptr;                 // [n][gtCols] transposed unique alphas

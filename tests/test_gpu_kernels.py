@@ -1,0 +1,48 @@
+"""Single kernels of the backup at the sizes where their tiles, splits and
+remainders can go wrong, against the oracle (bit for bit)."""
+import numpy as np
+import pytest
+
+from conftest import bits
+from oracle import oracle as orc
+from nova_gb300 import synth
+from nova_gb300.pomdp import POMDP
+from nova_gb300.pomdp_pbvi import POMDPPBVIGPU
+from nova_gb300 import nova_pomdp_pbvi as npp
+
+pytestmark = pytest.mark.gpu
+
+
+def backups(md, mode, steps, table=npp.TABLE_AUTO):
+    """The alphas, actions and statistics after `steps` GPU backups, and the oracle's."""
+    p = POMDP.from_arrays(md)
+    p.initialize_gpu()
+    alg = POMDPPBVIGPU(p, GammaInitial=md["GammaInitial"])
+    alg.set_scoring(mode)
+    alg.set_table(table)
+    stats = []
+    G, Gp, pi = md["GammaInitial"].copy(), md["GammaInitial"].copy(), np.zeros(md["r"], np.uint32)
+    for _ in range(steps):
+        alg.update()
+        stats.append(alg.stats())
+        orc.pbvi_update(md, G, Gp, pi)
+        G, Gp = Gp, G
+    pol = alg.get_policy()
+    return pol.gamma_array(), pol.pi_array(), stats, G, pi
+
+
+@pytest.mark.parametrize("r,n,distinct", [(1, 5, 1), (7, 33, 3), (8, 256, 8), (9, 257, 2), (255, 31, 40),
+                                          (257, 64, 257), (300, 513, 1), (1025, 12, 300)])
+def test_duplicate_alphas(r, n, distinct):
+    """Rows repeated at random: the unique count and the backup's results."""
+    md = synth.random_pomdp(n=n, m=2, z=3, ns=min(4, n), r=r, rz=min(5, n), gamma=0.9, horizon=2, seed=r + n)
+    rng = np.random.default_rng(r * n)
+    pool = rng.normal(-3.0, 1.0, size=(distinct, n)).astype(np.float32)
+    md["GammaInitial"] = pool[rng.integers(0, distinct, r)]
+    if r > 4:   # rows equal up to the sign of a zero are different rows
+        md["GammaInitial"][2] = md["GammaInitial"][1]
+        md["GammaInitial"][1, 0], md["GammaInitial"][2, 0] = 0.0, -0.0
+    G, pi, stats, Go, po = backups(md, npp.SCORING_EXACT, 2)
+    assert stats[0]["uniqueAlphas"] == len(np.unique(md["GammaInitial"].view(np.uint32), axis=0))
+    np.testing.assert_array_equal(bits(G), bits(Go))
+    np.testing.assert_array_equal(pi, po)

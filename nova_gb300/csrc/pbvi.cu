@@ -29,6 +29,7 @@
 
 #include <vector>
 #include <algorithm>
+#include <type_traits>
 
 #include <nova/constants.h>
 #include <nova/pomdp/algorithms/pomdp_pbvi_cpu.h>
@@ -614,29 +615,44 @@ __global__ void __launch_bounds__(256) proj_kernel(DevModel md, const unsigned *
 
 // The state-contiguous layout [m][z][uRows][sCols] (see proj_state_lanes_kernel).
 constexpr unsigned kProjTileS = 8;
-constexpr unsigned kStateMajorMinStates = 1024;
-constexpr int kProjUPL = 2;  // alphas per lane of the state-contiguous projection
+constexpr size_t kProjSmemMax = 200 * 1024;
 
 // State-contiguous table, register form: one block per (a, 8 consecutive
 // states) and column range of the alphas; lane (sl, ul) of every warp owns
-// state s0 + sl and UPL alphas (the block's 8 warps cover 32*UPL alphas per
-// step). Each lane reads its state's coefficients from shared memory
-// (per-state blocks padded by 4 floats, so the 8 states of a warp fall in
-// distinct banks) and keeps 32 observations' sums in registers; for every
-// (o, alpha) the 8 lanes of one alpha write the 8 states' values as one
-// 32-byte sector, straight from registers. Successor lists are staged
-// successor-major ([l][8 states]), so the 8 states' l-th successors sit in
-// 8 banks, and each lane's transposed-alpha gathers run two successors
-// ahead of the arithmetic.
-template <int ZC, int UPL>
-__global__ void __launch_bounds__(256, UPL == 1 ? 3 : 2) proj_state_lanes_kernel(
+// state s0 + sl and UPL adjacent alphas. Each lane reads its state's
+// coefficients from shared memory (per-state blocks padded by 4 floats, so
+// the 8 states of a warp fall in distinct banks) and keeps ZC observations'
+// sums of its alphas in registers; for every (o, alpha) the 8 lanes of one
+// alpha write the 8 states' values as one 32-byte sector, straight from
+// registers. Successor lists are staged successor-major ([l][8 states]), so
+// the 8 states' l-th successors sit in 8 banks, and each lane's vector
+// gathers of the transposed alphas run two successors ahead of the
+// arithmetic. Bound by FP32 issue (f32x2: 38 T operations/s measured) and by
+// the load/store unit's wavefronts (at z = 24 both over 50 % busy): one
+// vector gather per lane, guard-free stores for whole tiles and about eight
+// rounds of blocks took n = 512 (z = 16, r = 1,024) from 192 to 136 us, n =
+// 1,000 (z = 11, r = 1,500) from 332 to 188 us and n = 4,096 (z = 32, m = 16,
+// r = 4,096) from 29.6 to 23.2 ms.
+template <int UPL>
+__device__ __forceinline__ void load_alphas(const float *__restrict__ p, float (&g)[UPL]) {
+    if constexpr (UPL == 4) {
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
+        g[0] = v.x; g[1] = v.y; g[2] = v.z; g[3] = v.w;
+    } else {
+        const float2 v = __ldg(reinterpret_cast<const float2 *>(p));
+        g[0] = v.x; g[1] = v.y;
+    }
+}
+
+template <int ZC, int UPL, int THREADS, int BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS) proj_state_lanes_kernel(
         DevModel md, const unsigned *__restrict__ succLen, const float *__restrict__ C1,
         const float *__restrict__ Gt, size_t gtCols, unsigned nU, float *__restrict__ Proj, size_t uRows,
         size_t sCols, unsigned uRange, float one) {
     extern __shared__ float smem[];
     const unsigned cStride = md.ns * ZC + 4;
     float *Cs = smem;                                                   // [8][cStride]
-    int *Ss = reinterpret_cast<int *>(Cs + (size_t)kProjTileS * cStride);  // [ns][8]
+    int *Ss = reinterpret_cast<int *>(Cs + (size_t)kProjTileS * cStride);  // [ns + 2][8]
     __shared__ unsigned Ls[kProjTileS];
     const unsigned long long one2 = pack_f32x2(one, one);
     const unsigned tilesS = (md.n + kProjTileS - 1) / kProjTileS;
@@ -644,13 +660,14 @@ __global__ void __launch_bounds__(256, UPL == 1 ? 3 : 2) proj_state_lanes_kernel
     const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned sl = lane >> 2, ul = lane & 3;
     const unsigned s = s0 + sl;
-    const bool live = s < md.n;
     const float gamma = md.gamma;
     if (threadIdx.x < kProjTileS)
         Ls[threadIdx.x] = s0 + threadIdx.x < md.n ? succLen[(size_t)(s0 + threadIdx.x) * md.m + a] : 0u;
-    for (unsigned e = threadIdx.x; e < kProjTileS * md.ns; e += blockDim.x) {
-        const unsigned st = e / md.ns, l = e % md.ns;
-        Ss[l * kProjTileS + st] = s0 + st < md.n ? md.S[((size_t)(s0 + st) * md.m + a) * md.ns + l] : 0;
+    for (unsigned e = threadIdx.x; e < kProjTileS * (md.ns + 2); e += blockDim.x) {
+        const unsigned st = e / (md.ns + 2), l = e % (md.ns + 2);
+        int succ = 0;
+        if (s0 + st < md.n && l < md.ns) succ = md.S[((size_t)(s0 + st) * md.m + a) * md.ns + l];
+        Ss[l * kProjTileS + st] = max(succ, 0);  // past a row's end: state 0, gathered and not used
     }
     for (unsigned o0 = 0; o0 < md.z; o0 += ZC) {
         __syncthreads();
@@ -665,39 +682,26 @@ __global__ void __launch_bounds__(256, UPL == 1 ? 3 : 2) proj_state_lanes_kernel
         const float *cw = Cs + (size_t)sl * cStride;
         const int *sw = Ss + sl;
         const unsigned uBegin = blockIdx.y * uRange, uEnd = min(nU, uBegin + uRange);
-        for (unsigned u0 = uBegin + warp * 4u * UPL; u0 < uEnd; u0 += 32u * UPL) {
-            unsigned uu[UPL];
-            bool v[UPL];
-#pragma unroll
-            for (int j = 0; j < UPL; j++) {
-                uu[j] = u0 + ul + 4u * j;
-                v[j] = live && uu[j] < uEnd;
-            }
+        for (unsigned u0 = uBegin + (warp * 4u + ul) * UPL; u0 < uEnd; u0 += (THREADS / 8) * UPL) {
+            // Gt's columns are padded to 32, so a lane's UPL alphas are always readable.
+            const float *gcol = Gt + u0;
             unsigned long long acc[UPL][ZC / 2];
 #pragma unroll
             for (int j = 0; j < UPL; j++)
 #pragma unroll
                 for (int q = 0; q < ZC / 2; q++) acc[j][q] = 0ull;
             float gn[UPL], gn2[UPL];
-            if (L > 0) {
-                const float *grow = Gt + (size_t)sw[0] * gtCols;
-                const float *grow2 = Gt + (size_t)sw[(L > 1 ? 1 : 0) * kProjTileS] * gtCols;
-#pragma unroll
-                for (int j = 0; j < UPL; j++) {
-                    gn[j] = v[j] ? grow[uu[j]] : 0.0f;
-                    gn2[j] = v[j] ? grow2[uu[j]] : 0.0f;
-                }
-            }
+            load_alphas<UPL>(gcol + (size_t)sw[0] * gtCols, gn);
+            load_alphas<UPL>(gcol + (size_t)sw[kProjTileS] * gtCols, gn2);
+#pragma unroll 2
             for (unsigned l = 0; l < L; l++) {
                 unsigned long long gg[UPL];
 #pragma unroll
-                for (int j = 0; j < UPL; j++) gg[j] = pack_f32x2(gn[j], gn[j]);
-                const float *grow = Gt + (size_t)sw[(l + 2 < L ? l + 2 : L - 1) * kProjTileS] * gtCols;
-#pragma unroll
                 for (int j = 0; j < UPL; j++) {
+                    gg[j] = pack_f32x2(gn[j], gn[j]);
                     gn[j] = gn2[j];
-                    gn2[j] = v[j] ? grow[uu[j]] : 0.0f;
                 }
+                load_alphas<UPL>(gcol + (size_t)sw[(l + 2) * kProjTileS] * gtCols, gn2);
                 const ulonglong2 *c2 = reinterpret_cast<const ulonglong2 *>(cw + l * ZC);
 #pragma unroll
                 for (int q4 = 0; q4 < ZC / 4; q4++) {
@@ -709,14 +713,24 @@ __global__ void __launch_bounds__(256, UPL == 1 ? 3 : 2) proj_state_lanes_kernel
                     }
                 }
             }
+            if (s >= md.n) continue;
+            float *out = Proj + (((size_t)a * md.z + o0) * uRows + u0) * sCols + s;
+            const size_t slice = uRows * sCols;
+            if (zc == ZC && u0 + UPL <= uEnd) {
 #pragma unroll
-            for (int q = 0; q < ZC; q++) {
-                if ((unsigned)q < zc) {
+                for (int q = 0; q < ZC; q++) {
+#pragma unroll
+                    for (int j = 0; j < UPL; j++) out[j * sCols] = fmul(f32x2_part(acc[j][q / 2], q & 1), gamma);
+                    out += slice;
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < ZC; q++) {
 #pragma unroll
                     for (int j = 0; j < UPL; j++)
-                        if (v[j])
-                            Proj[(((size_t)a * md.z + o0 + q) * uRows + uu[j]) * sCols + s] =
-                                fmul(f32x2_part(acc[j][q / 2], q & 1), gamma);
+                        if ((unsigned)q < zc && u0 + j < uEnd)
+                            out[j * sCols] = fmul(f32x2_part(acc[j][q / 2], q & 1), gamma);
+                    out += slice;
                 }
             }
         }
@@ -1068,45 +1082,74 @@ bool BackupEngine::ensure_proj(unsigned nU) {
     return true;
 }
 
+// Observations a projection thread keeps in registers: the z observations in
+// ceil(z / 32) equal chunks, rounded up to 4 (one 16-byte coefficient read).
+// Both kernels are bound by FP32 issue, so lanes of padding cost their full
+// share: with chunks of 32 for z >= 16 and of 8 below, z = 16 computed twice
+// and z = 11 half again what it needed (alpha-contiguous, n = 512, z = 16:
+// 201 against 117 us).
+static int proj_chunk(unsigned z) {
+    const unsigned chunks = ceil_div(z, 32);
+    return (int)round_up(ceil_div(z, chunks), 4);
+}
+
+static size_t proj_rows_smem(const DevModel &md, int zc) {
+    return (size_t)md.ns * zc * sizeof(float) + md.ns * sizeof(int);
+}
+static size_t proj_state_smem(const DevModel &md, int zc) {
+    return (size_t)kProjTileS * (md.ns * zc + 4) * sizeof(float) +
+           (size_t)kProjTileS * (md.ns + 2) * sizeof(int);
+}
+
+// f(std::integral_constant<int, ZC>) for zc in {4, 8, ..., 32}.
+template <typename F>
+static void with_chunk(int zc, F f) {
+    switch (zc) {
+        case 4: f(std::integral_constant<int, 4>()); break;
+        case 8: f(std::integral_constant<int, 8>()); break;
+        case 12: f(std::integral_constant<int, 12>()); break;
+        case 16: f(std::integral_constant<int, 16>()); break;
+        case 20: f(std::integral_constant<int, 20>()); break;
+        case 24: f(std::integral_constant<int, 24>()); break;
+        case 28: f(std::integral_constant<int, 28>()); break;
+        default: f(std::integral_constant<int, 32>()); break;
+    }
+}
+
 int BackupEngine::project(unsigned nU, const char *fn) {
+    int zc = proj_chunk(md.z);
     if (projStateMajor) {
-        const unsigned zc = md.z >= 16 ? 32u : 8u;
-        const size_t smem = (size_t)kProjTileS * (md.ns * zc + 4) * sizeof(float) +
-                            (size_t)kProjTileS * md.ns * sizeof(int);
-        if (!projAttrDone) {
-            cudaFuncSetAttribute(proj_state_lanes_kernel<32, kProjUPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            cudaFuncSetAttribute(proj_state_lanes_kernel<8, kProjUPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            cudaFuncSetAttribute(proj_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            cudaFuncSetAttribute(proj_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            projAttrDone = true;
-        }
-        // Column ranges of about 32 MB of the transposed alphas (multiples of 32*UPL).
-        const unsigned uRange = (unsigned)std::max<size_t>(
-            32 * kProjUPL, ((32ull << 20) / ((size_t)md.n * sizeof(float))) / (32 * kProjUPL) * (32 * kProjUPL));
-        const dim3 blocks(md.m * ceil_div(md.n, kProjTileS), ceil_div(std::max(nU, 1u), uRange));
-        if (zc == 32)
-            proj_state_lanes_kernel<32, kProjUPL><<<blocks, 256, smem, stream>>>(md, succLen, C1, Gt, gtCols, nU, Proj,
-                                                                             projCols, projSCols, uRange, 1.0f);
-        else
-            proj_state_lanes_kernel<8, kProjUPL><<<blocks, 256, smem, stream>>>(md, succLen, C1, Gt, gtCols, nU, Proj,
-                                                                            projCols, projSCols, uRange, 1.0f);
+        const size_t smem = proj_state_smem(md, zc);
+        // Column ranges of at most 32 MB of the transposed alphas, and enough
+        // of them for about eight rounds of blocks (multiples of 128).
+        const unsigned tiles = md.m * ceil_div(md.n, kProjTileS);
+        const size_t byL2 = (32ull << 20) / ((size_t)md.n * sizeof(float)) / 128 * 128;
+        const size_t byRounds = round_up(ceil_div((size_t)nU * tiles, 152u * 2u * 8u), 128);
+        const unsigned uRange = (unsigned)std::max<size_t>(128, std::min(byL2, byRounds));
+        const dim3 blocks(tiles, ceil_div(std::max(nU, 1u), uRange));
+        with_chunk(zc, [&](auto c) {
+            // Up to 24 observations' sums of four alphas fit in registers, which
+            // halves the coefficient reads per product; above, two alphas a
+            // lane are faster (z = 30, n = 1,500: 3.2 against 3.7 ms).
+            constexpr int ZC = decltype(c)::value;
+            constexpr int UPL = ZC <= 24 ? 4 : 2, THREADS = ZC <= 24 ? 128 : 256, BLOCKS = ZC <= 24 ? 3 : 2;
+            auto kernel = proj_state_lanes_kernel<ZC, UPL, THREADS, BLOCKS>;
+            if (!projAttrDone) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjSmemMax);
+            kernel<<<blocks, THREADS, smem, stream>>>(md, succLen, C1, Gt, gtCols, nU, Proj, projCols, projSCols, uRange,
+                                                  1.0f);
+        });
+        projAttrDone = true;
         return check_launch(fn, "projection table");
     }
-    const size_t smem32 = (size_t)md.ns * 32 * sizeof(float) + md.ns * sizeof(int);
-    const unsigned blocks = md.m * md.n;
-    if (!projAttrDone) {
-        cudaFuncSetAttribute(proj_state_lanes_kernel<32, kProjUPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(proj_state_lanes_kernel<8, kProjUPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(proj_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(proj_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        projAttrDone = true;
-    }
-    if (md.z >= 16 && smem32 <= 200 * 1024) {
-        proj_kernel<32><<<blocks, 256, smem32, stream>>>(md, succLen, C1, Gt, gtCols, nU, Proj, projCols, 1.0f);
-    } else {
-        const size_t smem8 = (size_t)md.ns * 8 * sizeof(float) + md.ns * sizeof(int);
-        proj_kernel<8><<<blocks, 256, smem8, stream>>>(md, succLen, C1, Gt, gtCols, nU, Proj, projCols, 1.0f);
-    }
+    if (proj_rows_smem(md, zc) > kProjSmemMax) zc = std::min(zc, 8);  // long successor lists
+    const size_t smem = proj_rows_smem(md, zc);
+    with_chunk(zc, [&](auto c) {
+        auto kernel = proj_kernel<decltype(c)::value>;
+        if (!projRowsAttrDone)
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjSmemMax);
+        kernel<<<md.m * md.n, 256, smem, stream>>>(md, succLen, C1, Gt, gtCols, nU, Proj, projCols, 1.0f);
+    });
+    projRowsAttrDone = true;
     return check_launch(fn, "projection table");
 }
 
@@ -1242,18 +1285,15 @@ int BackupEngine::backup_all(const float *src, unsigned rGamma, float *dst, unsi
     useProjNow = ensure_proj(nU);
     const bool wantTc = (scoring == NOVA_SCORING_BF16 || scoring == NOVA_SCORING_FP16) &&
                         tc_supported(md) && nU >= kTcMinUnique && !tcUnavailable;
-    // Tensor-core updates of large models read the table by candidate and by
-    // chosen alpha (assembly reads whole columns) and, in FP16, leave almost
-    // no row to the exact scan, so they use the state-contiguous layout; the
-    // exact scan reads whole rows and keeps the alpha-contiguous one, as do
-    // smaller models and updates after one that left more than 1 % of its
-    // rows to the scan (BF16's wider margin does).
-    {
-        const unsigned zc = md.z >= 16 ? 32u : 8u;
-        const size_t smemSM = (size_t)kProjTileS * (md.ns * zc + 4) * sizeof(float) +
-                              (size_t)kProjTileS * md.ns * sizeof(int);
-        projStateMajor = wantTc && state_major_wanted(smemSM);
-    }
+    // Tensor-core updates read the table by candidate and by chosen alpha
+    // (assembly reads whole columns) and leave few rows to the exact scan, so
+    // they use the state-contiguous layout: its table costs up to a third more
+    // (n = 1,000, z = 11, r = 1,500: 188 against 139 us; n = 512: 136 against
+    // 117), its assembly and action values far less (39 against 205 us; 30
+    // against 128). The exact scan reads whole rows and keeps the
+    // alpha-contiguous one, as do updates after one that left more than 1 % of
+    // its rows to the scan.
+    projStateMajor = wantTc && state_major_wanted();
     if (useProjNow && (rc = project(nU, fn)) != NOVA_SUCCESS) return rc;
     if (wantTc && tc == nullptr && tc_build(*this, fn) != NOVA_SUCCESS) tcUnavailable = true;
     cudaEventRecord(ev[2], stream);
@@ -1305,8 +1345,8 @@ int BackupEngine::backup_all(const float *src, unsigned rGamma, float *dst, unsi
     return NOVA_SUCCESS;
 }
 
-bool BackupEngine::state_major_wanted(size_t smemSM) const {
-    return md.n > kStateMajorMinStates && smemSM <= 200 * 1024 &&
+bool BackupEngine::state_major_wanted() const {
+    return proj_state_smem(md, proj_chunk(md.z)) <= kProjSmemMax &&
            (scoring == NOVA_SCORING_FP16 || scoring == NOVA_SCORING_BF16) && lastScanFrac <= 0.01f;
 }
 
@@ -1326,12 +1366,7 @@ int BackupEngine::fixed_pre(const float *src, bool tensor, const char *fn) {
     if ((rc = check_launch(fn, "alpha transpose")) != NOVA_SUCCESS) return rc;
     useProjNow = ensure_proj(nU);
     if (!useProjNow) return NOVA_ERROR_KERNEL_EXECUTION;
-    {
-        const unsigned zc = md.z >= 16 ? 32u : 8u;
-        const size_t smemSM = (size_t)kProjTileS * (md.ns * zc + 4) * sizeof(float) +
-                              (size_t)kProjTileS * md.ns * sizeof(int);
-        projStateMajor = tensor && state_major_wanted(smemSM);
-    }
+    projStateMajor = tensor && state_major_wanted();
     if ((rc = project(nU, fn)) != NOVA_SUCCESS) return rc;
     return tensor ? tc_prepare(*this, src, nU, fn) : NOVA_SUCCESS;
 }

@@ -46,3 +46,21 @@ def test_duplicate_alphas(r, n, distinct):
     assert stats[0]["uniqueAlphas"] == len(np.unique(md["GammaInitial"].view(np.uint32), axis=0))
     np.testing.assert_array_equal(bits(G), bits(Go))
     np.testing.assert_array_equal(pi, po)
+
+
+@pytest.mark.parametrize("mode", [npp.SCORING_FP16, npp.SCORING_EXACT])
+@pytest.mark.parametrize("n,z,ns,r", [(33, 1, 5, 40), (64, 3, 1, 61), (70, 5, 7, 130), (31, 8, 31, 257),
+                                      (130, 13, 9, 100), (65, 17, 6, 97), (40, 24, 8, 131), (57, 25, 3, 66),
+                                      (90, 32, 16, 129), (41, 33, 5, 50), (48, 71, 4, 35)])
+def test_projection_chunks(n, z, ns, r, mode):
+    """Observation chunks of every width, state tiles with remainders, alpha
+    counts that are no multiple of a lane's share, successor rows of every
+    length (also none): both layouts of the projection table."""
+    md = synth.random_pomdp(n=n, m=2, z=z, ns=ns, r=r, rz=min(6, n), gamma=0.9, horizon=2, seed=n * z + r)
+    rng = np.random.default_rng(n + z)
+    length = rng.integers(0, ns + 1, size=(n, 2, 1))
+    md["S"] = np.where(np.arange(ns) < length, md["S"], -1).astype(np.int32)
+    md["GammaInitial"] = rng.normal(-3.0, 1.0, size=(r, n)).astype(np.float32)
+    G, pi, stats, Go, po = backups(md, mode, 2)
+    np.testing.assert_array_equal(bits(G), bits(Go))
+    np.testing.assert_array_equal(pi, po)

@@ -80,7 +80,6 @@ constexpr int STAGES = 4;
 constexpr int MAX_TOPK = 32;       // entries per candidate list (layout capacity)
 constexpr int MAX_LISTS = 8;       // candidate lists per row: two per alpha group
 constexpr int MAX_ENTRIES = MAX_LISTS * MAX_TOPK;
-constexpr int kLaneEntries = MAX_ENTRIES / 32;   // list entries per lane in the merge
 constexpr unsigned kNoneU = 0xffffffffu;
 constexpr int A_STAGE_BYTES = BM * BK * 2;   // 16 KB
 constexpr int B_STAGE_BYTES = BN * BK * 2;   // 32 KB
@@ -107,7 +106,7 @@ struct TcState {
     unsigned *rowFlag = nullptr;    // [MZ*r] rows needing the exact scan
     unsigned *rowCand = nullptr;    // [MZ*r] alphas each row re-scored exactly in the merge
     unsigned *rowList = nullptr;    // [MZ*r] their indices, compacted
-    unsigned *chunkCount = nullptr; // [ceil(MZ*r / 4096)] flagged rows per chunk, then chunk offsets
+    unsigned *chunkCount = nullptr; // [ceil(MZ*r / 4096)] flagged rows per chunk
     unsigned *badModel = nullptr;   // [1] set when a probability is negative or NaN
     PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     CUtensorMap tmA;
@@ -836,24 +835,6 @@ __global__ void tc_escale_kernel(unsigned *scal, float U, float gN) {
 // whose candidate set may be incomplete go to the exact row scan.
 // ---------------------------------------------------------------------------
 
-// score(u) = sum_k fl(Proj[s_k][u] * b_k) in support order
-// (pomdp_pbvi_cpu.cpp:50-83). Eight table entries are fetched before their
-// eight ordered additions, so the gathers overlap.
-__device__ __forceinline__ float proj_row_score(const float *__restrict__ P, const ProjView &pv, unsigned u,
-                                                const float *__restrict__ bk, const int *__restrict__ sk, unsigned Li) {
-    float v = 0.0f;
-    unsigned k = 0;
-    for (; k + 8 <= Li; k += 8) {
-        float pq[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) pq[q] = P[pv.at((unsigned)sk[k + q], u)];
-#pragma unroll
-        for (int q = 0; q < 8; q++) v = fadd(v, fmul(pq[q], bk[k + q]));
-    }
-    for (; k < Li; k++) v = fadd(v, fmul(P[pv.at((unsigned)sk[k], u)], bk[k]));
-    return v;
-}
-
 // Without the projection table: the same exact scores straight from the
 // model and the alpha rows, in the table's order: each support state's
 // entry fl(gamma * sum_l C * alpha(S)) (proj_state_lanes_kernel; C3 holds the
@@ -877,100 +858,141 @@ struct DirectScorer {
 
 // One warp per row; returns (in every lane) the number of candidates it
 // re-scored exactly, 0 when the row was settled without re-scoring or sent to
-// the exact scan. The row's lists hold K entries each; entry e of the warp's
-// view is entry e / nLists of list e % nLists, so the lists' leading entries
-// (where the candidates are) spread over the lanes.
-template <bool kDirect>
-__device__ __forceinline__ unsigned merge_row(size_t row, unsigned lane, DevModel md,
-                                              const unsigned *__restrict__ suppLen, const ProjView pv,
-                                              const DirectScorer ds, float *scratch,
+// the exact scan (*flagged). The row's lists hold K entries each; entry e of
+// the warp's view is entry e / nLists of list e % nLists, so the lists'
+// leading entries (where the candidates are) spread over the lanes. NE:
+// entries per lane, at least nLists * K / 32.
+//
+// Bound by the latency of dependent loads (lists, then the candidates' table
+// entries), so what a row needs before its candidates are known is loaded at
+// once, the candidates are scored together (each lane gathers one support
+// state's entry of up to kMergeBatch candidates before any is used, and lane
+// t adds candidate t's products in support order from shared memory), and
+// the entries per lane are fitted to the lists, which lets 40 warps share an
+// SM instead of 16: n = 512 (131,072 rows, 1.4 candidates each) 204 to 90 us,
+// n = 4,096 (2.1 M rows, 6.2 each) 6.2 to 5.3 ms, the latter near the DRAM
+// time of its 32-byte sectors.
+constexpr unsigned kMergeBatch = 8;    // candidates gathered together
+constexpr unsigned kMergePitch = 33;   // shared-memory row of one candidate's products
+
+template <bool kDirect, int NE>
+__device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const DevModel &md,
+                                              const unsigned *__restrict__ suppLen, const ProjView &pv,
+                                              const DirectScorer &ds, float *scratch, unsigned *list,
                                               const unsigned *__restrict__ uniqJ, unsigned nLists,
                                               unsigned K, size_t rPad, const float *__restrict__ a1,
                                               const float *__restrict__ d1,
                                               const float *__restrict__ a1raw, const unsigned *__restrict__ scal,
                                               const float *__restrict__ candV, const unsigned *__restrict__ candU,
                                               const float *__restrict__ candX, unsigned *__restrict__ ustar,
-                                              unsigned *__restrict__ jstar, unsigned *__restrict__ rowFlag,
+                                              unsigned *__restrict__ jstar, bool *flagged,
                                               const unsigned *__restrict__ badModel) {
-    const unsigned ao = (unsigned)(row / md.r), i = (unsigned)(row % md.r);
+    const unsigned ao = row / md.r, i = row % md.r;
     const unsigned a = ao / md.z, o = ao % md.z;
-    const size_t base = row * MAX_ENTRIES;
-    const unsigned nEnt = nLists * K;     // <= MAX_ENTRIES: each lane holds entries lane + 32 j, j < kLaneEntries
-    float v[kLaneEntries];
-    unsigned u[kLaneEntries];
-    float tmax = -INFINITY;
+    const size_t base = (size_t)row * MAX_ENTRIES;
+    const unsigned nEnt = nLists * K;
+    float v[NE];
+    unsigned u[NE];
 #pragma unroll
-    for (int j = 0; j < kLaneEntries; j++) {
+    for (int j = 0; j < NE; j++) {
         const unsigned e = lane + 32u * j;
         v[j] = -INFINITY;
         u[j] = kNoneU;
         if (e < nEnt) {
             const size_t idx = base + (size_t)(e % nLists) * MAX_TOPK + e / nLists;
-            u[j] = candU[idx];
-            if (u[j] != kNoneU) v[j] = candV[idx];
+            u[j] = __ldg(candU + idx);
+            v[j] = __ldg(candV + idx);
         }
+    }
+    float x = lane < nLists ? __ldg(candX + (size_t)row * MAX_LISTS + lane) : -INFINITY;
+    const float thr = row_margin(a1, d1, (size_t)ao * rPad + i, __uint_as_float(scal[2]), __uint_as_float(scal[7]));
+    const float rawBound = a1raw[(size_t)ao * rPad + i] * __uint_as_float(scal[1]);
+    const unsigned Li = suppLen[i];
+    const int *sk = md.Z + (size_t)i * md.rz;
+    const float *bk = md.B + (size_t)i * md.rz;
+    const unsigned s0 = lane < Li ? (unsigned)__ldg(sk + lane) : 0u;
+    const float b0 = lane < Li ? __ldg(bk + lane) : 0.0f;
+    float tmax = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < NE; j++) {
+        if (u[j] == kNoneU) v[j] = -INFINITY;
         tmax = fmaxf(tmax, v[j]);
     }
-    float x = lane < nLists ? candX[row * MAX_LISTS + lane] : -INFINITY;
     for (int off = 16; off > 0; off >>= 1) {
         tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, off));
         x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, off));
     }
-    const float thr = row_margin(a1, d1, (size_t)ao * rPad + i, __uint_as_float(scal[2]), __uint_as_float(scal[7]));
     // Usable only with a finite margin, non-negative probabilities, and
     // scores far from the reference's -1e10 sentinel.
-    const float Gmax = __uint_as_float(scal[1]);
-    const bool usable = (thr < 1e30f) && (tmax > -INFINITY) && *badModel == 0u &&
-                        (a1raw[(size_t)ao * rPad + i] * Gmax < 1e9f);
+    const bool usable = (thr < 1e30f) && (tmax > -INFINITY) && *badModel == 0u && (rawBound < 1e9f);
     const float cut = tmax - thr;
     if (!usable || x >= cut) {
-        if (lane == 0) rowFlag[row] = 1u;
+        *flagged = true;
         return 0u;
     }
-    bool c[kLaneEntries];
-    unsigned count = 0, first = kNoneU;
+    // The candidates, listed in shared memory.
+    unsigned count = 0;
 #pragma unroll
-    for (int j = 0; j < kLaneEntries; j++) {
-        c[j] = u[j] != kNoneU && v[j] >= cut;
-        const unsigned msk = __ballot_sync(0xffffffffu, c[j]);
+    for (int j = 0; j < NE; j++) {
+        const bool c = u[j] != kNoneU && v[j] >= cut;
+        const unsigned msk = __ballot_sync(0xffffffffu, c);
+        if (c) list[count + __popc(msk & ((1u << lane) - 1u))] = u[j];
         count += __popc(msk);
-        if (first == kNoneU && msk) first = 32u * j + __ffs(msk) - 1;
     }
+    __syncwarp();
     const size_t js = ((size_t)i * md.m + a) * md.z + o;
     if (count == 1) {
-        const unsigned src = first & 31u, jj = first >> 5;
-        unsigned mine = u[0];
-#pragma unroll
-        for (int j = 1; j < kLaneEntries; j++)
-            if (jj == (unsigned)j) mine = u[j];
-        const unsigned uu = __shfl_sync(0xffffffffu, mine, src);
-        if (lane == 0) { ustar[js] = uu; jstar[js] = uniqJ[uu]; }
+        if (lane == 0) {
+            const unsigned uu = list[0];
+            ustar[js] = uu;
+            jstar[js] = uniqJ[uu];
+        }
         return 0u;
     }
-    const unsigned Li = suppLen[i];
-    const int *sk = md.Z + (size_t)i * md.rz;
-    const float *bk = md.B + (size_t)i * md.rz;
+    // Several candidates: re-scored in the exact order, up to 32 at a time
+    // (candidate t of the batch in lane t).
     float best = -INFINITY;
     unsigned bu = kNoneU;
-    if constexpr (!kDirect) {
-        // Several candidates: each lane re-scores its own in the exact order.
-        const float *P = pv.slab(ao);
+    unsigned myU = kNoneU, nb = 0;
+    auto settle = [&](float total) {
+        if (lane < nb && (bu == kNoneU || total > best || (total == best && myU < bu))) { best = total; bu = myU; }
+    };
+    auto score_batch = [&]() {
+        if constexpr (!kDirect) {
+            const float *P = pv.slab(ao);
+            float total = 0.0f;
+            for (unsigned t0 = 0; t0 < nb; t0 += kMergeBatch) {
+                const unsigned nt = min(kMergeBatch, nb - t0);
+                for (unsigned k0 = 0; k0 < Li; k0 += 32u) {
+                    const unsigned k = k0 + lane;
+                    const bool kv = k < Li;
+                    const unsigned s = k0 == 0 ? s0 : (kv ? (unsigned)__ldg(sk + k) : 0u);
+                    const float b = k0 == 0 ? b0 : (kv ? __ldg(bk + k) : 0.0f);
+                    float pq[kMergeBatch];
 #pragma unroll
-        for (int j = 0; j < kLaneEntries; j++) {
-            if (c[j]) {
-                const float w = proj_row_score(P, pv, u[j], bk, sk, Li);
-                if (bu == kNoneU || w > best || (w == best && u[j] < bu)) { best = w; bu = u[j]; }
+                    for (unsigned t = 0; t < kMergeBatch; t++) {
+                        const unsigned uu = __shfl_sync(0xffffffffu, myU, t0 + t);
+                        pq[t] = t < nt && kv ? __ldg(P + pv.at(s, uu)) : 0.0f;
+                    }
+#pragma unroll
+                    for (unsigned t = 0; t < kMergeBatch; t++)
+                        if (t < nt) scratch[t * kMergePitch + lane] = fmul(pq[t], b);
+                    __syncwarp();
+                    if (lane >= t0 && lane < t0 + nt) {
+                        const float *mine = scratch + (lane - t0) * kMergePitch;
+                        const unsigned cnt = min(32u, Li - k0);
+#pragma unroll 8
+                        for (unsigned q = 0; q < cnt; q++) total = fadd(total, mine[q]);
+                    }
+                    __syncwarp();
+                }
             }
-        }
-    } else {
-        // Without the table the warp scores its candidates together, up to
-        // 32 at a time (candidate t held by lane t): for every 32 support
-        // states, lane k computes state k's term for each candidate of the
-        // batch into the warp's scratch (the gathers of one candidate stay
-        // in one alpha row), then lane t adds candidate t's terms in support
-        // order.
-        unsigned myU = kNoneU, nb = 0;
-        auto flush = [&]() {
+            settle(total);
+        } else {
+            // The gathers of one candidate stay within one alpha row: lane k
+            // computes support state k's term of every candidate of the
+            // batch into the warp's scratch, then lane t adds candidate t's
+            // terms in support order.
             float total = 0.0f;
             for (unsigned k0 = 0; k0 < Li; k0 += 32u) {
                 const unsigned k = k0 + lane;
@@ -1032,42 +1054,36 @@ __device__ __forceinline__ unsigned merge_row(size_t row, unsigned lane, DevMode
                 }
                 __syncwarp();
             }
-            if (lane < nb && (bu == kNoneU || total > best || (total == best && myU < bu))) { best = total; bu = myU; }
-            nb = 0;
-        };
-#pragma unroll
-        for (int j = 0; j < kLaneEntries; j++) {
-            unsigned msk = __ballot_sync(0xffffffffu, c[j]);
-            while (msk) {
-                const unsigned src = __ffs(msk) - 1;
-                msk &= msk - 1;
-                const unsigned uu = __shfl_sync(0xffffffffu, u[j], src);
-                if (lane == nb) myU = uu;
-                if (++nb == 32u) flush();
-            }
+            settle(total);
         }
-        if (nb) flush();
+    };
+    for (unsigned f = 0; f < count; f += 32u) {
+        nb = min(32u, count - f);
+        myU = lane < nb ? list[f + lane] : kNoneU;
+        score_batch();
     }
     for (int off = 16; off > 0; off >>= 1) {
         const float b2 = __shfl_xor_sync(0xffffffffu, best, off);
         const unsigned u2 = __shfl_xor_sync(0xffffffffu, bu, off);
         if (u2 != kNoneU && (bu == kNoneU || b2 > best || (b2 == best && u2 < bu))) { best = b2; bu = u2; }
     }
-    if (lane == 0) {
-        if (!(best > -1e10f)) {
-            rowFlag[row] = 1u;  // sentinel case: the exact scan applies the reference's rule
-        } else {
-            ustar[js] = bu;
-            jstar[js] = uniqJ[bu];
-        }
+    if (!(best > -1e10f)) {
+        *flagged = true;  // sentinel case: the exact scan applies the reference's rule
+    } else if (lane == 0) {
+        ustar[js] = bu;
+        jstar[js] = uniqJ[bu];
     }
     return count;
 }
 
 // Rows re-scored and candidates re-scored are counted per block in shared
-// memory, then added to the global counters once per block.
-template <bool kDirect>
-__global__ void __launch_bounds__(256, kDirect ? 1 : 2) tc_merge_kernel(DevModel md, const unsigned *__restrict__ suppLen,
+// memory, then added to the global counters once per block; rows left to the
+// exact scan are flagged and counted per compaction chunk.
+constexpr unsigned kCompactChunk = 4096;  // rows per block of the compaction (4 per thread)
+
+template <bool kDirect, int NE>
+__global__ void __launch_bounds__(256, kDirect ? 1 : NE <= 4 ? 5 : 4) tc_merge_kernel(
+                                DevModel md, const unsigned *__restrict__ suppLen,
                                 const ProjView pv, const DirectScorer ds, const unsigned *__restrict__ uniqJ,
                                 unsigned nLists, unsigned K,
                                 size_t rPad, const float *__restrict__ a1, const float *__restrict__ d1,
@@ -1076,23 +1092,32 @@ __global__ void __launch_bounds__(256, kDirect ? 1 : 2) tc_merge_kernel(DevModel
                                 const float *__restrict__ candX, unsigned *__restrict__ ustar,
                                 unsigned *__restrict__ jstar, unsigned *__restrict__ rowFlag,
                                 unsigned *__restrict__ rowCand, unsigned *__restrict__ counters,
-                                const unsigned *__restrict__ badModel) {
+                                unsigned *__restrict__ chunkCount, const unsigned *__restrict__ badModel) {
     __shared__ unsigned blockCount[2];
-    extern __shared__ float mergeScratch[];  // direct form: [warps][32 candidates][32 states]
+    // Direct form: [warps][32 candidates][32 states]; otherwise [warps][kMergeBatch][kMergePitch].
+    extern __shared__ float mergeScratch[];
+    // Then each warp's candidate list.
+    constexpr unsigned kWarpScratch = kDirect ? 1024u : kMergeBatch * kMergePitch;
     if (threadIdx.x == 0) { blockCount[0] = 0u; blockCount[1] = 0u; }
     __syncthreads();
-    const unsigned lane = threadIdx.x & 31;
-    const size_t row = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const size_t rows = (size_t)md.m * md.z * md.r;
-    unsigned rescored = 0;
-    if (row < rows)
-        rescored = merge_row<kDirect>(row, lane, md, suppLen, pv, ds, mergeScratch + (threadIdx.x >> 5) * 1024u,
-                                      uniqJ, nLists, K, rPad, a1, d1, a1raw, scal, candV, candU, candX, ustar, jstar,
-                                      rowFlag, badModel);
-    if (lane == 0 && row < rows) rowCand[row] = rescored;
-    if (lane == 0 && rescored) {
-        atomicAdd(&blockCount[0], 1u);
-        atomicAdd(&blockCount[1], rescored);
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned row = blockIdx.x * 8u + warp;  // fewer than 2^31 rows (tc_supported)
+    if (row < md.m * md.z * md.r) {
+        bool flagged = false;
+        unsigned *list = reinterpret_cast<unsigned *>(mergeScratch + 8u * kWarpScratch) + warp * (NE * 32u);
+        const unsigned rescored =
+            merge_row<kDirect, NE>(row, lane, md, suppLen, pv, ds, mergeScratch + warp * kWarpScratch, list, uniqJ,
+                                   nLists, K, rPad, a1, d1, a1raw, scal, candV, candU, candX, ustar, jstar,
+                                   &flagged, badModel);
+        if (lane == 0) {
+            rowCand[row] = rescored;
+            rowFlag[row] = flagged ? 1u : 0u;
+            if (flagged) atomicAdd(chunkCount + row / kCompactChunk, 1u);
+            if (rescored) {
+                atomicAdd(&blockCount[0], 1u);
+                atomicAdd(&blockCount[1], rescored);
+            }
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0 && blockCount[0]) {
@@ -1101,56 +1126,32 @@ __global__ void __launch_bounds__(256, kDirect ? 1 : 2) tc_merge_kernel(DevModel
     }
 }
 
-// List of flagged rows in increasing order, in three launches: flagged rows
-// per chunk of 4096, a one-block scan of the chunk counts, then each chunk
-// writes its rows at its offset.
-constexpr unsigned kCompactChunk = 4096;  // rows per block (4 per thread)
-
-__global__ void __launch_bounds__(1024) tc_compact_count_kernel(const unsigned *__restrict__ flag, unsigned count,
-                                                                unsigned *__restrict__ chunkCount) {
-    const unsigned base = blockIdx.x * kCompactChunk;
+// Indices of the flagged rows in increasing order, from the flagged rows per
+// chunk of kCompactChunk: every block adds up the chunks before its own (at
+// most a few thousand counts) and writes its rows behind them; the last
+// block also stores the total.
+__global__ void __launch_bounds__(1024) tc_compact_write_kernel(const unsigned *__restrict__ flag, unsigned count,
+                                                                const unsigned *__restrict__ chunkCount,
+                                                                unsigned *__restrict__ items,
+                                                                unsigned *__restrict__ nOut) {
+    const unsigned mine = chunkCount[blockIdx.x];
+    const bool lastBlock = blockIdx.x == gridDim.x - 1;
+    if (mine == 0 && !lastBlock) return;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ unsigned wsum[32], before;
     unsigned c = 0;
-    for (unsigned k = threadIdx.x; k < kCompactChunk; k += blockDim.x)
-        if (base + k < count && flag[base + k]) c++;
+    for (unsigned k = threadIdx.x; k < blockIdx.x; k += blockDim.x) c += chunkCount[k];
     for (int off = 16; off > 0; off >>= 1) c += __shfl_xor_sync(0xffffffffu, c, off);
-    __shared__ unsigned ws[32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
+    if (lane == 0) wsum[warp] = c;
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned t = 0;
-        for (unsigned w = 0; w < blockDim.x / 32; w++) t += ws[w];
-        chunkCount[blockIdx.x] = t;
+        for (unsigned w = 0; w < blockDim.x / 32; w++) t += wsum[w];
+        before = t;
+        if (lastBlock) *nOut = t + mine;
     }
-}
-
-// Exclusive scan of chunkCount[0..nChunks) in place; the total goes to *nOut.
-__global__ void __launch_bounds__(1024) tc_compact_scan_kernel(unsigned *__restrict__ chunkCount, unsigned nChunks,
-                                                               unsigned *__restrict__ nOut) {
-    __shared__ unsigned sums[1024];
-    const unsigned per = (nChunks + blockDim.x - 1) / blockDim.x;
-    const unsigned b = threadIdx.x * per, e = min(nChunks, b + per);
-    unsigned s = 0;
-    for (unsigned i = b; i < e; i++) s += chunkCount[i];
-    sums[threadIdx.x] = s;
     __syncthreads();
-    for (unsigned off = 1; off < blockDim.x; off <<= 1) {
-        const unsigned v = threadIdx.x >= off ? sums[threadIdx.x - off] : 0u;
-        __syncthreads();
-        sums[threadIdx.x] += v;
-        __syncthreads();
-    }
-    unsigned run = threadIdx.x ? sums[threadIdx.x - 1] : 0u;
-    for (unsigned i = b; i < e; i++) {
-        const unsigned c = chunkCount[i];
-        chunkCount[i] = run;
-        run += c;
-    }
-    if (threadIdx.x == blockDim.x - 1) *nOut = sums[blockDim.x - 1];
-}
-
-__global__ void __launch_bounds__(1024) tc_compact_write_kernel(const unsigned *__restrict__ flag, unsigned count,
-                                                                const unsigned *__restrict__ chunkStart,
-                                                                unsigned *__restrict__ items) {
+    if (mine == 0) return;
     const unsigned base = blockIdx.x * kCompactChunk + 4u * threadIdx.x;
     unsigned f[4], local = 0;
 #pragma unroll
@@ -1158,13 +1159,11 @@ __global__ void __launch_bounds__(1024) tc_compact_write_kernel(const unsigned *
         f[k] = (base + k < count && flag[base + k]) ? 1u : 0u;
         local += f[k];
     }
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned incl = local;
     for (int off = 1; off < 32; off <<= 1) {
         const unsigned y = __shfl_up_sync(0xffffffffu, incl, off);
         if (lane >= (unsigned)off) incl += y;
     }
-    __shared__ unsigned wsum[32];
     if (lane == 31) wsum[warp] = incl;
     __syncthreads();
     if (warp == 0) {
@@ -1176,7 +1175,7 @@ __global__ void __launch_bounds__(1024) tc_compact_write_kernel(const unsigned *
         wsum[lane] = x;
     }
     __syncthreads();
-    unsigned pos = chunkStart[blockIdx.x] + (warp ? wsum[warp - 1] : 0u) + incl - local;
+    unsigned pos = before + (warp ? wsum[warp - 1] : 0u) + incl - local;
 #pragma unroll
     for (int k = 0; k < 4; k++)
         if (f[k]) items[pos++] = base + k;
@@ -1404,34 +1403,40 @@ int tc_finish(BackupEngine &eng, const char *fn) {
     const DevModel &md = eng.md;
     int rc;
     const size_t rows = (size_t)tc->MZ * md.r;
-    cudaMemsetAsync(tc->rowFlag, 0, rows * sizeof(unsigned), eng.stream);
-    const DirectScorer ds{eng.succLen, eng.C3, tc->src};
-    auto merge = eng.useProjNow ? tc_merge_kernel<false> : tc_merge_kernel<true>;
-    const size_t mergeSmem = eng.useProjNow ? 0 : (256 / 32) * 1024 * sizeof(float);
-    merge<<<(unsigned)ceil_div(rows * 32, 256), 256, mergeSmem, eng.stream>>>(
-        md, eng.suppLen, eng.useProjNow ? eng.proj_view() : ProjView{}, ds, eng.uniqJ, L.lists, L.topk, tc->rPad,
-        tc->a1, tc->d1, tc->a1raw, tc->scal, tc->candV, tc->candU, tc->candX, eng.ustar, eng.jstar, tc->rowFlag,
-        tc->rowCand, tc->scal + 3, tc->badModel);
-    if ((rc = check_launch(fn, "candidate merge")) != NOVA_SUCCESS) return rc;
     // The list can hold every row: it is sized m*z*r like the flags.
     const unsigned nChunks = ceil_div(rows, kCompactChunk);
-    tc_compact_count_kernel<<<nChunks, 1024, 0, eng.stream>>>(tc->rowFlag, (unsigned)rows, tc->chunkCount);
-    if ((rc = check_launch(fn, "exact-scan list (count)")) != NOVA_SUCCESS) return rc;
-    tc_compact_scan_kernel<<<1, 1024, 0, eng.stream>>>(tc->chunkCount, nChunks, eng.itemCount);
-    if ((rc = check_launch(fn, "exact-scan list (scan)")) != NOVA_SUCCESS) return rc;
+    cudaMemsetAsync(tc->chunkCount, 0, nChunks * sizeof(unsigned), eng.stream);
+    const DirectScorer ds{eng.succLen, eng.C3, tc->src};
+    // Entries per lane: the fewest that hold the row's lists.
+    const unsigned perLane = ceil_div(L.lists * L.topk, 32);
+    const bool table = eng.useProjNow;
+    const unsigned NE = !table ? 8u : perLane <= 1 ? 1u : perLane <= 2 ? 2u : perLane <= 4 ? 4u : 8u;
+    const size_t mergeSmem = 8 * ((table ? kMergeBatch * kMergePitch : 1024u) + NE * 32u) * sizeof(float);
+    auto merge = !table ? tc_merge_kernel<true, 8>
+                 : NE == 1u ? tc_merge_kernel<false, 1>
+                 : NE == 2u ? tc_merge_kernel<false, 2>
+                 : NE == 4u ? tc_merge_kernel<false, 4> : tc_merge_kernel<false, 8>;
+    merge<<<(unsigned)ceil_div(rows * 32, 256), 256, mergeSmem, eng.stream>>>(
+        md, eng.suppLen, table ? eng.proj_view() : ProjView{}, ds, eng.uniqJ, L.lists, L.topk, tc->rPad,
+        tc->a1, tc->d1, tc->a1raw, tc->scal, tc->candV, tc->candU, tc->candX, eng.ustar, eng.jstar, tc->rowFlag,
+        tc->rowCand, tc->scal + 3, tc->chunkCount, tc->badModel);
+    if ((rc = check_launch(fn, "candidate merge")) != NOVA_SUCCESS) return rc;
     tc_compact_write_kernel<<<nChunks, 1024, 0, eng.stream>>>(tc->rowFlag, (unsigned)rows, tc->chunkCount,
-                                                              tc->rowList);
-    return check_launch(fn, "exact-scan list (write)");
+                                                              tc->rowList, eng.itemCount);
+    return check_launch(fn, "exact-scan list");
 }
 
-// Flag the (belief, action) item of every listed row.
+// Flag the (belief, action) item of every listed row; each item is counted
+// once, in its compaction chunk.
 __global__ void tc_row_items_kernel(const unsigned *__restrict__ rowList, unsigned nRows, unsigned r, unsigned m,
-                                    unsigned z, unsigned *__restrict__ itemFlag) {
+                                    unsigned z, unsigned *__restrict__ itemFlag,
+                                    unsigned *__restrict__ chunkCount) {
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nRows) return;
     const unsigned row = rowList[t];
     const unsigned ao = row / r, i = row % r;
-    itemFlag[(size_t)i * m + ao / z] = 1u;
+    const size_t item = (size_t)i * m + ao / z;
+    if (atomicExch(itemFlag + item, 1u) == 0u) atomicAdd(chunkCount + item / kCompactChunk, 1u);
 }
 
 // The distinct (belief, action) items of the listed rows, in increasing
@@ -1442,17 +1447,15 @@ int tc_rows_to_items(BackupEngine &eng, const unsigned *rowList, unsigned nRows,
     const DevModel &md = eng.md;
     const unsigned count = md.r * md.m;
     int rc;
-    cudaMemsetAsync(tc->rowFlag, 0, (size_t)count * sizeof(unsigned), eng.stream);
-    tc_row_items_kernel<<<ceil_div(nRows, 256), 256, 0, eng.stream>>>(rowList, nRows, md.r, md.m, md.z,
-                                                                      tc->rowFlag);
-    if ((rc = check_launch(fn, "rows to items")) != NOVA_SUCCESS) return rc;
     const unsigned nChunks = ceil_div(count, kCompactChunk);
-    tc_compact_count_kernel<<<nChunks, 1024, 0, eng.stream>>>(tc->rowFlag, count, tc->chunkCount);
-    if ((rc = check_launch(fn, "item list (count)")) != NOVA_SUCCESS) return rc;
-    tc_compact_scan_kernel<<<1, 1024, 0, eng.stream>>>(tc->chunkCount, nChunks, eng.itemCount);
-    if ((rc = check_launch(fn, "item list (scan)")) != NOVA_SUCCESS) return rc;
-    tc_compact_write_kernel<<<nChunks, 1024, 0, eng.stream>>>(tc->rowFlag, count, tc->chunkCount, eng.items);
-    return check_launch(fn, "item list (write)");
+    cudaMemsetAsync(tc->rowFlag, 0, (size_t)count * sizeof(unsigned), eng.stream);
+    cudaMemsetAsync(tc->chunkCount, 0, nChunks * sizeof(unsigned), eng.stream);
+    tc_row_items_kernel<<<ceil_div(nRows, 256), 256, 0, eng.stream>>>(rowList, nRows, md.r, md.m, md.z,
+                                                                      tc->rowFlag, tc->chunkCount);
+    if ((rc = check_launch(fn, "rows to items")) != NOVA_SUCCESS) return rc;
+    tc_compact_write_kernel<<<nChunks, 1024, 0, eng.stream>>>(tc->rowFlag, count, tc->chunkCount, eng.items,
+                                                              eng.itemCount);
+    return check_launch(fn, "item list");
 }
 
 int tc_score_launch(BackupEngine &eng, const float *src, unsigned nU, bool timed, const char *fn) {

@@ -64,3 +64,20 @@ def test_projection_chunks(n, z, ns, r, mode):
     G, pi, stats, Go, po = backups(md, mode, 2)
     np.testing.assert_array_equal(bits(G), bits(Go))
     np.testing.assert_array_equal(pi, po)
+
+
+@pytest.mark.parametrize("table", [npp.TABLE_AUTO, npp.TABLE_NEVER])
+@pytest.mark.parametrize("mode", [npp.SCORING_FP16, npp.SCORING_BF16])
+@pytest.mark.parametrize("r,rz,spread", [(64, 1, 1.0), (300, 31, 1.0), (260, 33, 1e-3), (515, 64, 1e-4),
+                                         (1100, 65, 2e-5), (700, 97, 0.0)])
+def test_merge_candidate_counts(r, rz, spread, mode, table):
+    """Rows with one, a few, more than 8 and more than 32 candidates, up to
+    lists that overflow (alphas that differ by `spread`), over supports
+    around and past multiples of 32."""
+    md = synth.random_pomdp(n=100, m=2, z=3, ns=7, r=r, rz=rz, gamma=0.9, horizon=2, seed=r)
+    rng = np.random.default_rng(r)
+    base = rng.normal(-3.0, 1.0, size=(1, 100))
+    md["GammaInitial"] = (base + max(spread, 1e-7) * rng.normal(size=(r, 100))).astype(np.float32)
+    G, pi, stats, Go, po = backups(md, mode, 2, table)
+    np.testing.assert_array_equal(bits(G), bits(Go))
+    np.testing.assert_array_equal(pi, po)

@@ -81,3 +81,39 @@ def test_merge_candidate_counts(r, rz, spread, mode, table):
     G, pi, stats, Go, po = backups(md, mode, 2, table)
     np.testing.assert_array_equal(bits(G), bits(Go))
     np.testing.assert_array_equal(pi, po)
+
+
+@pytest.mark.parametrize("r,n,count,nz", [(5, 1, 1, 1), (9, 70, 129, 1), (7, 130, 128, 130), (70, 128, 300, 128),
+                                          (131, 61, 257, 30), (130, 100, 400, 0), (6, 7900, 3, 40),
+                                          (5, 15000, 2, 15000), (3, 4097, 140, 2000), (4200, 50, 1400, 50)])
+@pytest.mark.parametrize("odd", [False, True])
+def test_belief_values(r, n, count, nz, odd):
+    """Listed beliefs, dense ones and both in one call (nz 0), one and two
+    planes of alphas and too many states for either, tiles with remainders,
+    arrays at odd addresses, ties, zeros of both signs, and alphas that are
+    not finite."""
+    import torch
+    from nova_gb300 import nova_pomdp_alpha_vectors as npav
+    rng = np.random.default_rng(r * n + count)
+    G = rng.uniform(-5, 5, size=(r, n)).astype(np.float32)
+    if r > 6:
+        G[5] = G[2]
+    if odd:
+        G[r // 2, n // 2], G[r // 3, 0] = np.inf, np.nan
+        G[0, n - 1] = -0.0
+    pi = rng.integers(0, 9, size=r).astype(np.int32)
+    B = np.zeros((count, n), np.float32)
+    for i in range(count):
+        k = nz if nz else (3 if i % 200 < 100 else n)
+        B[i, rng.choice(n, min(k, n), replace=False)] = rng.uniform(0, 1, min(k, n))
+    B[0, 0] = -0.0
+    dG, dB = (torch.as_tensor(np.concatenate([[0], x.ravel()]).astype(np.float32), device="cuda")[1:] for x in (G, B))
+    dPi = torch.as_tensor(pi, device="cuda")
+    dV, dA = torch.empty(count, device="cuda"), torch.empty(count, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert npav._nova.pomdp_alpha_vectors_value_batched_gpu(dG.data_ptr(), dPi.data_ptr(), r, n, dB.data_ptr(), count,
+                                                            dV.data_ptr(), dA.data_ptr()) == 0
+    some = range(count) if count * r * n < 4e6 else rng.choice(count, 40, replace=False)
+    for i in some:
+        V, a = orc.alpha_value(G, pi.astype(np.uint32), B[i])
+        assert bits(dV[i].cpu().numpy()) == bits(np.float32(V)) and int(dA[i]) == a, i

@@ -59,48 +59,180 @@ __global__ void adj_len_kernel(unsigned rows, unsigned ns, const int *__restrict
     len[row] = L;
 }
 
-// C3[a][o][s][l] = fl(O(a,S(s,a,l),o) * T(s,a,l)) (the reference's first
-// product), 0 past the row end.
-__global__ void adj_coef_kernel(AdjModel md, const unsigned *__restrict__ len, float *__restrict__ C3) {
-    const size_t total = (size_t)md.m * md.z * md.n * md.ns;
+// State-contiguous tables for the replay, so that the 32 states of a warp read
+// consecutive entries: ST[a][l][s] = S(s,a,l) (0 past the row end) and
+// CT[a][o][l][s] = fl(O(a,S(s,a,l),o) * T(s,a,l)), the reference's first
+// product (0 past the row end).
+__global__ void adj_coef_kernel(AdjModel md, const unsigned *__restrict__ len, unsigned *__restrict__ ST,
+                                float *__restrict__ CT) {
+    const size_t total = (size_t)md.m * md.ns * md.n;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const unsigned l = (unsigned)(e % md.ns);
-        size_t t = e / md.ns;
-        const unsigned s = (unsigned)(t % md.n);
-        t /= md.n;
-        const unsigned o = (unsigned)(t % md.z);
-        const unsigned a = (unsigned)(t / md.z);
-        float c = 0.0f;
-        if (l < len[(size_t)s * md.m + a]) {
-            const size_t row = ((size_t)s * md.m + a) * md.ns + l;
-            c = fmul(md.O[((size_t)a * md.n + md.S[row]) * md.z + o], md.T[row]);
+        const unsigned s = (unsigned)(e % md.n);
+        size_t t = e / md.n;
+        const unsigned l = (unsigned)(t % md.ns);
+        const unsigned a = (unsigned)(t / md.ns);
+        const bool live = l < len[(size_t)s * md.m + a];
+        const size_t row = ((size_t)s * md.m + a) * md.ns + l;
+        const unsigned sp = live ? (unsigned)md.S[row] : 0u;
+        const float T = live ? md.T[row] : 0.0f;
+        ST[e] = sp;
+        for (unsigned o = 0; o < md.z; o++)
+            CT[(((size_t)a * md.z + o) * md.ns + l) * md.n + s] =
+                live ? fmul(md.O[((size_t)a * md.n + sp) * md.z + o], T) : 0.0f;
+    }
+}
+
+// Beliefs of one action in groups of kGroup, for the replays of all steps at
+// once (one block per step): group g of step t backs up beliefs
+// ids[(t * groups + g) * kGroup ..] (kNoRow: none) with action
+// acts[t * groups + g] (kNoRow: no such group); groups = ceil(r / kGroup) + m.
+constexpr unsigned kGroup = 4;
+
+__global__ void __launch_bounds__(1024) replay_groups_kernel(unsigned r, unsigned m, unsigned groups,
+                                                             const unsigned *__restrict__ act,
+                                                             unsigned *__restrict__ acts, unsigned *__restrict__ ids,
+                                                             unsigned *__restrict__ wideCursor) {
+    extern __shared__ unsigned narrowCursor[];
+    const size_t t = blockIdx.x;
+    // [m] next place of each action's beliefs (in global memory for very many actions)
+    unsigned *cursor = wideCursor != nullptr ? wideCursor + t * m : narrowCursor;
+    act += t * r;
+    acts += t * groups;
+    ids += t * groups * kGroup;
+    for (unsigned a = threadIdx.x; a < m; a += blockDim.x) cursor[a] = 0u;
+    for (unsigned g = threadIdx.x; g < groups; g += blockDim.x) acts[g] = kNoRow;
+    for (unsigned k = threadIdx.x; k < groups * kGroup; k += blockDim.x) ids[k] = kNoRow;
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < r; i += blockDim.x) atomicAdd(cursor + min(act[i], m - 1), 1u);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned g = 0;
+        for (unsigned a = 0; a < m; a++) {
+            const unsigned n = (cursor[a] + kGroup - 1) / kGroup;
+            cursor[a] = g * kGroup;
+            g += n;
         }
-        C3[e] = c;
+    }
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < r; i += blockDim.x) {
+        const unsigned a = min(act[i], m - 1);
+        const unsigned k = atomicAdd(cursor + a, 1u);
+        ids[k] = i;
+        acts[k / kGroup] = a;
     }
 }
 
 // Gamma_t from Gamma_{t-1} with recorded selections, in the reference's
-// order: alpha = R(s,a); for each o, alpha += gamma * sum_l C3 * G_j(S).
-__global__ void replay_kernel(AdjModel md, const unsigned *__restrict__ len, const float *__restrict__ C3,
-                              const float *__restrict__ Gin, const unsigned *__restrict__ act,
-                              const unsigned *__restrict__ sel, float *__restrict__ Gout) {
-    const unsigned i = blockIdx.x;
-    extern __shared__ unsigned jsh[];  // [z]
-    const unsigned a = min(act[i], md.m - 1);
-    for (unsigned o = threadIdx.x; o < md.z; o += blockDim.x) jsh[o] = min(sel[(size_t)i * md.z + o], md.r - 1);
-    __syncthreads();
-    for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) {
-        float alpha = md.R[(size_t)s * md.m + a];
-        const unsigned L = len[(size_t)s * md.m + a];
-        const int *sp = md.S + ((size_t)s * md.m + a) * md.ns;
-        for (unsigned o = 0; o < md.z; o++) {
-            const float *c = C3 + (((size_t)a * md.z + o) * md.n + s) * md.ns;
-            const float *Gj = Gin + (size_t)jsh[o] * md.n;
-            float vt = 0.0f;
-            for (unsigned l = 0; l < L; l++) vt = fadd(vt, fmul(c[l], Gj[sp[l]]));
-            alpha = fadd(alpha, fmul(vt, md.gamma));
+// order: alpha = R(s,a); for each o, alpha += gamma * sum_l CT * G_j(S).
+// One block per (group of beliefs with one action, 1,024 states): the
+// beliefs' alphas of one observation lie in shared memory (the next
+// observation's are copied in meanwhile) and every coefficient is read once
+// for the whole group. Bound by the shared-memory gathers (random states,
+// about 3.5 passes each): 2.7e8 of them (n = r = 1,024, z = ns = 16) take
+// 189 us; one belief per block reading 64-byte coefficient rows per lane
+// and gathering from L1 took 1,490 us.
+constexpr unsigned kReplayThreads = 256;
+constexpr unsigned kReplayStates = 4;  // states per thread
+
+__device__ __forceinline__ void copy_async(float *dst, const float *src, bool wide) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if (wide) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+
+template <bool kShared>
+__global__ void __launch_bounds__(kReplayThreads) replay_kernel(AdjModel md, const unsigned *__restrict__ len,
+                                                                const unsigned *__restrict__ ST,
+                                                                const float *__restrict__ CT,
+                                                                const float *__restrict__ Gin,
+                                                                const unsigned *__restrict__ acts,
+                                                                const unsigned *__restrict__ ids,
+                                                                const unsigned *__restrict__ sel, int wide,
+                                                                float *__restrict__ Gout) {
+    extern __shared__ __align__(16) float rows[];  // [2][kGroup][pitch]
+    const unsigned a = acts[blockIdx.x];
+    if (a == kNoRow) return;
+    const unsigned pitch = (md.n + 3u) & ~3u;
+    unsigned id[kGroup];
+#pragma unroll
+    for (unsigned b = 0; b < kGroup; b++) id[b] = ids[blockIdx.x * kGroup + b];
+    auto chosen = [&](unsigned b, unsigned o) { return Gin + (size_t)min(sel[(size_t)id[b] * md.z + o], md.r - 1) * md.n; };
+    auto stage = [&](unsigned o) {
+        if constexpr (kShared) {
+#pragma unroll
+            for (unsigned b = 0; b < kGroup; b++) {
+                if (id[b] == kNoRow) continue;
+                const float *src = chosen(b, o);
+                float *dst = rows + ((o & 1u) * kGroup + b) * pitch;
+                const unsigned w = wide ? 4u : 1u;
+                for (unsigned s = threadIdx.x * w; s < md.n; s += kReplayThreads * w) copy_async(dst + s, src + s, wide != 0);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
         }
-        Gout[(size_t)i * md.n + s] = alpha;
+    };
+    const unsigned s0 = blockIdx.y * (kReplayThreads * kReplayStates) + threadIdx.x;
+    float alpha[kReplayStates][kGroup];
+    unsigned L[kReplayStates];
+#pragma unroll
+    for (unsigned q = 0; q < kReplayStates; q++) {
+        const unsigned s = s0 + q * kReplayThreads;
+        const bool live = s < md.n;
+        L[q] = live ? len[(size_t)s * md.m + a] : 0u;
+        const float R = live ? md.R[(size_t)s * md.m + a] : 0.0f;
+#pragma unroll
+        for (unsigned b = 0; b < kGroup; b++) alpha[q][b] = R;
+    }
+    stage(0);
+    for (unsigned o = 0; o < md.z; o++) {
+        const float *g[kGroup];
+        if constexpr (kShared) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();  // observation o's rows are in, observation o - 1's free
+            if (o + 1 < md.z) stage(o + 1);
+#pragma unroll
+            for (unsigned b = 0; b < kGroup; b++) g[b] = rows + ((o & 1u) * kGroup + b) * pitch;
+        } else {
+#pragma unroll
+            for (unsigned b = 0; b < kGroup; b++) g[b] = id[b] == kNoRow ? Gin : chosen(b, o);
+        }
+        const float *C = CT + ((size_t)a * md.z + o) * md.ns * md.n;
+        const unsigned *Sa = ST + (size_t)a * md.ns * md.n;
+#pragma unroll
+        for (unsigned q = 0; q < kReplayStates; q++) {
+            const unsigned s = s0 + q * kReplayThreads;
+            float vt[kGroup];
+#pragma unroll
+            for (unsigned b = 0; b < kGroup; b++) vt[b] = 0.0f;
+            for (unsigned l0 = 0; l0 < L[q]; l0 += 4) {
+                float c[4];
+                unsigned sp[4];
+#pragma unroll
+                for (unsigned k = 0; k < 4; k++) {
+                    const bool v = l0 + k < L[q];
+                    c[k] = v ? __ldg(C + (size_t)(l0 + k) * md.n + s) : 0.0f;
+                    sp[k] = v ? __ldg(Sa + (size_t)(l0 + k) * md.n + s) : 0u;
+                }
+#pragma unroll
+                for (unsigned k = 0; k < 4; k++) {
+                    if (l0 + k < L[q]) {
+#pragma unroll
+                        for (unsigned b = 0; b < kGroup; b++)
+                            if (kShared || id[b] != kNoRow) vt[b] = fadd(vt[b], fmul(c[k], g[b][sp[k]]));
+                    }
+                }
+            }
+#pragma unroll
+            for (unsigned b = 0; b < kGroup; b++) alpha[q][b] = fadd(alpha[q][b], fmul(vt[b], md.gamma));
+        }
+    }
+#pragma unroll
+    for (unsigned q = 0; q < kReplayStates; q++) {
+        const unsigned s = s0 + q * kReplayThreads;
+        if (s < md.n) {
+#pragma unroll
+            for (unsigned b = 0; b < kGroup; b++)
+                if (id[b] != kNoRow) Gout[(size_t)id[b] * md.n + s] = alpha[q][b];
+        }
     }
 }
 
@@ -203,12 +335,12 @@ __global__ void adjoint_step_kernel(AdjModel md, const unsigned *__restrict__ le
 }
 
 struct AdjBuffers {
-    unsigned *len = nullptr;
-    float *C3 = nullptr, *seg = nullptr;
+    unsigned *len = nullptr, *ST = nullptr, *acts = nullptr, *ids = nullptr, *cursor = nullptr;
+    float *CT = nullptr, *seg = nullptr;
     double *lamA = nullptr, *lamB = nullptr, *vals = nullptr, *V = nullptr;
     unsigned *istar = nullptr;
     ~AdjBuffers() {
-        cudaFree(len); cudaFree(C3); cudaFree(seg);
+        cudaFree(len); cudaFree(ST); cudaFree(acts); cudaFree(ids); cudaFree(cursor); cudaFree(CT); cudaFree(seg);
         cudaFree(lamA); cudaFree(lamB); cudaFree(vals); cudaFree(V); cudaFree(istar);
     }
 };
@@ -303,7 +435,11 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
     AdjBuffers bf;
     int rc;
     if ((rc = dev_alloc(&bf.len, (size_t)n * m, fn, "the successor lengths")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&bf.C3, (size_t)m * z * n * ns, fn, "the projection coefficients")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&bf.ST, (size_t)m * n * ns, fn, "the successors")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&bf.CT, (size_t)m * z * n * ns, fn, "the projection coefficients")) != NOVA_SUCCESS) return rc;
+    const unsigned groups = ceil_div(r, kGroup) + m;
+    if ((rc = dev_alloc(&bf.acts, (size_t)horizon * groups, fn, "the belief groups")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&bf.ids, (size_t)horizon * groups * kGroup, fn, "the belief groups")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&bf.seg, (size_t)(k + 1) * rn, fn, "the recomputed alphas")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&bf.lamA, rn, fn, "the adjoint")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&bf.lamB, rn, fn, "the adjoint")) != NOVA_SUCCESS) return rc;
@@ -314,8 +450,29 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
 
     adj_len_kernel<<<ceil_div((size_t)n * m, 256), 256>>>(n * m, ns, md.S, bf.len);
     if ((rc = check_launch(fn, "successor lengths")) != NOVA_SUCCESS) return rc;
-    adj_coef_kernel<<<std::min<size_t>(ceil_div((size_t)m * z * n * ns, 256), 65535u * 8u), 256>>>(md, bf.len, bf.C3);
+    adj_coef_kernel<<<std::min<size_t>(ceil_div((size_t)m * n * ns, 256), 65535u * 8u), 256>>>(md, bf.len, bf.ST,
+                                                                                              bf.CT);
     if ((rc = check_launch(fn, "projection coefficients")) != NOVA_SUCCESS) return rc;
+    const bool manyActions = m > 8192;
+    if (manyActions && (rc = dev_alloc(&bf.cursor, (size_t)horizon * m, fn, "the action counts")) != NOVA_SUCCESS)
+        return rc;
+    replay_groups_kernel<<<horizon, 1024, manyActions ? 0 : m * sizeof(unsigned)>>>(r, m, groups, d_actions, bf.acts,
+                                                                                  bf.ids, bf.cursor);
+    if ((rc = check_launch(fn, "belief groups")) != NOVA_SUCCESS) return rc;
+    // Two observations' alphas of a group in shared memory, where they fit;
+    // larger models gather from the alpha rows themselves.
+    const size_t rowsSmem = 2 * (size_t)kGroup * round_up(n, 4) * sizeof(float);
+    const bool rowsShared = rowsSmem + 1024 <= (size_t)optin;
+    if (rowsShared && rowsSmem > 48 * 1024 &&
+            cudaFuncSetAttribute(replay_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rowsSmem) !=
+                cudaSuccess) {
+        cudaGetLastError();
+        NOVA_ERR(fn, "Failed to configure the replay kernel.");
+        return NOVA_ERROR_KERNEL_EXECUTION;
+    }
+    // 16-byte copies where every alpha row starts on a 16-byte boundary (the
+    // segment buffer itself does).
+    const int wide = n % 4u == 0u ? 1 : 0;
     if (cudaMemset(d_dR, 0, (size_t)n * m * sizeof(double)) != cudaSuccess ||
             cudaMemset(d_dT, 0, (size_t)n * m * ns * sizeof(double)) != cudaSuccess ||
             cudaMemset(d_dO, 0, (size_t)m * n * z * sizeof(double)) != cudaSuccess ||
@@ -338,9 +495,11 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
         }
         for (unsigned q = 1; q <= last; q++) {
             const size_t step = base + q - 1;
-            replay_kernel<<<r, 256, z * sizeof(unsigned)>>>(md, bf.len, bf.C3, bf.seg + (size_t)(q - 1) * rn,
-                                                             d_actions + step * r, d_selects + step * r * z,
-                                                             bf.seg + (size_t)q * rn);
+            auto kernel = rowsShared ? replay_kernel<true> : replay_kernel<false>;
+            kernel<<<dim3(groups, ceil_div(n, kReplayThreads * kReplayStates)), kReplayThreads,
+                     rowsShared ? rowsSmem : 0>>>(md, bf.len, bf.ST, bf.CT, bf.seg + (size_t)(q - 1) * rn,
+                                                  bf.acts + step * groups, bf.ids + step * groups * kGroup,
+                                                  d_selects + step * r * z, wide, bf.seg + (size_t)q * rn);
             int e = check_launch(fn, "alpha recomputation");
             if (e != NOVA_SUCCESS) return e;
         }

@@ -117,3 +117,28 @@ def test_belief_values(r, n, count, nz, odd):
     for i in some:
         V, a = orc.alpha_value(G, pi.astype(np.uint32), B[i])
         assert bits(dV[i].cpu().numpy()) == bits(np.float32(V)) and int(dA[i]) == a, i
+
+
+@pytest.mark.parametrize("n,m,z,ns,r", [(5, 1, 1, 2, 3), (33, 3, 2, 5, 41), (1026, 2, 3, 9, 10), (130, 7, 5, 31, 9),
+                                        (2051, 2, 2, 3, 7), (7300, 2, 2, 4, 6)])
+def test_replayed_backups(n, m, z, ns, r):
+    """The alphas recomputed between checkpoints carry the forward pass's
+    bits, so the gradient does not depend on where the checkpoints lie
+    (selections of several actions, ragged successor rows, one to several
+    blocks of states, alphas in and out of shared memory)."""
+    from nova_gb300.pomdp_adjoint import pbvi_record_and_adjoint
+    md = synth.random_pomdp(n=n, m=m, z=z, ns=ns, r=r, rz=min(5, n), gamma=0.9, horizon=5, seed=n + r)
+    rng = np.random.default_rng(n)
+    length = rng.integers(0, ns + 1, size=(n, m, 1))
+    md["S"] = np.where(np.arange(ns) < length, md["S"], -1).astype(np.int32)
+    md["GammaInitial"] = rng.normal(-3.0, 1.0, size=(r, n)).astype(np.float32)
+    b0 = np.full(n, 1.0 / n, np.float32)
+    every = pbvi_record_and_adjoint(md, b0, 5, 1)    # each step's alphas stored
+    once = pbvi_record_and_adjoint(md, b0, 5, 5)     # all but the first recomputed
+    assert every[0] == once[0] and every[1] == once[1]
+    for x, y in zip(every[2:6], once[2:6]):
+        # The same FP64 terms in whatever order the atomics land: the sums
+        # have at most r * (horizon + z) of them.
+        np.testing.assert_allclose(x, y, rtol=0, atol=2.0 ** -52 * r * (5 + z) * max(1e-30, np.abs(y).max()))
+    np.testing.assert_array_equal(every[6], once[6])
+    np.testing.assert_array_equal(every[7], once[7])

@@ -566,60 +566,99 @@ __global__ void vi_plan_scan_rows_kernel(unsigned n, unsigned m, unsigned ns, co
 struct PlanGeometry {
     unsigned n, m, ns, Vt, T, Sb, L, rowsPerWarp;
     float gamma;
-    // Slice (block, tile, row warp) of a row of the block.
-    __device__ __forceinline__ size_t slice(unsigned blk, unsigned t, unsigned rowLocal) const {
-        return ((size_t)blk * T + t) * kRowWarps + rowLocal / rowsPerWarp;
+};
+
+// Calls f(tile, first list index, run length) for every run of the row. The
+// successors are read four at a time where rows allow it (kVec: ns a multiple
+// of 4, S 16-byte aligned), a quarter of the sector requests.
+template <bool kVec, typename F>
+__device__ __forceinline__ void for_each_run(const int *Sr, unsigned ns, unsigned Vt, F f) {
+    unsigned tile = 0, l0 = 0, len = 0;
+    auto take = [&](unsigned l, int sp) {
+        const unsigned t = (unsigned)sp / Vt;
+        if (len != 0 && t == tile) {
+            len++;
+        } else {
+            if (len != 0) f(tile, l0, len);
+            tile = t;
+            l0 = l;
+            len = 1;
+        }
+    };
+    if constexpr (kVec) {
+        for (unsigned l = 0; l < ns; l += 4) {
+            const int4 sp = __ldg(reinterpret_cast<const int4 *>(Sr + l));
+            if (sp.x < 0) break;
+            take(l, sp.x);
+            if (sp.y < 0) break;
+            take(l + 1, sp.y);
+            if (sp.z < 0) break;
+            take(l + 2, sp.z);
+            if (sp.w < 0) break;
+            take(l + 3, sp.w);
+        }
+    } else {
+        for (unsigned l = 0; l < ns; l++) {
+            const int sp = __ldg(Sr + l);
+            if (sp < 0) break;
+            take(l, sp);
+        }
+    }
+    if (len != 0) f(tile, l0, len);
+}
+
+// The plan's counting and filling run one CTA per (block, row warp): its
+// slices' counters stay in shared memory, for kTiles tiles at a time.
+constexpr unsigned kPlanThreads = 256;
+
+// The rows [row0, row1) of the whole model that CTA `cta` plans for, and the
+// first of its block; its slice of tile t is (blk * T + t) * kRowWarps + warp.
+struct PlanRows {
+    unsigned blk, warp;
+    unsigned long long first, row0, row1;
+    __device__ __forceinline__ PlanRows(const PlanGeometry &g, unsigned cta) {
+        blk = cta / kRowWarps;
+        warp = cta % kRowWarps;
+        const unsigned long long all = (unsigned long long)g.n * g.m, perBlock = (unsigned long long)g.Sb * g.m;
+        first = blk * perBlock;
+        const unsigned long long end = min(all, first + perBlock);
+        row0 = min(end, first + (unsigned long long)warp * g.rowsPerWarp);
+        row1 = min(end, row0 + g.rowsPerWarp);
+    }
+    __device__ __forceinline__ size_t slice(const PlanGeometry &g, unsigned t) const {
+        return ((size_t)blk * g.T + t) * kRowWarps + warp;
     }
 };
 
-// Calls f(tile, first list index, run length) for every run of the row.
-template <typename F>
-__device__ __forceinline__ void for_each_run(const int *Sr, unsigned ns, unsigned Vt, F f) {
-    unsigned l = 0;
-    while (l < ns) {
-        const int sp = Sr[l];
-        if (sp < 0) break;
-        const unsigned t = (unsigned)sp / Vt;
-        unsigned e = l + 1;
-        while (e < ns && Sr[e] >= 0 && (unsigned)Sr[e] / Vt == t) e++;
-        f(t, l, e - l);
-        l = e;
-    }
-}
-
-// Per slice: levelCnt[sl*L + q] = runs with more than q records;
-// bucket[sl*32 + b] = single-record runs whose partial sum lies in shared-
-// memory bank b (row mod 32); longCnt[sl*(L+1) + len] = runs of len >= 2.
-__global__ void vi_plan_count_kernel(PlanGeometry g, const int *__restrict__ S, unsigned *__restrict__ levelCnt,
-                                     unsigned *__restrict__ bucket, unsigned *__restrict__ longCnt) {
-    const unsigned long long row = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= (unsigned long long)g.n * g.m) return;
-    const unsigned blk = (unsigned)(row / g.m) / g.Sb;
-    const unsigned rowLocal = (unsigned)(row - (unsigned long long)blk * g.Sb * g.m);
-    const int *Sr = S + row * g.ns;
-    for_each_run(Sr, g.ns, g.Vt, [&](unsigned t, unsigned, unsigned len) {
-        const size_t sl = g.slice(blk, t, rowLocal);
-        for (unsigned q = 0; q < len; q++) atomicAdd(levelCnt + sl * g.L + q, 1u);
-        if (len == 1) atomicAdd(bucket + sl * 32 + (rowLocal & 31u), 1u);
-        else atomicAdd(longCnt + sl * (g.L + 1) + len, 1u);
-    });
-}
-
-// Per slice: its record count, and the long runs' exclusive prefix by
-// length, longest first (in place in longCnt).
-__global__ void vi_plan_slice_kernel(size_t nSlices, unsigned L, const unsigned *__restrict__ levelCnt,
-                                     unsigned *__restrict__ longCnt, unsigned *__restrict__ sliceSize) {
-    const size_t sl = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (sl >= nSlices) return;
-    unsigned total = 0;
-    for (unsigned q = 0; q < L; q++) total += levelCnt[sl * L + q];
-    sliceSize[sl] = total;
-    unsigned run = 0;
-    for (unsigned len = L; len >= 2; len--) {
-        unsigned *p = longCnt + sl * (L + 1) + len;
-        const unsigned v = *p;
-        *p = run;
-        run += v;
+// Per slice: levelCnt[sl*L + q] = runs with more than q records, and their sum.
+template <bool kVec>
+__global__ void __launch_bounds__(kPlanThreads) vi_plan_count_kernel(PlanGeometry g, const int *__restrict__ S,
+                                                                     unsigned tilesPerPass,
+                                                                     unsigned *__restrict__ levelCnt,
+                                                                     unsigned *__restrict__ sliceSize) {
+    extern __shared__ unsigned planShared[];   // [tilesPerPass][L]
+    const PlanRows rows(g, blockIdx.x);
+    for (unsigned t0 = 0; t0 < g.T; t0 += tilesPerPass) {
+        const unsigned nt = min(tilesPerPass, g.T - t0);
+        for (unsigned k = threadIdx.x; k < nt * g.L; k += kPlanThreads) planShared[k] = 0u;
+        __syncthreads();
+        for (unsigned long long row = rows.row0 + threadIdx.x; row < rows.row1; row += kPlanThreads)
+            for_each_run<kVec>(S + row * g.ns, g.ns, g.Vt, [&](unsigned t, unsigned, unsigned len) {
+                if (t - t0 < nt)
+                    for (unsigned q = 0; q < len; q++) atomicAdd(planShared + (t - t0) * g.L + q, 1u);
+            });
+        __syncthreads();
+        for (unsigned t = threadIdx.x; t < nt; t += kPlanThreads) {
+            const size_t sl = rows.slice(g, t0 + t);
+            unsigned total = 0;
+            for (unsigned q = 0; q < g.L; q++) {
+                const unsigned c = planShared[t * g.L + q];
+                levelCnt[sl * g.L + q] = c;
+                total += c;
+            }
+            sliceSize[sl] = total;
+        }
+        __syncthreads();
     }
 }
 
@@ -634,42 +673,99 @@ __global__ void vi_plan_hdr_kernel(size_t nSlices, unsigned L, const unsigned *_
 }
 
 // Write every record at its place. The position j of a run in its slice's
-// levels: long runs first, by length (ties in the order threads arrive,
+// levels: long runs first, by length (as many runs lie before the class of
+// length len as have more than len records; ties in the order threads arrive,
 // which changes nothing: the rows of one slice are distinct), then the
 // single-record runs dealt round-robin over the 32 banks, the k-th run of
-// bank b's bucket in round k.
-__global__ void vi_plan_fill_kernel(PlanGeometry g, const int *__restrict__ S, const float *__restrict__ Tm,
-                                    const unsigned *__restrict__ sliceStart, const unsigned *__restrict__ levelCnt,
-                                    const unsigned *__restrict__ bucket, unsigned *__restrict__ ticket,
-                                    unsigned *__restrict__ longCnt, uint2 *__restrict__ rec) {
-    const unsigned long long row = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= (unsigned long long)g.n * g.m) return;
-    const unsigned blk = (unsigned)(row / g.m) / g.Sb;
-    const unsigned rowLocal = (unsigned)(row - (unsigned long long)blk * g.Sb * g.m);
-    const int *Sr = S + row * g.ns;
-    const float *Tr = Tm + row * g.ns;
-    for_each_run(Sr, g.ns, g.Vt, [&](unsigned t, unsigned l0, unsigned len) {
-        const size_t sl = g.slice(blk, t, rowLocal);
-        unsigned j;
-        if (len >= 2) {
-            j = atomicAdd(longCnt + sl * (g.L + 1) + len, 1u);
-        } else {
-            const unsigned qb = rowLocal & 31u;
-            const unsigned rank = atomicAdd(ticket + sl * 32 + qb, 1u);
-            j = g.L > 1 ? levelCnt[sl * g.L + 1] : 0u;   // the long runs come first
-            const unsigned *bs = bucket + sl * 32;
-            for (unsigned b = 0; b < 32; b++) {
-                const unsigned sz = bs[b];
-                j += min(sz, rank) + ((b < qb && sz > rank) ? 1u : 0u);
+// bank b's bucket in round k. Rounds up to kPlanRounds are looked up: runs in
+// the rounds before, and the banks that still deal in this one. (Adding up the
+// 32 bucket sizes for every record, with the counters in global memory, took
+// 9.8 ms of a solve at n = 2^20, m = 8, ns = 16; this kernel 2.1 ms.)
+constexpr unsigned kPlanRounds = 32;
+constexpr size_t kPlanFillWords = 32 + 32 + 2 * kPlanRounds;  // per tile, and 2 L + 2 for the levels
+
+template <bool kVec>
+__global__ void __launch_bounds__(kPlanThreads) vi_plan_fill_kernel(PlanGeometry g, const int *__restrict__ S,
+                                                                    const float *__restrict__ Tm,
+                                                                    unsigned tilesPerPass,
+                                                                    const unsigned *__restrict__ sliceStart,
+                                                                    const unsigned *__restrict__ levelCnt,
+                                                                    uint2 *__restrict__ rec) {
+    extern __shared__ unsigned planShared[];
+    unsigned *bucket = planShared;                                   // [tiles][32] single runs per bank
+    unsigned *ticket = bucket + (size_t)tilesPerPass * 32;           // [tiles][32] dealt so far
+    unsigned *before = ticket + (size_t)tilesPerPass * 32;           // [tiles][kPlanRounds] runs of earlier rounds
+    unsigned *banks = before + (size_t)tilesPerPass * kPlanRounds;   // [tiles][kPlanRounds] banks in the round
+    unsigned *longs = banks + (size_t)tilesPerPass * kPlanRounds;    // [tiles][L + 1] next place per run length
+    unsigned *level = longs + (size_t)tilesPerPass * (g.L + 1);      // [tiles][L]
+    unsigned *start = level + (size_t)tilesPerPass * g.L;            // [tiles]
+    const PlanRows rows(g, blockIdx.x);
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (unsigned t0 = 0; t0 < g.T; t0 += tilesPerPass) {
+        const unsigned nt = min(tilesPerPass, g.T - t0);
+        for (unsigned k = threadIdx.x; k < nt * 32; k += kPlanThreads) bucket[k] = ticket[k] = 0u;
+        for (unsigned k = threadIdx.x; k < nt * g.L; k += kPlanThreads)
+            level[k] = levelCnt[rows.slice(g, t0 + k / g.L) * g.L + k % g.L];
+        for (unsigned t = threadIdx.x; t < nt; t += kPlanThreads) start[t] = sliceStart[rows.slice(g, t0 + t)];
+        __syncthreads();
+        for (unsigned k = threadIdx.x; k < nt * (g.L + 1); k += kPlanThreads) {
+            const unsigned len = k % (g.L + 1);
+            longs[k] = len < g.L ? level[k / (g.L + 1) * g.L + len] : 0u;
+        }
+        for (unsigned long long row = rows.row0 + threadIdx.x; row < rows.row1; row += kPlanThreads) {
+            const unsigned qb = (unsigned)(row - rows.first) & 31u;
+            for_each_run<kVec>(S + row * g.ns, g.ns, g.Vt, [&](unsigned t, unsigned, unsigned len) {
+                if (t - t0 < nt && len == 1) atomicAdd(bucket + (t - t0) * 32 + qb, 1u);
+            });
+        }
+        __syncthreads();
+        for (unsigned t = warp; t < nt; t += kPlanThreads / 32) {
+            const unsigned size = bucket[t * 32 + lane];
+            unsigned run = 0;
+            for (unsigned k = 0; k < kPlanRounds; k++) {
+                const unsigned msk = __ballot_sync(0xffffffffu, size > k);
+                if (lane == 0) {
+                    before[t * kPlanRounds + k] = run;
+                    banks[t * kPlanRounds + k] = msk;
+                }
+                run += __popc(msk);
+                if (msk == 0) break;
             }
         }
-        unsigned base = sliceStart[sl];
-        for (unsigned q = 0; q < len; q++) {
-            const unsigned sp = (unsigned)Sr[l0 + q];
-            rec[base + j] = make_uint2((rowLocal << 16) | ((sp - t * g.Vt) * 4u), __float_as_uint(fmul(g.gamma, Tr[l0 + q])));
-            base += levelCnt[sl * g.L + q];
+        __syncthreads();
+        for (unsigned long long row = rows.row0 + threadIdx.x; row < rows.row1; row += kPlanThreads) {
+            const unsigned rowLocal = (unsigned)(row - rows.first), qb = rowLocal & 31u;
+            const int *Sr = S + row * g.ns;
+            const float *Tr = Tm + row * g.ns;
+            for_each_run<kVec>(Sr, g.ns, g.Vt, [&](unsigned tile, unsigned l0, unsigned len) {
+                const unsigned t = tile - t0;
+                if (t >= nt) return;
+                unsigned j;
+                if (len >= 2) {
+                    j = atomicAdd(longs + t * (g.L + 1) + len, 1u);
+                } else {
+                    const unsigned rank = atomicAdd(ticket + t * 32 + qb, 1u);
+                    j = g.L > 1 ? level[t * g.L + 1] : 0u;   // the long runs come first
+                    if (rank < kPlanRounds) {
+                        j += before[t * kPlanRounds + rank] + __popc(banks[t * kPlanRounds + rank] & ((1u << qb) - 1u));
+                    } else {
+                        for (unsigned b = 0; b < 32; b++) {
+                            const unsigned sz = bucket[t * 32 + b];
+                            j += min(sz, rank) + ((b < qb && sz > rank) ? 1u : 0u);
+                        }
+                    }
+                }
+                unsigned base = start[t];
+                for (unsigned q = 0; q < len; q++) {
+                    const unsigned sp = (unsigned)Sr[l0 + q];
+                    rec[base + j] = make_uint2((rowLocal << 16) | ((sp - tile * g.Vt) * 4u),
+                                               __float_as_uint(fmul(g.gamma, __ldg(Tr + l0 + q))));
+                    base += level[t * g.L + q];
+                }
+            });
         }
-    });
+        __syncthreads();
+    }
 }
 
 // Exclusive scan of in[0..N) into out[0..N] (out[N] = total) in three
@@ -896,36 +992,30 @@ int vi_plan_build(ViTilePlan *plan, const MDP *mdp, const int *S, const float *T
     const unsigned long long nSlices = (unsigned long long)blocks * tiles * kRowWarps;
     if (nSlices * 32ull >= (1ull << 32) || nSlices * (L + 1) >= (1ull << 32)) { release(plan); return NOVA_SUCCESS; }
 
-    // Pass 2: per-slice counts (levels, banks, long runs) and the slice starts.
-    unsigned *bucket = nullptr, *ticket = nullptr, *longCnt = nullptr, *sliceSize = nullptr;
+    // Pass 2: per-slice counts and the slice starts. Tiles per pass of a CTA:
+    // what 64 KB of counters hold (three CTAs an SM).
+    unsigned *sliceSize = nullptr;
     auto freeScratch = [&]() {
-        cudaFree(bucket); cudaFree(ticket); cudaFree(longCnt); cudaFree(sliceSize);
-        bucket = ticket = longCnt = sliceSize = nullptr;
+        cudaFree(sliceSize);
+        sliceSize = nullptr;
     };
-    if (!try_alloc(&plan->levelCnt, nSlices * L) || !try_alloc(&bucket, nSlices * 32) ||
-            !try_alloc(&ticket, nSlices * 32) || !try_alloc(&longCnt, nSlices * (L + 1)) ||
-            !try_alloc(&sliceSize, nSlices) || !try_alloc(&plan->sliceStart, nSlices + 1)) {
+    if (!try_alloc(&plan->levelCnt, nSlices * L) || !try_alloc(&sliceSize, nSlices) ||
+            !try_alloc(&plan->sliceStart, nSlices + 1)) {
         freeScratch();
         release(plan);
         return NOVA_SUCCESS;
     }
-    if (cudaMemsetAsync(plan->levelCnt, 0, nSlices * L * sizeof(unsigned), stream) != cudaSuccess ||
-            cudaMemsetAsync(bucket, 0, nSlices * 32 * sizeof(unsigned), stream) != cudaSuccess ||
-            cudaMemsetAsync(ticket, 0, nSlices * 32 * sizeof(unsigned), stream) != cudaSuccess ||
-            cudaMemsetAsync(longCnt, 0, nSlices * (L + 1) * sizeof(unsigned), stream) != cudaSuccess) {
-        cudaGetLastError();
-        freeScratch();
-        release(plan);
-        NOVA_ERR(fn, "Failed to clear the sweep plan counters.");
-        return NOVA_ERROR_KERNEL_EXECUTION;
-    }
-    vi_plan_count_kernel<<<rowBlocks, 256, 0, stream>>>(g, S, plan->levelCnt, bucket, longCnt);
+    const size_t tileWords = kPlanFillWords + 2 * (size_t)L + 2;
+    const unsigned perPass = (unsigned)std::min<size_t>(tiles, std::max<size_t>(1, 64 * 1024 / (tileWords * 4)));
+    const size_t fillBytes = perPass * tileWords * 4;
+    const bool vec = ns % 4u == 0u && (uintptr_t)S % 16u == 0u;
+    auto countKernel = vec ? vi_plan_count_kernel<true> : vi_plan_count_kernel<false>;
+    auto fillKernel = vec ? vi_plan_fill_kernel<true> : vi_plan_fill_kernel<false>;
+    if (fillBytes > 48 * 1024)
+        cudaFuncSetAttribute(fillKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fillBytes);
+    const unsigned ctas = blocks * kRowWarps;
+    countKernel<<<ctas, kPlanThreads, (size_t)perPass * L * 4, stream>>>(g, S, perPass, plan->levelCnt, sliceSize);
     rc = check_launch(fn, "sweep plan (count)");
-    if (rc == NOVA_SUCCESS) {
-        vi_plan_slice_kernel<<<ceil_div(nSlices, 256), 256, 0, stream>>>((size_t)nSlices, L, plan->levelCnt, longCnt,
-                                                                         sliceSize);
-        rc = check_launch(fn, "sweep plan (slices)");
-    }
     if (rc == NOVA_SUCCESS) rc = scan_counts(sliceSize, nSlices, plan->sliceStart, stream, fn);
     // Headers, with (kDepth + 1) * kRowWarps zeroed ones after the last slice
     // for the row warps' unconditional look-ahead loads.
@@ -947,13 +1037,13 @@ int vi_plan_build(ViTilePlan *plan, const MDP *mdp, const int *S, const float *T
     // Pass 3: the records (two spare ones at the end for the bulk prefetch).
     if (rc == NOVA_SUCCESS && !try_alloc(&plan->rec, (size_t)total + 2)) rc = NOVA_ERROR_DEVICE_MALLOC;
     if (rc == NOVA_SUCCESS &&
-            cudaMemsetAsync(plan->rec, 0xFF, ((size_t)total + 2) * sizeof(uint2), stream) != cudaSuccess) {
+            cudaMemsetAsync(plan->rec + total, 0xFF, 2 * sizeof(uint2), stream) != cudaSuccess) {
         cudaGetLastError();
         rc = NOVA_ERROR_KERNEL_EXECUTION;
     }
     if (rc == NOVA_SUCCESS) {
-        vi_plan_fill_kernel<<<rowBlocks, 256, 0, stream>>>(g, S, T, plan->sliceStart, plan->levelCnt, bucket, ticket,
-                                                           longCnt, plan->rec);
+        fillKernel<<<ctas, kPlanThreads, fillBytes, stream>>>(g, S, T, perPass, plan->sliceStart, plan->levelCnt,
+                                                              plan->rec);
         rc = check_launch(fn, "sweep plan (fill)");
     }
     if (rc == NOVA_SUCCESS) rc = sync_device(fn);

@@ -142,3 +142,36 @@ def test_replayed_backups(n, m, z, ns, r):
         np.testing.assert_allclose(x, y, rtol=0, atol=2.0 ** -52 * r * (5 + z) * max(1e-30, np.abs(y).max()))
     np.testing.assert_array_equal(every[6], once[6])
     np.testing.assert_array_equal(every[7], once[7])
+
+
+@pytest.mark.parametrize("n,m,ns,tile,ragged,crowd", [(5, 1, 1, 64, False, 0), (300, 3, 7, 64, True, 0),
+                                                      (1025, 2, 8, 64, True, 60), (40000, 1, 4, 64, False, 0),
+                                                      (9000, 4, 12, 256, True, 4000), (2500, 33, 6, 1024, False, 2400)])
+def test_sweep_plan(n, m, ns, tile, ragged, crowd):
+    """Plans with one and with many tiles (also more than a CTA counts at
+    once), row counts that are no multiple of a warp's share, ragged rows, and
+    more than 32 single records of one bank in a tile (`crowd` states share
+    their successors' tile)."""
+    from nova_gb300 import mdp_vi as mvi
+    from nova_gb300 import nova_mdp_vi as nmvi
+    from nova_gb300.mdp import MDP
+    md = synth.random_mdp(n=n, m=m, ns=ns, gamma=0.95, horizon=3, seed=n)
+    rng = np.random.default_rng(n)
+    if crowd:
+        lead = rng.integers(0, min(tile, n), size=(crowd, m))
+        md["S"][:crowd, :, 0] = lead
+        md["S"][:crowd, :, 1:] = np.sort(rng.integers(tile, n, size=(crowd, m, ns - 1)), axis=2)
+    if ragged:
+        md["S"] = np.where(np.arange(ns) < rng.integers(0, ns + 1, size=(n, m, 1)), md["S"], -1).astype(np.int32)
+    V0 = rng.normal(size=n).astype(np.float32)
+    p = MDP.from_arrays(md)
+    p.initialize_gpu()
+    mvi.set_tiling(nmvi.TILING_ALWAYS, tile)
+    try:
+        pol = mvi.MDPValueIterationGPU(p, Vinitial=V0).solve()
+        assert mvi.tiling_status() == 1
+    finally:
+        mvi.set_tiling(nmvi.TILING_AUTO)
+    V, pi = orc.mdp_vi_solve(md, horizon=3, VInitial=V0)
+    np.testing.assert_array_equal(bits(pol.V_array()), bits(V))
+    np.testing.assert_array_equal(pol.pi_array(), pi)

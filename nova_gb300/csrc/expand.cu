@@ -15,9 +15,13 @@
 //     probabilities, normalisers, L1 distances, error bounds) is formed the
 //     same way: the terms are computed in parallel and one thread adds them in
 //     order.
-//   * one block per belief (distinct, PEMA) or per trajectory (random); the
-//     L1 distances to all r beliefs run one belief per thread over a dense,
+//   * one block per belief (PEMA) or per trajectory (random); PEMA's L1
+//     distances to all r beliefs run one belief per thread over a dense,
 //     state-major copy of B.
+//   * the distinct expansion needs the exact distances only where they decide
+//     something: every successor's smallest distance is first bounded from the
+//     beliefs' nonzeros, and the sums the reference forms are added up for the
+//     successors and beliefs within that bound's error of the best.
 //
 // The random expansions draw from libc rand() on the host exactly as the
 // reference does (srand(time(nullptr)), or a fixed seed set with
@@ -68,8 +72,10 @@ struct ExpModel {
     const int *Z;
     const float *B;
     const unsigned *predStart;  // [m][n+1]
-    const unsigned *predIdx;    // entries (s*m + a)*ns + i, sorted by (s, i) per (a, s')
+    const unsigned *predState;  // predecessor s of each entry, sorted by (s, i) per (a, s')
+    const float *predT;         // its T(s,a,i)
     const float *BT;            // [n][r] dense beliefs, state-major
+    const float *PO;            // [m][n][z] sum_i fl(T(s,a,i) O(a,S,o)), added in i order
 };
 
 // Shared-memory layout of one block: b, bp, aux, tmp (n floats each) plus
@@ -90,19 +96,33 @@ __device__ float seq_sum(const float *v, unsigned n, float *slot) {
     return *slot;
 }
 
+// PO[a][s][o]: the belief-independent part of
 // pomdp_expand_probability_observation_cpu (pomdp_expand_cpu.cpp:56-78).
-__device__ float prob_obs_dense(const ExpModel &md, const float *b, float *tmp, unsigned a, unsigned o, float *slot) {
-    for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) {
-        const size_t row = ((size_t)s * md.m + a) * md.ns;
+__global__ void prob_table_kernel(unsigned n, unsigned ns, unsigned m, unsigned z, const int *__restrict__ S,
+                                  const float *__restrict__ T, const float *__restrict__ O, float *__restrict__ PO) {
+    const size_t total = (size_t)m * n * z;
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
+        const unsigned o = (unsigned)(e % z);
+        const size_t as = e / z;
+        const unsigned s = (unsigned)(as % n), a = (unsigned)(as / n);
+        const size_t row = ((size_t)s * m + a) * ns;
         float val = 0.0f;
-        for (unsigned i = 0; i < md.ns; i++) {
-            const int sp = md.S[row + i];
+        for (unsigned i = 0; i < ns; i++) {
+            const int sp = S[row + i];
             if (sp < 0) break;
-            val = fadd(val, fmul(md.T[row + i], md.O[((size_t)a * md.n + sp) * md.z + o]));
+            val = fadd(val, fmul(T[row + i], O[((size_t)a * n + sp) * z + o]));
         }
-        tmp[s] = fmul(val, b[s]);
+        PO[e] = val;
     }
-    return seq_sum(tmp, md.n, slot);
+}
+
+// Pr(o | b, a) for one observation: sum_s fl(PO * b(s)) in state order.
+__device__ __forceinline__ float prob_obs_dense(const ExpModel &md, const float *b, unsigned a, unsigned o) {
+    const float *po = md.PO + (size_t)a * md.n * md.z + o;
+    float acc = 0.0f;
+#pragma unroll 8
+    for (unsigned s = 0; s < md.n; s++) acc = fadd(acc, fmul(__ldg(po + (size_t)s * md.z), b[s]));
+    return acc;
 }
 
 // pomdp_belief_update_cpu (pomdp_model_cpu.cpp:89-137). Returns true when
@@ -114,9 +134,7 @@ __device__ bool belief_update(const ExpModel &md, const float *b, float *bp, uns
         const unsigned e1 = md.predStart[(size_t)a * (md.n + 1) + sp + 1];
         float v = 0.0f;
         for (unsigned k = e0; k < e1; k++) {
-            const unsigned e = md.predIdx[k];
-            const unsigned s = e / (md.m * md.ns);
-            v = fadd(v, fmul(md.T[e], b[s]));
+            v = fadd(v, fmul(md.predT[k], b[md.predState[k]]));
         }
         bp[sp] = fmul(v, md.O[((size_t)a * md.n + sp) * md.z + o]);
     }
@@ -162,36 +180,279 @@ __device__ BlockBufs carve(float *smem, unsigned n) {
     return BlockBufs{smem, smem + n, smem + 2 * (size_t)n, smem + 3 * (size_t)n};
 }
 
+// ---------------------------------------------------------------------------
 // pomdp_expand_distinct_beliefs_cpu (pomdp_expand_cpu.cpp:153-241): for
 // belief i, the successor b'(b_i, a, o) farthest (in min L1 distance) from
-// the belief set. One block per belief.
-__global__ void __launch_bounds__(kThreads) distinct_kernel(ExpModel md, float *__restrict__ Bnew) {
+// the belief set. Beliefs are expanded in chunks that share the buffers below;
+// row ao = a*z + o of belief i is a successor.
+// ---------------------------------------------------------------------------
+struct Distinct {
+    unsigned first, chunk;      // beliefs first .. first + chunk - 1
+    float *W;                   // [chunk][m][n] sum over predecessors of fl(T b), before O
+    float *bp;                  // [chunk][n][m*z] normalised successors, row-contiguous
+    float *mass;                // [chunk][m*z] sum_s b'(s); negative: no successor
+    float *bound;               // [chunk][m*z] approximate smallest distance
+    uint2 *list;                // [r][cap] the beliefs' nonzeros (state, value bits) in state order
+    unsigned *nnz;              // [r]
+    float *total;               // [r] sum_s b_j(s)
+    unsigned *odd;              // [2] a value below 0 or not finite somewhere; the largest total's bits
+    unsigned cap;               // min(n, rz)
+};
+
+// Whether some observation probability sum is not finite (a zero of a belief
+// then still decides something).
+__global__ void distinct_check_kernel(ExpModel md, unsigned *__restrict__ odd) {
+    const size_t total = (size_t)md.m * md.n * md.z;
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x)
+        if (!(fabsf(md.PO[e]) <= 3.402823466e38f)) atomicOr(odd, 1u);
+}
+
+// Nonzeros of every belief in state order (one warp each), their sums, and
+// whether any value is negative or not finite.
+__global__ void __launch_bounds__(kThreads) distinct_list_kernel(ExpModel md, Distinct d) {
+    const unsigned lane = threadIdx.x & 31, j = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    if (j >= md.r) return;
+    unsigned filled = 0;
+    float sum = 0.0f;
+    bool odd = false;
+    for (unsigned s0 = 0; s0 < md.n; s0 += 32) {
+        const unsigned s = s0 + lane;
+        const float v = s < md.n ? md.BT[(size_t)s * md.r + j] : 0.0f;
+        const bool some = !(v == 0.0f);
+        const unsigned msk = __ballot_sync(0xffffffffu, some);
+        if (some) d.list[(size_t)j * d.cap + filled + __popc(msk & ((1u << lane) - 1u))] = make_uint2(s, __float_as_uint(v));
+        filled += __popc(msk);
+        odd |= !(v >= 0.0f && v <= NOVA_FLT_MAX);
+        sum += v;
+    }
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    if (__any_sync(0xffffffffu, odd) && lane == 0) atomicOr(d.odd, 1u);
+    if (lane == 0) {
+        d.nnz[j] = filled;
+        d.total[j] = sum;
+        if (sum >= 0.0f) atomicMax(d.odd + 1, __float_as_uint(sum));
+    }
+}
+
+// W[i][a][s'] in the reference's order (belief_update's first sum; it does
+// not depend on o). One block per belief and action.
+__global__ void __launch_bounds__(kThreads) distinct_mass_kernel(ExpModel md, Distinct d) {
     extern __shared__ __align__(16) float smem[];
-    __shared__ float slot, sv[kThreads];
-    __shared__ unsigned si[kThreads];
-    __shared__ int take;
-    BlockBufs w = carve(smem, md.n);
-    float *star = w.aux;
-    const unsigned i = blockIdx.x;
-    load_belief(md, i, w.b);
-    for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) star[s] = 0.0f;
-    float starValue = NOVA_FLT_MIN;
-    for (unsigned a = 0; a < md.m; a++) {
-        for (unsigned o = 0; o < md.z; o++) {
-            const float pr = prob_obs_dense(md, w.b, w.tmp, a, o, &slot);
-            if (pr == 0.0f) continue;
-            if (!belief_update(md, w.b, w.bp, a, o, &slot)) continue;
-            const float jStar = min_distance(md, w.bp, nullptr, sv, si);
-            if (threadIdx.x == 0) take = jStar > starValue ? 1 : 0;
-            __syncthreads();
-            if (take) {
-                starValue = jStar;
-                for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) star[s] = w.bp[s];
+    const unsigned i = blockIdx.x / md.m, a = blockIdx.x % md.m;
+    load_belief(md, d.first + i, smem);
+    for (unsigned sp = threadIdx.x; sp < md.n; sp += blockDim.x) {
+        const unsigned e0 = md.predStart[(size_t)a * (md.n + 1) + sp];
+        const unsigned e1 = md.predStart[(size_t)a * (md.n + 1) + sp + 1];
+        float v = 0.0f;
+        for (unsigned k = e0; k < e1; k++) v = fadd(v, fmul(md.predT[k], smem[md.predState[k]]));
+        d.W[((size_t)i * md.m + a) * md.n + sp] = v;
+    }
+}
+
+// One thread per (belief, action, observation), observations adjacent:
+// whether the successor exists (Pr(o|b,a) != 0 and the normaliser reaches
+// FLT_ERR_TOL), its values and their sum. The sums the reference adds in state
+// order are chains of n additions, but r*m*z of them run side by side (the
+// serial form was one thread's work per block and successor).
+__global__ void __launch_bounds__(kThreads) distinct_rows_kernel(ExpModel md, Distinct d) {
+    const unsigned mz = md.m * md.z;
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (size_t)d.chunk * mz) return;
+    const unsigned i = (unsigned)(t / mz), ao = (unsigned)(t % mz), a = ao / md.z, o = ao % md.z;
+    const float *po = md.PO + (size_t)a * md.n * md.z + o;
+    float pr = 0.0f;
+    if (d.odd[0] == 0u) {
+        // Zeros of the belief add fl(PO * 0) = 0 to the sum of finite products.
+        const unsigned j = d.first + i, L = d.nnz[j];
+        const uint2 *list = d.list + (size_t)j * d.cap;
+        for (unsigned k = 0; k < L; k++) {
+            const uint2 e = list[k];
+            pr = fadd(pr, fmul(po[(size_t)e.x * md.z], __uint_as_float(e.y)));
+        }
+    } else {
+        for (unsigned s = 0; s < md.n; s++) pr = fadd(pr, fmul(po[(size_t)s * md.z], md.BT[(size_t)s * md.r + d.first + i]));
+    }
+    float mass = -1.0f;
+    if (!(pr == 0.0f)) {
+        const float *W = d.W + ((size_t)i * md.m + a) * md.n;
+        const float *Oa = md.O + (size_t)a * md.n * md.z + o;
+        float norm = 0.0f;
+#pragma unroll 8
+        for (unsigned s = 0; s < md.n; s++) norm = fadd(norm, fmul(W[s], Oa[(size_t)s * md.z]));
+        if (!(fabs((double)fabsf(norm)) < NOVA_FLT_ERR_TOL)) {
+            float *out = d.bp + (size_t)i * md.n * mz + ao;
+            mass = 0.0f;
+            bool odd = false;
+#pragma unroll 4
+            for (unsigned s = 0; s < md.n; s++) {
+                const float v = __fdiv_rn(fmul(W[s], Oa[(size_t)s * md.z]), norm);
+                out[(size_t)s * mz] = v;
+                odd |= !(v >= 0.0f && v <= NOVA_FLT_MAX);
+                mass += fabsf(v);
             }
-            __syncthreads();
+            if (odd) atomicOr(d.odd, 1u);
         }
     }
-    for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) Bnew[(size_t)i * md.n + s] = star[s];
+    d.mass[t] = mass;
+}
+
+// Half-width of the interval around an approximate distance in which the
+// reference's FP32 sum lies. With both beliefs non-negative,
+//     sum_s |b_j - b'| = mass - total_j + 2 sum_{s in supp j} max(b_j - b', 0).
+// The reference's n-term sum rounds by at most (n + 1) u (mass + total), u =
+// 2^-24; mass by n u mass, total by (n / 32 + 6) u total, the sum of the
+// maxima by (nnz + 2) u total, twice, and the last three operations by 3 u
+// (mass + 2 total): at most (2 n + 4) u mass + (3.1 n + 20) u total together.
+__device__ __forceinline__ float distance_error(const ExpModel &md, const Distinct &d, float mass) {
+    if (d.odd[0] != 0u) return INFINITY;
+    return 2.0f * (float)(2 * md.n + 16) * 5.97e-8f * (mass + 2.0f * __uint_as_float(d.odd[1]));
+}
+
+// bound[i][ao] = min_j of the approximate distance. A block keeps ROWS
+// successors of one belief in shared memory ([state][ROWS], kShared) and its
+// warps walk the beliefs' nonzeros, lane = successor: one conflict-free read,
+// a subtraction, a maximum and an addition per nonzero and successor, 16 times
+// fewer terms than the sums over all states at n = 512 (32 nonzeros). Bound by
+// issue: r = 1,024, m z = 128 takes 1.4 ms, the whole expansion 2.0 ms on the
+// device; one block per belief forming every sum in full took 33 ms.
+template <int ROWS, bool kShared>
+__global__ void __launch_bounds__(1024) distinct_bound_kernel(ExpModel md, Distinct d) {
+    constexpr int PER = ROWS / 32;
+    extern __shared__ __align__(16) float tile[];   // [n][ROWS]; then [warps][ROWS]
+    const unsigned mz = md.m * md.z, tiles = (mz + ROWS - 1) / ROWS;
+    const unsigned i = blockIdx.x / tiles, r0 = (blockIdx.x % tiles) * ROWS;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const float *src = d.bp + (size_t)i * md.n * mz + r0;
+    const unsigned live = min((unsigned)ROWS, mz - r0);
+    float *best = tile;
+    if constexpr (kShared) {
+        best = tile + (size_t)md.n * ROWS;
+        for (unsigned e = threadIdx.x; e < md.n * ROWS; e += blockDim.x) {
+            const unsigned s = e / ROWS, q = e % ROWS;
+            tile[e] = q < live ? src[(size_t)s * mz + q] : 0.0f;
+        }
+        __syncthreads();
+    }
+    float low[PER];
+    unsigned at[PER];
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+        low[q] = INFINITY;
+        at[q] = min(lane + 32u * q, live - 1);
+    }
+    for (unsigned j = warp; j < md.r; j += warps) {
+        const uint2 *list = d.list + (size_t)j * d.cap;
+        const unsigned L = d.nnz[j];
+        float acc[PER];
+#pragma unroll
+        for (int q = 0; q < PER; q++) acc[q] = 0.0f;
+#pragma unroll 8
+        for (unsigned k = 0; k < L; k++) {
+            const uint2 e = __ldg(list + k);
+            const float b = __uint_as_float(e.y);
+#pragma unroll
+            for (int q = 0; q < PER; q++) {
+                const float p = kShared ? tile[e.x * ROWS + lane + 32u * q] : __ldg(src + (size_t)e.x * mz + at[q]);
+                acc[q] += fmaxf(b - p, 0.0f);
+            }
+        }
+        const float t = d.total[j];
+#pragma unroll
+        for (int q = 0; q < PER; q++) low[q] = fminf(low[q], 2.0f * acc[q] - t);
+    }
+#pragma unroll
+    for (int q = 0; q < PER; q++) best[warp * ROWS + lane + 32 * q] = low[q];
+    __syncthreads();
+    for (unsigned q = threadIdx.x; q < live; q += blockDim.x) {
+        float v = INFINITY;
+        for (unsigned w = 0; w < warps; w++) v = fminf(v, best[w * ROWS + q]);
+        const float mass = d.mass[(size_t)i * mz + r0 + q];
+        d.bound[(size_t)i * mz + r0 + q] = v + mass;
+    }
+}
+
+// Per belief: the successors whose bound lies within the error of the largest,
+// in (a, o) order; for each, the reference's sums to the beliefs within the
+// error of its smallest, one warp per belief: the lanes form 32 terms, lane 0
+// adds them in state order. The first successor with the strictly largest
+// smallest distance becomes the new belief.
+__global__ void __launch_bounds__(kThreads) distinct_select_kernel(ExpModel md, Distinct d, float *__restrict__ Bnew) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ float red[kThreads / 32], terms[kThreads / 32][32];
+    const unsigned mz = md.m * md.z, i = blockIdx.x;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float *row = smem, *star = smem + md.n;
+    const float *bound = d.bound + (size_t)i * mz, *mass = d.mass + (size_t)i * mz;
+    float top = -INFINITY, heaviest = 0.0f;
+    for (unsigned ao = threadIdx.x; ao < mz; ao += blockDim.x) {
+        if (mass[ao] < 0.0f) continue;
+        top = fmaxf(top, bound[ao]);
+        heaviest = fmaxf(heaviest, mass[ao]);
+    }
+    auto block_max = [&](float v) {
+        for (int off = 16; off > 0; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
+        __syncthreads();
+        if (lane == 0) red[warp] = v;
+        __syncthreads();
+        for (unsigned w = 0; w < kThreads / 32; w++) v = fmaxf(v, red[w]);
+        return v;
+    };
+    top = block_max(top);
+    heaviest = block_max(heaviest);
+    const float err = distance_error(md, d, heaviest);
+    for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) star[s] = 0.0f;
+    float starValue = NOVA_FLT_MIN;
+    for (unsigned ao = 0; ao < mz; ao++) {
+        // A NaN mass is a successor too (err is infinite then).
+        if (mass[ao] < 0.0f || bound[ao] < top - 2.0f * err) continue;
+        __syncthreads();
+        for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) row[s] = d.bp[((size_t)i * md.n + s) * mz + ao];
+        __syncthreads();
+        const float cut = bound[ao] + 2.0f * err;
+        float low = NOVA_FLT_MAX;
+        for (unsigned j0 = warp * 32; j0 < md.r; j0 += kThreads) {
+            const unsigned j = j0 + lane;
+            bool near = j < md.r;
+            if (near) {
+                const uint2 *list = d.list + (size_t)j * d.cap;
+                const unsigned L = d.nnz[j];
+                float acc = 0.0f;
+                for (unsigned k = 0; k < L; k++) {
+                    const uint2 e = list[k];
+                    acc += fmaxf(__uint_as_float(e.y) - row[e.x], 0.0f);
+                }
+                near = !(mass[ao] + (2.0f * acc - d.total[j]) > cut);
+            }
+            for (unsigned msk = __ballot_sync(0xffffffffu, near); msk != 0; msk &= msk - 1) {
+                const unsigned jj = j0 + __ffs(msk) - 1;
+                float dist = 0.0f;
+                for (unsigned s0 = 0; s0 < md.n; s0 += 32) {
+                    const unsigned s = s0 + lane;
+                    terms[warp][lane] = s < md.n ? fabsf(__fsub_rn(md.BT[(size_t)s * md.r + jj], row[s])) : 0.0f;
+                    __syncwarp();
+                    const unsigned cnt = min(32u, md.n - s0);
+                    if (lane == 0)
+#pragma unroll 8
+                        for (unsigned q = 0; q < cnt; q++) dist = fadd(dist, terms[warp][q]);
+                    __syncwarp();
+                }
+                dist = __shfl_sync(0xffffffffu, dist, 0);
+                if (dist < low) low = dist;
+            }
+        }
+        __syncthreads();
+        if (lane == 0) red[warp] = low;
+        __syncthreads();
+        float jStar = NOVA_FLT_MAX;
+        for (unsigned w = 0; w < kThreads / 32; w++)
+            if (red[w] < jStar) jStar = red[w];
+        if (jStar > starValue) {
+            starValue = jStar;
+            for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) star[s] = row[s];
+        }
+    }
+    __syncthreads();
+    for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) Bnew[(size_t)(d.first + i) * md.n + s] = star[s];
 }
 
 // One step of a random trajectory, laid out by the host.
@@ -207,24 +468,28 @@ struct Step {
 __global__ void __launch_bounds__(kThreads) random_kernel(ExpModel md, const unsigned *__restrict__ start,
                                                           const unsigned *__restrict__ first,
                                                           const Step *__restrict__ steps, int checkPositive,
-                                                          float *__restrict__ Bnew) {
+                                                          float *__restrict__ probs, float *__restrict__ Bnew) {
     extern __shared__ __align__(16) float smem[];
     __shared__ float slot;
     __shared__ unsigned chosen;
     BlockBufs w = carve(smem, md.n);
     const unsigned k = blockIdx.x;
+    volatile float *pr = probs + (size_t)k * md.z;
     load_belief(md, start[k], w.b);
     for (unsigned q = first[k]; q < first[k + 1]; q++) {
         const Step st = steps[q];
-        float cur = 0.0f;
-        if (threadIdx.x == 0) chosen = 0;
-        for (unsigned op = 0; op < md.z; op++) {
-            const float pr = prob_obs_dense(md, w.b, w.tmp, st.a, op, &slot);
-            cur = fadd(cur, pr);
-            if (cur >= st.target && (!checkPositive || pr > 0.0f)) {
-                if (threadIdx.x == 0) chosen = op;
-                break;
+        // Every observation's probability is a chain of n additions, one
+        // thread each side by side.
+        for (unsigned o = threadIdx.x; o < md.z; o += blockDim.x) pr[o] = prob_obs_dense(md, w.b, st.a, o);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float cur = 0.0f;
+            unsigned c = 0;
+            for (unsigned op = 0; op < md.z; op++) {
+                cur = fadd(cur, pr[op]);
+                if (cur >= st.target && (!checkPositive || pr[op] > 0.0f)) { c = op; break; }
             }
+            chosen = c;
         }
         __syncthreads();
         belief_update(md, w.b, w.bp, st.a, chosen, &slot);
@@ -355,12 +620,12 @@ __global__ void dense_beliefs_kernel(unsigned n, unsigned r, unsigned rz, const 
 struct ExpWorkspace {
     ExpModel md{};
     int *S = nullptr, *Z = nullptr;
-    float *T = nullptr, *O = nullptr, *R = nullptr, *B = nullptr, *BT = nullptr;
-    unsigned *predStart = nullptr, *predIdx = nullptr;
+    float *T = nullptr, *O = nullptr, *R = nullptr, *B = nullptr, *BT = nullptr, *PO = nullptr, *predT = nullptr;
+    unsigned *predStart = nullptr, *predState = nullptr;
     size_t smem = 0;
     ~ExpWorkspace() {
         cudaFree(S); cudaFree(Z); cudaFree(T); cudaFree(O); cudaFree(R); cudaFree(B); cudaFree(BT);
-        cudaFree(predStart); cudaFree(predIdx);
+        cudaFree(PO); cudaFree(predStart); cudaFree(predState); cudaFree(predT);
     }
 };
 
@@ -370,7 +635,9 @@ int build_workspace(const POMDP *p, ExpWorkspace &ws, const char *fn) {
     int rc;
     // Predecessors of each (a, s'), in (s, i) order: action a's lists are
     // start[a*(n+1) + s'] .. start[a*(n+1) + s' + 1] of one global array.
-    std::vector<unsigned> count((size_t)m * n, 0u), start((size_t)m * (n + 1), 0u), idx(std::max<size_t>(nms, 1));
+    std::vector<unsigned> count((size_t)m * n, 0u), start((size_t)m * (n + 1), 0u),
+        state(std::max<size_t>(nms, 1));
+    std::vector<float> prob(std::max<size_t>(nms, 1));
     for (unsigned s = 0; s < n; s++)
         for (unsigned a = 0; a < m; a++)
             for (unsigned i = 0; i < ns; i++) {
@@ -396,7 +663,9 @@ int build_workspace(const POMDP *p, ExpWorkspace &ws, const char *fn) {
             for (unsigned i = 0; i < ns; i++) {
                 const int sp = p->S[((size_t)s * m + a) * ns + i];
                 if (sp < 0) break;
-                idx[cursor[(size_t)a * (n + 1) + sp]++] = (unsigned)(((size_t)s * m + a) * ns + i);
+                const unsigned k = cursor[(size_t)a * (n + 1) + sp]++;
+                state[k] = s;
+                prob[k] = p->T[((size_t)s * m + a) * ns + i];
             }
     if ((rc = dev_alloc(&ws.S, nms, fn, "the successor states")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&ws.T, nms, fn, "the state transitions")) != NOVA_SUCCESS) return rc;
@@ -406,7 +675,9 @@ int build_workspace(const POMDP *p, ExpWorkspace &ws, const char *fn) {
     if ((rc = dev_alloc(&ws.B, (size_t)r * rz, fn, "the belief values")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&ws.BT, (size_t)n * r, fn, "the dense beliefs")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&ws.predStart, start.size(), fn, "the predecessor offsets")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws.predIdx, std::max<size_t>(nms, 1), fn, "the predecessors")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&ws.predState, std::max<size_t>(nms, 1), fn, "the predecessors")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&ws.predT, std::max<size_t>(nms, 1), fn, "the predecessors")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&ws.PO, (size_t)m * n * z, fn, "the observation probabilities")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws.S, p->S, nms * sizeof(int), fn, "the successor states")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws.T, p->T, nms * sizeof(float), fn, "the state transitions")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws.O, p->O, (size_t)m * n * z * sizeof(float), fn, "the observation transitions")) != NOVA_SUCCESS)
@@ -417,11 +688,15 @@ int build_workspace(const POMDP *p, ExpWorkspace &ws, const char *fn) {
     if ((rc = h2d(ws.predStart, start.data(), start.size() * sizeof(unsigned), fn, "the predecessor offsets")) !=
             NOVA_SUCCESS)
         return rc;
-    if ((rc = h2d(ws.predIdx, idx.data(), nms * sizeof(unsigned), fn, "the predecessors")) != NOVA_SUCCESS) return rc;
+    if ((rc = h2d(ws.predState, state.data(), nms * sizeof(unsigned), fn, "the predecessors")) != NOVA_SUCCESS) return rc;
+    if ((rc = h2d(ws.predT, prob.data(), nms * sizeof(float), fn, "the predecessors")) != NOVA_SUCCESS) return rc;
+    prob_table_kernel<<<std::min<size_t>(ceil_div((size_t)m * n * z, 256), 65535u * 8u), 256>>>(n, ns, m, z, ws.S, ws.T,
+                                                                                               ws.O, ws.PO);
+    if ((rc = check_launch(fn, "observation probabilities")) != NOVA_SUCCESS) return rc;
     dense_beliefs_kernel<<<r, 256>>>(n, r, rz, ws.Z, ws.B, ws.BT);
     if ((rc = check_launch(fn, "dense beliefs")) != NOVA_SUCCESS) return rc;
-    ws.md = ExpModel{n, ns, m, z, r, rz, p->gamma, ws.S, ws.T, ws.O, ws.R, ws.Z, ws.B, ws.predStart, ws.predIdx,
-                     ws.BT};
+    ws.md = ExpModel{n, ns, m, z, r, rz, p->gamma, ws.S, ws.T, ws.O, ws.R, ws.Z, ws.B, ws.predStart, ws.predState,
+                     ws.predT, ws.BT, ws.PO};
     ws.smem = 4 * (size_t)n * sizeof(float);
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
@@ -432,7 +707,8 @@ int build_workspace(const POMDP *p, ExpWorkspace &ws, const char *fn) {
         return NOVA_ERROR_INVALID_DATA;
     }
     if (ws.smem > 40 * 1024) {
-        cudaFuncSetAttribute(distinct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws.smem);
+        cudaFuncSetAttribute(distinct_mass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws.smem);
+        cudaFuncSetAttribute(distinct_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws.smem);
         cudaFuncSetAttribute(random_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws.smem);
         cudaFuncSetAttribute(pema_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws.smem);
         cudaFuncSetAttribute(update_one_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws.smem);
@@ -478,14 +754,14 @@ int run_random(const POMDP *p, unsigned total, bool fromB0, std::vector<float> &
     for (size_t k = 0; k + 1 < first.size(); k++)
         if (first[k + 1] > first[k]) { s2.push_back(start[k]); f2.push_back(first[k]); }
     f2.push_back((unsigned)steps.size());
-    float *dB = nullptr;
+    float *dB = nullptr, *dProbs = nullptr;
     unsigned *dStart = nullptr, *dFirst = nullptr;
     Step *dSteps = nullptr;
     const size_t n = p->n;
     struct Free {
-        float *&b; unsigned *&s, *&f; Step *&st;
-        ~Free() { cudaFree(b); cudaFree(s); cudaFree(f); cudaFree(st); }
-    } guard{dB, dStart, dFirst, dSteps};
+        float *&b, *&q; unsigned *&s, *&f; Step *&st;
+        ~Free() { cudaFree(b); cudaFree(q); cudaFree(s); cudaFree(f); cudaFree(st); }
+    } guard{dB, dProbs, dStart, dFirst, dSteps};
     if ((rc = dev_alloc(&dB, (size_t)total * n, fn, "the new beliefs")) != NOVA_SUCCESS) return rc;
     if (cudaMemset(dB, 0, (size_t)total * n * sizeof(float)) != cudaSuccess) {
         cudaGetLastError();
@@ -502,7 +778,9 @@ int run_random(const POMDP *p, unsigned total, bool fromB0, std::vector<float> &
             return rc;
         if ((rc = h2d(dSteps, steps.data(), steps.size() * sizeof(Step), fn, "the trajectory steps")) != NOVA_SUCCESS)
             return rc;
-        random_kernel<<<(unsigned)s2.size(), kThreads, ws.smem>>>(ws.md, dStart, dFirst, dSteps, fromB0 ? 0 : 1, dB);
+        if ((rc = dev_alloc(&dProbs, s2.size() * p->z, fn, "the observation draws")) != NOVA_SUCCESS) return rc;
+        random_kernel<<<(unsigned)s2.size(), kThreads, ws.smem>>>(ws.md, dStart, dFirst, dSteps, fromB0 ? 0 : 1, dProbs,
+                                                                  dB);
         if ((rc = check_launch(fn, "random trajectories")) != NOVA_SUCCESS) return rc;
     }
     if (fromB0) {
@@ -517,6 +795,80 @@ int run_random(const POMDP *p, unsigned total, bool fromB0, std::vector<float> &
     }
     Bnew.assign((size_t)total * n, 0.0f);
     return d2h(Bnew.data(), dB, (size_t)total * n * sizeof(float), fn, "the new beliefs");
+}
+
+// The successor farthest from the belief set for every belief, into Bnew [r][n].
+int run_distinct(const ExpWorkspace &ws, std::vector<float> &Bnew, const char *fn) {
+    const ExpModel &md = ws.md;
+    const size_t n = md.n, mz = (size_t)md.m * md.z, rn = md.r * n;
+    int dev = 0, optin = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+        cudaGetLastError();
+        optin = 48 * 1024;
+    }
+    Distinct d{};
+    d.cap = std::min(md.n, md.rz);
+    // Beliefs whose successors are held at once: about 512 MB of them.
+    const size_t perBelief = (n * mz + md.m * n + 2 * mz) * sizeof(float);
+    d.chunk = (unsigned)std::min<size_t>(md.r, std::max<size_t>(1, (512ull << 20) / perBelief));
+    float *dB = nullptr;
+    struct Free {
+        Distinct &d; float *&b;
+        ~Free() {
+            cudaFree(d.W); cudaFree(d.bp); cudaFree(d.mass); cudaFree(d.bound); cudaFree(d.list); cudaFree(d.nnz);
+            cudaFree(d.total); cudaFree(d.odd); cudaFree(b);
+        }
+    } guard{d, dB};
+    int rc;
+    if ((rc = dev_alloc(&dB, rn, fn, "the new beliefs")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&d.W, (size_t)d.chunk * md.m * n, fn, "the successor masses")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&d.bp, (size_t)d.chunk * n * mz, fn, "the successor beliefs")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&d.mass, (size_t)d.chunk * mz, fn, "the successor sums")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&d.bound, (size_t)d.chunk * mz, fn, "the distance bounds")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&d.list, (size_t)md.r * d.cap, fn, "the belief nonzeros")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&d.nnz, md.r, fn, "the belief nonzeros")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&d.total, md.r, fn, "the belief sums")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&d.odd, 2, fn, "the belief check")) != NOVA_SUCCESS) return rc;
+    if (cudaMemsetAsync(d.odd, 0, 2 * sizeof(unsigned)) != cudaSuccess) {
+        cudaGetLastError();
+        NOVA_ERR(fn, "Failed to clear the belief check.");
+        return NOVA_ERROR_KERNEL_EXECUTION;
+    }
+    distinct_check_kernel<<<std::min<size_t>(ceil_div(mz * n, 256), 65535u), 256>>>(md, d.odd);
+    if ((rc = check_launch(fn, "observation probabilities")) != NOVA_SUCCESS) return rc;
+    distinct_list_kernel<<<ceil_div(md.r, kThreads / 32), kThreads>>>(md, d);
+    if ((rc = check_launch(fn, "belief nonzeros")) != NOVA_SUCCESS) return rc;
+    // Successors per block of the bound kernel: 64 where they fit in shared
+    // memory (each nonzero is read once for all of them), else 32, else 32
+    // read through the cache.
+    const size_t tile64 = (n + 32) * 64 * sizeof(float), tile32 = (n + 32) * 32 * sizeof(float);
+    const bool wide = mz > 32 && tile64 <= (size_t)optin, shared = wide || tile32 <= (size_t)optin;
+    const unsigned rows = wide ? 64u : 32u;
+    const size_t boundSmem = wide ? tile64 : shared ? tile32 : 32 * 32 * sizeof(float);
+    auto bound = wide ? distinct_bound_kernel<64, true> : shared ? distinct_bound_kernel<32, true>
+                                                                 : distinct_bound_kernel<32, false>;
+    if (boundSmem > 48 * 1024 &&
+            cudaFuncSetAttribute(bound, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)boundSmem) != cudaSuccess) {
+        cudaGetLastError();
+        NOVA_ERR(fn, "Failed to configure the distance kernel.");
+        return NOVA_ERROR_KERNEL_EXECUTION;
+    }
+    for (d.first = 0; d.first < md.r; d.first += d.chunk) {
+        const unsigned count = std::min(d.chunk, md.r - d.first);
+        Distinct part = d;
+        part.chunk = count;
+        distinct_mass_kernel<<<count * md.m, kThreads, n * sizeof(float)>>>(md, part);
+        if ((rc = check_launch(fn, "successor masses")) != NOVA_SUCCESS) return rc;
+        distinct_rows_kernel<<<ceil_div((size_t)count * mz, kThreads), kThreads>>>(md, part);
+        if ((rc = check_launch(fn, "successor beliefs")) != NOVA_SUCCESS) return rc;
+        bound<<<count * ceil_div(mz, rows), 1024, boundSmem>>>(md, part);
+        if ((rc = check_launch(fn, "distance bounds")) != NOVA_SUCCESS) return rc;
+        distinct_select_kernel<<<count, kThreads, 2 * n * sizeof(float)>>>(md, part, dB);
+        if ((rc = check_launch(fn, "distinct beliefs")) != NOVA_SUCCESS) return rc;
+    }
+    Bnew.assign(rn, 0.0f);
+    return d2h(Bnew.data(), dB, rn * sizeof(float), fn, "the new beliefs");
 }
 
 }  // namespace
@@ -572,17 +924,7 @@ extern "C" int pomdp_expand_distinct_beliefs_cpu(POMDP *pomdp) {
         ExpWorkspace ws;
         int rc = build_workspace(pomdp, ws, fn);
         if (rc != NOVA_SUCCESS) return rc;
-        float *dB = nullptr;
-        const size_t rn = (size_t)pomdp->r * pomdp->n;
-        if ((rc = dev_alloc(&dB, rn, fn, "the new beliefs")) != NOVA_SUCCESS) return rc;
-        distinct_kernel<<<pomdp->r, kThreads, ws.smem>>>(ws.md, dB);
-        rc = check_launch(fn, "distinct beliefs");
-        if (rc == NOVA_SUCCESS) {
-            Bnew.assign(rn, 0.0f);
-            rc = d2h(Bnew.data(), dB, rn * sizeof(float), fn, "the new beliefs");
-        }
-        cudaFree(dB);
-        if (rc != NOVA_SUCCESS) return rc;
+        if ((rc = run_distinct(ws, Bnew, fn)) != NOVA_SUCCESS) return rc;
     }
     return pomdp_add_new_raw_beliefs_cpu(pomdp, pomdp->r, Bnew.data());
 }

@@ -175,3 +175,29 @@ def test_sweep_plan(n, m, ns, tile, ragged, crowd):
     V, pi = orc.mdp_vi_solve(md, horizon=3, VInitial=V0)
     np.testing.assert_array_equal(bits(pol.V_array()), bits(V))
     np.testing.assert_array_equal(pol.pi_array(), pi)
+
+
+@pytest.mark.parametrize("n,m,z,r,rz,odd", [(3, 1, 1, 2, 2, ""), (40, 3, 11, 33, 9, ""), (65, 2, 40, 20, 65, "negative"),
+                                            (90, 2, 3, 70, 7, "same"), (50, 2, 4, 30, 6, "infinite"),
+                                            (900, 2, 17, 12, 30, "zero"), (1800, 2, 3, 9, 40, "")])
+def test_distinct_expansion(n, m, z, r, rz, odd):
+    """One and several tiles of successors, successors in and out of shared
+    memory, beliefs at equal distances, observations that cannot occur, and
+    probabilities for which no bound holds."""
+    md = synth.random_pomdp(n=n, m=m, z=z, ns=min(5, n), r=r, rz=rz, gamma=0.9, horizon=2, seed=n + r)
+    if odd == "negative":
+        md["T"][::7, 0, 0] *= -1
+    elif odd == "infinite":
+        md["O"][0, ::9, 1] = np.inf
+    elif odd == "zero":
+        md["O"][:, :, 0] = 0.0
+    elif odd == "same":
+        md["Z"][r // 2:], md["B"][r // 2:] = md["Z"][0], md["B"][0]
+    md["Z"] = md["Z"][:, ::-1].copy()   # supports in no ascending order
+    md["B"] = md["B"][:, ::-1].copy()
+    p = POMDP.from_arrays(md)
+    p.expand(method="distinct_beliefs")
+    Z, B = orc.merge_raw_beliefs(md["Z"], md["B"], orc.expand_distinct(md))
+    out = p.arrays()
+    np.testing.assert_array_equal(out["Z"], Z)
+    np.testing.assert_array_equal(bits(out["B"]), bits(B))

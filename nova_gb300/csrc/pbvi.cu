@@ -411,12 +411,11 @@ __device__ __forceinline__ unsigned load_succ(const DevModel &md, const unsigned
 __global__ void __launch_bounds__(256) action_value_kernel(DevModel md, const unsigned *__restrict__ succLen,
                                     const unsigned *__restrict__ suppLen, const float *__restrict__ C3,
                                     const float *__restrict__ G, const unsigned *__restrict__ jstar,
-                                    const unsigned *__restrict__ items, unsigned nItems,
-                                    float *__restrict__ actVal) {
+                                    unsigned nItems, float *__restrict__ actVal) {
     const unsigned warpGlobal = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned lane = threadIdx.x & 31;
     if (warpGlobal >= nItems) return;
-    const unsigned ia = items ? items[warpGlobal] : warpGlobal;
+    const unsigned ia = warpGlobal;
     const unsigned i = ia / md.m, a = ia % md.m;
     const unsigned Li = suppLen[i];
     const bool regs = reg_form(md);
@@ -452,9 +451,9 @@ __global__ void __launch_bounds__(256) action_value_kernel(DevModel md, const un
 // and action, as in the reference.
 __global__ void assemble_kernel(DevModel md, const unsigned *__restrict__ succLen, const float *__restrict__ C3,
                                 const float *__restrict__ G, const unsigned *__restrict__ jstar,
-                                const float *__restrict__ actVal, unsigned beliefBegin, float *__restrict__ dst,
-                                unsigned *__restrict__ pi, float *__restrict__ rowOut, unsigned *__restrict__ actionOut) {
-    const unsigned i = beliefBegin + blockIdx.x;
+                                const float *__restrict__ actVal, float *__restrict__ dst,
+                                unsigned *__restrict__ pi) {
+    const unsigned i = blockIdx.x;
     __shared__ unsigned bestA;
     extern __shared__ unsigned jsh[];  // [z]
     if (threadIdx.x == 0) {
@@ -465,13 +464,12 @@ __global__ void assemble_kernel(DevModel md, const unsigned *__restrict__ succLe
             if (v > best) { best = v; ba = a; }
         }
         bestA = ba;
-        if (actionOut) *actionOut = ba;
     }
     __syncthreads();
     const unsigned a = bestA;
     if (a == kNone) return;
-    if (pi && threadIdx.x == 0) pi[i] = a;
-    float *out = rowOut ? rowOut : dst + (size_t)i * md.n;
+    if (threadIdx.x == 0) pi[i] = a;
+    float *out = dst + (size_t)i * md.n;
     const unsigned *js = jstar + ((size_t)i * md.m + a) * md.z;
     for (unsigned o = threadIdx.x; o < md.z; o += blockDim.x) jsh[o] = js[o];
     __syncthreads();
@@ -923,7 +921,7 @@ BackupEngine::~BackupEngine() {
     cudaFree(jstar); cudaFree(actVal); cudaFree(partV); cudaFree(partU); cudaFree(items); cudaFree(itemCount);
     cudaFree(keptCount);
     cudaFree(dotScratch); cudaFree(bDense); cudaFree(resultA); cudaFree(resultV); cudaFree(rowScratch);
-    cudaFree(vnb); cudaFree(vnp1b); cudaFree(btilde);
+    cudaFree(vnb); cudaFree(vnp1b);
     cudaFree(Proj); cudaFree(ustar); cudaFree(scanV); cudaFree(scanU);
     if (eventsMade)
         for (auto &e : ev) cudaEventDestroy(e);
@@ -1207,33 +1205,21 @@ int BackupEngine::fill_items(unsigned first, unsigned count, const char *fn) {
     return check_launch(fn, "work list");
 }
 
-int BackupEngine::assemble(const float *src, float *dst, unsigned *pi, int onlyBelief, float *dstRowOverride,
-                           unsigned *actionOut, const char *fn) {
+int BackupEngine::assemble(const float *src, float *dst, unsigned *pi, const char *fn) {
     int rc;
-    const unsigned firstBelief = onlyBelief >= 0 ? (unsigned)onlyBelief : 0u;
-    const unsigned nBeliefs = onlyBelief >= 0 ? 1u : md.r;
-    const unsigned nItems = nBeliefs * md.m;
-    const unsigned *itemList = nullptr;
-    if (onlyBelief >= 0) {
-        iota_items_kernel<<<ceil_div(nItems, 256), 256, 0, stream>>>(items, nItems, firstBelief * md.m);
-        if ((rc = check_launch(fn, "work list")) != NOVA_SUCCESS) return rc;
-        itemList = items;
-    }
-    if (useProjNow && onlyBelief < 0)
+    const unsigned nItems = md.r * md.m;
+    if (useProjNow)
         action_value_proj_kernel<<<ceil_div((size_t)nItems * 32, 256), 256, 0, stream>>>(md, suppLen, proj_view(),
                                                                                          ustar, actVal);
     else
         action_value_kernel<<<ceil_div((size_t)nItems * 32, 256), 256, 0, stream>>>(md, succLen, suppLen, C3, src,
-                                                                                    jstar, itemList, nItems, actVal);
+                                                                                    jstar, nItems, actVal);
     if ((rc = check_launch(fn, "action values")) != NOVA_SUCCESS) return rc;
-    if (onlyBelief < 0 && !capturing) cudaEventRecord(ev[6], stream);
-    if (useProjNow && onlyBelief < 0)
-        assemble_proj_kernel<<<nBeliefs, 256, md.z * sizeof(unsigned), stream>>>(md, proj_view(), ustar, actVal,
-                                                                                  dst, pi);
+    if (!capturing) cudaEventRecord(ev[6], stream);
+    if (useProjNow)
+        assemble_proj_kernel<<<md.r, 256, md.z * sizeof(unsigned), stream>>>(md, proj_view(), ustar, actVal, dst, pi);
     else
-        assemble_kernel<<<nBeliefs, 256, md.z * sizeof(unsigned), stream>>>(md, succLen, C3, src, jstar, actVal,
-                                                                             firstBelief, dst, pi, dstRowOverride,
-                                                                             actionOut);
+        assemble_kernel<<<md.r, 256, md.z * sizeof(unsigned), stream>>>(md, succLen, C3, src, jstar, actVal, dst, pi);
     return check_launch(fn, "alpha assembly");
 }
 
@@ -1322,7 +1308,7 @@ int BackupEngine::backup_all(const float *src, unsigned rGamma, float *dst, unsi
         if ((rc = exact_score(items, allItems, nU, fn)) != NOVA_SUCCESS) return rc;
     }
     cudaEventRecord(ev[3], stream);
-    if ((rc = assemble(src, dst, pi, -1, nullptr, nullptr, fn)) != NOVA_SUCCESS) return rc;
+    if ((rc = assemble(src, dst, pi, fn)) != NOVA_SUCCESS) return rc;
     cudaEventRecord(ev[4], stream);
     if (cudaEventSynchronize(ev[4]) != cudaSuccess) {
         cudaGetLastError();
@@ -1381,7 +1367,7 @@ int BackupEngine::fixed_post(const float *src, float *dst, unsigned *pi, bool te
         rc = scan_rows(nullptr, md.m * md.z * md.r, nU, fn);
     }
     if (rc != NOVA_SUCCESS) return rc;
-    return assemble(src, dst, pi, -1, nullptr, nullptr, fn);
+    return assemble(src, dst, pi, fn);
 }
 
 int BackupEngine::backup_fixed(const float *src, float *dst, unsigned *pi, const char *fn) {

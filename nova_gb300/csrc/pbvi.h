@@ -88,7 +88,6 @@ struct BackupEngine {
     double *resultV = nullptr;           // [1]
     float *rowScratch = nullptr;         // [n] single-belief alpha (Perseus)
     float *vnb = nullptr, *vnp1b = nullptr;  // [r] Perseus values over V_n and V_{n+1}
-    unsigned *btilde = nullptr;          // [r] Perseus compacted belief list
     cudaStream_t stream = 0;
     cudaEvent_t ev[8] = {};
     bool eventsMade = false;
@@ -152,9 +151,8 @@ struct BackupEngine {
     // Write the last backup's selections (action per belief, alpha per
     // (belief, observation) under that action) to device arrays.
     int record(const unsigned *pi, unsigned *actOut, unsigned *selOut, const char *fn);
-    // Action values and best-action assembly for all beliefs (or one).
-    int assemble(const float *src, float *dst, unsigned *pi, int onlyBelief, float *dstRowOverride,
-                 unsigned *actionOut, const char *fn);
+    // Action values and best-action assembly for all beliefs.
+    int assemble(const float *src, float *dst, unsigned *pi, const char *fn);
     // After backup_all: the number of beliefs whose every action value
     // failed to beat the -1e10 sentinel (their row and action were left as
     // they were in dst and pi).

@@ -3,17 +3,29 @@
 //
 // One update (pomdp_perseus_cpu.cpp:312-429):
 //   * draw a belief from B~ with rand() on the host (the reference formula);
-//   * back it up against V_n = Gamma[0, rGamma) with the exact-order engine
-//     (dedup + scoring + assembly of pbvi.cu, restricted to one belief);
+//   * back it up against V_n = Gamma[0, rGamma) (perseus_score_kernel,
+//     perseus_action_kernel, perseus_assemble_kernel: the FP32 operations of
+//     the point-based backup in the reference's order, for one belief);
 //   * keep the new alpha if it does not lose value at the belief, else copy
-//     the belief's best old alpha (pomdp_perseus_cpu.cpp:367-374);
-//   * rebuild B~ = {i : V_{n+1}(b_i) < V_n(b_i)} (pomdp_perseus_cpu.cpp:387-402).
+//     the belief's best old alpha (pomdp_perseus_cpu.cpp:367-374), and rebuild
+//     B~ = {i : V_{n+1}(b_i) < V_n(b_i)} (pomdp_perseus_cpu.cpp:387-402), in
+//     perseus_commit_kernel.
 // V_n(b_i) is constant within a horizon step and is computed once per step;
 // V_{n+1}(b_i) is a running maximum updated with the one new alpha, which is
 // exact because only the maximum value (not its index) enters the test.
+//
+// One belief's backup is little work (n = 512, m = 8, z = ns = 16, rz = 32,
+// three alphas: 0.2 M products) and is bound by the latency of its dependent
+// loads, so each of the four launches spreads it as widely as its order of
+// additions allows, and the chosen alphas' projections are kept from the
+// scoring for the action values. An update took 310 us with the kernels made
+// for whole belief sets (one block per (belief, action) stepping through the
+// support, one block for the assembly, eleven launches and three
+// synchronisations); it takes 75 us.
 
 #include "pbvi.h"
 
+#include <algorithm>
 #include <cstdlib>
 #include <vector>
 
@@ -55,85 +67,282 @@ __global__ void perseus_vb_kernel(DevModel md, const unsigned *__restrict__ supp
         const float d = belief_dot(md, Li, i, G + (size_t)j * md.n);
         if (best < d) { best = d; bj = j; }
     }
-    __shared__ float sv[256];
-    __shared__ unsigned si[256];
-    sv[threadIdx.x] = best; si[threadIdx.x] = bj;
+    // Larger value, lower index on ties; kNoneP: none above -1e10.
+    auto take = [&](float v, unsigned j) {
+        if (j != kNoneP && (bj == kNoneP || v > best || (v == best && j < bj))) { best = v; bj = j; }
+    };
+    __shared__ float sv[8];
+    __shared__ unsigned si[8];
+    for (int off = 16; off > 0; off >>= 1) {
+        const float v = __shfl_xor_sync(0xffffffffu, best, off);
+        take(v, __shfl_xor_sync(0xffffffffu, bj, off));
+    }
+    if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = best; si[threadIdx.x >> 5] = bj; }
     __syncthreads();
     if (threadIdx.x == 0) {
-        float b = NOVA_FLT_MIN;
-        unsigned bi = kNoneP;
-        for (unsigned t = 0; t < blockDim.x; t++) {
-            if (si[t] == kNoneP) continue;
-            if (bi == kNoneP || sv[t] > b || (sv[t] == b && si[t] < bi)) { b = sv[t]; bi = si[t]; }
-        }
-        vOut[i] = b;
+        for (unsigned w = 1; w < 8; w++) take(sv[w], si[w]);
+        vOut[i] = best;
         // The reference's caller starts alphaPrimeIndex at 0 (pomdp_perseus_cpu.cpp:361).
-        if (idxOut) idxOut[i] = bi == kNoneP ? 0u : bi;
+        if (idxOut) idxOut[i] = bj == kNoneP ? 0u : bj;
     }
 }
 
-// Keep the new alpha or copy the belief's best old one, into slot `slot`.
-__global__ void perseus_commit_kernel(DevModel md, const unsigned *__restrict__ suppLen, unsigned bIndex,
-                                      const float *__restrict__ alpha, const unsigned *__restrict__ alphaAction,
-                                      const float *__restrict__ vnb, const unsigned *__restrict__ vnbIdx,
-                                      const float *__restrict__ G, const unsigned *__restrict__ pi,
-                                      float *__restrict__ Gp, unsigned *__restrict__ piP, unsigned slot) {
-    __shared__ int keepNew;
-    if (threadIdx.x == 0) {
-        const float bDotAlpha = belief_dot(md, suppLen[bIndex], bIndex, alpha);
-        keepNew = bDotAlpha >= vnb[bIndex] ? 1 : 0;
-        const unsigned act = *alphaAction == kNoneP ? 0u : *alphaAction;
-        piP[slot] = keepNew ? act : pi[vnbIdx[bIndex]];
-    }
-    __syncthreads();
-    const float *srcRow = keepNew ? alpha : G + (size_t)vnbIdx[bIndex] * md.n;
-    for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) Gp[(size_t)slot * md.n + s] = srcRow[s];
+__device__ __forceinline__ bool better(float v1, unsigned u1, float v2, unsigned u2) {
+    return v1 > v2 || (v1 == v2 && u1 < u2);
 }
 
-// V_{n+1}(b_i) <- max(V_{n+1}(b_i), b_i . newRow) with the reference's strict '<'.
-__global__ void perseus_raise_kernel(DevModel md, const unsigned *__restrict__ suppLen, const float *__restrict__ row,
-                                     float *__restrict__ vnp1b) {
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= md.r) return;
-    const float d = belief_dot(md, suppLen[i], i, row);
-    if (vnp1b[i] < d) vnp1b[i] = d;
-}
-
-// B~ = {i : V_{n+1}(b_i) < V_n(b_i)} in increasing i (single block).
-__global__ void __launch_bounds__(1024) perseus_btilde_kernel(unsigned r, const float *__restrict__ vnb,
-                                                              const float *__restrict__ vnp1b,
-                                                              unsigned *__restrict__ out, unsigned *__restrict__ count) {
-    __shared__ unsigned warpSums[32];
-    __shared__ unsigned carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (unsigned base = 0; base < r; base += blockDim.x) {
-        const unsigned i = base + threadIdx.x;
-        const unsigned flag = (i < r && vnp1b[i] < vnb[i]) ? 1u : 0u;
-        unsigned v = flag;
-        for (int off = 1; off < 32; off <<= 1) {
-            const unsigned y = __shfl_up_sync(0xffffffffu, v, off);
-            if (lane >= (unsigned)off) v += y;
+// fl(gamma * sum_l C3 * G_j(S)) for state s under action a, observation o
+// (the reference's order). Four successors' loads are issued together.
+__device__ __forceinline__ float projected_at(const DevModel &md, const float *__restrict__ C3, unsigned Ls,
+                                              const float *__restrict__ Gj, unsigned a, unsigned o, unsigned s) {
+    const float *c = C3 + (((size_t)a * md.z + o) * md.n + s) * md.ns;
+    const int *sp = md.S + ((size_t)s * md.m + a) * md.ns;
+    float vt = 0.0f;
+    unsigned l = 0;
+    for (; l + 8 <= Ls; l += 8) {
+        float g[8], cc[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            g[q] = Gj[__ldg(sp + l + q)];
+            cc[q] = __ldg(c + l + q);
         }
-        if (lane == 31) warpSums[warp] = v;
-        __syncthreads();
-        if (warp == 0) {
-            unsigned w = lane < (blockDim.x >> 5) ? warpSums[lane] : 0u;
-            for (int off = 1; off < 32; off <<= 1) {
-                const unsigned y = __shfl_up_sync(0xffffffffu, w, off);
-                if (lane >= (unsigned)off) w += y;
+#pragma unroll
+        for (int q = 0; q < 8; q++) vt = fadd(vt, fmul(cc[q], g[q]));
+    }
+    for (; l < Ls; l++) vt = fadd(vt, fmul(__ldg(c + l), Gj[__ldg(sp + l)]));
+    return fmul(vt, md.gamma);
+}
+
+// Belief i against alphas [0, rows): warp (a*z+o, split) scores its share of
+// them, lane k taking support state k (32 at a time), and keeps the best and
+// its index (kNoneP: none above -1e10) and, in one of its two slots of
+// proj [m*z][splits][2][rz], the best one's projections at the support.
+__global__ void __launch_bounds__(128) perseus_score_kernel(DevModel md, const unsigned *__restrict__ succLen,
+                                                            const unsigned *__restrict__ suppLen,
+                                                            const float *__restrict__ C3, const float *__restrict__ G,
+                                                            unsigned rows, unsigned i, unsigned splits, unsigned share,
+                                                            float *__restrict__ partV, unsigned *__restrict__ partU,
+                                                            float *__restrict__ proj) {
+    const unsigned lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (w >= md.m * md.z * splits) return;
+    const unsigned ao = w / splits, split = w % splits, a = ao / md.z, o = ao % md.z;
+    const unsigned Li = suppLen[i];
+    float *slots = proj + (size_t)w * 2 * md.rz;
+    float best = NOVA_FLT_MIN;
+    unsigned bu = kNoneP, slot = 0;
+    for (unsigned u = split * share; u < min(rows, (split + 1) * share); u++) {
+        float *mine = slots + (slot ^ 1u) * md.rz;
+        float score = 0.0f;
+        for (unsigned k0 = 0; k0 < Li; k0 += 32) {
+            const unsigned k = k0 + lane;
+            float p = 0.0f;
+            if (k < Li) {
+                const unsigned s = (unsigned)md.Z[(size_t)i * md.rz + k];
+                p = projected_at(md, C3, succLen[(size_t)s * md.m + a], G + (size_t)u * md.n, a, o, s);
+                mine[k] = p;
+                p = fmul(p, md.B[(size_t)i * md.rz + k]);
             }
-            warpSums[lane] = w;
+            const unsigned cnt = min(32u, Li - k0);
+            for (unsigned t = 0; t < cnt; t++) score = fadd(score, __shfl_sync(0xffffffffu, p, t));
         }
+        if (score > best) {
+            best = score;
+            bu = u;
+            slot ^= 1u;
+        }
+    }
+    if (lane == 0) {
+        partV[w] = best;
+        partU[w] = bu == kNoneP ? kNoneP : bu << 1 | slot;
+    }
+}
+
+// One warp per action: per observation the best alpha of all splits (the
+// lowest index among equals; where none beat -1e10 the previous observation's,
+// row 0 for the first), then the action's value at the belief: alpha_a(s_k) =
+// R(s_k,a) + sum_o projection, times b_k, summed in support order.
+__global__ void __launch_bounds__(32) perseus_action_kernel(DevModel md, const unsigned *__restrict__ succLen,
+                                                            const unsigned *__restrict__ suppLen,
+                                                            const float *__restrict__ C3, const float *__restrict__ G,
+                                                            unsigned i, unsigned splits,
+                                                            const float *__restrict__ partV,
+                                                            const unsigned *__restrict__ partU,
+                                                            const float *__restrict__ proj,
+                                                            unsigned *__restrict__ jstar, float *__restrict__ actVal) {
+    extern __shared__ unsigned from[];  // [z] split and slot of the choice, or kNoneP
+    const unsigned a = blockIdx.x, lane = threadIdx.x;
+    unsigned *js = jstar + ((size_t)i * md.m + a) * md.z;
+    unsigned prev = 0;
+    for (unsigned o0 = 0; o0 < md.z; o0 += 32) {
+        const unsigned o = o0 + lane;
+        float v = NOVA_FLT_MIN;
+        unsigned u = kNoneP, at = kNoneP;
+        if (o < md.z) {
+            const size_t w0 = ((size_t)a * md.z + o) * splits;
+            for (unsigned sp = 0; sp < splits; sp++) {
+                const unsigned pu = partU[w0 + sp];
+                const float pv = partV[w0 + sp];
+                if (pu != kNoneP && (u == kNoneP || better(pv, pu >> 1, v, u))) {
+                    v = pv;
+                    u = pu >> 1;
+                    at = sp << 1 | (pu & 1u);
+                }
+            }
+            from[o] = at;
+        }
+        const unsigned cnt = min(32u, md.z - o0);
+        for (unsigned t = 0; t < cnt; t++) {
+            const unsigned ut = __shfl_sync(0xffffffffu, u, t);
+            if (ut != kNoneP) prev = ut;
+            if (lane == t) u = prev;
+        }
+        if (o < md.z) js[o] = u;
+    }
+    __syncwarp();
+    const unsigned Li = suppLen[i];
+    float value = 0.0f;
+    for (unsigned k0 = 0; k0 < Li; k0 += 32) {
+        const unsigned k = k0 + lane;
+        float p = 0.0f;
+        if (k < Li) {
+            const unsigned s = (unsigned)md.Z[(size_t)i * md.rz + k];
+            float alpha = md.R[(size_t)s * md.m + a];
+            for (unsigned o = 0; o < md.z; o += 8) {
+                float q[8];
+#pragma unroll
+                for (unsigned t = 0; t < 8; t++) {
+                    if (o + t >= md.z) break;
+                    const unsigned at = from[o + t];
+                    q[t] = at != kNoneP
+                        ? proj[((((size_t)a * md.z + o + t) * splits + (at >> 1)) * 2 + (at & 1u)) * md.rz + k]
+                        : projected_at(md, C3, succLen[(size_t)s * md.m + a], G + (size_t)js[o + t] * md.n, a, o + t, s);
+                }
+#pragma unroll
+                for (unsigned t = 0; t < 8; t++)
+                    if (o + t < md.z) alpha = fadd(alpha, q[t]);
+            }
+            p = fmul(alpha, md.B[(size_t)i * md.rz + k]);
+        }
+        const unsigned cnt = min(32u, Li - k0);
+        for (unsigned t = 0; t < cnt; t++) value = fadd(value, __shfl_sync(0xffffffffu, p, t));
+    }
+    if (lane == 0) actVal[a] = value;
+}
+
+// The best action's alpha (strict '>' from -1e10, lowest action on ties; none:
+// *action = kNoneP and the row stays) over 32 states a block: thread (x, y)
+// projects state x for observations y, y + 16, ...; sixteen at a time they are
+// added in observation order.
+constexpr unsigned kAssembleObs = 16;
+
+__global__ void __launch_bounds__(32 * kAssembleObs) perseus_assemble_kernel(
+        DevModel md, const unsigned *__restrict__ succLen, const float *__restrict__ C3, const float *__restrict__ G,
+        unsigned i, const unsigned *__restrict__ jstar, const float *__restrict__ actVal, float *__restrict__ row,
+        unsigned *__restrict__ action) {
+    __shared__ float part[kAssembleObs][32];
+    __shared__ unsigned bestA;
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        float best = NOVA_FLT_MIN;
+        unsigned ba = kNoneP;
+        for (unsigned a = 0; a < md.m; a++) {
+            const float v = actVal[a];
+            if (v > best) { best = v; ba = a; }
+        }
+        bestA = ba;
+        if (blockIdx.x == 0) *action = ba;
+    }
+    __syncthreads();
+    const unsigned a = bestA, s = blockIdx.x * 32 + threadIdx.x;
+    if (a == kNoneP) return;
+    const unsigned *js = jstar + ((size_t)i * md.m + a) * md.z;
+    const unsigned Ls = s < md.n ? succLen[(size_t)s * md.m + a] : 0u;
+    float alpha = s < md.n ? md.R[(size_t)s * md.m + a] : 0.0f;
+    for (unsigned o0 = 0; o0 < md.z; o0 += kAssembleObs) {
+        const unsigned o = o0 + threadIdx.y;
+        if (s < md.n && o < md.z)
+            part[threadIdx.y][threadIdx.x] = projected_at(md, C3, Ls, G + (size_t)js[o] * md.n, a, o, s);
         __syncthreads();
-        const unsigned pos = carry + (warp > 0 ? warpSums[warp - 1] : 0u) + v - flag;
-        if (flag) out[pos] = i;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += warpSums[(blockDim.x >> 5) - 1];
+        if (threadIdx.y == 0)
+            for (unsigned q = 0; q < min(kAssembleObs, md.z - o0); q++) alpha = fadd(alpha, part[q][threadIdx.x]);
         __syncthreads();
     }
-    if (threadIdx.x == 0) *count = carry;
+    if (threadIdx.y == 0 && s < md.n) row[s] = alpha;
+}
+
+// belief_dot by a whole warp: the products side by side, added in support order.
+__device__ __forceinline__ float belief_dot_warp(const DevModel &md, unsigned Li, unsigned i, const float *alpha,
+                                                 unsigned lane) {
+    float acc = 0.0f;
+    for (unsigned k0 = 0; k0 < Li; k0 += 32) {
+        const unsigned k = k0 + lane;
+        const float p = k < Li ? fmul(md.B[(size_t)i * md.rz + k], alpha[md.Z[(size_t)i * md.rz + k]]) : 0.0f;
+        const unsigned cnt = min(32u, Li - k0);
+        for (unsigned t = 0; t < cnt; t++) acc = fadd(acc, __shfl_sync(0xffffffffu, p, t));
+    }
+    return acc;
+}
+
+// Keep the new alpha or take the belief's best old one, as row `slot` of V_{n+1};
+// raise V_{n+1}(b_i) <- max(V_{n+1}(b_i), b_i . row) with the reference's strict
+// '<'; and list B~ = {i : V_{n+1}(b_i) < V_n(b_i)} in increasing i, behind its
+// size, in out [1 + r]. Every block decides about the row by itself; the one
+// that finishes last makes the list. *done is 0 before and after.
+__global__ void __launch_bounds__(256) perseus_commit_kernel(DevModel md, const unsigned *__restrict__ suppLen,
+                                                             unsigned bIndex, const float *__restrict__ alpha,
+                                                             const unsigned *__restrict__ alphaAction,
+                                                             const float *__restrict__ vnb,
+                                                             const unsigned *__restrict__ vnbIdx,
+                                                             const float *__restrict__ G,
+                                                             const unsigned *__restrict__ pi, float *__restrict__ Gp,
+                                                             unsigned *__restrict__ piP, unsigned slot, float *vnp1b,
+                                                             unsigned *__restrict__ out, unsigned *__restrict__ done) {
+    __shared__ int keepNew;
+    __shared__ bool last;
+    __shared__ unsigned warpSums[8];
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp == 0) {
+        const float acc = belief_dot_warp(md, suppLen[bIndex], bIndex, alpha, lane);
+        if (lane == 0) {
+            keepNew = acc >= vnb[bIndex] ? 1 : 0;
+            if (blockIdx.x == 0) {
+                const unsigned act = *alphaAction == kNoneP ? 0u : *alphaAction;
+                piP[slot] = keepNew ? act : pi[vnbIdx[bIndex]];
+            }
+        }
+    }
+    __syncthreads();
+    const float *row = keepNew ? alpha : G + (size_t)vnbIdx[bIndex] * md.n;
+    for (unsigned s = blockIdx.x * 256 + threadIdx.x; s < md.n; s += gridDim.x * 256) Gp[(size_t)slot * md.n + s] = row[s];
+    for (unsigned i = blockIdx.x * 8 + warp; i < md.r; i += gridDim.x * 8) {
+        const float d = belief_dot_warp(md, suppLen[i], i, row, lane);
+        if (lane == 0 && vnp1b[i] < d) vnp1b[i] = d;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // Every thread takes a range of beliefs; a block scan gives its first place.
+    const unsigned per = (md.r + 255) / 256;
+    const unsigned b = min(md.r, threadIdx.x * per), e = min(md.r, b + per);
+    unsigned cnt = 0;
+    for (unsigned i = b; i < e; i++) cnt += __ldcg(vnp1b + i) < vnb[i] ? 1u : 0u;
+    unsigned v = cnt;
+    for (int off = 1; off < 32; off <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, v, off);
+        if (lane >= (unsigned)off) v += y;
+    }
+    if (lane == 31) warpSums[warp] = v;
+    __syncthreads();
+    unsigned pos = v - cnt;
+    for (unsigned w = 0; w < warp; w++) pos += warpSums[w];
+    for (unsigned i = b; i < e; i++)
+        if (__ldcg(vnp1b + i) < vnb[i]) out[1 + pos++] = i;
+    if (threadIdx.x == 255) {
+        out[0] = pos;
+        *done = 0u;
+    }
 }
 
 __global__ void fill_float_kernel(float *p, unsigned count, float v) {
@@ -146,25 +355,39 @@ struct PerseusCore {
     BackupEngine eng;
     bool built = false;
     unsigned *vnbIdx = nullptr;
-    // Validity of the per-horizon-step caches (V_n values, V_n dedup).
+    // Validity of the per-horizon-step cache (V_n values).
     bool cacheValid = false;
     unsigned cacheHorizon = 0;
-    unsigned nU = 0;
-    ~PerseusCore() { cudaFree(vnbIdx); }
+    unsigned *bt = nullptr;       // [1 + r] |B~| and B~
+    unsigned *done = nullptr;     // [1] finished blocks of perseus_commit_kernel
+    float *partV = nullptr, *proj = nullptr;   // the scoring's partial maxima and projections
+    unsigned *partU = nullptr;
+    size_t partCap = 0;
+    std::vector<unsigned> btHost;
+    ~PerseusCore() {
+        cudaFree(vnbIdx); cudaFree(bt); cudaFree(done); cudaFree(partV); cudaFree(partU); cudaFree(proj);
+    }
 
     int build(const DevModel &md, const char *fn) {
         int rc = eng.build(md, fn);
         if (rc != NOVA_SUCCESS) return rc;
         if ((rc = dev_alloc(&eng.vnb, md.r, fn, "V_n(b)")) != NOVA_SUCCESS) return rc;
         if ((rc = dev_alloc(&eng.vnp1b, md.r, fn, "V_n+1(b)")) != NOVA_SUCCESS) return rc;
-        if ((rc = dev_alloc(&eng.btilde, md.r, fn, "B~")) != NOVA_SUCCESS) return rc;
+        if ((rc = dev_alloc(&bt, (size_t)md.r + 1, fn, "B~")) != NOVA_SUCCESS) return rc;
+        if ((rc = dev_alloc(&done, 1, fn, "the block counter")) != NOVA_SUCCESS) return rc;
         if ((rc = dev_alloc(&vnbIdx, md.r, fn, "argmax V_n(b)")) != NOVA_SUCCESS) return rc;
+        if (cudaMemsetAsync(done, 0, sizeof(unsigned), eng.stream) != cudaSuccess) {
+            cudaGetLastError();
+            NOVA_ERR(fn, "Failed to clear the block counter.");
+            return NOVA_ERROR_KERNEL_EXECUTION;
+        }
+        btHost.resize((size_t)md.r + 1);
         built = true;
         return NOVA_SUCCESS;
     }
 
-    // Per-step caches: V_n(b_i) with maximisers, the dedup of V_n, and
-    // V_{n+1}(b_i) over the rows already in Gamma'.
+    // Per-step cache: V_n(b_i) with maximisers, and V_{n+1}(b_i) over the rows
+    // already in Gamma'.
     int refresh(const float *G, unsigned rGamma, const float *Gp, unsigned rGammaPrime, const char *fn) {
         const DevModel &md = eng.md;
         int rc;
@@ -180,8 +403,6 @@ struct PerseusCore {
         else
             fill_float_kernel<<<ceil_div(md.r, 256), 256, 0, eng.stream>>>(eng.vnp1b, md.r, NOVA_FLT_MIN);
         if ((rc = check_launch(fn, "V_n+1(b)")) != NOVA_SUCCESS) return rc;
-        nU = 0;
-        if (rGamma > 0 && (rc = eng.dedup(G, rGamma, &nU, fn)) != NOVA_SUCCESS) return rc;
         cacheValid = true;
         return NOVA_SUCCESS;
     }
@@ -212,34 +433,51 @@ struct PerseusCore {
             NOVA_ERR(fn, "Out of memory. Too many alpha-vectors added.");
             return NOVA_ERROR_OUT_OF_MEMORY;
         }
-        // Backup of belief bIndex against V_n.
-        if (rGamma == 0) {
-            // The reference's best-alpha index is never assigned when V_n is
-            // empty (pomdp_perseus_cpu.cpp:78-84); row 0 is used here.
-            cudaMemsetAsync(eng.jstar + (size_t)bIndex * md.m * md.z, 0, (size_t)md.m * md.z * sizeof(unsigned),
-                            eng.stream);
-        } else {
-            if ((rc = eng.fill_items(bIndex * md.m, md.m, fn)) != NOVA_SUCCESS) return rc;
-            if ((rc = eng.exact_score(eng.items, md.m, nU, fn)) != NOVA_SUCCESS) return rc;
+        // Backup of belief bIndex against V_n: about 8,192 scoring warps, each
+        // with as many alphas as that leaves it. With V_n empty no warp has an
+        // alpha, and every observation takes row 0 (the reference's best-alpha
+        // index is never assigned there, pomdp_perseus_cpu.cpp:78-84).
+        const unsigned mz = md.m * md.z;
+        const unsigned splits = std::max(1u, std::min(rGamma, 8192u / mz));
+        const unsigned share = ceil_div(rGamma, splits);
+        const size_t need = (size_t)mz * splits;
+        if (need > partCap) {
+            // Room for every later step's splits, allocated once.
+            const size_t most = (size_t)mz * std::max(1u, std::min(md.r, 8192u / mz));
+            cudaFree(partV); cudaFree(partU); cudaFree(proj);
+            partV = proj = nullptr;
+            partU = nullptr;
+            partCap = 0;
+            if ((rc = dev_alloc(&partV, most, fn, "the partial maxima")) != NOVA_SUCCESS) return rc;
+            if ((rc = dev_alloc(&partU, most, fn, "the partial arg-maxima")) != NOVA_SUCCESS) return rc;
+            if ((rc = dev_alloc(&proj, most * 2 * md.rz, fn, "the projections")) != NOVA_SUCCESS) return rc;
+            partCap = most;
         }
-        if ((rc = eng.assemble(G, nullptr, nullptr, (int)bIndex, eng.rowScratch, eng.resultA, fn)) != NOVA_SUCCESS)
-            return rc;
+        perseus_score_kernel<<<ceil_div(need, 4), 128, 0, eng.stream>>>(md, eng.succLen, eng.suppLen, eng.C3, G, rGamma,
+                                                                        bIndex, splits, share, partV, partU, proj);
+        if ((rc = check_launch(fn, "belief scoring")) != NOVA_SUCCESS) return rc;
+        perseus_action_kernel<<<md.m, 32, md.z * sizeof(unsigned), eng.stream>>>(
+            md, eng.succLen, eng.suppLen, eng.C3, G, bIndex, splits, partV, partU, proj, eng.jstar, eng.actVal);
+        if ((rc = check_launch(fn, "action values")) != NOVA_SUCCESS) return rc;
+        perseus_assemble_kernel<<<ceil_div(md.n, 32), dim3(32, kAssembleObs), 0, eng.stream>>>(
+            md, eng.succLen, eng.C3, G, bIndex, eng.jstar, eng.actVal, eng.rowScratch, eng.resultA);
+        if ((rc = check_launch(fn, "alpha assembly")) != NOVA_SUCCESS) return rc;
         const unsigned slot = rGammaPrime;
-        perseus_commit_kernel<<<1, 256, 0, eng.stream>>>(md, eng.suppLen, bIndex, eng.rowScratch, eng.resultA,
-                                                         eng.vnb, vnbIdx, G, pi, Gp, piP, slot);
+        perseus_commit_kernel<<<std::min(608u, ceil_div(md.r, 8)), 256, 0, eng.stream>>>(
+            md, eng.suppLen, bIndex, eng.rowScratch, eng.resultA, eng.vnb, vnbIdx, G, pi, Gp, piP, slot, eng.vnp1b, bt,
+            done);
         if ((rc = check_launch(fn, "Perseus commit")) != NOVA_SUCCESS) return rc;
         rGammaPrime++;
         *newSlot = slot;
-        perseus_raise_kernel<<<ceil_div(md.r, 256), 256, 0, eng.stream>>>(md, eng.suppLen, Gp + (size_t)slot * md.n,
-                                                                          eng.vnp1b);
-        if ((rc = check_launch(fn, "V_n+1(b) update")) != NOVA_SUCCESS) return rc;
-        perseus_btilde_kernel<<<1, 1024, 0, eng.stream>>>(md.r, eng.vnb, eng.vnp1b, eng.btilde, eng.itemCount);
-        if ((rc = check_launch(fn, "B~")) != NOVA_SUCCESS) return rc;
-        unsigned count = 0;
-        if ((rc = sync_device(fn)) != NOVA_SUCCESS) return rc;
-        if ((rc = d2h(&count, eng.itemCount, sizeof(unsigned), fn, "|B~|")) != NOVA_SUCCESS) return rc;
-        if (count > 0 && (rc = d2h(BTilde, eng.btilde, count * sizeof(unsigned), fn, "B~")) != NOVA_SUCCESS)
-            return rc;
+        // One read-back: the size and, whatever it is, the whole list.
+        if (cudaMemcpyAsync(btHost.data(), bt, btHost.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, eng.stream) !=
+                cudaSuccess || cudaStreamSynchronize(eng.stream) != cudaSuccess) {
+            cudaGetLastError();
+            NOVA_ERR(fn, "Failed to copy B~ from device to host.");
+            return NOVA_ERROR_MEMCPY_TO_HOST;
+        }
+        const unsigned count = std::min(btHost[0], md.r);
+        memcpy(BTilde, btHost.data() + 1, count * sizeof(unsigned));
         rTilde = count;
         if (rTilde == 0) {
             // pomdp_perseus_cpu.cpp:405-426

@@ -201,3 +201,24 @@ def test_distinct_expansion(n, m, z, r, rz, odd):
     out = p.arrays()
     np.testing.assert_array_equal(out["Z"], Z)
     np.testing.assert_array_equal(bits(out["B"]), bits(B))
+
+
+@pytest.mark.parametrize("n,m,z,ns,r,rz", [(2, 1, 1, 1, 3, 1), (33, 3, 33, 5, 60, 31), (70, 2, 16, 33, 90, 64),
+                                           (40, 300, 40, 3, 12, 7), (300, 2, 5, 8, 1100, 3), (64, 5, 17, 12, 257, 33)])
+def test_perseus_backups(n, m, z, ns, r, rz):
+    """Single-belief backups: supports and observations around multiples of 32
+    and 16, more (action, observation) pairs than scoring warps, one and many
+    splits of the alphas, blocks of states and beliefs with remainders."""
+    from nova_gb300.pomdp_perseus import POMDPPerseusGPU
+    md = synth.random_pomdp(n=n, m=m, z=z, ns=min(ns, n), r=r, rz=min(rz, n), gamma=0.9, horizon=5, seed=n + r)
+    rng = np.random.default_rng(n)
+    length = rng.integers(1, md["ns"] + 1, size=(n, m, 1))
+    md["S"] = np.where(np.arange(md["ns"]) < length, md["S"], -1).astype(np.int32)
+    Go, po = orc.perseus_solve(md, seed=r)
+    p = POMDP.from_arrays(md)
+    p.initialize_gpu()
+    alg = POMDPPerseusGPU(p, GammaInitial=md["GammaInitial"])
+    orc.lib().oracle_srand(r)
+    pol = alg.solve()
+    np.testing.assert_array_equal(bits(pol.gamma_array()), bits(Go))
+    np.testing.assert_array_equal(pol.pi_array(), po)

@@ -801,28 +801,29 @@ __global__ void scan_finish_kernel(DevModel md, const unsigned *__restrict__ row
                                    const unsigned *__restrict__ nRowsDev,
                                    const unsigned *__restrict__ runU, const unsigned *__restrict__ uniqJ,
                                    unsigned *__restrict__ ustar, unsigned *__restrict__ jstar) {
-    const unsigned w = blockIdx.x * blockDim.x + threadIdx.x;
     if (nRowsDev) nRows = min(nRows, *nRowsDev);
-    if (w >= nRows) return;
-    const unsigned row = rowList ? rowList[w] : w;
-    const unsigned ao = row / md.r, i = row % md.r;
-    const size_t js = ((size_t)i * md.m + ao / md.z) * md.z + ao % md.z;
-    const unsigned bu = runU[w];
-    ustar[js] = bu;
-    jstar[js] = bu == kNone ? kNone : uniqJ[bu];
+    for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < nRows; w += gridDim.x * blockDim.x) {
+        const unsigned row = rowList ? rowList[w] : w;
+        const unsigned ao = row / md.r, i = row % md.r;
+        const size_t js = ((size_t)i * md.m + ao / md.z) * md.z + ao % md.z;
+        const unsigned bu = runU[w];
+        ustar[js] = bu;
+        jstar[js] = bu == kNone ? kNone : uniqJ[bu];
+    }
 }
 
 // Rows with no alpha above the -1e10 sentinel take the previous
 // observation's choice (0 for the first), as the reference's bestj does.
-__global__ void sentinel_fixup_kernel(DevModel md, const unsigned *__restrict__ uniqJ, unsigned *__restrict__ ustar,
+// Only scanned rows can be such (nRowsDev: how many there are).
+__global__ void sentinel_fixup_kernel(DevModel md, const unsigned *__restrict__ nRowsDev, unsigned *__restrict__ ustar,
                                       unsigned *__restrict__ jstar) {
     const unsigned ia = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ia >= md.r * md.m) return;
+    if (ia >= md.r * md.m || (nRowsDev && *nRowsDev == 0u)) return;
     unsigned prevU = 0, prevJ = 0;
     for (unsigned o = 0; o < md.z; o++) {
         const size_t js = (size_t)ia * md.z + o;
         if (jstar[js] == kNone) {
-            // uniqJ[0] == 0: the first row is always its own representative
+            // Alpha 0 has unique index 0: the first row is its own representative.
             jstar[js] = prevJ;
             ustar[js] = prevU;
         }
@@ -917,8 +918,8 @@ BackupEngine::~BackupEngine() {
         if (g) cudaGraphExecDestroy(g);
     if (tc) tc_release(tc);
     cudaFree(succLen); cudaFree(suppLen); cudaFree(C1); cudaFree(C3);
-    cudaFree(hash); cudaFree(rep); cudaFree(dedupKeys); cudaFree(dedupLow); cudaFree(dedupDone); cudaFree(uniqJ); cudaFree(nUniqueDev); cudaFree(Gt);
-    cudaFree(jstar); cudaFree(actVal); cudaFree(partV); cudaFree(partU); cudaFree(items); cudaFree(itemCount);
+    cudaFree(hash); cudaFree(rep); cudaFree(dedupKeys); cudaFree(dedupLow); cudaFree(dedupDone); cudaFree(uniqJ); cudaFree(uniqIota); cudaFree(report); cudaFree(Gt);
+    cudaFree(jstar); cudaFree(actVal); cudaFree(partV); cudaFree(partU); cudaFree(items);
     cudaFree(keptCount);
     cudaFree(dotScratch); cudaFree(bDense); cudaFree(resultA); cudaFree(resultV); cudaFree(rowScratch);
     cudaFree(vnb); cudaFree(vnp1b);
@@ -947,14 +948,16 @@ int BackupEngine::build(const DevModel &model, const char *fn) {
     if ((rc = dev_alloc(&dedupLow, dedupCap, fn, "the alpha dedup table")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&dedupDone, 1, fn, "the alpha dedup counter")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&uniqJ, md.r, fn, "the unique alphas")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&nUniqueDev, 1, fn, "the unique alpha count")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&uniqIota, md.r, fn, "the alpha indices")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&report, kReport, fn, "the update's report")) != NOVA_SUCCESS) return rc;
+    nUniqueDev = report;
+    itemCount = report + 1;
     gtCols = round_up(md.r, 32);
     if ((rc = dev_alloc(&Gt, (size_t)md.n * gtCols, fn, "the transposed alphas")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&jstar, (size_t)md.r * md.m * md.z, fn, "the chosen alphas")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&ustar, (size_t)md.r * md.m * md.z, fn, "the chosen unique alphas")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&actVal, (size_t)md.r * md.m, fn, "the action values")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&items, (size_t)md.r * md.m, fn, "the work list")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&itemCount, 1, fn, "the work list count")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&keptCount, 1, fn, "the kept-belief count")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&dotScratch, md.r, fn, "the FP64 values")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&bDense, md.n, fn, "the belief")) != NOVA_SUCCESS) return rc;
@@ -965,6 +968,9 @@ int BackupEngine::build(const DevModel &model, const char *fn) {
         for (auto &e : ev) cudaEventCreate(&e);
         eventsMade = true;
     }
+    iota_items_kernel<<<ceil_div(md.r, 256), 256>>>(uniqIota, md.r, 0);
+    if ((rc = check_launch(fn, "alpha indices")) != NOVA_SUCCESS) return rc;
+    uniqMap = uniqIota;
     tables_len_kernel<<<ceil_div(nm, 256), 256>>>((unsigned)nm, md.ns, md.S, succLen);
     if ((rc = check_launch(fn, "successor lengths")) != NOVA_SUCCESS) return rc;
     tables_len_kernel<<<ceil_div(md.r, 256), 256>>>(md.r, md.rz, md.Z, suppLen);
@@ -974,7 +980,7 @@ int BackupEngine::build(const DevModel &model, const char *fn) {
     return sync_device(fn);
 }
 
-int BackupEngine::dedup(const float *src, unsigned rows, unsigned *nUnique, const char *fn) {
+int BackupEngine::dedup(const float *src, unsigned rows, bool own, unsigned *nUnique, const char *fn) {
     int rc;
     if (rows == 0) { *nUnique = 0; return NOVA_SUCCESS; }
     // The transpose below leaves the table free; after an update that failed
@@ -993,17 +999,18 @@ int BackupEngine::dedup(const float *src, unsigned rows, unsigned *nUnique, cons
     dedup_rep_kernel<<<ceil_div(rows, 8), 256, 0, stream>>>(hash, dedupKeys, dedupLow, dedupCap, src, md.n, rows,
                                                             rep, uniqJ, nUniqueDev, dedupDone);
     if ((rc = check_launch(fn, "alpha dedup")) != NOVA_SUCCESS) return rc;
-    unsigned h = 0;
-    if (cudaMemcpyAsync(&h, nUniqueDev, sizeof(unsigned), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
-            cudaStreamSynchronize(stream) != cudaSuccess) {
+    unsigned h = rows;
+    if (!own && (cudaMemcpyAsync(&h, nUniqueDev, sizeof(unsigned), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+                 cudaStreamSynchronize(stream) != cudaSuccess)) {
         cudaGetLastError();
         NOVA_ERR(fn, "Failed to read the number of unique alpha-vectors.");
         return NOVA_ERROR_MEMCPY_TO_HOST;
     }
     *nUnique = h;
+    uniqMap = own ? uniqIota : uniqJ;
     // Transposed unique alphas for the exact scan.
     dim3 grid(ceil_div(std::max(h, 1u), 32), ceil_div(md.n, 32));
-    gather_transpose_kernel<<<grid, dim3(32, 8), 0, stream>>>(src, md.n, uniqJ, h, Gt, gtCols, dedupKeys, dedupLow,
+    gather_transpose_kernel<<<grid, dim3(32, 8), 0, stream>>>(src, md.n, uniqMap, h, Gt, gtCols, dedupKeys, dedupLow,
                                                               dedupCap);
     if ((rc = check_launch(fn, "alpha transpose")) != NOVA_SUCCESS) return rc;
     dedupClean = true;
@@ -1048,7 +1055,7 @@ int BackupEngine::exact_score(const unsigned *itemList, unsigned nItems, unsigne
     }
     if ((rc = check_launch(fn, "exact belief scoring")) != NOVA_SUCCESS) return rc;
     exact_finalize_kernel<<<ceil_div(nItems, 128), 128, 0, stream>>>(md, itemList, nItems, splits, partV, partU,
-                                                                      uniqJ, jstar);
+                                                                      uniqMap, jstar);
     return check_launch(fn, "exact belief scoring (merge)");
 }
 
@@ -1151,17 +1158,22 @@ int BackupEngine::project(unsigned nU, const char *fn) {
     return check_launch(fn, "projection table");
 }
 
+int BackupEngine::scan_capacity(size_t rows, const char *fn) {
+    if (rows <= scanCap) return NOVA_SUCCESS;
+    int rc;
+    cudaFree(scanV); cudaFree(scanU);
+    scanV = nullptr; scanU = nullptr; scanCap = 0;
+    if ((rc = dev_alloc(&scanV, rows, fn, "the scan maxima")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&scanU, rows, fn, "the scan arg-maxima")) != NOVA_SUCCESS) return rc;
+    scanCap = rows;
+    return NOVA_SUCCESS;
+}
+
 int BackupEngine::scan_rows(const unsigned *rowList, unsigned nRows, unsigned nU, const char *fn,
                             const unsigned *nRowsDev) {
     if (nRows == 0) return NOVA_SUCCESS;
     int rc;
-    if ((size_t)nRows > scanCap) {
-        cudaFree(scanV); cudaFree(scanU);
-        scanV = nullptr; scanU = nullptr; scanCap = 0;
-        if ((rc = dev_alloc(&scanV, nRows, fn, "the scan maxima")) != NOVA_SUCCESS) return rc;
-        if ((rc = dev_alloc(&scanU, nRows, fn, "the scan arg-maxima")) != NOVA_SUCCESS) return rc;
-        scanCap = nRows;
-    }
+    if ((rc = scan_capacity(nRows, fn)) != NOVA_SUCCESS) return rc;
     // Column chunk: one (a, o) slice of at most ~48 MB stays L2-resident.
     size_t chunk = ((48ull << 20) / ((size_t)md.n * sizeof(float))) / 256 * 256;
     if (chunk < 256) chunk = 256;
@@ -1173,10 +1185,10 @@ int BackupEngine::scan_rows(const unsigned *rowList, unsigned nRows, unsigned nU
                                                                           scanU, u0 == 0 ? 1 : 0);
         if ((rc = check_launch(fn, "exact row scan")) != NOVA_SUCCESS) return rc;
     }
-    scan_finish_kernel<<<ceil_div(nRows, 256), 256, 0, stream>>>(md, rowList, nRows, nRowsDev, scanU, uniqJ, ustar,
-                                                                 jstar);
+    scan_finish_kernel<<<std::min(ceil_div(nRows, 256), 152u * 8u), 256, 0, stream>>>(md, rowList, nRows, nRowsDev,
+                                                                                     scanU, uniqMap, ustar, jstar);
     if ((rc = check_launch(fn, "exact row scan (finish)")) != NOVA_SUCCESS) return rc;
-    sentinel_fixup_kernel<<<ceil_div((size_t)md.r * md.m, 256), 256, 0, stream>>>(md, uniqJ, ustar, jstar);
+    sentinel_fixup_kernel<<<ceil_div((size_t)md.r * md.m, 256), 256, 0, stream>>>(md, nRowsDev, ustar, jstar);
     return check_launch(fn, "sentinel fixup");
 }
 
@@ -1254,12 +1266,15 @@ int BackupEngine::count_kept(unsigned *out, const char *fn) {
 int BackupEngine::backup_all(const float *src, unsigned rGamma, float *dst, unsigned *pi, const char *fn) {
     int rc;
     memset(&stats, 0, sizeof(stats));
-    identityUniq = false;  // the dedup below rewrites uniqJ
     const unsigned long long launches0 = launch_count();
     cudaEventRecord(ev[0], stream);
+    // Duplicate alphas cost work, never a result (equal rows score equally
+    // and the lowest index wins), so an update after one whose alphas were all
+    // distinct, or with too few for it to matter, takes every alpha as its own
+    // and does not wait for the count; what it finds decides for the next.
+    const bool own = distinctLast || rGamma < kTcMinUnique;
     unsigned nU = 0;
-    if ((rc = dedup(src, rGamma, &nU, fn)) != NOVA_SUCCESS) return rc;
-    stats.uniqueAlphas = nU;
+    if ((rc = dedup(src, rGamma, own, &nU, fn)) != NOVA_SUCCESS) return rc;
     cudaEventRecord(ev[1], stream);
     const unsigned allItems = md.r * md.m;
     // With room for the projection table every exact score is a 64-term
@@ -1283,18 +1298,27 @@ int BackupEngine::backup_all(const float *src, unsigned rGamma, float *dst, unsi
     if (useProjNow && (rc = project(nU, fn)) != NOVA_SUCCESS) return rc;
     if (wantTc && tc == nullptr && tc_build(*this, fn) != NOVA_SUCCESS) tcUnavailable = true;
     cudaEventRecord(ev[2], stream);
-    if (wantTc && tc != nullptr) {
-        unsigned nRows = 0;
-        const unsigned *rowList = nullptr;
-        if ((rc = tc_score(*this, src, nU, &nRows, &rowList, fn)) != NOVA_SUCCESS) return rc;
-        cudaEventRecord(ev[5], stream);
+    const size_t allRows = (size_t)md.m * md.z * md.r;
+    const bool scored = wantTc && tc != nullptr;
+    // With the table, and with few rows expected to be left open, the exact
+    // scan reads their number on the device, and nothing is waited for before
+    // the update's end (n = 64, r = 256: a read-back and its gap cost 15 us of
+    // an update of 85).
+    const bool deferred = scored && useProjNow && allRows <= kDeferredRows && lastScanFrac <= 0.01f;
+    if (scored) {
         stats.scoring = scoring;
-        stats.rowsOverflow = nRows;
-        lastScanFrac = (float)nRows / (float)((size_t)md.m * md.z * md.r);
-        if (useProjNow) {
-            if ((rc = scan_rows(rowList, nRows, nU, fn)) != NOVA_SUCCESS) return rc;
-        } else if ((rc = scan_rows_direct(rowList, nRows, nU, fn)) != NOVA_SUCCESS) {
-            return rc;
+        if (deferred) {
+            if ((rc = scan_capacity(allRows, fn)) != NOVA_SUCCESS) return rc;
+            if ((rc = tc_score_launch(*this, src, nU, true, fn)) != NOVA_SUCCESS) return rc;
+            cudaEventRecord(ev[5], stream);
+            if ((rc = scan_rows(tc_row_list(*this), (unsigned)allRows, nU, fn, itemCount)) != NOVA_SUCCESS) return rc;
+        } else {
+            unsigned nRows = 0;
+            const unsigned *rowList = nullptr;
+            if ((rc = tc_score(*this, src, nU, &nRows, &rowList, fn)) != NOVA_SUCCESS) return rc;
+            cudaEventRecord(ev[5], stream);
+            rc = useProjNow ? scan_rows(rowList, nRows, nU, fn) : scan_rows_direct(rowList, nRows, nU, fn);
+            if (rc != NOVA_SUCCESS) return rc;
         }
     } else if (useProjNow) {
         cudaEventRecord(ev[5], stream);
@@ -1310,10 +1334,14 @@ int BackupEngine::backup_all(const float *src, unsigned rGamma, float *dst, unsi
     cudaEventRecord(ev[3], stream);
     if ((rc = assemble(src, dst, pi, fn)) != NOVA_SUCCESS) return rc;
     cudaEventRecord(ev[4], stream);
-    if (cudaEventSynchronize(ev[4]) != cudaSuccess) {
+    unsigned h[kReport];
+    if (cudaMemcpyAsync(h, report, sizeof(h), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+            cudaStreamSynchronize(stream) != cudaSuccess) {
         cudaGetLastError();
         return sync_device(fn);
     }
+    stats.uniqueAlphas = h[0];
+    distinctLast = h[0] == rGamma;
     cudaEventElapsedTime(&stats.msDedup, ev[0], ev[1]);
     cudaEventElapsedTime(&stats.msProject, ev[1], ev[2]);
     cudaEventElapsedTime(&stats.msScore, ev[2], ev[5]);
@@ -1322,11 +1350,10 @@ int BackupEngine::backup_all(const float *src, unsigned rGamma, float *dst, unsi
     cudaEventElapsedTime(&stats.msAssemble, ev[6], ev[4]);
     cudaEventElapsedTime(&stats.msTotal, ev[0], ev[4]);
     stats.launches = (unsigned)(launch_count() - launches0);
-    if (stats.tcGroups != 0) tc_tune_feedback(*this, stats.msScore + stats.msRescore, nU);
-    const unsigned derr = tc_device_error();
-    if (derr != 0) {
-        NOVA_ERR(fn, "A device-side wait timed out; results of this update are invalid.");
-        return NOVA_ERROR_KERNEL_EXECUTION;
+    if (deferred && (rc = tc_take_report(*this, h, fn)) != NOVA_SUCCESS) return rc;
+    if (scored) {
+        lastScanFrac = (float)stats.rowsOverflow / (float)allRows;
+        tc_tune_feedback(*this, stats.msScore + stats.msRescore, nU);
     }
     return NOVA_SUCCESS;
 }
@@ -1339,7 +1366,7 @@ bool BackupEngine::state_major_wanted() const {
 bool BackupEngine::fixed_ready() const {
     return tc != nullptr && !tcUnavailable && tc_schedule_fixed(*this) && Proj != nullptr && !projUnavailable &&
            projCap >= (size_t)md.m * md.z * std::max(projSCols, (size_t)md.n) * round_up(md.r, 32) &&
-           scanCap >= (size_t)md.m * md.z * md.r && identityUniq &&
+           scanCap >= (size_t)md.m * md.z * md.r &&
            (scoring == NOVA_SCORING_BF16 || scoring == NOVA_SCORING_FP16);
 }
 
@@ -1347,7 +1374,8 @@ int BackupEngine::fixed_pre(const float *src, bool tensor, const char *fn) {
     int rc;
     const unsigned nU = md.r;
     dim3 grid(ceil_div(nU, 32), ceil_div(md.n, 32));
-    gather_transpose_kernel<<<grid, dim3(32, 8), 0, stream>>>(src, md.n, uniqJ, nU, Gt, gtCols, nullptr, nullptr,
+    uniqMap = uniqIota;
+    gather_transpose_kernel<<<grid, dim3(32, 8), 0, stream>>>(src, md.n, uniqMap, nU, Gt, gtCols, nullptr, nullptr,
                                                               0u);
     if ((rc = check_launch(fn, "alpha transpose")) != NOVA_SUCCESS) return rc;
     useProjNow = ensure_proj(nU);
@@ -1377,27 +1405,7 @@ int BackupEngine::backup_fixed(const float *src, float *dst, unsigned *pi, const
     return fixed_post(src, dst, pi, true, fn);
 }
 
-int BackupEngine::fixed_setup(const char *fn) {
-    int rc;
-    if (!identityUniq) {
-        if ((rc = fill_items(0, md.r, fn)) != NOVA_SUCCESS) return rc;
-        if (cudaMemcpyAsync(uniqJ, items, (size_t)md.r * sizeof(unsigned), cudaMemcpyDeviceToDevice, stream) !=
-                cudaSuccess) {
-            cudaGetLastError();
-            return NOVA_ERROR_KERNEL_EXECUTION;
-        }
-        identityUniq = true;
-    }
-    const size_t rows = (size_t)md.m * md.z * md.r;
-    if (scanCap < rows) {
-        cudaFree(scanV); cudaFree(scanU);
-        scanV = nullptr; scanU = nullptr; scanCap = 0;
-        if ((rc = dev_alloc(&scanV, rows, fn, "the scan maxima")) != NOVA_SUCCESS) return rc;
-        if ((rc = dev_alloc(&scanU, rows, fn, "the scan arg-maxima")) != NOVA_SUCCESS) return rc;
-        scanCap = rows;
-    }
-    return NOVA_SUCCESS;
-}
+int BackupEngine::fixed_setup(const char *fn) { return scan_capacity((size_t)md.m * md.z * md.r, fn); }
 
 // Selections of the last backup: for belief i, the action a = pi[i] whose
 // alpha became GammaPrime[i] and, per observation o, the alpha index j* that
@@ -1428,7 +1436,7 @@ __global__ void record_selection_kernel(unsigned r, unsigned m, unsigned z, cons
 
 int BackupEngine::record(const unsigned *pi, unsigned *actOut, unsigned *selOut, const char *fn) {
     record_selection_kernel<<<ceil_div((size_t)md.r * md.z, 256), 256, 0, stream>>>(
-        md.r, md.m, md.z, pi, useProjNow ? 1 : 0, ustar, uniqJ, jstar, actOut, selOut);
+        md.r, md.m, md.z, pi, useProjNow ? 1 : 0, ustar, uniqMap, jstar, actOut, selOut);
     int rc = check_launch(fn, "selection record");
     if (rc != NOVA_SUCCESS) return rc;
     return sync_device(fn);
@@ -1647,7 +1655,7 @@ static int graph_dir(const BackupEngine &e, const float *src) {
 
 static bool graph_needs_capture(const BackupEngine &e, const float *src) {
     const int dir = graph_dir(e, src);
-    return !e.identityUniq || e.graph[dir] == nullptr || e.graphSrc[dir] != src;
+    return e.graph[dir] == nullptr || e.graphSrc[dir] != src;
 }
 
 // Under capture_lock() held exclusively.

@@ -61,7 +61,13 @@ struct BackupEngine {
     unsigned dedupCap = 0;
     bool dedupClean = false;             // the table is free (left so by a finished dedup)
     unsigned *uniqJ = nullptr;           // [r] unique index -> lowest original index
-    unsigned *nUniqueDev = nullptr;      // device scalar
+    unsigned *uniqIota = nullptr;        // [r] 0 .. r-1: every alpha as its own
+    const unsigned *uniqMap = nullptr;   // the one of the two that this update's alpha indices refer to
+    // What an update leaves for the host to read: distinct alphas, rows left
+    // to the exact scan, rows and candidates re-scored, the error word.
+    static constexpr unsigned kReport = 5;
+    unsigned *report = nullptr;          // [kReport], device
+    unsigned *nUniqueDev = nullptr;      // report[0]
     float *Gt = nullptr;                 // [n][gtCols] transposed unique alphas
     size_t gtCols = 0;
     unsigned *jstar = nullptr;           // [r][m][z] chosen alpha per (belief, action, observation)
@@ -80,7 +86,7 @@ struct BackupEngine {
     unsigned *partU = nullptr;
     size_t partCap = 0;
     unsigned *items = nullptr;           // [r*m] work list (belief*m + action)
-    unsigned *itemCount = nullptr;       // device scalar
+    unsigned *itemCount = nullptr;       // report[1]; also the length of other lists
     unsigned *keptCount = nullptr;       // device scalar (count_kept)
     double *dotScratch = nullptr;        // [r] FP64 V(b) row values
     float *bDense = nullptr;             // [n]
@@ -101,8 +107,11 @@ struct BackupEngine {
     int build(const DevModel &model, const char *fn);
     // One backup of every belief (PBVI): Gamma rows [0, rGamma) -> dst, pi.
     int backup_all(const float *src, unsigned rGamma, float *dst, unsigned *pi, const char *fn);
-    // Dedup of Gamma rows [0, rows); returns the number of unique rows.
-    int dedup(const float *src, unsigned rows, unsigned *nUnique, const char *fn);
+    // Dedup of Gamma rows [0, rows), and their transpose. With `own` every
+    // row counts as its own alpha (*nUnique = rows, nothing is read back; the
+    // number of distinct ones still goes to the report), else *nUnique is the
+    // number of distinct rows.
+    int dedup(const float *src, unsigned rows, bool own, unsigned *nUnique, const char *fn);
     // Exact scoring of the listed (belief, action) items over the unique rows.
     int exact_score(const unsigned *items, unsigned nItems, unsigned nU, const char *fn);
     // Without the table: exact scoring of the (belief, action) items of the
@@ -120,17 +129,18 @@ struct BackupEngine {
     int scan_rows(const unsigned *rowList, unsigned nRows, unsigned nU, const char *fn,
                   const unsigned *nRowsDev = nullptr);
     // One update without host read-backs, for graph capture: every alpha
-    // is scored as its own (uniqJ must be the identity), tensor-core
-    // scoring with the solver's fixed schedule, the exact scan sized on the
-    // device. Same results as backup_all.
+    // is scored as its own, tensor-core scoring with the solver's fixed
+    // schedule, the exact scan sized on the device. Same results as
+    // backup_all.
     int backup_fixed(const float *src, float *dst, unsigned *pi, const char *fn);
     // backup_fixed in two halves around the scoring GEMM (tensor) or, with
     // tensor false, an update that scans every row exactly; no host
     // read-back in either.
     int fixed_pre(const float *src, bool tensor, const char *fn);
     int fixed_post(const float *src, float *dst, unsigned *pi, bool tensor, const char *fn);
-    // Identity unique-alpha map and exact-scan capacity for every row, which
-    // the fixed updates need.
+    // Exact-scan capacity for every row, which updates that read nothing back
+    // before it need.
+    int scan_capacity(size_t rows, const char *fn);
     int fixed_setup(const char *fn);
     // Ready for backup_fixed: tensor-core scoring built with a fixed
     // schedule, the projection table allocated for all r alphas.
@@ -140,7 +150,8 @@ struct BackupEngine {
     const float *graphSrc[2] = {nullptr, nullptr};
     unsigned graphLaunches[2] = {0, 0};
     bool graphMode = false;
-    bool identityUniq = false;     // uniqJ holds 0 .. r-1
+    bool distinctLast = false;     // the last update's alphas were all distinct
+    static constexpr size_t kDeferredRows = 1u << 24;  // rows up to which an update may size its exact scan on the device
     bool capturing = false;        // launches are being captured, not run
     bool projAttrDone = false;     // shared-memory attribute of the state-contiguous projection set
     bool projRowsAttrDone = false; // and of the alpha-contiguous one
@@ -172,7 +183,7 @@ bool tc_supported(const DevModel &md);
 // Builds the BF16 operand tables once; returns NOVA_SUCCESS or an error.
 int tc_build(BackupEngine &eng, const char *fn);
 // Scores every (belief, action, observation) row against the nU unique rows
-// of src (gathered through eng.uniqJ), writes eng.jstar for rows whose argmax
+// of src (gathered through eng.uniqMap), writes eng.jstar for rows whose argmax
 // is proven, and appends the (belief, action) items that need the exact full
 // scan to *rowList / *nRows as (a*z+o)*r + i row indices (a device list
 // owned by the tensor-core state, sized for every row).
@@ -202,6 +213,9 @@ bool tc_schedule_fixed(const BackupEngine &eng);  // and built for eng.scoring
 const unsigned *tc_row_list(const BackupEngine &eng);
 int tc_score(BackupEngine &eng, const float *src, unsigned nU, unsigned *nRows, const unsigned **rowList,
              const char *fn);
+// Takes what a tensor-core update left in the report (on the host) into the
+// statistics; an error code if a wait of the scoring kernel ran out.
+int tc_take_report(BackupEngine &eng, const unsigned (&h)[BackupEngine::kReport], const char *fn);
 void tc_release(TcState *tc);
 // Per-belief detail of the last tensor-core update: alphas re-scored exactly
 // and rows sent to the exact scan, summed over the belief's (a, o) rows.

@@ -99,7 +99,10 @@ struct TcState {
     float *d1 = nullptr;            // [MZ][rPad] sum_s |A - half(A)| (scaled units): A's actual operand rounding
     uint16_t *Gb = nullptr;         // [capN][nPad] FP16, or [capN][2 nPad] split BF16, bits of (alpha - c) * 2^gexp
     float *shift = nullptr;         // [n]
-    unsigned *scal = nullptr;       // [0] gmax, [1] Gmax, [2] escale, [3..4] counters, [5] max half-range, [6] G scale, [7] dscale (float bits)
+    // [0] gmax, [1] Gmax, [2] escale, [3..4] counters, [5] max half-range, [7] dscale (float bits), [8] finished
+    // packing blocks; what is accumulated is 0 again after an update (scalClean).
+    unsigned *scal = nullptr;
+    bool scalClean = false;
     float *candV = nullptr;         // [MZ][r][MAX_LISTS][MAX_TOPK] (the first K entries of each list used)
     unsigned *candU = nullptr;
     float *candX = nullptr;         // [MZ][r][MAX_LISTS]
@@ -760,11 +763,11 @@ __global__ void tc_shift_kernel(const float *__restrict__ Gt, size_t gtCols, uns
 
 // Power-of-two scale for the packed alphas: the largest |alpha - c| lands
 // in [2^13, 2^14) (half-range plus slack for the rounding of c).
-__global__ void tc_gscale_kernel(unsigned *scal) {
+__device__ __forceinline__ float pack_scale(const unsigned *scal) {
     const float hr = __uint_as_float(scal[5]) * 1.001f + 1e-30f;
     int e = 0;
     frexpf(hr, &e);
-    scal[6] = __float_as_uint(hr < 1e30f ? ldexpf(1.0f, 13 - e) : 1.0f);
+    return hr < 1e30f ? ldexpf(1.0f, 13 - e) : 1.0f;
 }
 
 // Gb[u] = half((alpha_u(s) - c[s]) * gscale); rows >= nU, states >= n are 0.
@@ -773,12 +776,18 @@ __global__ void tc_gscale_kernel(unsigned *scal) {
 // (v - hi is exact in FP32), so |v - hi - lo| <= 2^-16 |v|; the row holds,
 // for every 64-state block kb, the 64 hi values and then the 64 lo values
 // (row length 2 nPad), and the GEMM multiplies one A block by both.
-// Records gmax = max |(alpha - c) * gscale| over the FP32 values.
+// Records gmax = max |(alpha - c) * gscale| over the FP32 values; the block
+// that finishes last turns it into the margin's scales, escale = U * gmax +
+// gN * Gmax * gscale and dscale = gmax (1 + 2^-22), all in the packed units
+// (the per-row bound is a1 * escale + d1 * dscale). Also clears the merge's
+// chunk counts.
 __global__ void tc_pack_kernel(const float *__restrict__ G, unsigned n, size_t nPad, const unsigned *__restrict__ uniqJ,
                                unsigned nU, const float *__restrict__ shift, int fp16, int split,
-                               uint16_t *__restrict__ Gb, unsigned *__restrict__ scal) {
+                               uint16_t *__restrict__ Gb, unsigned *scal, float U, float gN,
+                               unsigned *__restrict__ chunkCount, unsigned nChunks) {
     const unsigned u = blockIdx.x;
-    const float gscale = __uint_as_float(scal[6]);
+    const float gscale = pack_scale(scal);
+    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < nChunks; k += gridDim.x * blockDim.x) chunkCount[k] = 0u;
     const size_t rowLen = split ? 2 * nPad : nPad;
     uint16_t *out = Gb + (size_t)u * rowLen;
     float m = 0.0f;
@@ -816,17 +825,15 @@ __global__ void tc_pack_kernel(const float *__restrict__ G, unsigned n, size_t n
     if (threadIdx.x == 0) {
         for (unsigned w = 0; w < blockDim.x / 32; w++) m = fmaxf(m, red[w]);
         atomic_max_nonneg(&scal[0], snan ? __uint_as_float(0x7fc00000u) : m);
+        __threadfence();
+        if (atomicAdd(&scal[8], 1u) == gridDim.x - 1) {
+            __threadfence();
+            const float gmax = __uint_as_float(atomicAdd(&scal[0], 0u));
+            const float Gmax = __uint_as_float(scal[1]);
+            scal[2] = __float_as_uint(U * gmax + gN * Gmax * gscale);
+            scal[7] = __float_as_uint(gmax * (1.0f + 2.4e-7f));
+        }
     }
-}
-
-// escale = U * gmax + gN * Gmax * gscale and dscale = gmax (1 + 2^-22), all
-// in the packed units; the per-row bound is a1 * escale + d1 * dscale.
-__global__ void tc_escale_kernel(unsigned *scal, float U, float gN) {
-    const float gmax = __uint_as_float(scal[0]);
-    const float Gmax = __uint_as_float(scal[1]);
-    const float gscale = __uint_as_float(scal[6]);
-    scal[2] = __float_as_uint(U * gmax + gN * Gmax * gscale);
-    scal[7] = __float_as_uint(gmax * (1.0f + 2.4e-7f));
 }
 
 // ---------------------------------------------------------------------------
@@ -1129,11 +1136,13 @@ __global__ void __launch_bounds__(256, kDirect ? 1 : NE <= 4 ? 5 : 4) tc_merge_k
 // Indices of the flagged rows in increasing order, from the flagged rows per
 // chunk of kCompactChunk: every block adds up the chunks before its own (at
 // most a few thousand counts) and writes its rows behind them; the last
-// block also stores the total.
+// block also stores the total in out[0] and, with scal (after a merge), the
+// merge's counters and the error word behind it, and clears what the next
+// update accumulates.
 __global__ void __launch_bounds__(1024) tc_compact_write_kernel(const unsigned *__restrict__ flag, unsigned count,
                                                                 const unsigned *__restrict__ chunkCount,
                                                                 unsigned *__restrict__ items,
-                                                                unsigned *__restrict__ nOut) {
+                                                                unsigned *__restrict__ out, unsigned *scal) {
     const unsigned mine = chunkCount[blockIdx.x];
     const bool lastBlock = blockIdx.x == gridDim.x - 1;
     if (mine == 0 && !lastBlock) return;
@@ -1148,7 +1157,15 @@ __global__ void __launch_bounds__(1024) tc_compact_write_kernel(const unsigned *
         unsigned t = 0;
         for (unsigned w = 0; w < blockDim.x / 32; w++) t += wsum[w];
         before = t;
-        if (lastBlock) *nOut = t + mine;
+        if (lastBlock) {
+            out[0] = t + mine;
+            if (scal != nullptr) {
+                out[1] = scal[3];
+                out[2] = scal[4];
+                out[3] = atomicAdd(&g_device_error, 0u);
+                scal[0] = scal[1] = scal[3] = scal[4] = scal[5] = scal[8] = 0u;
+            }
+        }
     }
     __syncthreads();
     if (mine == 0) return;
@@ -1285,7 +1302,7 @@ int tc_build(BackupEngine &eng, const char *fn) {
     if ((rc = dev_alloc(&tc->d1, (size_t)tc->MZ * tc->rPad, fn, "the row bounds")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&tc->Gb, tc->capN * tc->nPad * 2, fn, "the packed alphas")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&tc->shift, md.n, fn, "the alpha shift")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&tc->scal, 8, fn, "the scoring scalars")) != NOVA_SUCCESS) return rc;
+    if ((rc = dev_alloc(&tc->scal, 9, fn, "the scoring scalars")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&tc->candV, slots * MAX_TOPK, fn, "the candidate scores")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&tc->candU, slots * MAX_TOPK, fn, "the candidate alphas")) != NOVA_SUCCESS) return rc;
     if ((rc = dev_alloc(&tc->candX, slots, fn, "the dropped-score bounds")) != NOVA_SUCCESS) return rc;
@@ -1324,15 +1341,11 @@ int tc_prepare(BackupEngine &eng, const float *src, unsigned nU, const char *fn)
     const unsigned kSplit = fp16 ? 1u : 2u;
     const size_t nPadRows = round_up(nU, BN);
     const unsigned nTiles = (unsigned)(nPadRows / BN);
-    // ---- pack the shifted, scaled unique alphas ----
-    cudaMemsetAsync(tc->scal, 0, 8 * sizeof(unsigned), eng.stream);
+    // ---- shift, scale and pack the unique alphas ----
+    if (!tc->scalClean) cudaMemsetAsync(tc->scal, 0, 9 * sizeof(unsigned), eng.stream);
+    tc->scalClean = false;  // until the merge's list has cleared it again
     tc_shift_kernel<<<md.n, 256, 0, eng.stream>>>(eng.Gt, eng.gtCols, md.n, nU, tc->shift, tc->scal);
     if ((rc = check_launch(fn, "alpha shift")) != NOVA_SUCCESS) return rc;
-    tc_gscale_kernel<<<1, 1, 0, eng.stream>>>(tc->scal);
-    if ((rc = check_launch(fn, "alpha scale")) != NOVA_SUCCESS) return rc;
-    tc_pack_kernel<<<(unsigned)nPadRows, 256, 0, eng.stream>>>(src, md.n, tc->nPad, eng.uniqJ, nU, tc->shift,
-                                                              fp16 ? 1 : 0, kSplit == 2u ? 1 : 0, tc->Gb, tc->scal);
-    if ((rc = check_launch(fn, "alpha packing")) != NOVA_SUCCESS) return rc;
     // The row bound is a1 * escale + d1 * dscale (packed units), with
     // escale = U * gmax + gN * Gmax * gscale and dscale = gmax (1 + 2^-22).
     // Against the reference's FP32 score, the tensor-core score of a row
@@ -1357,8 +1370,11 @@ int tc_prepare(BackupEngine &eng, const float *src, unsigned nU, const char *fn)
                             steps / 4194304.0 * (1.0 + uA) * (1.0 + uG) * (1.0 + 2.0 * u24) +
                             (fp16 ? (double)tc->nPad / 33554432.0 / 8192.0 : 0.0) + 1.0 / 1048576.0);
     const float gN = (float)((double)(md.ns + md.rz + 3) * u24 * 1.01);
-    tc_escale_kernel<<<1, 1, 0, eng.stream>>>(tc->scal, U, gN);
-    if ((rc = check_launch(fn, "margin")) != NOVA_SUCCESS) return rc;
+    const unsigned nChunks = ceil_div((size_t)tc->MZ * md.r, kCompactChunk);
+    tc_pack_kernel<<<(unsigned)nPadRows, 256, 0, eng.stream>>>(src, md.n, tc->nPad, eng.uniqMap, nU, tc->shift,
+                                                              fp16 ? 1 : 0, kSplit == 2u ? 1 : 0, tc->Gb, tc->scal, U,
+                                                              gN, tc->chunkCount, nChunks);
+    if ((rc = check_launch(fn, "alpha packing")) != NOVA_SUCCESS) return rc;
     // ---- schedule and the alphas' tensor map ----
     TcState::Launch &L = tc->last;
     if ((rc = encode_map(tc, &L.tmB, tc->Gb, nPadRows, tc->nPad * kSplit, BN, fn)) != NOVA_SUCCESS) return rc;
@@ -1405,7 +1421,6 @@ int tc_finish(BackupEngine &eng, const char *fn) {
     const size_t rows = (size_t)tc->MZ * md.r;
     // The list can hold every row: it is sized m*z*r like the flags.
     const unsigned nChunks = ceil_div(rows, kCompactChunk);
-    cudaMemsetAsync(tc->chunkCount, 0, nChunks * sizeof(unsigned), eng.stream);
     const DirectScorer ds{eng.succLen, eng.C3, tc->src};
     // Entries per lane: the fewest that hold the row's lists.
     const unsigned perLane = ceil_div(L.lists * L.topk, 32);
@@ -1417,13 +1432,15 @@ int tc_finish(BackupEngine &eng, const char *fn) {
                  : NE == 2u ? tc_merge_kernel<false, 2>
                  : NE == 4u ? tc_merge_kernel<false, 4> : tc_merge_kernel<false, 8>;
     merge<<<(unsigned)ceil_div(rows * 32, 256), 256, mergeSmem, eng.stream>>>(
-        md, eng.suppLen, table ? eng.proj_view() : ProjView{}, ds, eng.uniqJ, L.lists, L.topk, tc->rPad,
+        md, eng.suppLen, table ? eng.proj_view() : ProjView{}, ds, eng.uniqMap, L.lists, L.topk, tc->rPad,
         tc->a1, tc->d1, tc->a1raw, tc->scal, tc->candV, tc->candU, tc->candX, eng.ustar, eng.jstar, tc->rowFlag,
         tc->rowCand, tc->scal + 3, tc->chunkCount, tc->badModel);
     if ((rc = check_launch(fn, "candidate merge")) != NOVA_SUCCESS) return rc;
     tc_compact_write_kernel<<<nChunks, 1024, 0, eng.stream>>>(tc->rowFlag, (unsigned)rows, tc->chunkCount,
-                                                              tc->rowList, eng.itemCount);
-    return check_launch(fn, "exact-scan list");
+                                                              tc->rowList, eng.itemCount, tc->scal);
+    if ((rc = check_launch(fn, "exact-scan list")) != NOVA_SUCCESS) return rc;
+    tc->scalClean = true;
+    return NOVA_SUCCESS;
 }
 
 // Flag the (belief, action) item of every listed row; each item is counted
@@ -1454,7 +1471,7 @@ int tc_rows_to_items(BackupEngine &eng, const unsigned *rowList, unsigned nRows,
                                                                       tc->rowFlag, tc->chunkCount);
     if ((rc = check_launch(fn, "rows to items")) != NOVA_SUCCESS) return rc;
     tc_compact_write_kernel<<<nChunks, 1024, 0, eng.stream>>>(tc->rowFlag, count, tc->chunkCount, eng.items,
-                                                              eng.itemCount);
+                                                              eng.itemCount, nullptr);
     return check_launch(fn, "item list");
 }
 
@@ -1574,25 +1591,28 @@ int tc_score(BackupEngine &eng, const float *src, unsigned nU, unsigned *nRows, 
              const char *fn) {
     int rc;
     if ((rc = tc_score_launch(eng, src, nU, true, fn)) != NOVA_SUCCESS) return rc;
-    TcState *tc = eng.tc;
-    unsigned h[8];
-    unsigned cnt = 0;
-    if (cudaMemcpyAsync(h, tc->scal, sizeof(h), cudaMemcpyDeviceToHost, eng.stream) != cudaSuccess ||
-            cudaMemcpyAsync(&cnt, eng.itemCount, sizeof(unsigned), cudaMemcpyDeviceToHost, eng.stream) !=
-                cudaSuccess ||
+    unsigned h[BackupEngine::kReport];
+    if (cudaMemcpyAsync(h, eng.report, sizeof(h), cudaMemcpyDeviceToHost, eng.stream) != cudaSuccess ||
             cudaStreamSynchronize(eng.stream) != cudaSuccess) {
         cudaGetLastError();
         NOVA_ERR(fn, "Failed to read the scoring counters.");
         return NOVA_ERROR_MEMCPY_TO_HOST;
     }
-    if (tc_device_error() != 0) {
-        NOVA_ERR(fn, "The tensor-core scoring kernel timed out waiting on a barrier.");
+    *nRows = h[1];
+    *rowList = eng.tc->rowList;
+    return tc_take_report(eng, h, fn);
+}
+
+int tc_take_report(BackupEngine &eng, const unsigned (&h)[BackupEngine::kReport], const char *fn) {
+    const TcState *tc = eng.tc;
+    if (h[4] != 0) {
+        read_and_clear_device_error();
+        NOVA_ERR(fn, "The tensor-core scoring kernel timed out waiting on a barrier; results are invalid.");
         return NOVA_ERROR_KERNEL_EXECUTION;
     }
-    *nRows = cnt;
-    *rowList = tc->rowList;
-    eng.stats.rowsMultiCand = h[3];
-    eng.stats.candidates = h[4];
+    eng.stats.rowsOverflow = h[1];
+    eng.stats.rowsMultiCand = h[2];
+    eng.stats.candidates = h[3];
     cudaEventElapsedTime(&eng.stats.msGemm, tc->g0, tc->g1);
     eng.stats.tcGroups = tc->groupsUsed;
     return NOVA_SUCCESS;

@@ -37,43 +37,60 @@ using nova::MDPValueFunction;
 
 namespace nova_gb300 {
 
+// Q(s,a) in list order. A batch of kBatch successors is loaded before any of
+// their values of V, and those before any is added, so a row costs two round
+// trips to memory per batch instead of two per successor.
+constexpr unsigned kBatch = 8;
+constexpr unsigned kResident = 5;   // 256-thread blocks per SM
+
 template <bool VEC>
 __device__ __forceinline__ float bellman_q(unsigned s, unsigned a, unsigned m, unsigned ns, float gamma,
                                            const int *__restrict__ S, const float *__restrict__ T,
                                            const float *__restrict__ R, const float *__restrict__ V) {
     float q = __ldg(R + (size_t)s * m + a);
     const size_t row = ((size_t)s * m + a) * ns;
-    if (VEC) {
-        const int4 *S4 = reinterpret_cast<const int4 *>(S + row);
-        const float4 *T4 = reinterpret_cast<const float4 *>(T + row);
-        const unsigned nv = ns >> 2;
-        for (unsigned c = 0; c < nv; c++) {
-            const int4 sv = __ldg(S4 + c);
-            const float4 tv = __ldg(T4 + c);
-            if (sv.x < 0) break;
-            q = fadd(q, fmul(fmul(gamma, tv.x), __ldg(V + sv.x)));
-            if (sv.y < 0) break;
-            q = fadd(q, fmul(fmul(gamma, tv.y), __ldg(V + sv.y)));
-            if (sv.z < 0) break;
-            q = fadd(q, fmul(fmul(gamma, tv.z), __ldg(V + sv.z)));
-            if (sv.w < 0) break;
-            q = fadd(q, fmul(fmul(gamma, tv.w), __ldg(V + sv.w)));
+    for (unsigned l0 = 0; l0 < ns; l0 += kBatch) {
+        int sp[kBatch];
+        float t[kBatch], v[kBatch];
+#pragma unroll
+        for (unsigned k = 0; k < kBatch; k += VEC ? 4 : 1) {
+            if constexpr (VEC) {
+                // ns is a multiple of 4 here.
+                const bool in = l0 + k < ns;
+                const int4 s4 = in ? __ldg(reinterpret_cast<const int4 *>(S + row + l0 + k)) : make_int4(-1, -1, -1, -1);
+                const float4 t4 = in ? __ldg(reinterpret_cast<const float4 *>(T + row + l0 + k)) : make_float4(0, 0, 0, 0);
+                sp[k] = s4.x; sp[k + 1] = s4.y; sp[k + 2] = s4.z; sp[k + 3] = s4.w;
+                t[k] = t4.x; t[k + 1] = t4.y; t[k + 2] = t4.z; t[k + 3] = t4.w;
+            } else {
+                const bool in = l0 + k < ns;
+                sp[k] = in ? __ldg(S + row + l0 + k) : -1;
+                t[k] = in ? __ldg(T + row + l0 + k) : 0.0f;
+            }
         }
-    } else {
-        for (unsigned l = 0; l < ns; l++) {
-            const int sp = __ldg(S + row + l);
-            if (sp < 0) break;
-            q = fadd(q, fmul(fmul(gamma, __ldg(T + row + l)), __ldg(V + sp)));
+        // The row ends at its first negative entry, whatever follows.
+        bool live[kBatch];
+#pragma unroll
+        for (unsigned k = 0; k < kBatch; k++) {
+            live[k] = (k == 0 || live[k - 1]) && sp[k] >= 0;
+            v[k] = live[k] ? __ldg(V + sp[k]) : 0.0f;
         }
+#pragma unroll
+        for (unsigned k = 0; k < kBatch; k++)
+            if (live[k]) q = fadd(q, fmul(fmul(gamma, t[k]), v[k]));
+        if (!live[kBatch - 1]) break;
     }
     return q;
 }
 
 // One Bellman sweep. G lanes per state, G a power of two in [1, 32], m <= G.
+// Bound by the L2's rate of 32-byte sectors (a random gather of V each: 7.5
+// TB/s measured at n = 2^20), or, on small models, by the latency of a row's
+// loads. Five blocks an SM leave room for a batch in registers: n = 150,001,
+// m = 5, ns <= 11 41 to 36 us a sweep, n = 20,000, m = 6, ns = 10 13.6 to 12.7.
 // The grid is a few waves of resident blocks that stride over 256-thread
 // tiles, so the residual costs two atomics per block, not per tile.
 template <int G, bool VEC>
-__global__ void __launch_bounds__(256) bellman_sweep_kernel(unsigned n, unsigned ns, unsigned m, float gamma,
+__global__ void __launch_bounds__(256, kResident) bellman_sweep_kernel(unsigned n, unsigned ns, unsigned m, float gamma,
         const int *__restrict__ S, const float *__restrict__ T, const float *__restrict__ R,
         const float *__restrict__ V, float *__restrict__ Vp, unsigned *__restrict__ pi,
         ViDeviceState *st, double tol, int early_exit) {
@@ -145,7 +162,7 @@ static unsigned resident_blocks() {
             cudaGetLastError();
             sms = 152;
         }
-        cache[dev] = (unsigned)sms * 8u;
+        cache[dev] = (unsigned)sms * kResident;
     }
     return cache[dev];
 }
@@ -415,6 +432,23 @@ extern "C" int mdp_vi_execute_gpu(const MDP *mdp, MDPVIGPU *vi, MDPValueFunction
     }
     // Sweeps are queued back to back on the stream; one synchronisation at
     // the end replaces the reference's per-sweep cudaDeviceSynchronize.
+    {
+        ViDeviceState *st = nullptr;
+        {
+            std::lock_guard<std::mutex> lock(registry_mutex());
+            auto *ws = find_workspace<ViGpuWorkspace>(vi);
+            if (ws != nullptr) st = ws->st;
+        }
+        unsigned done = 0;
+        if (st != nullptr)
+            rc = vi_resident_sweeps(mdp, mdp->d_S, mdp->d_T, mdp->d_R, vi->d_V, vi->d_VPrime, vi->d_pi, st,
+                                    mdp->horizon, 0.0, 0, &done, 0, fn);
+        if (rc != NOVA_SUCCESS) {
+            mdp_vi_uninitialize_gpu(mdp, vi);
+            return rc;
+        }
+        vi->currentHorizon += done;
+    }
     while (vi->currentHorizon < mdp->horizon) {
         rc = vi_gpu_sweep(mdp, vi, 0.0, 0, false, fn);
         if (rc != NOVA_SUCCESS) {
@@ -488,6 +522,13 @@ extern "C" int mdp_vi_execute_until_converged_gpu(const MDP *mdp, MDPVIGPU *vi, 
     unsigned launched = 0;
     ViDeviceState h;
     memset(&h, 0, sizeof(h));
+    rc = vi_resident_sweeps(mdp, mdp->d_S, mdp->d_T, mdp->d_R, vi->d_V, vi->d_VPrime, vi->d_pi, st, maxSweeps, tol, 1,
+                            &launched, 0, fn);
+    if (rc == NOVA_SUCCESS && launched != 0) {
+        rc = d2h(&h, st, sizeof(h), fn, "the convergence state");
+        if (rc == NOVA_SUCCESS) rc = vi_state_error(st, fn);
+    }
+    if (rc != NOVA_SUCCESS) { mdp_vi_uninitialize_gpu(mdp, vi); return rc; }
     while (launched < maxSweeps) {
         const unsigned b = (maxSweeps - launched) < kBatch ? (maxSweeps - launched) : kBatch;
         for (unsigned k = 0; k < b; k++) {
@@ -649,6 +690,12 @@ extern "C" int mdp_vi_execute_cpu(const MDP *mdp, MDPVICPU *vi, MDPValueFunction
     // The whole solve stays on the device; V, V' and pi are copied back once.
     rc = h2d(ws->V, vi->V, n * sizeof(float), fn, "the value function");
     if (rc == NOVA_SUCCESS) rc = h2d(ws->VPrime, vi->VPrime, n * sizeof(float), fn, "the value function (prime)");
+    if (rc == NOVA_SUCCESS) {
+        unsigned done = 0;
+        rc = vi_resident_sweeps(mdp, ws->S, ws->T, ws->R, ws->V, ws->VPrime, ws->pi, ws->st, mdp->horizon, 0.0, 0,
+                                &done, 0, fn);
+        vi->currentHorizon += done;
+    }
     while (rc == NOVA_SUCCESS && vi->currentHorizon < mdp->horizon) {
         const bool even = (vi->currentHorizon % 2u) == 0u;
         rc = launch_sweep(mdp, ws->S, ws->T, ws->R, even ? ws->V : ws->VPrime, even ? ws->VPrime : ws->V, ws->pi,

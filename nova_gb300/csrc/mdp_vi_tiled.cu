@@ -1076,6 +1076,10 @@ int vi_tiled_sweep(const ViTilePlan *plan, const MDP *mdp, const float *R, const
 
 unsigned vi_last_plan_status() { return g_last_status.load(); }
 
+void vi_note_gather() { g_last_status.store(ViTilePlan::kGather); }
+
+bool vi_tiling_forced() { return g_mode.load() != NOVA_VI_TILING_AUTO; }
+
 int vi_state_error(ViDeviceState *st, const char *fn) {
     unsigned err = 0;
     int rc = d2h(&err, &st->err, sizeof(unsigned), fn, "the sweep error word");

@@ -15,8 +15,11 @@ struct ViDeviceState {
     unsigned int blocks_done;        // blocks finished in the current sweep
     unsigned int sweeps_done;        // sweeps that ran (early-exit mode)
     unsigned int converged;          // 1 once a sweep's residual fell below tol
-    unsigned int err;                // 1 if a bounded wait of the tiled sweep ran out
+    unsigned int err;                // 1 if a bounded wait of the tiled or the resident sweeps ran out
     double last_resid;               // residual of the last finished sweep
+    // The resident sweeps', cleared before each launch (from here to the end):
+    unsigned long long resid[3];     // residuals of the sweep, the last and the next, as FP64 bits
+    unsigned int arrived;            // arrivals at the grid barrier
 };
 
 #ifdef __CUDACC__
@@ -83,6 +86,21 @@ int vi_plan_build(ViTilePlan *plan, const nova::MDP *mdp, const int *S, const fl
 int vi_tiled_sweep(const ViTilePlan *plan, const nova::MDP *mdp, const float *R, const float *V, float *Vp,
                    unsigned *pi, ViDeviceState *st, double tol, int early_exit, cudaStream_t stream,
                    const char *fn);
+
+// All `sweeps` sweeps of a solve, V -> Vp -> V ..., in launches that keep the
+// model in the SMs (mdp_vi_resident.cu), or none (*done = 0) where it does not
+// fit or would not pay; with early_exit the sweeps stop once a residual falls
+// below tol. *done: the sweeps asked of the launches (sweeps or 0). Queued, not
+// waited for.
+int vi_resident_sweeps(const nova::MDP *mdp, const int *S, const float *T, const float *R, float *V, float *Vp,
+                       unsigned *pi, ViDeviceState *st, unsigned sweeps, double tol, int early_exit, unsigned *done,
+                       cudaStream_t stream, const char *fn);
+
+// Whether the tiling setting names a sweep kernel (it is not AUTO).
+bool vi_tiling_forced();
+
+// Records that the last solve swept without a tile plan.
+void vi_note_gather();
 
 // Reads (and clears) the state's error word after the sweeps queued so far
 // finished: NOVA_ERROR_KERNEL_EXECUTION if a bounded wait ran out.

@@ -222,3 +222,48 @@ def test_perseus_backups(n, m, z, ns, r, rz):
     pol = alg.solve()
     np.testing.assert_array_equal(bits(pol.gamma_array()), bits(Go))
     np.testing.assert_array_equal(pol.pi_array(), po)
+
+
+@pytest.mark.parametrize("n,m,ns,horizon", [(1, 1, 1, 2), (37, 3, 5, 7), (1500, 1, 9, 6), (5000, 7, 3, 5),
+                                            (3001, 16, 8, 4), (40000, 5, 6, 3), (900, 200, 2, 4), (60000, 1, 64, 3),
+                                            (30, 2, 30, 5001)])
+@pytest.mark.parametrize("api", ["gpu", "cpu", "converged"])
+def test_resident_sweeps(n, m, ns, horizon, api):
+    """One and many blocks, several rows a thread, V in and out of shared
+    memory, models too large to stay in the SMs, unordered rows with entries
+    after their end, more sweeps than one launch runs, and a stop between."""
+    from nova_gb300.mdp import MDP
+    from nova_gb300.mdp_vi import MDPValueIterationCPU, MDPValueIterationGPU
+    md = synth.random_mdp(n=n, m=m, ns=min(ns, n), gamma=0.9, horizon=horizon, seed=n + m)
+    rng = np.random.default_rng(n)
+    k = md["ns"]
+    order = np.argsort(rng.random((n, m, k)), axis=2)
+    md["S"] = np.take_along_axis(md["S"], order, 2)
+    md["T"] = np.take_along_axis(md["T"], order, 2)
+    end = rng.integers(1, k + 1, size=(n, m))
+    hit = np.arange(k) == end[..., None]
+    md["S"] = np.where(hit, -1, md["S"]).astype(np.int32)   # entries behind it stay
+    V0 = rng.normal(size=n).astype(np.float32)
+    p = MDP.from_arrays(md)
+    if api == "cpu":
+        pol = MDPValueIterationCPU(p, Vinitial=V0).solve()
+    else:
+        p.initialize_gpu()
+        alg = MDPValueIterationGPU(p, Vinitial=V0)
+        if api == "gpu":
+            pol = alg.solve()
+        else:
+            sweep, prev = 0, V0
+            while True:      # where the oracle's residual first falls below the tolerance
+                sweep += 1
+                V, pi = orc.mdp_vi_solve(dict(md, horizon=1), horizon=1, VInitial=prev)
+                resid = float(np.max(np.abs(V.astype(np.float64) - prev.astype(np.float64))))
+                if resid < 0.3 or sweep == min(horizon, 40):
+                    break
+                prev = V
+            pol, ran, residual = alg.solve_until_converged(tol=0.3, maxSweeps=min(horizon, 40))
+            assert ran == sweep and residual == resid
+    if api != "converged":
+        V, pi = orc.mdp_vi_solve(md, horizon=horizon, VInitial=V0)
+    np.testing.assert_array_equal(bits(pol.V_array()), bits(V))
+    np.testing.assert_array_equal(pol.pi_array(), pi)

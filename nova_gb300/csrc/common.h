@@ -10,6 +10,7 @@
 #include <mutex>
 #include <unordered_map>
 #include <memory>
+#include <vector>
 
 #include <nova/error_codes.h>
 
@@ -38,6 +39,44 @@ template <typename T>
 inline int dev_alloc(T **p, size_t count, const char *fn, const char *what) {
     return dev_malloc(reinterpret_cast<void **>(p), count * sizeof(T), fn, what);
 }
+
+// Device arrays that live and die together, in one allocation: a solver's 30
+// to 40 arrays cost 0.6 ms to allocate and 0.5 ms to free one by one (an eighth
+// of a Perseus solve of n = 512). add() each array, then commit() once; the
+// arrays are 256-byte aligned.
+class Arena {
+    struct Item {
+        void **p;
+        size_t bytes;
+    };
+    std::vector<Item> items;
+    void *base = nullptr;
+
+public:
+    Arena() = default;
+    Arena(const Arena &) = delete;
+    Arena &operator=(const Arena &) = delete;
+    ~Arena() { cudaFree(base); }
+    template <typename T>
+    void add(T **p, size_t count) {
+        *p = nullptr;
+        items.push_back(Item{reinterpret_cast<void **>(p), count * sizeof(T)});
+    }
+    int commit(const char *fn, const char *what) {
+        size_t total = 0;
+        for (const Item &i : items) total += (i.bytes + 255) / 256 * 256;
+        const int rc = dev_malloc(&base, total, fn, what);
+        if (rc == NOVA_SUCCESS) {
+            size_t at = 0;
+            for (const Item &i : items) {
+                *i.p = static_cast<unsigned char *>(base) + at;
+                at += (i.bytes + 255) / 256 * 256;
+            }
+        }
+        items.clear();
+        return rc;
+    }
+};
 
 // Device-side error word: bounded waits write a code here instead of hanging.
 // Codes: 1 = mbarrier wait timed out in the scoring GEMM. Defined with the

@@ -618,15 +618,12 @@ __global__ void dense_beliefs_kernel(unsigned n, unsigned r, unsigned rz, const 
 // Device copies of a host-array POMDP plus the predecessor lists and the
 // dense beliefs, freed on destruction.
 struct ExpWorkspace {
+    Arena arena;
     ExpModel md{};
     int *S = nullptr, *Z = nullptr;
     float *T = nullptr, *O = nullptr, *R = nullptr, *B = nullptr, *BT = nullptr, *PO = nullptr, *predT = nullptr;
     unsigned *predStart = nullptr, *predState = nullptr;
     size_t smem = 0;
-    ~ExpWorkspace() {
-        cudaFree(S); cudaFree(Z); cudaFree(T); cudaFree(O); cudaFree(R); cudaFree(B); cudaFree(BT);
-        cudaFree(PO); cudaFree(predStart); cudaFree(predState); cudaFree(predT);
-    }
 };
 
 int build_workspace(const POMDP *p, ExpWorkspace &ws, const char *fn) {
@@ -667,17 +664,18 @@ int build_workspace(const POMDP *p, ExpWorkspace &ws, const char *fn) {
                 state[k] = s;
                 prob[k] = p->T[((size_t)s * m + a) * ns + i];
             }
-    if ((rc = dev_alloc(&ws.S, nms, fn, "the successor states")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws.T, nms, fn, "the state transitions")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws.O, (size_t)m * n * z, fn, "the observation transitions")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws.R, (size_t)n * m, fn, "the rewards")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws.Z, (size_t)r * rz, fn, "the belief states")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws.B, (size_t)r * rz, fn, "the belief values")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws.BT, (size_t)n * r, fn, "the dense beliefs")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws.predStart, start.size(), fn, "the predecessor offsets")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws.predState, std::max<size_t>(nms, 1), fn, "the predecessors")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws.predT, std::max<size_t>(nms, 1), fn, "the predecessors")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws.PO, (size_t)m * n * z, fn, "the observation probabilities")) != NOVA_SUCCESS) return rc;
+    ws.arena.add(&ws.S, nms);
+    ws.arena.add(&ws.T, nms);
+    ws.arena.add(&ws.O, (size_t)m * n * z);
+    ws.arena.add(&ws.R, (size_t)n * m);
+    ws.arena.add(&ws.Z, (size_t)r * rz);
+    ws.arena.add(&ws.B, (size_t)r * rz);
+    ws.arena.add(&ws.BT, (size_t)n * r);
+    ws.arena.add(&ws.predStart, start.size());
+    ws.arena.add(&ws.predState, std::max<size_t>(nms, 1));
+    ws.arena.add(&ws.predT, std::max<size_t>(nms, 1));
+    ws.arena.add(&ws.PO, (size_t)m * n * z);
+    if ((rc = ws.arena.commit(fn, "the model and the beliefs")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws.S, p->S, nms * sizeof(int), fn, "the successor states")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws.T, p->T, nms * sizeof(float), fn, "the state transitions")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws.O, p->O, (size_t)m * n * z * sizeof(float), fn, "the observation transitions")) != NOVA_SUCCESS)
@@ -813,23 +811,18 @@ int run_distinct(const ExpWorkspace &ws, std::vector<float> &Bnew, const char *f
     const size_t perBelief = (n * mz + md.m * n + 2 * mz) * sizeof(float);
     d.chunk = (unsigned)std::min<size_t>(md.r, std::max<size_t>(1, (512ull << 20) / perBelief));
     float *dB = nullptr;
-    struct Free {
-        Distinct &d; float *&b;
-        ~Free() {
-            cudaFree(d.W); cudaFree(d.bp); cudaFree(d.mass); cudaFree(d.bound); cudaFree(d.list); cudaFree(d.nnz);
-            cudaFree(d.total); cudaFree(d.odd); cudaFree(b);
-        }
-    } guard{d, dB};
+    Arena arena;
     int rc;
-    if ((rc = dev_alloc(&dB, rn, fn, "the new beliefs")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&d.W, (size_t)d.chunk * md.m * n, fn, "the successor masses")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&d.bp, (size_t)d.chunk * n * mz, fn, "the successor beliefs")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&d.mass, (size_t)d.chunk * mz, fn, "the successor sums")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&d.bound, (size_t)d.chunk * mz, fn, "the distance bounds")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&d.list, (size_t)md.r * d.cap, fn, "the belief nonzeros")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&d.nnz, md.r, fn, "the belief nonzeros")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&d.total, md.r, fn, "the belief sums")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&d.odd, 2, fn, "the belief check")) != NOVA_SUCCESS) return rc;
+    arena.add(&dB, rn);
+    arena.add(&d.W, (size_t)d.chunk * md.m * n);
+    arena.add(&d.bp, (size_t)d.chunk * n * mz);
+    arena.add(&d.mass, (size_t)d.chunk * mz);
+    arena.add(&d.bound, (size_t)d.chunk * mz);
+    arena.add(&d.list, (size_t)md.r * d.cap);
+    arena.add(&d.nnz, md.r);
+    arena.add(&d.total, md.r);
+    arena.add(&d.odd, 2);
+    if ((rc = arena.commit(fn, "the successor beliefs")) != NOVA_SUCCESS) return rc;
     if (cudaMemsetAsync(d.odd, 0, 2 * sizeof(unsigned)) != cudaSuccess) {
         cudaGetLastError();
         NOVA_ERR(fn, "Failed to clear the belief check.");

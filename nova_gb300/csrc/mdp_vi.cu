@@ -223,17 +223,16 @@ static int launch_sweep(const MDP *mdp, const int *S, const float *T, const floa
 
 // Device-side solver state of MDPVIGPU beyond its ABI fields.
 struct ViGpuWorkspace : Workspace {
+    Arena arena;
     float *d_V = nullptr, *d_VPrime = nullptr;
     unsigned *d_pi = nullptr;
     ViDeviceState *st = nullptr;
     ViTilePlan plan;
-    ~ViGpuWorkspace() override {
-        cudaFree(d_V); cudaFree(d_VPrime); cudaFree(d_pi); cudaFree(st);
-    }
 };
 
 // Host-buffer solver (MDPVICPU): device copies of the model and of V, V', pi.
 struct ViCpuWorkspace : Workspace {
+    Arena arena;
     int *S = nullptr;
     float *T = nullptr, *R = nullptr;
     float *V = nullptr, *VPrime = nullptr;
@@ -242,15 +241,10 @@ struct ViCpuWorkspace : Workspace {
     float *hostV = nullptr, *hostVPrime = nullptr;   // the arrays this library gave the struct
     unsigned *hostPi = nullptr;
     ViTilePlan plan;
-    ~ViCpuWorkspace() override {
-        cudaFree(S); cudaFree(T); cudaFree(R); cudaFree(V); cudaFree(VPrime); cudaFree(pi); cudaFree(st);
-    }
 };
 
-static int alloc_state(ViDeviceState **st, const char *fn) {
-    int rc = dev_alloc(st, 1, fn, "the convergence state");
-    if (rc != NOVA_SUCCESS) return rc;
-    if (cudaMemset(*st, 0, sizeof(ViDeviceState)) != cudaSuccess) {
+static int clear_state(ViDeviceState *st, const char *fn) {
+    if (cudaMemset(st, 0, sizeof(ViDeviceState)) != cudaSuccess) {
         cudaGetLastError();
         NOVA_ERR(fn, "Failed to clear the convergence state.");
         return NOVA_ERROR_MEMCPY_TO_DEVICE;
@@ -320,10 +314,12 @@ extern "C" int mdp_vi_initialize_gpu(const MDP *mdp, MDPVIGPU *vi) {
     const unsigned n = mdp->n;
     std::unique_ptr<ViGpuWorkspace> ws(new ViGpuWorkspace());
     int rc;
-    if ((rc = dev_alloc(&ws->d_V, n, fn, "the value function")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->d_VPrime, n, fn, "the value function (prime)")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->d_pi, n, fn, "the policy (pi)")) != NOVA_SUCCESS) return rc;
-    if ((rc = alloc_state(&ws->st, fn)) != NOVA_SUCCESS) return rc;
+    ws->arena.add(&ws->d_V, n);
+    ws->arena.add(&ws->d_VPrime, n);
+    ws->arena.add(&ws->d_pi, n);
+    ws->arena.add(&ws->st, 1);
+    if ((rc = ws->arena.commit(fn, "the value functions")) != NOVA_SUCCESS) return rc;
+    if ((rc = clear_state(ws->st, fn)) != NOVA_SUCCESS) return rc;
     // VInitial == nullptr means V = 0 (mdp_vi_gpu.cu:100-106).
     std::vector<float> zeros;
     const float *init = vi->VInitial;
@@ -607,13 +603,15 @@ extern "C" int mdp_vi_initialize_cpu(const MDP *mdp, MDPVICPU *vi) {
     if (mdp->S != nullptr && mdp->T != nullptr && mdp->R != nullptr && mdp->ns > 0 && mdp->m > 0) {
         const size_t nms = (size_t)n * mdp->m * mdp->ns;
         int rc;
-        if ((rc = dev_alloc(&ws->S, nms, fn, "the successor states")) != NOVA_SUCCESS) return rc;
-        if ((rc = dev_alloc(&ws->T, nms, fn, "the state transitions")) != NOVA_SUCCESS) return rc;
-        if ((rc = dev_alloc(&ws->R, (size_t)n * mdp->m, fn, "the rewards")) != NOVA_SUCCESS) return rc;
-        if ((rc = dev_alloc(&ws->V, n, fn, "the value function")) != NOVA_SUCCESS) return rc;
-        if ((rc = dev_alloc(&ws->VPrime, n, fn, "the value function (prime)")) != NOVA_SUCCESS) return rc;
-        if ((rc = dev_alloc(&ws->pi, n, fn, "the policy (pi)")) != NOVA_SUCCESS) return rc;
-        if ((rc = alloc_state(&ws->st, fn)) != NOVA_SUCCESS) return rc;
+        ws->arena.add(&ws->S, nms);
+        ws->arena.add(&ws->T, nms);
+        ws->arena.add(&ws->R, (size_t)n * mdp->m);
+        ws->arena.add(&ws->V, n);
+        ws->arena.add(&ws->VPrime, n);
+        ws->arena.add(&ws->pi, n);
+        ws->arena.add(&ws->st, 1);
+        if ((rc = ws->arena.commit(fn, "the model and the value functions")) != NOVA_SUCCESS) return rc;
+        if ((rc = clear_state(ws->st, fn)) != NOVA_SUCCESS) return rc;
         if ((rc = h2d(ws->S, mdp->S, nms * sizeof(int), fn, "the successor states")) != NOVA_SUCCESS) return rc;
         if ((rc = h2d(ws->T, mdp->T, nms * sizeof(float), fn, "the state transitions")) != NOVA_SUCCESS) return rc;
         if ((rc = h2d(ws->R, mdp->R, (size_t)n * mdp->m * sizeof(float), fn, "the rewards")) != NOVA_SUCCESS) return rc;

@@ -917,13 +917,8 @@ BackupEngine::~BackupEngine() {
     for (auto &g : graph)
         if (g) cudaGraphExecDestroy(g);
     if (tc) tc_release(tc);
-    cudaFree(succLen); cudaFree(suppLen); cudaFree(C1); cudaFree(C3);
-    cudaFree(hash); cudaFree(rep); cudaFree(dedupKeys); cudaFree(dedupLow); cudaFree(dedupDone); cudaFree(uniqJ); cudaFree(uniqIota); cudaFree(report); cudaFree(Gt);
-    cudaFree(jstar); cudaFree(actVal); cudaFree(partV); cudaFree(partU); cudaFree(items);
-    cudaFree(keptCount);
-    cudaFree(dotScratch); cudaFree(bDense); cudaFree(resultA); cudaFree(resultV); cudaFree(rowScratch);
-    cudaFree(vnb); cudaFree(vnp1b);
-    cudaFree(Proj); cudaFree(ustar); cudaFree(scanV); cudaFree(scanU);
+    cudaFree(partV); cudaFree(partU);
+    cudaFree(Proj); cudaFree(scanV); cudaFree(scanU);
     if (eventsMade)
         for (auto &e : ev) cudaEventDestroy(e);
 }
@@ -936,34 +931,35 @@ int BackupEngine::build(const DevModel &model, const char *fn) {
     if ((rc = sync_device(fn)) != NOVA_SUCCESS) return rc;
     const size_t nm = (size_t)md.n * md.m;
     const size_t coef = nm * md.ns * md.z;
-    if ((rc = dev_alloc(&succLen, nm, fn, "the successor lengths")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&suppLen, md.r, fn, "the belief support lengths")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&C1, coef, fn, "the projection coefficients")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&C3, coef, fn, "the projection coefficients (successor-major)")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&hash, md.r, fn, "the alpha hashes")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&rep, md.r, fn, "the alpha representatives")) != NOVA_SUCCESS) return rc;
+    arena.add(&succLen, nm);
+    arena.add(&suppLen, md.r);
+    arena.add(&C1, coef);
+    arena.add(&C3, coef);
+    arena.add(&hash, md.r);
+    arena.add(&rep, md.r);
     dedupCap = 64;
     while (dedupCap < 2ull * md.r) dedupCap *= 2;
-    if ((rc = dev_alloc(&dedupKeys, dedupCap, fn, "the alpha dedup table")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&dedupLow, dedupCap, fn, "the alpha dedup table")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&dedupDone, 1, fn, "the alpha dedup counter")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&uniqJ, md.r, fn, "the unique alphas")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&uniqIota, md.r, fn, "the alpha indices")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&report, kReport, fn, "the update's report")) != NOVA_SUCCESS) return rc;
+    arena.add(&dedupKeys, dedupCap);
+    arena.add(&dedupLow, dedupCap);
+    arena.add(&dedupDone, 1);
+    arena.add(&uniqJ, md.r);
+    arena.add(&uniqIota, md.r);
+    arena.add(&report, kReport);
+    gtCols = round_up(md.r, 32);
+    arena.add(&Gt, (size_t)md.n * gtCols);
+    arena.add(&jstar, (size_t)md.r * md.m * md.z);
+    arena.add(&ustar, (size_t)md.r * md.m * md.z);
+    arena.add(&actVal, (size_t)md.r * md.m);
+    arena.add(&items, (size_t)md.r * md.m);
+    arena.add(&keptCount, 1);
+    arena.add(&dotScratch, md.r);
+    arena.add(&bDense, md.n);
+    arena.add(&resultA, 1);
+    arena.add(&resultV, 1);
+    arena.add(&rowScratch, md.n);
+    if ((rc = arena.commit(fn, "the backup tables")) != NOVA_SUCCESS) return rc;
     nUniqueDev = report;
     itemCount = report + 1;
-    gtCols = round_up(md.r, 32);
-    if ((rc = dev_alloc(&Gt, (size_t)md.n * gtCols, fn, "the transposed alphas")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&jstar, (size_t)md.r * md.m * md.z, fn, "the chosen alphas")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ustar, (size_t)md.r * md.m * md.z, fn, "the chosen unique alphas")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&actVal, (size_t)md.r * md.m, fn, "the action values")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&items, (size_t)md.r * md.m, fn, "the work list")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&keptCount, 1, fn, "the kept-belief count")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&dotScratch, md.r, fn, "the FP64 values")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&bDense, md.n, fn, "the belief")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&resultA, 1, fn, "the action")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&resultV, 1, fn, "the value")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&rowScratch, md.n, fn, "the alpha row")) != NOVA_SUCCESS) return rc;
     if (!eventsMade) {
         for (auto &e : ev) cudaEventCreate(&e);
         eventsMade = true;
@@ -976,8 +972,7 @@ int BackupEngine::build(const DevModel &model, const char *fn) {
     tables_len_kernel<<<ceil_div(md.r, 256), 256>>>(md.r, md.rz, md.Z, suppLen);
     if ((rc = check_launch(fn, "support lengths")) != NOVA_SUCCESS) return rc;
     tables_coef_kernel<<<std::min<size_t>(ceil_div(coef, 256), 65535u * 8u), 256>>>(md, succLen, C1, C3);
-    if ((rc = check_launch(fn, "projection coefficients")) != NOVA_SUCCESS) return rc;
-    return sync_device(fn);
+    return check_launch(fn, "projection coefficients");
 }
 
 int BackupEngine::dedup(const float *src, unsigned rows, bool own, unsigned *nUnique, const char *fn) {
@@ -1450,17 +1445,16 @@ struct PbviGpuWorkspace : Workspace {
     BackupEngine eng;
     bool built = false;
     const void *modelKey[6] = {};   // device model pointers the tables were built from
+    Arena arena;
     float *d_Gamma = nullptr, *d_GammaPrime = nullptr;
     unsigned *d_pi = nullptr;
-    ~PbviGpuWorkspace() override {
-        cudaDeviceSynchronize();
-        cudaFree(d_Gamma); cudaFree(d_GammaPrime); cudaFree(d_pi);
-    }
+    ~PbviGpuWorkspace() override { cudaDeviceSynchronize(); }
 };
 
 struct PbviCpuWorkspace : Workspace {
     BackupEngine eng;
     bool built = false;
+    Arena arena;
     int *S = nullptr; float *T = nullptr, *O = nullptr, *R = nullptr; int *Z = nullptr; float *B = nullptr;
     float *Gamma = nullptr, *GammaPrime = nullptr;
     unsigned *pi = nullptr;
@@ -1475,8 +1469,6 @@ struct PbviCpuWorkspace : Workspace {
             cudaHostUnregister(hostPi);
             cudaGetLastError();
         }
-        cudaFree(S); cudaFree(T); cudaFree(O); cudaFree(R); cudaFree(Z); cudaFree(B);
-        cudaFree(Gamma); cudaFree(GammaPrime); cudaFree(pi);
     }
 };
 
@@ -1487,18 +1479,24 @@ static DevModel device_model(const POMDP *p) {
     return md;
 }
 
-// Upload a host POMDP into device arrays owned by a workspace.
+// Upload a host POMDP into device arrays owned by a workspace, beside its
+// alpha sets.
 template <typename W>
 static int upload_model(W *ws, const POMDP *p, DevModel *md, const char *fn) {
     const size_t nms = (size_t)p->n * p->m * p->ns, mnz = (size_t)p->m * p->n * p->z, nm = (size_t)p->n * p->m,
                  rrz = (size_t)p->r * p->rz;
     int rc;
-    if ((rc = dev_alloc(&ws->S, nms, fn, "the successor states")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->T, nms, fn, "the state transitions")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->O, mnz, fn, "the observation transitions")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->R, nm, fn, "the rewards")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->Z, rrz, fn, "the non-zero belief states")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->B, rrz, fn, "the belief points")) != NOVA_SUCCESS) return rc;
+    ws->arena.add(&ws->S, nms);
+    ws->arena.add(&ws->T, nms);
+    ws->arena.add(&ws->O, mnz);
+    ws->arena.add(&ws->R, nm);
+    ws->arena.add(&ws->Z, rrz);
+    ws->arena.add(&ws->B, rrz);
+    const size_t rn = (size_t)p->r * p->n;
+    ws->arena.add(&ws->Gamma, rn);
+    ws->arena.add(&ws->GammaPrime, rn);
+    ws->arena.add(&ws->pi, p->r);
+    if ((rc = ws->arena.commit(fn, "the model and the alpha sets")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws->S, p->S, nms * sizeof(int), fn, "the successor states")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws->T, p->T, nms * sizeof(float), fn, "the state transitions")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws->O, p->O, mnz * sizeof(float), fn, "the observation transitions")) != NOVA_SUCCESS) return rc;
@@ -1591,11 +1589,12 @@ extern "C" int pomdp_pbvi_initialize_gpu(const POMDP *pomdp, POMDPPBVIGPU *pbvi)
     ws->eng.scoring = scoring;
     const size_t rn = (size_t)pomdp->r * pomdp->n;
     int rc;
-    if ((rc = dev_alloc(&ws->d_Gamma, rn, fn, "Gamma")) != NOVA_SUCCESS) return rc;
+    ws->arena.add(&ws->d_Gamma, rn);
+    ws->arena.add(&ws->d_GammaPrime, rn);
+    ws->arena.add(&ws->d_pi, pomdp->r);
+    if ((rc = ws->arena.commit(fn, "the alpha sets")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws->d_Gamma, pbvi->GammaInitial, rn * sizeof(float), fn, "Gamma")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->d_GammaPrime, rn, fn, "Gamma (prime)")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws->d_GammaPrime, pbvi->GammaInitial, rn * sizeof(float), fn, "Gamma (prime)")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->d_pi, pomdp->r, fn, "pi")) != NOVA_SUCCESS) return rc;
     if (cudaMemset(ws->d_pi, 0, pomdp->r * sizeof(unsigned)) != cudaSuccess) {
         cudaGetLastError();
         NOVA_ERR(fn, "Failed to clear pi.");
@@ -2037,10 +2036,6 @@ static int pbvi_cpu_prepare(PbviCpuWorkspace *ws, const POMDP *pomdp, const char
     DevModel md;
     int rc = upload_model(ws, pomdp, &md, fn);
     if (rc != NOVA_SUCCESS) return rc;
-    const size_t rn = (size_t)pomdp->r * pomdp->n;
-    if ((rc = dev_alloc(&ws->Gamma, rn, fn, "Gamma")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->GammaPrime, rn, fn, "Gamma (prime)")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->pi, pomdp->r, fn, "pi")) != NOVA_SUCCESS) return rc;
     if ((rc = ws->eng.build(md, fn)) != NOVA_SUCCESS) return rc;
     ws->built = true;
     return NOVA_SUCCESS;

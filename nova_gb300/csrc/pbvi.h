@@ -47,6 +47,7 @@ struct ProjView {
 // Exact-order kernel workspace and tables.
 struct BackupEngine {
     DevModel md{};
+    Arena arena;                   // what build() allocates
     // Step-invariant tables (built once per model):
     unsigned *succLen = nullptr;   // [n*m]  successors before the first negative entry of row (s,a)
     unsigned *suppLen = nullptr;   // [r]    support entries before the first negative state of belief i

@@ -335,14 +335,11 @@ __global__ void adjoint_step_kernel(AdjModel md, const unsigned *__restrict__ le
 }
 
 struct AdjBuffers {
+    Arena arena;
     unsigned *len = nullptr, *ST = nullptr, *acts = nullptr, *ids = nullptr, *cursor = nullptr;
     float *CT = nullptr, *seg = nullptr;
     double *lamA = nullptr, *lamB = nullptr, *vals = nullptr, *V = nullptr;
     unsigned *istar = nullptr;
-    ~AdjBuffers() {
-        cudaFree(len); cudaFree(ST); cudaFree(acts); cudaFree(ids); cudaFree(cursor); cudaFree(CT); cudaFree(seg);
-        cudaFree(lamA); cudaFree(lamB); cudaFree(vals); cudaFree(V); cudaFree(istar);
-    }
 };
 
 // Gamma_t from Gamma_{t-1} in FP64 with recorded selections:
@@ -434,18 +431,21 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
     const size_t rn = (size_t)r * n;
     AdjBuffers bf;
     int rc;
-    if ((rc = dev_alloc(&bf.len, (size_t)n * m, fn, "the successor lengths")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&bf.ST, (size_t)m * n * ns, fn, "the successors")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&bf.CT, (size_t)m * z * n * ns, fn, "the projection coefficients")) != NOVA_SUCCESS) return rc;
+    bf.arena.add(&bf.len, (size_t)n * m);
+    bf.arena.add(&bf.ST, (size_t)m * n * ns);
+    bf.arena.add(&bf.CT, (size_t)m * z * n * ns);
     const unsigned groups = ceil_div(r, kGroup) + m;
-    if ((rc = dev_alloc(&bf.acts, (size_t)horizon * groups, fn, "the belief groups")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&bf.ids, (size_t)horizon * groups * kGroup, fn, "the belief groups")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&bf.seg, (size_t)(k + 1) * rn, fn, "the recomputed alphas")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&bf.lamA, rn, fn, "the adjoint")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&bf.lamB, rn, fn, "the adjoint")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&bf.vals, r, fn, "the values")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&bf.V, 1, fn, "the value")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&bf.istar, 1, fn, "the maximising alpha")) != NOVA_SUCCESS) return rc;
+    bf.arena.add(&bf.acts, (size_t)horizon * groups);
+    bf.arena.add(&bf.ids, (size_t)horizon * groups * kGroup);
+    bf.arena.add(&bf.seg, (size_t)(k + 1) * rn);
+    bf.arena.add(&bf.lamA, rn);
+    bf.arena.add(&bf.lamB, rn);
+    bf.arena.add(&bf.vals, r);
+    bf.arena.add(&bf.V, 1);
+    bf.arena.add(&bf.istar, 1);
+    const bool manyActions = m > 8192;
+    if (manyActions) bf.arena.add(&bf.cursor, (size_t)horizon * m);
+    if ((rc = bf.arena.commit(fn, "the adjoint")) != NOVA_SUCCESS) return rc;
     if ((rc = sync_device(fn)) != NOVA_SUCCESS) return rc;
 
     adj_len_kernel<<<ceil_div((size_t)n * m, 256), 256>>>(n * m, ns, md.S, bf.len);
@@ -453,9 +453,6 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
     adj_coef_kernel<<<std::min<size_t>(ceil_div((size_t)m * n * ns, 256), 65535u * 8u), 256>>>(md, bf.len, bf.ST,
                                                                                               bf.CT);
     if ((rc = check_launch(fn, "projection coefficients")) != NOVA_SUCCESS) return rc;
-    const bool manyActions = m > 8192;
-    if (manyActions && (rc = dev_alloc(&bf.cursor, (size_t)horizon * m, fn, "the action counts")) != NOVA_SUCCESS)
-        return rc;
     replay_groups_kernel<<<horizon, 1024, manyActions ? 0 : m * sizeof(unsigned)>>>(r, m, groups, d_actions, bf.acts,
                                                                                   bf.ids, bf.cursor);
     if ((rc = check_launch(fn, "belief groups")) != NOVA_SUCCESS) return rc;

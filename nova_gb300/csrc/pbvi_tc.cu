@@ -89,6 +89,7 @@ constexpr size_t GEMM_SMEM = (size_t)STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + 
 constexpr long long kWaitCycles = 4000000000ll;  // ~2 s at 2 GHz
 
 struct TcState {
+    Arena arena;
     size_t nPad = 0, rPad = 0, capN = 0;
     unsigned MZ = 0, mTiles = 0;
     unsigned mode = 0;              // NOVA_SCORING_BF16 or NOVA_SCORING_FP16: element type of A and Gb
@@ -149,10 +150,6 @@ constexpr size_t kTuneMaxNPad = 2048;
 
 void tc_release(TcState *tc) {
     if (!tc) return;
-    cudaFree(tc->A); cudaFree(tc->a1); cudaFree(tc->a1raw); cudaFree(tc->d1); cudaFree(tc->Gb); cudaFree(tc->shift); cudaFree(tc->scal);
-    cudaFree(tc->candV); cudaFree(tc->candU); cudaFree(tc->candX); cudaFree(tc->rowFlag); cudaFree(tc->rowCand); cudaFree(tc->rowList);
-    cudaFree(tc->chunkCount);
-    cudaFree(tc->badModel);
     if (tc->g0) cudaEventDestroy(tc->g0);
     if (tc->g1) cudaEventDestroy(tc->g1);
     delete tc;
@@ -1296,24 +1293,22 @@ int tc_build(BackupEngine &eng, const char *fn) {
     }
     tc->encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fnPtr);
     int rc;
-    if ((rc = dev_alloc(&tc->A, aElems, fn, "the tensor-core scoring operand")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&tc->a1, (size_t)tc->MZ * tc->rPad, fn, "the row bounds")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&tc->a1raw, (size_t)tc->MZ * tc->rPad, fn, "the row bounds")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&tc->d1, (size_t)tc->MZ * tc->rPad, fn, "the row bounds")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&tc->Gb, tc->capN * tc->nPad * 2, fn, "the packed alphas")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&tc->shift, md.n, fn, "the alpha shift")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&tc->scal, 9, fn, "the scoring scalars")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&tc->candV, slots * MAX_TOPK, fn, "the candidate scores")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&tc->candU, slots * MAX_TOPK, fn, "the candidate alphas")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&tc->candX, slots, fn, "the dropped-score bounds")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&tc->rowFlag, (size_t)tc->MZ * md.r, fn, "the exact-scan flags")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&tc->rowCand, (size_t)tc->MZ * md.r, fn, "the per-row re-score counts")) != NOVA_SUCCESS)
-        return rc;
-    if ((rc = dev_alloc(&tc->rowList, (size_t)tc->MZ * md.r, fn, "the exact-scan rows")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&tc->chunkCount, ceil_div((size_t)tc->MZ * md.r, kCompactChunk), fn,
-                        "the exact-scan chunk counts")) != NOVA_SUCCESS)
-        return rc;
-    if ((rc = dev_alloc(&tc->badModel, 1, fn, "the model check")) != NOVA_SUCCESS) return rc;
+    tc->arena.add(&tc->A, aElems);
+    tc->arena.add(&tc->a1, (size_t)tc->MZ * tc->rPad);
+    tc->arena.add(&tc->a1raw, (size_t)tc->MZ * tc->rPad);
+    tc->arena.add(&tc->d1, (size_t)tc->MZ * tc->rPad);
+    tc->arena.add(&tc->Gb, tc->capN * tc->nPad * 2);
+    tc->arena.add(&tc->shift, md.n);
+    tc->arena.add(&tc->scal, 9);
+    tc->arena.add(&tc->candV, slots * MAX_TOPK);
+    tc->arena.add(&tc->candU, slots * MAX_TOPK);
+    tc->arena.add(&tc->candX, slots);
+    tc->arena.add(&tc->rowFlag, (size_t)tc->MZ * md.r);
+    tc->arena.add(&tc->rowCand, (size_t)tc->MZ * md.r);
+    tc->arena.add(&tc->rowList, (size_t)tc->MZ * md.r);
+    tc->arena.add(&tc->chunkCount, ceil_div((size_t)tc->MZ * md.r, kCompactChunk));
+    tc->arena.add(&tc->badModel, 1);
+    if ((rc = tc->arena.commit(fn, "the tensor-core operands")) != NOVA_SUCCESS) return rc;
     if ((rc = tc_build_operand(eng, tc.get(), fn)) != NOVA_SUCCESS) return rc;
     cudaDeviceProp prop;
     cudaGetDeviceProperties(&prop, 0);

@@ -353,6 +353,7 @@ __global__ void fill_float_kernel(float *p, unsigned count, float v) {
 // Device-side Perseus state shared by the _gpu and _cpu front ends.
 struct PerseusCore {
     BackupEngine eng;
+    Arena arena;
     bool built = false;
     unsigned *vnbIdx = nullptr;
     // Validity of the per-horizon-step cache (V_n values).
@@ -365,17 +366,18 @@ struct PerseusCore {
     size_t partCap = 0;
     std::vector<unsigned> btHost;
     ~PerseusCore() {
-        cudaFree(vnbIdx); cudaFree(bt); cudaFree(done); cudaFree(partV); cudaFree(partU); cudaFree(proj);
+        cudaFree(partV); cudaFree(partU); cudaFree(proj);
     }
 
     int build(const DevModel &md, const char *fn) {
         int rc = eng.build(md, fn);
         if (rc != NOVA_SUCCESS) return rc;
-        if ((rc = dev_alloc(&eng.vnb, md.r, fn, "V_n(b)")) != NOVA_SUCCESS) return rc;
-        if ((rc = dev_alloc(&eng.vnp1b, md.r, fn, "V_n+1(b)")) != NOVA_SUCCESS) return rc;
-        if ((rc = dev_alloc(&bt, (size_t)md.r + 1, fn, "B~")) != NOVA_SUCCESS) return rc;
-        if ((rc = dev_alloc(&done, 1, fn, "the block counter")) != NOVA_SUCCESS) return rc;
-        if ((rc = dev_alloc(&vnbIdx, md.r, fn, "argmax V_n(b)")) != NOVA_SUCCESS) return rc;
+        arena.add(&eng.vnb, md.r);
+        arena.add(&eng.vnp1b, md.r);
+        arena.add(&bt, (size_t)md.r + 1);
+        arena.add(&done, 1);
+        arena.add(&vnbIdx, md.r);
+        if ((rc = arena.commit(fn, "the Perseus values")) != NOVA_SUCCESS) return rc;
         if (cudaMemsetAsync(done, 0, sizeof(unsigned), eng.stream) != cudaSuccess) {
             cudaGetLastError();
             NOVA_ERR(fn, "Failed to clear the block counter.");
@@ -494,26 +496,21 @@ struct PerseusCore {
 
 struct PerseusGpuWorkspace : Workspace {
     PerseusCore core;
+    Arena arena;
     const void *modelKey[6] = {};
     float *d_Gamma = nullptr, *d_GammaPrime = nullptr;
     unsigned *d_pi = nullptr, *d_piPrime = nullptr;
     unsigned *hostBTilde = nullptr;
-    ~PerseusGpuWorkspace() override {
-        cudaDeviceSynchronize();
-        cudaFree(d_Gamma); cudaFree(d_GammaPrime); cudaFree(d_pi); cudaFree(d_piPrime);
-    }
+    ~PerseusGpuWorkspace() override { cudaDeviceSynchronize(); }
 };
 
 struct PerseusCpuWorkspace : Workspace {
     PerseusCore core;
+    Arena arena;
     int *S = nullptr; float *T = nullptr, *O = nullptr, *R = nullptr; int *Z = nullptr; float *B = nullptr;
     float *Gamma = nullptr, *GammaPrime = nullptr;
     unsigned *pi = nullptr, *piPrime = nullptr;
-    ~PerseusCpuWorkspace() override {
-        cudaDeviceSynchronize();
-        cudaFree(S); cudaFree(T); cudaFree(O); cudaFree(R); cudaFree(Z); cudaFree(B);
-        cudaFree(Gamma); cudaFree(GammaPrime); cudaFree(pi); cudaFree(piPrime);
-    }
+    ~PerseusCpuWorkspace() override { cudaDeviceSynchronize(); }
 };
 
 static bool perseus_shape_invalid(const POMDP *p) {
@@ -569,10 +566,11 @@ extern "C" int pomdp_perseus_initialize_gpu(const POMDP *pomdp, POMDPPerseusGPU 
     const size_t rn = (size_t)pomdp->r * pomdp->n;
     std::unique_ptr<PerseusGpuWorkspace> ws(new PerseusGpuWorkspace());
     int rc;
-    if ((rc = dev_alloc(&ws->d_Gamma, rn, fn, "Gamma")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->d_GammaPrime, rn, fn, "Gamma (prime)")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->d_pi, pomdp->r, fn, "pi")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->d_piPrime, pomdp->r, fn, "pi (prime)")) != NOVA_SUCCESS) return rc;
+    ws->arena.add(&ws->d_Gamma, rn);
+    ws->arena.add(&ws->d_GammaPrime, rn);
+    ws->arena.add(&ws->d_pi, pomdp->r);
+    ws->arena.add(&ws->d_piPrime, pomdp->r);
+    if ((rc = ws->arena.commit(fn, "the alpha sets")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws->d_Gamma, per->GammaInitial, rn * sizeof(float), fn, "Gamma")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws->d_GammaPrime, per->GammaInitial, rn * sizeof(float), fn, "Gamma (prime)")) != NOVA_SUCCESS)
         return rc;
@@ -747,16 +745,17 @@ static int perseus_cpu_prepare(PerseusCpuWorkspace *ws, const POMDP *p, POMDPPer
     const size_t nms = (size_t)p->n * p->m * p->ns, mnz = (size_t)p->m * p->n * p->z, nm = (size_t)p->n * p->m,
                  rrz = (size_t)p->r * p->rz, rn = (size_t)p->r * p->n;
     int rc;
-    if ((rc = dev_alloc(&ws->S, nms, fn, "the successor states")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->T, nms, fn, "the state transitions")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->O, mnz, fn, "the observation transitions")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->R, nm, fn, "the rewards")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->Z, rrz, fn, "the non-zero belief states")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->B, rrz, fn, "the belief points")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->Gamma, rn, fn, "Gamma")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->GammaPrime, rn, fn, "Gamma (prime)")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->pi, p->r, fn, "pi")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&ws->piPrime, p->r, fn, "pi (prime)")) != NOVA_SUCCESS) return rc;
+    ws->arena.add(&ws->S, nms);
+    ws->arena.add(&ws->T, nms);
+    ws->arena.add(&ws->O, mnz);
+    ws->arena.add(&ws->R, nm);
+    ws->arena.add(&ws->Z, rrz);
+    ws->arena.add(&ws->B, rrz);
+    ws->arena.add(&ws->Gamma, rn);
+    ws->arena.add(&ws->GammaPrime, rn);
+    ws->arena.add(&ws->pi, p->r);
+    ws->arena.add(&ws->piPrime, p->r);
+    if ((rc = ws->arena.commit(fn, "the model and the alpha sets")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws->S, p->S, nms * sizeof(int), fn, "the successor states")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws->T, p->T, nms * sizeof(float), fn, "the state transitions")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(ws->O, p->O, mnz * sizeof(float), fn, "the observation transitions")) != NOVA_SUCCESS) return rc;

@@ -423,16 +423,14 @@ extern "C" int pomdp_alpha_vectors_value_and_action_batched(const POMDPAlphaVect
     const unsigned r = policy->r, n = policy->n;
     float *dG = nullptr, *dB = nullptr, *dV = nullptr;
     unsigned *dPi = nullptr, *dA = nullptr;
-    struct Free {
-        float *&g, *&b, *&v; unsigned *&p, *&a;
-        ~Free() { cudaFree(g); cudaFree(b); cudaFree(v); cudaFree(p); cudaFree(a); }
-    } guard{dG, dB, dV, dPi, dA};
+    Arena arena;
     int rc;
-    if ((rc = dev_alloc(&dG, (size_t)r * n, fn, "the alpha-vectors")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&dPi, r, fn, "the policy actions")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&dB, (size_t)count * n, fn, "the beliefs")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&dV, count, fn, "the values")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&dA, count, fn, "the actions")) != NOVA_SUCCESS) return rc;
+    arena.add(&dG, (size_t)r * n);
+    arena.add(&dPi, r);
+    arena.add(&dB, (size_t)count * n);
+    arena.add(&dV, count);
+    arena.add(&dA, count);
+    if ((rc = arena.commit(fn, "the policy and the beliefs")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(dG, policy->Gamma, (size_t)r * n * sizeof(float), fn, "the alpha-vectors")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(dPi, policy->pi, r * sizeof(unsigned), fn, "the policy actions")) != NOVA_SUCCESS) return rc;
     if ((rc = h2d(dB, B, (size_t)count * n * sizeof(float), fn, "the beliefs")) != NOVA_SUCCESS) return rc;

@@ -735,10 +735,108 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) proj_state_lanes_kernel(
     }
 }
 
-// Exact scan of whole (a*z+o, belief) rows over the unique alphas using the
-// projection table: value(u) = sum_k fl(Proj[ao][s_k][u] * B[i,k]) in
-// support order (pomdp_pbvi_cpu.cpp:50-83), argmax with the lowest index on
-// ties and the -1e10 sentinel. One block per row. The alphas are scanned in
+// Exact scan of every (a*z+o, belief) row: value(u) = sum_k fl(Proj[ao][s_k][u]
+// * B[i,k]) in support order (pomdp_pbvi_cpu.cpp:50-83), argmax with the lowest
+// index on ties and the -1e10 sentinel. A block holds the entries of UC alphas
+// at every state of one (a, o) in shared memory and walks its share of the
+// beliefs, UC / 4 lanes to a belief, so a table entry is read from
+// memory once instead of once per belief whose support holds its state. Bound
+// by the shared-memory reads: 4.3e9 terms (n = 512, r = 1,024, m z = 128, rz =
+// 32) take 1.04 ms; reading every row's entries through L2 took 2.06 ms.
+//
+// The best alpha of a row is a 64-bit key, the value's order-preserving bits
+// above the complement of the index (0: none above the sentinel), raised with
+// atomicMax where several blocks score a row. A value is never -0 (it starts
+// at +0), so equal values have equal bits.
+__device__ __forceinline__ unsigned long long scan_key(float v, unsigned u) {
+    const unsigned b = __float_as_uint(v);
+    const unsigned order = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+    return ((unsigned long long)order << 32) | (unsigned)~u;
+}
+
+template <int UC>
+__global__ void __launch_bounds__(1024) scan_all_kernel(DevModel md, const unsigned *__restrict__ suppLen,
+                                                        const ProjView pv, unsigned nU, unsigned chunks,
+                                                        unsigned share, unsigned long long *__restrict__ keys,
+                                                        float one) {
+    // LANES lanes share a belief, four adjacent alphas each (one vector read a
+    // term). Odd list pitches keep a warp's lists in distinct banks.
+    constexpr unsigned LANES = UC / 4, GROUPS = 32 / LANES, PITCH = UC + 4;
+    extern __shared__ __align__(16) float smem[];
+    float *tile = smem;                                                          // [n][PITCH]
+    uint2 *lists = reinterpret_cast<uint2 *>(tile + (size_t)md.n * PITCH);       // [warps * GROUPS][rz | 1]
+    const unsigned ao = blockIdx.x / chunks, chunk = blockIdx.x % chunks, u0 = chunk * UC;
+    const float *P = pv.slab(ao);
+    const unsigned live = min((unsigned)UC, nU - u0);
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    for (unsigned e = warp; e < UC * ((md.n + 31) / 32); e += warps) {
+        const unsigned u = e % UC, s = e / UC * 32 + lane;
+        if (s < md.n) tile[s * PITCH + u] = u < live ? __ldg(P + pv.at(s, u0 + u)) : 0.0f;
+    }
+    __syncthreads();
+    const unsigned long long one2 = pack_f32x2(one, one);
+    const unsigned group = lane / LANES, gl = lane % LANES;
+    uint2 *list = lists + (size_t)(warp * GROUPS + group) * (md.rz | 1u);
+    const float *mine = tile + 4 * gl;
+    const unsigned iEnd = min(md.r, (blockIdx.y + 1) * share);
+    for (unsigned i0 = blockIdx.y * share + warp * GROUPS; i0 < iEnd; i0 += warps * GROUPS) {
+        const unsigned i = i0 + group;
+        const unsigned Li = i < iEnd ? suppLen[i] : 0u;
+        for (unsigned k = gl; k < Li; k += LANES)
+            list[k] = make_uint2((unsigned)md.Z[(size_t)i * md.rz + k] * PITCH,
+                                 __float_as_uint(md.B[(size_t)i * md.rz + k]));
+        __syncwarp();
+        unsigned long long lo = 0ull, hi = 0ull;
+#pragma unroll 8
+        for (unsigned k = 0; k < Li; k++) {
+            const uint2 e = list[k];
+            const ulonglong2 p = *reinterpret_cast<const ulonglong2 *>(mine + e.x);
+            const float b = __uint_as_float(e.y);
+            const unsigned long long bb = pack_f32x2(b, b);
+            lo = fma_f32x2(mul_f32x2(p.x, bb), one2, lo);
+            hi = fma_f32x2(mul_f32x2(p.y, bb), one2, hi);
+        }
+        float best = NOVA_FLT_MIN;
+        unsigned bu = kNone;
+#pragma unroll
+        for (unsigned q = 0; q < 4; q++) {
+            const float v = f32x2_part(q < 2 ? lo : hi, q & 1);
+            if (4 * gl + q < live && v > best) { best = v; bu = u0 + 4 * gl + q; }
+        }
+#pragma unroll
+        for (int off = LANES / 2; off > 0; off >>= 1) {
+            const float v2 = __shfl_xor_sync(0xffffffffu, best, off);
+            const unsigned u2 = __shfl_xor_sync(0xffffffffu, bu, off);
+            if (u2 != kNone && (bu == kNone || better(v2, u2, best, bu))) { best = v2; bu = u2; }
+        }
+        if (gl == 0 && i < iEnd) {
+            unsigned long long *key = keys + (size_t)ao * md.r + i;
+            const unsigned long long k = bu == kNone ? 0ull : scan_key(best, bu);
+            if (chunks == 1) *key = k;
+            else if (k != 0ull) atomicMax(key, k);
+        }
+        __syncwarp();
+    }
+}
+
+// The choices of scan_all_kernel (kNone where nothing beat the sentinel).
+__global__ void scan_all_finish_kernel(DevModel md, const unsigned long long *__restrict__ keys,
+                                       const unsigned *__restrict__ uniqJ, unsigned *__restrict__ ustar,
+                                       unsigned *__restrict__ jstar) {
+    const unsigned rows = md.m * md.z * md.r;
+    for (unsigned row = blockIdx.x * blockDim.x + threadIdx.x; row < rows; row += gridDim.x * blockDim.x) {
+        const unsigned ao = row / md.r, i = row % md.r;
+        const size_t js = ((size_t)i * md.m + ao / md.z) * md.z + ao % md.z;
+        const unsigned long long k = keys[row];
+        const unsigned bu = k == 0ull ? kNone : ~(unsigned)k;
+        ustar[js] = bu;
+        jstar[js] = bu == kNone ? kNone : uniqJ[bu];
+    }
+}
+
+// The same for listed rows (those a tensor-core update leaves open), or for
+// all of them where a state column of four alphas does not fit in shared
+// memory. One block per row. The alphas are scanned in
 // column chunks [u0, u1) so that the (a, o) slice being read stays in L2
 // while the rows of that (a, o) (consecutive in the list) use it; a chunk
 // after the first merges with the running best of the earlier ones, which
@@ -918,7 +1016,7 @@ BackupEngine::~BackupEngine() {
         if (g) cudaGraphExecDestroy(g);
     if (tc) tc_release(tc);
     cudaFree(partV); cudaFree(partU);
-    cudaFree(Proj); cudaFree(scanV); cudaFree(scanU);
+    cudaFree(Proj); cudaFree(scanLate);
     if (eventsMade)
         for (auto &e : ev) cudaEventDestroy(e);
 }
@@ -945,6 +1043,9 @@ int BackupEngine::build(const DevModel &model, const char *fn) {
     arena.add(&uniqJ, md.r);
     arena.add(&uniqIota, md.r);
     arena.add(&report, kReport);
+    const size_t allRows = (size_t)md.m * md.z * md.r;
+    unsigned long long *scanBuf = nullptr;
+    if (allRows <= kDeferredRows) arena.add(&scanBuf, allRows);
     gtCols = round_up(md.r, 32);
     arena.add(&Gt, (size_t)md.n * gtCols);
     arena.add(&jstar, (size_t)md.r * md.m * md.z);
@@ -960,6 +1061,7 @@ int BackupEngine::build(const DevModel &model, const char *fn) {
     if ((rc = arena.commit(fn, "the backup tables")) != NOVA_SUCCESS) return rc;
     nUniqueDev = report;
     itemCount = report + 1;
+    if (scanBuf != nullptr) scan_buffer(scanBuf, allRows);
     if (!eventsMade) {
         for (auto &e : ev) cudaEventCreate(&e);
         eventsMade = true;
@@ -1155,19 +1257,77 @@ int BackupEngine::project(unsigned nU, const char *fn) {
 
 int BackupEngine::scan_capacity(size_t rows, const char *fn) {
     if (rows <= scanCap) return NOVA_SUCCESS;
-    int rc;
-    cudaFree(scanV); cudaFree(scanU);
-    scanV = nullptr; scanU = nullptr; scanCap = 0;
-    if ((rc = dev_alloc(&scanV, rows, fn, "the scan maxima")) != NOVA_SUCCESS) return rc;
-    if ((rc = dev_alloc(&scanU, rows, fn, "the scan arg-maxima")) != NOVA_SUCCESS) return rc;
-    scanCap = rows;
+    cudaFree(scanLate);
+    scanLate = nullptr;
+    scanCap = 0;
+    const int rc = dev_alloc(&scanLate, rows, fn, "the scan's choices");
+    if (rc != NOVA_SUCCESS) return rc;
+    scan_buffer(scanLate, rows);
     return NOVA_SUCCESS;
+}
+
+// Shared memory of scan_all_kernel with `threads` threads, and its shape: as
+// many alphas per block as fit beside the belief lists of at least 256
+// threads' groups (alphas 0: not even four do).
+constexpr size_t kScanSmemMax = 222 * 1024;
+
+static size_t scan_all_smem(const DevModel &md, unsigned alphas, unsigned threads) {
+    const size_t groups = threads / (alphas / 4);
+    return (size_t)md.n * (alphas + 4) * sizeof(float) + groups * (md.rz | 1u) * sizeof(uint2);
+}
+struct ScanShape {
+    unsigned alphas, threads;
+};
+static ScanShape scan_all_shape(const DevModel &md) {
+    for (unsigned alphas = 64; alphas >= 4; alphas /= 2)
+        for (unsigned threads = 1024; threads >= 256; threads /= 2)
+            if (scan_all_smem(md, alphas, threads) <= kScanSmemMax && scan_all_smem(md, 4, 128) <= kScanSmemMax)
+                return ScanShape{alphas, threads};
+    return ScanShape{0, 0};
+}
+
+int BackupEngine::scan_all(unsigned nU, const char *fn) {
+    int rc;
+    const size_t rows = (size_t)md.m * md.z * md.r;
+    if ((rc = scan_capacity(rows, fn)) != NOVA_SUCCESS) return rc;
+    // No more alphas than there are, no more warps than the beliefs keep
+    // busy; 512 threads where two blocks then share an SM.
+    ScanShape shape = scan_all_shape(md);
+    while (shape.alphas > 4 && shape.alphas / 2 >= nU) shape.alphas /= 2;
+    const unsigned uc = shape.alphas, lanes = uc / 4;
+    unsigned threads = 2 * scan_all_smem(md, uc, 512) <= kScanSmemMax ? 512u : shape.threads;
+    while (threads > 128 && (threads / lanes > md.r || scan_all_smem(md, uc, threads) > kScanSmemMax)) threads /= 2;
+    const size_t smem = scan_all_smem(md, uc, threads);
+    const unsigned chunks = ceil_div(std::max(nU, 1u), uc);
+    // Shares of the beliefs so that about four rounds of blocks fill the device.
+    const unsigned tiles = md.m * md.z * chunks;
+    const unsigned perSM = (unsigned)std::max<size_t>(1, std::min<size_t>(2048 / threads, kScanSmemMax / (smem + 1024)));
+    const unsigned shares =
+        std::max(1u, std::min(ceil_div(4ull * 152 * perSM, tiles), ceil_div(md.r, threads / lanes)));
+    const unsigned share = ceil_div(md.r, shares);
+    if (chunks > 1 && cudaMemsetAsync(scanKeys, 0, rows * sizeof(unsigned long long), stream) != cudaSuccess) {
+        cudaGetLastError();
+        NOVA_ERR(fn, "Failed to clear the scan keys.");
+        return NOVA_ERROR_KERNEL_EXECUTION;
+    }
+    auto kernel = uc == 64 ? scan_all_kernel<64> : uc == 32 ? scan_all_kernel<32> : uc == 16 ? scan_all_kernel<16>
+                  : uc == 8 ? scan_all_kernel<8> : scan_all_kernel<4>;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kernel<<<dim3(tiles, ceil_div(md.r, share)), threads, smem, stream>>>(md, suppLen, proj_view(), nU, chunks, share,
+                                                                        scanKeys, 1.0f);
+    if ((rc = check_launch(fn, "exact scan")) != NOVA_SUCCESS) return rc;
+    scan_all_finish_kernel<<<std::min(ceil_div(rows, 256), 152u * 8u), 256, 0, stream>>>(md, scanKeys, uniqMap, ustar,
+                                                                                        jstar);
+    if ((rc = check_launch(fn, "exact scan (finish)")) != NOVA_SUCCESS) return rc;
+    sentinel_fixup_kernel<<<ceil_div((size_t)md.r * md.m, 256), 256, 0, stream>>>(md, nullptr, ustar, jstar);
+    return check_launch(fn, "sentinel fixup");
 }
 
 int BackupEngine::scan_rows(const unsigned *rowList, unsigned nRows, unsigned nU, const char *fn,
                             const unsigned *nRowsDev) {
     if (nRows == 0) return NOVA_SUCCESS;
     int rc;
+    if (rowList == nullptr && projStateMajor) return scan_all(nU, fn);
     if ((rc = scan_capacity(nRows, fn)) != NOVA_SUCCESS) return rc;
     // Column chunk: one (a, o) slice of at most ~48 MB stays L2-resident.
     size_t chunk = ((48ull << 20) / ((size_t)md.n * sizeof(float))) / 256 * 256;
@@ -1286,10 +1446,11 @@ int BackupEngine::backup_all(const float *src, unsigned rGamma, float *dst, unsi
     // they use the state-contiguous layout: its table costs up to a third more
     // (n = 1,000, z = 11, r = 1,500: 188 against 139 us; n = 512: 136 against
     // 117), its assembly and action values far less (39 against 205 us; 30
-    // against 128). The exact scan reads whole rows and keeps the
-    // alpha-contiguous one, as do updates after one that left more than 1 % of
-    // its rows to the scan.
-    projStateMajor = wantTc && state_major_wanted();
+    // against 128). So do exact updates whose scan holds the table's columns
+    // in shared memory (scan_all). The scan of listed rows reads whole rows,
+    // and an update after one that left more than 1 % of its rows to it keeps
+    // the alpha-contiguous layout.
+    projStateMajor = state_major_wanted(wantTc);
     if (useProjNow && (rc = project(nU, fn)) != NOVA_SUCCESS) return rc;
     if (wantTc && tc == nullptr && tc_build(*this, fn) != NOVA_SUCCESS) tcUnavailable = true;
     cudaEventRecord(ev[2], stream);
@@ -1353,9 +1514,9 @@ int BackupEngine::backup_all(const float *src, unsigned rGamma, float *dst, unsi
     return NOVA_SUCCESS;
 }
 
-bool BackupEngine::state_major_wanted() const {
-    return proj_state_smem(md, proj_chunk(md.z)) <= kProjSmemMax &&
-           (scoring == NOVA_SCORING_FP16 || scoring == NOVA_SCORING_BF16) && lastScanFrac <= 0.01f;
+bool BackupEngine::state_major_wanted(bool tensor) const {
+    if (proj_state_smem(md, proj_chunk(md.z)) > kProjSmemMax) return false;
+    return tensor ? lastScanFrac <= 0.01f : scan_all_shape(md).alphas != 0;
 }
 
 bool BackupEngine::fixed_ready() const {
@@ -1375,7 +1536,7 @@ int BackupEngine::fixed_pre(const float *src, bool tensor, const char *fn) {
     if ((rc = check_launch(fn, "alpha transpose")) != NOVA_SUCCESS) return rc;
     useProjNow = ensure_proj(nU);
     if (!useProjNow) return NOVA_ERROR_KERNEL_EXECUTION;
-    projStateMajor = tensor && state_major_wanted();
+    projStateMajor = state_major_wanted(tensor);
     if ((rc = project(nU, fn)) != NOVA_SUCCESS) return rc;
     return tensor ? tc_prepare(*this, src, nU, fn) : NOVA_SUCCESS;
 }

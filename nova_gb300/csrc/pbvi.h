@@ -79,9 +79,19 @@ struct BackupEngine {
     size_t projSCols = 0;                // states per column in the state-contiguous layout (n rounded to 8)
     bool projUnavailable = false, useProjNow = false;
     bool tableNever = false;             // NOVA_PBVI_TABLE_NEVER: no projection table, ever
-    float *scanV = nullptr;              // running best of the chunked row scan
+    // The exact scans' best per row, for scanCap rows: the chunked row scan's
+    // running values and indices, or scan_all's keys, in the same memory (from
+    // the arena for up to kDeferredRows rows, else scanLate).
+    unsigned long long *scanKeys = nullptr, *scanLate = nullptr;
+    float *scanV = nullptr;
     unsigned *scanU = nullptr;
     size_t scanCap = 0;
+    void scan_buffer(unsigned long long *buf, size_t rows) {
+        scanKeys = buf;
+        scanV = reinterpret_cast<float *>(buf);
+        scanU = reinterpret_cast<unsigned *>(scanV + rows);
+        scanCap = rows;
+    }
     float *actVal = nullptr;             // [r][m] value of each action's assembled alpha at the belief
     float *partV = nullptr;              // [items][z][splits] split-scan partial maxima
     unsigned *partU = nullptr;
@@ -129,6 +139,8 @@ struct BackupEngine {
     // With nRowsDev the row count is read on the device (nRows is then its upper bound).
     int scan_rows(const unsigned *rowList, unsigned nRows, unsigned nU, const char *fn,
                   const unsigned *nRowsDev = nullptr);
+    // The same for all rows over a state-contiguous table.
+    int scan_all(unsigned nU, const char *fn);
     // One update without host read-backs, for graph capture: every alpha
     // is scored as its own, tensor-core scoring with the solver's fixed
     // schedule, the exact scan sized on the device. Same results as
@@ -157,7 +169,7 @@ struct BackupEngine {
     bool projAttrDone = false;     // shared-memory attribute of the state-contiguous projection set
     bool projRowsAttrDone = false; // and of the alpha-contiguous one
     float lastScanFrac = 0.0f;     // share of rows the last tensor-core update left to the exact scan
-    bool state_major_wanted() const;
+    bool state_major_wanted(bool tensor) const;
     // Work list of `count` consecutive items starting at `first`.
     int fill_items(unsigned first, unsigned count, const char *fn);
     // Write the last backup's selections (action per belief, alpha per

@@ -267,3 +267,23 @@ def test_resident_sweeps(n, m, ns, horizon, api):
         V, pi = orc.mdp_vi_solve(md, horizon=horizon, VInitial=V0)
     np.testing.assert_array_equal(bits(pol.V_array()), bits(V))
     np.testing.assert_array_equal(pol.pi_array(), pi)
+
+
+@pytest.mark.parametrize("n,r,rz,m,z,distinct", [(2, 5, 2, 3, 2, 5), (5, 40, 5, 2, 3, 1), (64, 300, 33, 2, 5, 300),
+                                                 (830, 130, 7, 2, 2, 130), (1500, 67, 64, 1, 3, 67),
+                                                 (3000, 40, 9, 2, 1, 40), (9000, 21, 100, 1, 2, 6),
+                                                 (40, 1300, 40, 1, 2, 1300), (14000, 6, 3, 1, 1, 6)])
+def test_exact_scan(n, r, rz, m, z, distinct):
+    """4 to 64 alphas per block (as many as shared memory holds, and no more
+    than there are), one and several blocks and shares per row, equal scores,
+    and states too many for the shared-memory form."""
+    md = synth.random_pomdp(n=n, m=m, z=z, ns=min(4, n), r=r, rz=rz, gamma=0.9, horizon=2, seed=n + r)
+    rng = np.random.default_rng(n)
+    pool = rng.normal(-3.0, 1.0, size=(distinct, n)).astype(np.float32)
+    md["GammaInitial"] = pool[np.arange(r) % distinct]
+    if r > 20:   # alphas that differ only outside some beliefs' successors tie there
+        md["GammaInitial"][7] = md["GammaInitial"][3]
+        md["GammaInitial"][7, 0] += 1.0
+    G, pi, stats, Go, po = backups(md, npp.SCORING_EXACT, 2)
+    np.testing.assert_array_equal(bits(G), bits(Go))
+    np.testing.assert_array_equal(pi, po)

@@ -33,9 +33,9 @@
 // ring; with split alphas each A tile is loaded for the hi and then for the
 // lo block), warp 1 issues tcgen05.mma (M=128, N=256, K=16, cta_group::1) into
 // two 256-column TMEM accumulators, warps 2-9 drain TMEM with tcgen05.ld
-// (two warps per lane quarter, alternate 32-column chunks) and run the top-8
-// epilogue, skipping scores that lie below the row's margin under the
-// running best, while the next tile accumulates. Work units are
+// (two warps per lane quarter, alternate 32-column chunks) and list the scores
+// within the row's margin of the running best, while the next tile
+// accumulates. Work units are
 // (a*z+o, 128-row tile, alpha group); units that run concurrently share
 // their A tile and stream the same alphas, so both stay in L2. Every
 // mbarrier wait is bounded; on timeout the kernel records an error word,
@@ -77,15 +77,15 @@ constexpr int BM = 128;            // rows (beliefs) per tile
 constexpr int BN = 256;            // alphas per tile
 constexpr int BK = 64;             // K (states) per stage: 128 bytes of BF16
 constexpr int STAGES = 4;
-constexpr int MAX_TOPK = 32;       // entries per candidate list (layout capacity)
 constexpr int MAX_LISTS = 8;       // candidate lists per row: two per alpha group
-constexpr int MAX_ENTRIES = MAX_LISTS * MAX_TOPK;
+constexpr unsigned LIST_SLOTS = 32;            // a list's header and entries: 256 bytes
+constexpr unsigned LIST_CAP = LIST_SLOTS - 1;  // entries per list
 constexpr unsigned kNoneU = 0xffffffffu;
 constexpr int A_STAGE_BYTES = BM * BK * 2;   // 16 KB
 constexpr int B_STAGE_BYTES = BN * BK * 2;   // 32 KB
 constexpr int EPI_WARPS = 8;          // two per TMEM lane quarter
 constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS;
-constexpr size_t GEMM_SMEM = (size_t)STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + 1024 + 256;
+constexpr size_t GEMM_SMEM = (size_t)STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + 1024 + 256 + 2 * BM * 8;
 constexpr long long kWaitCycles = 4000000000ll;  // ~2 s at 2 GHz
 
 struct TcState {
@@ -104,9 +104,9 @@ struct TcState {
     // packing blocks; what is accumulated is 0 again after an update (scalClean).
     unsigned *scal = nullptr;
     bool scalClean = false;
-    float *candV = nullptr;         // [MZ][r][MAX_LISTS][MAX_TOPK] (the first K entries of each list used)
-    unsigned *candU = nullptr;
-    float *candX = nullptr;         // [MZ][r][MAX_LISTS]
+    // [MZ][r][MAX_LISTS][LIST_SLOTS]: slot 0 of a list is {best score that found no room, entries}, then
+    // {score, unique alpha} in the order of the alphas.
+    uint2 *cand = nullptr;
     unsigned *rowFlag = nullptr;    // [MZ*r] rows needing the exact scan
     unsigned *rowCand = nullptr;    // [MZ*r] alphas each row re-scored exactly in the merge
     unsigned *rowList = nullptr;    // [MZ*r] their indices, compacted
@@ -116,12 +116,12 @@ struct TcState {
     CUtensorMap tmA;
     cudaEvent_t g0 = nullptr, g1 = nullptr;
     int numSMs = 0;
-    // Scoring schedule: alpha groups per row tile and entries per candidate
-    // list. Fewer groups and shorter lists make the epilogue cheaper; more
-    // room in the lists leaves fewer rows to the exact scan. The best choice
-    // depends on the shape, so each solver times kSchedules on its first
-    // tensor-core updates (scoring plus the exact scan it leaves, per unique
-    // alpha) and keeps the fastest. Results are identical for every choice.
+    // Scoring schedule: alpha groups per row tile. Fewer groups restart the
+    // running bests less often (fewer scores are listed, fewer lists merged);
+    // more split the work more evenly over the SMs. The best choice depends
+    // on the shape, so each solver times kSchedules on its first tensor-core
+    // updates (scoring plus the exact scan it leaves, per unique alpha) and
+    // keeps the fastest. Results are identical for every choice.
     int schedFixed = -1;            // chosen schedule, -1 while tuning
     unsigned tuneNext = 0;          // next trial
     bool tuneWarm = false;          // the first tensor-core update (lazy set-up) is not timed
@@ -129,23 +129,18 @@ struct TcState {
     float tuneCost[3] = {0, 0, 0};  // one per tuned schedule
     // The launch prepared by tc_prepare for tc_gemm / tc_finish.
     struct Launch {
-        unsigned nU = 0, nTiles = 0, groups = 0, lists = 0, topk = 0, kSplit = 1;
+        unsigned nU = 0, nTiles = 0, groups = 0, lists = 0, kSplit = 1;
         bool fp16 = true;
         CUtensorMap tmB;
     } last;
 };
 
-// Schedules: alpha groups per row tile and entries per candidate list.
-struct TcSchedule {
-    unsigned groups, topk;
-};
-constexpr TcSchedule kSchedules[4] = {{4u, 16u}, {4u, 8u}, {2u, 8u}, {4u, 32u}};
-constexpr int kTunedSchedules = 3;  // the first three are timed on small models
-// Deep contractions use the most lists without tuning: FP16 with 16 entries
-// per list; BF16, whose margin admits several times more candidates, 32.
-constexpr int kDeepScheduleFp16 = 0, kDeepScheduleBf16 = 3;
-// Deep contractions keep the epilogue hidden behind the MMAs; they use the
-// most lists (best resolution) without tuning.
+// Alpha groups per row tile that small models time.
+constexpr unsigned kSchedules[3] = {4u, 2u, 1u};
+constexpr int kTunedSchedules = 3;
+// Deep contractions keep the epilogue hidden behind the MMAs and take the most
+// groups (the evenest split) without tuning.
+constexpr int kDeepSchedule = 0;
 constexpr size_t kTuneMaxNPad = 2048;
 
 void tc_release(TcState *tc) {
@@ -264,7 +259,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 }
 
 // ---------------------------------------------------------------------------
-// The scoring GEMM with the top-8 epilogue
+// The scoring GEMM with the listing epilogue
 // ---------------------------------------------------------------------------
 
 struct GemmBarriers {
@@ -274,6 +269,9 @@ struct GemmBarriers {
     uint64_t accEmpty[2];
     uint32_t tmemBase;
     int abortFlag;
+    // Running best of each row in each epilogue half, below the unit it
+    // belongs to (plus 1), for the other half to read.
+    unsigned long long best[2][BM];
 };
 
 __device__ __forceinline__ void decode_unit(unsigned unit, unsigned groups, unsigned mTiles, unsigned nTiles,
@@ -286,76 +284,24 @@ __device__ __forceinline__ void decode_unit(unsigned unit, unsigned groups, unsi
     nt1 = (unsigned)((unsigned long long)(g + 1) * nTiles / groups);
 }
 
-// Sorted top-K of (score, alpha) in registers; `excl` is the best score
-// that fell off (or never entered) the list.
-template <int K>
-struct TopList {
-    float v[K];
-    unsigned u[K];
-    float excl;
-    __device__ __forceinline__ void reset() {
-#pragma unroll
-        for (int k = 0; k < K; k++) { v[k] = -INFINITY; u[k] = kNoneU; }
-        excl = -INFINITY;
+// The larger of three / eight scores, ignoring NaN unless all are.
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float max8(const float *v) {
+    return max3(max3(max3(v[0], v[1], v[2]), v[3], v[4]), max3(v[5], v[6], v[7]), v[7]);
+}
+// Drops a list's entries below the limit; returns how many are left.
+__device__ __forceinline__ unsigned list_trim(uint2 *list, unsigned count, float lim) {
+    unsigned kept = 0;
+#pragma unroll 1
+    for (unsigned k = 1; k <= count; k++) {
+        const uint2 e = list[k];
+        if (__uint_as_float(e.x) >= lim) list[++kept] = e;
     }
-    __device__ __forceinline__ void push(float x, unsigned idx) {
-        if (!(x > v[K - 1])) {   // also drops NaN
-            excl = fmaxf(excl, x);
-            return;
-        }
-        excl = fmaxf(excl, v[K - 1]);
-        // insertion from the bottom; equal scores keep the earlier (lower) index first
-#pragma unroll
-        for (int k = K - 1; k > 0; k--) {
-            const bool shift = x > v[k - 1];
-            const bool place = !shift && x > v[k];
-            if (shift) { v[k] = v[k - 1]; u[k] = u[k - 1]; }
-            else if (place) { v[k] = x; u[k] = idx; }
-        }
-        if (x > v[0]) { v[0] = x; u[0] = idx; }
-    }
-};
-
-// Branch-free helpers over one 32-column chunk of a row's scores.
-__device__ __forceinline__ float chunk_max(const float (&v)[32]) {
-    float t[16];
-#pragma unroll
-    for (int k = 0; k < 16; k++) t[k] = fmaxf(v[2 * k], v[2 * k + 1]);
-#pragma unroll
-    for (int w = 8; w > 0; w >>= 1)
-#pragma unroll
-        for (int k = 0; k < w; k++) t[k] = fmaxf(t[2 * k], t[2 * k + 1]);
-    return t[0];
-}
-__device__ __forceinline__ unsigned chunk_mask(const float (&v)[32], float lim) {
-    unsigned t[16];
-#pragma unroll
-    for (int k = 0; k < 16; k++)
-        t[k] = (v[2 * k] >= lim ? 1u << (2 * k) : 0u) | (v[2 * k + 1] >= lim ? 1u << (2 * k + 1) : 0u);
-#pragma unroll
-    for (int w = 8; w > 0; w >>= 1)
-#pragma unroll
-        for (int k = 0; k < w; k++) t[k] = t[2 * k] | t[2 * k + 1];
-    return t[0];
-}
-// The smallest float above a finite or -inf f (+0 and -0 step to the
-// smallest subnormal): x > f is x >= next_up(f) for every non-NaN x.
-__device__ __forceinline__ float next_up(float f) {
-    const unsigned b = __float_as_uint(f);
-    if ((b & 0x7fffffffu) == 0u) return __uint_as_float(1u);
-    return __uint_as_float((b & 0x80000000u) ? b - 1u : b + 1u);
-}
-// v[c] for a run-time c without indexing the register array.
-__device__ __forceinline__ float chunk_select(const float (&v)[32], unsigned c) {
-    float t[16];
-#pragma unroll
-    for (int k = 0; k < 16; k++) t[k] = (c & 1u) ? v[2 * k + 1] : v[2 * k];
-    unsigned bit = 2u;
-#pragma unroll
-    for (int w = 8; w > 0; w >>= 1, bit <<= 1)
-#pragma unroll
-        for (int k = 0; k < w; k++) t[k] = (c & bit) ? t[2 * k + 1] : t[2 * k];
-    return t[0];
+    return kept;
 }
 
 // Twice the row's proven error bound (scaled units): the score gap within
@@ -375,9 +321,7 @@ struct UnitParams {
     unsigned rPad, r, nU, kBlocks, kSplit;
     const float *a1, *d1;
     const unsigned *scal;
-    float *candV;
-    unsigned *candU;
-    float *candX;
+    uint2 *cand;
 };
 
 // One solver's units (the tensor maps are kernel parameters).
@@ -385,14 +329,12 @@ struct SingleUnits {
     unsigned MZ, rPad, r, mTiles, nTiles, groups, nU, kBlocks, kSplit;
     const float *a1, *d1;
     const unsigned *scal;
-    float *candV;
-    unsigned *candU;
-    float *candX;
+    uint2 *cand;
     __device__ __forceinline__ unsigned total() const { return MZ * mTiles * groups; }
     __device__ __forceinline__ void get(unsigned unit, UnitParams &p) const {
         decode_unit(unit, groups, mTiles, nTiles, p.ao, p.mt, p.g, p.nt0, p.nt1);
         p.rPad = rPad; p.r = r; p.nU = nU; p.kBlocks = kBlocks; p.kSplit = kSplit;
-        p.a1 = a1; p.d1 = d1; p.scal = scal; p.candV = candV; p.candU = candU; p.candX = candX;
+        p.a1 = a1; p.d1 = d1; p.scal = scal; p.cand = cand;
     }
 };
 
@@ -404,9 +346,7 @@ struct BatchModel {
     unsigned unitStart, MZ, rPad, r, mTiles, nTiles, groups, nU, kBlocks, kSplit;
     const float *a1, *d1;
     const unsigned *scal;
-    float *candV;
-    unsigned *candU;
-    float *candX;
+    uint2 *cand;
 };
 
 // The units of many solvers in one sequence (solver k owns units
@@ -427,11 +367,11 @@ struct BatchUnits {
         decode_unit(unit - b.unitStart, b.groups, b.mTiles, b.nTiles, p.ao, p.mt, p.g, p.nt0, p.nt1);
         p.tmA = &b.tmA; p.tmB = &b.tmB;
         p.rPad = b.rPad; p.r = b.r; p.nU = b.nU; p.kBlocks = b.kBlocks; p.kSplit = b.kSplit;
-        p.a1 = b.a1; p.d1 = b.d1; p.scal = b.scal; p.candV = b.candV; p.candU = b.candU; p.candX = b.candX;
+        p.a1 = b.a1; p.d1 = b.d1; p.scal = b.scal; p.cand = b.cand;
     }
 };
 
-template <int K, class Units>
+template <class Units>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) tc_score_gemm_kernel(
         const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, uint32_t idesc,
         const Units units) {
@@ -447,6 +387,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) tc_score_gemm_kernel(
             mbar_init(smem_u32(&bar->full[s]), 1);
             mbar_init(smem_u32(&bar->empty[s]), 1);
         }
+        for (int k = 0; k < 2 * BM; k++) bar->best[0][k] = 0ull;  // unit 0 - 1: nobody's
         for (int a = 0; a < 2; a++) {
             mbar_init(smem_u32(&bar->accFull[a]), 1);
             mbar_init(smem_u32(&bar->accEmpty[a]), EPI_WARPS);
@@ -525,7 +466,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) tc_score_gemm_kernel(
             }
         }
     } else {
-        // ---- epilogue: TMEM -> registers -> running top-8 per row ----
+        // ---- epilogue: TMEM -> registers -> the row's candidate list ----
         // Eight warps: warps w and w+4 read the same TMEM lane quarter
         // (w & 3), one row per thread, and take alternate 32-column chunks
         // of every tile, each keeping its own list for the unit (list
@@ -533,35 +474,55 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) tc_score_gemm_kernel(
         // A score below (running best - thr), thr being the row's margin as
         // the merge computes it, lies below the merge's cut for every later
         // best (the cut is fl(final best - thr) and rounding is monotonic):
-        // it can be neither a candidate nor the dropped score that sends the
-        // row to the exact scan, so it is skipped without touching the list.
-        // A chunk whose maximum is below the limit costs a few branch-free
-        // instructions; otherwise the limit is raised to the chunk's maximum
-        // minus thr and only the chunk's scores at or above it go through
-        // the list, one set bit of the chunk's mask at a time.
+        // it cannot be a candidate, so it is skipped.
+        //
+        // With few states the MMAs of a tile take less time than reading it,
+        // and compares and selects run at half rate: what counts is the
+        // instructions per chunk. Some row of the 32 has a new best in most
+        // chunks (records of 79 chunks in random order), so the listing path
+        // matters as much as the skipping one. Listed scores are therefore
+        // appended to the row's list in global memory, unsorted, without
+        // selecting them out of the registers: each 8 columns whose maximum
+        // passes are compared and stored in turn. n = 150 (2,500 alphas,
+        // 400,000 rows): 591 us with a sorted list in registers, 348 so; 200
+        // states: 692 to 395; 512: 135 to 101 (its MMAs need 71); 700 with
+        // 12 candidates a row: 354 to 225.
         const unsigned quarter = warp & 3u;   // TMEM lanes this warp may access
         const unsigned half = (warp - 2u) >> 2;
         const unsigned rowInTile = quarter * 32u + lane;
         const float qnan = __uint_as_float(0x7fc00000u);
         unsigned acc = 0, accPhase = 0;
-        TopList<K> top;
         for (unsigned unit = blockIdx.x; unit < totalUnits && !*abortFlag; unit += gridDim.x) {
             UnitParams p;
             unit_params(unit, p);
-            const unsigned ao = p.ao, g = p.g, r = p.r, nU = p.nU;
+            const unsigned ao = p.ao, nU = p.nU;
             const float escale = __uint_as_float(p.scal[2]);
             const float dscale = __uint_as_float(p.scal[7]);
-            top.reset();
             const unsigned iRow = p.mt * BM + rowInTile;
+            const bool real = iRow < p.r;
             // Same expression as the merge's margin. An infinite margin skips
             // nothing; a NaN one skips everything, and the merge sends such
-            // rows to the exact scan whatever their lists hold.
-            const float thr = iRow < r ? row_margin(p.a1, p.d1, (size_t)ao * p.rPad + iRow, escale, dscale) : INFINITY;
-            float best = -INFINITY, lim = -INFINITY;
+            // rows to the exact scan whatever their lists hold. Rows of the
+            // tile's padding skip everything.
+            const float thr = real ? row_margin(p.a1, p.d1, (size_t)ao * p.rPad + iRow, escale, dscale) : 0.0f;
+            float best = real ? -INFINITY : INFINITY, lim = best;
+            uint2 *list = p.cand + (((size_t)ao * p.r + (real ? iRow : 0u)) * MAX_LISTS + 2u * p.g + half) * LIST_SLOTS;
+            unsigned count = 0;
+            float excl = -INFINITY, limTrim = -INFINITY;
+            volatile unsigned long long *myBest = &bar->best[half][rowInTile];
+            volatile unsigned long long *otherBest = &bar->best[half ^ 1u][rowInTile];
+            const unsigned long long tag = (unsigned long long)(unit + 1u) << 32;
             bool ok = true;
             for (unsigned nt = p.nt0; nt < p.nt1; nt++) {
                 if (!mbar_wait(smem_u32(&bar->accFull[acc]), accPhase, abortFlag)) { ok = false; break; }
                 tc_fence_after();
+                // The other half's best of this row is a listed score too, so
+                // it bounds the final best from below just as well.
+                const unsigned long long other = *otherBest;
+                if ((other & 0xffffffff00000000ull) == tag) {
+                    best = fmaxf(best, __uint_as_float((unsigned)other));
+                    lim = fmaxf(lim, best - thr);
+                }
                 const uint32_t base = tmem + ((quarter * 32u) << 16) + acc * BN;
 #pragma unroll 1
                 for (unsigned ch = half; ch < BN / 32; ch += 2) {
@@ -574,44 +535,54 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) tc_score_gemm_kernel(
                         for (int c = 0; c < 32; c++)
                             if (u0 + c >= nU) v[c] = qnan;
                     }
-                    const float mx = chunk_max(v);
+                    float m8[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) m8[q] = max8(v + 8 * q);
+                    const float mx = max3(max3(m8[0], m8[1], m8[2]), m8[3], m8[3]);
                     if (mx >= lim) {
                         // The chunk's maximum raises the running best first,
                         // so only its scores within thr of the new best are
-                        // listed (the list's first entry is that best).
+                        // listed.
                         best = fmaxf(best, mx);
                         lim = best - thr;
-                        // Scores at or below the list's last entry f would
-                        // only raise the dropped maximum (push's first
-                        // branch). If any score of the chunk is above f, its
-                        // insertion drops f itself, which bounds them all;
-                        // otherwise the chunk's maximum is the largest of
-                        // them. Either way the list and the dropped maximum
-                        // end as if every score >= lim had been pushed.
-                        unsigned mask = chunk_mask(v, fmaxf(lim, next_up(top.v[K - 1])));
-                        if (mask == 0u) top.excl = fmaxf(top.excl, mx);
-                        while (mask) {
-                            const unsigned c = __ffs(mask) - 1;
-                            mask &= mask - 1;
-                            top.push(chunk_select(v, c), u0 + c);
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            if (!(m8[q] >= lim)) continue;
+                            if (count + 8u <= LIST_CAP) {
+#pragma unroll
+                                for (int c = 0; c < 8; c++)
+                                    if (v[8 * q + c] >= lim)
+                                        list[++count] = make_uint2(__float_as_uint(v[8 * q + c]), u0 + 8 * q + c);
+                            } else {
+                                // Room may run out: entries that the risen
+                                // limit has left behind go first; what then
+                                // finds no room only raises the best dropped
+                                // score, which the merge compares to its cut.
+                                if (lim > limTrim) {
+                                    count = list_trim(list, count, lim);
+                                    limTrim = lim;
+                                }
+#pragma unroll
+                                for (int c = 0; c < 8; c++)
+                                    if (v[8 * q + c] >= lim) {
+                                        if (count < LIST_CAP)
+                                            list[++count] = make_uint2(__float_as_uint(v[8 * q + c]), u0 + 8 * q + c);
+                                        else
+                                            excl = fmaxf(excl, v[8 * q + c]);
+                                    }
+                            }
                         }
                     }
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&bar->accEmpty[acc]));
+                *myBest = tag | __float_as_uint(best);
                 acc ^= 1u;
                 if (acc == 0) accPhase ^= 1u;
             }
             if (!ok) break;
-            if (iRow < r) {
-                const size_t slot = ((size_t)ao * r + iRow) * MAX_LISTS + 2u * g + half;
-                float *cv = p.candV + slot * MAX_TOPK;
-                unsigned *cu = p.candU + slot * MAX_TOPK;
-#pragma unroll
-                for (int k = 0; k < K; k++) { cv[k] = top.v[k]; cu[k] = top.u[k]; }
-                p.candX[slot] = top.excl;
-            }
+            if (real) list[0] = make_uint2(__float_as_uint(excl), count);
         }
     }
     tc_fence_before();
@@ -862,18 +833,18 @@ struct DirectScorer {
 
 // One warp per row; returns (in every lane) the number of candidates it
 // re-scored exactly, 0 when the row was settled without re-scoring or sent to
-// the exact scan (*flagged). The row's lists hold K entries each; entry e of
-// the warp's view is entry e / nLists of list e % nLists, so the lists'
-// leading entries (where the candidates are) spread over the lanes. NE:
-// entries per lane, at least nLists * K / 32.
+// the exact scan (*flagged). Slot e of the warp's view is slot e / nLists of
+// list e % nLists, so the lists' headers (slot 0) come first, in lanes
+// 0 .. nLists - 1; NE slots per lane are loaded before the lists' lengths are
+// known, what is beyond them (rare: lists of more than 7 entries, 15 of two)
+// after that.
 //
 // Bound by the latency of dependent loads (lists, then the candidates' table
 // entries), so what a row needs before its candidates are known is loaded at
 // once, the candidates are scored together (each lane gathers one support
 // state's entry of up to kMergeBatch candidates before any is used, and lane
 // t adds candidate t's products in support order from shared memory), and
-// the entries per lane are fitted to the lists, which lets 40 warps share an
-// SM instead of 16: n = 512 (131,072 rows, 1.4 candidates each) 204 to 90 us,
+// few entries are held per lane, which lets 40 warps share an SM: n = 512 (131,072 rows, 1.4 candidates each) 204 to 90 us,
 // n = 4,096 (2.1 M rows, 6.2 each) 6.2 to 5.3 ms, the latter near the DRAM
 // time of its 32-byte sectors.
 constexpr unsigned kMergeBatch = 8;    // candidates gathered together
@@ -884,31 +855,23 @@ __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const
                                               const unsigned *__restrict__ suppLen, const ProjView &pv,
                                               const DirectScorer &ds, float *scratch, unsigned *list,
                                               const unsigned *__restrict__ uniqJ, unsigned nLists,
-                                              unsigned K, size_t rPad, const float *__restrict__ a1,
+                                              size_t rPad, const float *__restrict__ a1,
                                               const float *__restrict__ d1,
                                               const float *__restrict__ a1raw, const unsigned *__restrict__ scal,
-                                              const float *__restrict__ candV, const unsigned *__restrict__ candU,
-                                              const float *__restrict__ candX, unsigned *__restrict__ ustar,
+                                              const uint2 *__restrict__ cand, unsigned *__restrict__ ustar,
                                               unsigned *__restrict__ jstar, bool *flagged,
                                               const unsigned *__restrict__ badModel) {
     const unsigned ao = row / md.r, i = row % md.r;
     const unsigned a = ao / md.z, o = ao % md.z;
-    const size_t base = (size_t)row * MAX_ENTRIES;
-    const unsigned nEnt = nLists * K;
-    float v[NE];
-    unsigned u[NE];
+    const uint2 *lists = cand + (size_t)row * (MAX_LISTS * LIST_SLOTS);
+    const unsigned nEnt = nLists * LIST_SLOTS;
+    auto slot_of = [&](unsigned e) { return lists + (size_t)(e % nLists) * LIST_SLOTS + e / nLists; };
+    uint2 ent[NE];
 #pragma unroll
     for (int j = 0; j < NE; j++) {
         const unsigned e = lane + 32u * j;
-        v[j] = -INFINITY;
-        u[j] = kNoneU;
-        if (e < nEnt) {
-            const size_t idx = base + (size_t)(e % nLists) * MAX_TOPK + e / nLists;
-            u[j] = __ldg(candU + idx);
-            v[j] = __ldg(candV + idx);
-        }
+        ent[j] = e < nEnt ? __ldg(slot_of(e)) : make_uint2(0u, 0u);
     }
-    float x = lane < nLists ? __ldg(candX + (size_t)row * MAX_LISTS + lane) : -INFINITY;
     const float thr = row_margin(a1, d1, (size_t)ao * rPad + i, __uint_as_float(scal[2]), __uint_as_float(scal[7]));
     const float rawBound = a1raw[(size_t)ao * rPad + i] * __uint_as_float(scal[1]);
     const unsigned Li = suppLen[i];
@@ -916,19 +879,35 @@ __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const
     const float *bk = md.B + (size_t)i * md.rz;
     const unsigned s0 = lane < Li ? (unsigned)__ldg(sk + lane) : 0u;
     const float b0 = lane < Li ? __ldg(bk + lane) : 0.0f;
+    // Lane l < nLists holds list l's header.
+    const unsigned held = lane < nLists ? min(ent[0].y, LIST_CAP) : 0u;
+    float x = lane < nLists ? __uint_as_float(ent[0].x) : -INFINITY;
+    const unsigned steps = (__reduce_max_sync(0xffffffffu, held) + 1u) * nLists;  // e beyond these is in no list
+    // The score of the warp's entry e (-inf where e's list is shorter).
+    auto score_of = [&](unsigned e, uint2 en) {
+        const unsigned len = __shfl_sync(0xffffffffu, held, e % nLists), k = e / nLists;
+        return k != 0u && k <= len ? __uint_as_float(en.x) : -INFINITY;
+    };
+    float v[NE];
     float tmax = -INFINITY;
 #pragma unroll
     for (int j = 0; j < NE; j++) {
-        if (u[j] == kNoneU) v[j] = -INFINITY;
+        v[j] = score_of(lane + 32u * j, ent[j]);
         tmax = fmaxf(tmax, v[j]);
+    }
+    for (unsigned e0 = 32u * NE; e0 < steps; e0 += 32u) {
+        const unsigned e = e0 + lane;
+        tmax = fmaxf(tmax, score_of(e, e < nEnt ? __ldg(slot_of(e)) : make_uint2(0u, 0u)));
     }
     for (int off = 16; off > 0; off >>= 1) {
         tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, off));
         x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, off));
     }
-    // Usable only with a finite margin, non-negative probabilities, and
-    // scores far from the reference's -1e10 sentinel.
-    const bool usable = (thr < 1e30f) && (tmax > -INFINITY) && *badModel == 0u && (rawBound < 1e9f);
+    // Usable only with lists that the GEMM has finished, a finite margin,
+    // non-negative probabilities, and scores far from the reference's -1e10
+    // sentinel.
+    const bool usable = (thr < 1e30f) && (tmax > -INFINITY) && *badModel == 0u && (rawBound < 1e9f) &&
+                        g_device_error == 0u;
     const float cut = tmax - thr;
     if (!usable || x >= cut) {
         *flagged = true;
@@ -936,12 +915,18 @@ __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const
     }
     // The candidates, listed in shared memory.
     unsigned count = 0;
-#pragma unroll
-    for (int j = 0; j < NE; j++) {
-        const bool c = u[j] != kNoneU && v[j] >= cut;
+    auto keep = [&](float score, unsigned u) {
+        const bool c = score >= cut;
         const unsigned msk = __ballot_sync(0xffffffffu, c);
-        if (c) list[count + __popc(msk & ((1u << lane) - 1u))] = u[j];
+        if (c) list[count + __popc(msk & ((1u << lane) - 1u))] = u;
         count += __popc(msk);
+    };
+#pragma unroll
+    for (int j = 0; j < NE; j++) keep(v[j], ent[j].y);
+    for (unsigned e0 = 32u * NE; e0 < steps; e0 += 32u) {
+        const unsigned e = e0 + lane;
+        const uint2 en = e < nEnt ? __ldg(slot_of(e)) : make_uint2(0u, 0u);
+        keep(score_of(e, en), en.y);
     }
     __syncwarp();
     const size_t js = ((size_t)i * md.m + a) * md.z + o;
@@ -1086,14 +1071,13 @@ __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const
 constexpr unsigned kCompactChunk = 4096;  // rows per block of the compaction (4 per thread)
 
 template <bool kDirect, int NE>
-__global__ void __launch_bounds__(256, kDirect ? 1 : NE <= 4 ? 5 : 4) tc_merge_kernel(
+__global__ void __launch_bounds__(256, kDirect ? 1 : 5) tc_merge_kernel(
                                 DevModel md, const unsigned *__restrict__ suppLen,
                                 const ProjView pv, const DirectScorer ds, const unsigned *__restrict__ uniqJ,
-                                unsigned nLists, unsigned K,
+                                unsigned nLists,
                                 size_t rPad, const float *__restrict__ a1, const float *__restrict__ d1,
                                 const float *__restrict__ a1raw, const unsigned *__restrict__ scal,
-                                const float *__restrict__ candV, const unsigned *__restrict__ candU,
-                                const float *__restrict__ candX, unsigned *__restrict__ ustar,
+                                const uint2 *__restrict__ cand, unsigned *__restrict__ ustar,
                                 unsigned *__restrict__ jstar, unsigned *__restrict__ rowFlag,
                                 unsigned *__restrict__ rowCand, unsigned *__restrict__ counters,
                                 unsigned *__restrict__ chunkCount, const unsigned *__restrict__ badModel) {
@@ -1108,10 +1092,10 @@ __global__ void __launch_bounds__(256, kDirect ? 1 : NE <= 4 ? 5 : 4) tc_merge_k
     const unsigned row = blockIdx.x * 8u + warp;  // fewer than 2^31 rows (tc_supported)
     if (row < md.m * md.z * md.r) {
         bool flagged = false;
-        unsigned *list = reinterpret_cast<unsigned *>(mergeScratch + 8u * kWarpScratch) + warp * (NE * 32u);
+        unsigned *list = reinterpret_cast<unsigned *>(mergeScratch + 8u * kWarpScratch) + warp * (nLists * LIST_SLOTS);
         const unsigned rescored =
             merge_row<kDirect, NE>(row, lane, md, suppLen, pv, ds, mergeScratch + warp * kWarpScratch, list, uniqJ,
-                                   nLists, K, rPad, a1, d1, a1raw, scal, candV, candU, candX, ustar, jstar,
+                                   nLists, rPad, a1, d1, a1raw, scal, cand, ustar, jstar,
                                    &flagged, badModel);
         if (lane == 0) {
             rowCand[row] = rescored;
@@ -1221,7 +1205,7 @@ static int encode_map(TcState *tc, CUtensorMap *map, const void *base, size_t ro
 static int tc_build_operand(BackupEngine &eng, TcState *tc, const char *fn) {
     const DevModel &md = eng.md;
     // A new operand form starts its schedule choice afresh (the margins,
-    // and with them the best list length, differ between forms).
+    // and with them the best split, differ between forms).
     if (tc->mode != eng.scoring) {
         tc->schedFixed = -1;
         tc->tuneNext = 0;
@@ -1254,12 +1238,8 @@ static bool gemm_attributes_set() {
     std::call_once(once, [] {
         const int b = (int)GEMM_SMEM;
         const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        ok = cudaFuncSetAttribute(tc_score_gemm_kernel<8, SingleUnits>, attr, b) == cudaSuccess &&
-             cudaFuncSetAttribute(tc_score_gemm_kernel<16, SingleUnits>, attr, b) == cudaSuccess &&
-             cudaFuncSetAttribute(tc_score_gemm_kernel<32, SingleUnits>, attr, b) == cudaSuccess &&
-             cudaFuncSetAttribute(tc_score_gemm_kernel<8, BatchUnits>, attr, b) == cudaSuccess &&
-             cudaFuncSetAttribute(tc_score_gemm_kernel<16, BatchUnits>, attr, b) == cudaSuccess &&
-             cudaFuncSetAttribute(tc_score_gemm_kernel<32, BatchUnits>, attr, b) == cudaSuccess;
+        ok = cudaFuncSetAttribute(tc_score_gemm_kernel<SingleUnits>, attr, b) == cudaSuccess &&
+             cudaFuncSetAttribute(tc_score_gemm_kernel<BatchUnits>, attr, b) == cudaSuccess;
         if (!ok) cudaGetLastError();
     });
     return ok;
@@ -1278,7 +1258,7 @@ int tc_build(BackupEngine &eng, const char *fn) {
     size_t freeB = 0, totalB = 0;
     cudaMemGetInfo(&freeB, &totalB);
     const size_t slots = (size_t)tc->MZ * md.r * MAX_LISTS;
-    const size_t need = aElems * 2 + tc->capN * tc->nPad * 4 + slots * (MAX_TOPK * 8 + 4) + (size_t)tc->MZ * md.r * 12;
+    const size_t need = aElems * 2 + tc->capN * tc->nPad * 4 + slots * LIST_SLOTS * 8 + (size_t)tc->MZ * md.r * 12;
     if (need + (256ull << 20) > freeB) {
         NOVA_ERR(fn, "Not enough device memory for the tensor-core operands; using exact scoring.");
         return NOVA_ERROR_DEVICE_MALLOC;
@@ -1300,9 +1280,7 @@ int tc_build(BackupEngine &eng, const char *fn) {
     tc->arena.add(&tc->Gb, tc->capN * tc->nPad * 2);
     tc->arena.add(&tc->shift, md.n);
     tc->arena.add(&tc->scal, 9);
-    tc->arena.add(&tc->candV, slots * MAX_TOPK);
-    tc->arena.add(&tc->candU, slots * MAX_TOPK);
-    tc->arena.add(&tc->candX, slots);
+    tc->arena.add(&tc->cand, slots * LIST_SLOTS);
     tc->arena.add(&tc->rowFlag, (size_t)tc->MZ * md.r);
     tc->arena.add(&tc->rowCand, (size_t)tc->MZ * md.r);
     tc->arena.add(&tc->rowList, (size_t)tc->MZ * md.r);
@@ -1374,13 +1352,12 @@ int tc_prepare(BackupEngine &eng, const float *src, unsigned nU, const char *fn)
     TcState::Launch &L = tc->last;
     if ((rc = encode_map(tc, &L.tmB, tc->Gb, nPadRows, tc->nPad * kSplit, BN, fn)) != NOVA_SUCCESS) return rc;
     // Each alpha group leaves two lists per row (one per epilogue half).
-    if (tc->schedFixed < 0 && tc->nPad > kTuneMaxNPad) tc->schedFixed = fp16 ? kDeepScheduleFp16 : kDeepScheduleBf16;
-    const TcSchedule sched = kSchedules[tc->schedFixed >= 0 ? tc->schedFixed : (tc->tuneWarm ? (int)tc->tuneNext : 0)];
+    if (tc->schedFixed < 0 && tc->nPad > kTuneMaxNPad) tc->schedFixed = kDeepSchedule;
+    const unsigned groups = kSchedules[tc->schedFixed >= 0 ? tc->schedFixed : (tc->tuneWarm ? (int)tc->tuneNext : 0)];
     L.nU = nU;
     L.nTiles = nTiles;
-    L.groups = std::max(1u, std::min<unsigned>(sched.groups, nTiles));
+    L.groups = std::max(1u, std::min<unsigned>(groups, nTiles));
     L.lists = 2u * L.groups;
-    L.topk = sched.topk;
     L.kSplit = kSplit;
     L.fp16 = fp16;
     tc->groupsUsed = L.groups;
@@ -1394,12 +1371,9 @@ int tc_gemm(BackupEngine &eng, bool timed, const char *fn) {
     const unsigned totalUnits = tc->MZ * tc->mTiles * L.groups;
     const unsigned grid = std::min<unsigned>(totalUnits, (unsigned)tc->numSMs);
     if (timed) cudaEventRecord(tc->g0, eng.stream);
-    auto gemm = L.topk == 32u ? tc_score_gemm_kernel<32, SingleUnits>
-                : (L.topk == 16u ? tc_score_gemm_kernel<16, SingleUnits> : tc_score_gemm_kernel<8, SingleUnits>);
     const SingleUnits units{tc->MZ, (unsigned)tc->rPad, eng.md.r, tc->mTiles, L.nTiles, L.groups, L.nU,
-                            (unsigned)(tc->nPad / BK), L.kSplit, tc->a1, tc->d1, tc->scal, tc->candV, tc->candU,
-                            tc->candX};
-    gemm<<<grid, GEMM_THREADS, GEMM_SMEM, eng.stream>>>(tc->tmA, L.tmB, make_idesc(L.fp16 ? 0u : 1u), units);
+                            (unsigned)(tc->nPad / BK), L.kSplit, tc->a1, tc->d1, tc->scal, tc->cand};
+    tc_score_gemm_kernel<SingleUnits><<<grid, GEMM_THREADS, GEMM_SMEM, eng.stream>>>(tc->tmA, L.tmB, make_idesc(L.fp16 ? 0u : 1u), units);
     int rc = check_launch(fn, "tensor-core scoring");
     if (rc != NOVA_SUCCESS) return rc;
     if (timed) cudaEventRecord(tc->g1, eng.stream);
@@ -1417,18 +1391,13 @@ int tc_finish(BackupEngine &eng, const char *fn) {
     // The list can hold every row: it is sized m*z*r like the flags.
     const unsigned nChunks = ceil_div(rows, kCompactChunk);
     const DirectScorer ds{eng.succLen, eng.C3, tc->src};
-    // Entries per lane: the fewest that hold the row's lists.
-    const unsigned perLane = ceil_div(L.lists * L.topk, 32);
     const bool table = eng.useProjNow;
-    const unsigned NE = !table ? 8u : perLane <= 1 ? 1u : perLane <= 2 ? 2u : perLane <= 4 ? 4u : 8u;
-    const size_t mergeSmem = 8 * ((table ? kMergeBatch * kMergePitch : 1024u) + NE * 32u) * sizeof(float);
-    auto merge = !table ? tc_merge_kernel<true, 8>
-                 : NE == 1u ? tc_merge_kernel<false, 1>
-                 : NE == 2u ? tc_merge_kernel<false, 2>
-                 : NE == 4u ? tc_merge_kernel<false, 4> : tc_merge_kernel<false, 8>;
+    const size_t mergeSmem =
+        8 * ((table ? kMergeBatch * kMergePitch : 1024u) + L.lists * LIST_SLOTS) * sizeof(float);
+    auto merge = !table ? tc_merge_kernel<true, 2> : L.lists <= 2u ? tc_merge_kernel<false, 1> : tc_merge_kernel<false, 2>;
     merge<<<(unsigned)ceil_div(rows * 32, 256), 256, mergeSmem, eng.stream>>>(
-        md, eng.suppLen, table ? eng.proj_view() : ProjView{}, ds, eng.uniqMap, L.lists, L.topk, tc->rPad,
-        tc->a1, tc->d1, tc->a1raw, tc->scal, tc->candV, tc->candU, tc->candX, eng.ustar, eng.jstar, tc->rowFlag,
+        md, eng.suppLen, table ? eng.proj_view() : ProjView{}, ds, eng.uniqMap, L.lists, tc->rPad,
+        tc->a1, tc->d1, tc->a1raw, tc->scal, tc->cand, eng.ustar, eng.jstar, tc->rowFlag,
         tc->rowCand, tc->scal + 3, tc->chunkCount, tc->badModel);
     if ((rc = check_launch(fn, "candidate merge")) != NOVA_SUCCESS) return rc;
     tc_compact_write_kernel<<<nChunks, 1024, 0, eng.stream>>>(tc->rowFlag, (unsigned)rows, tc->chunkCount,
@@ -1483,11 +1452,11 @@ int tc_score_launch(BackupEngine &eng, const float *src, unsigned nU, bool timed
 
 struct TcBatch {
     struct Group {
-        unsigned topk = 0, totalUnits = 0, nModels = 0;
+        unsigned totalUnits = 0, nModels = 0;
         bool fp16 = true;
         BatchModel *models = nullptr;   // device work table
     };
-    std::vector<Group> groups;   // one per list length and operand form
+    std::vector<Group> groups;   // one per operand form
     int numSMs = 0;
     ~TcBatch() {
         for (auto &g : groups) cudaFree(g.models);
@@ -1500,20 +1469,15 @@ int tc_batch_create(BackupEngine *const *engs, unsigned count, TcBatch **out, co
     for (unsigned k = 0; k < count; k++) {
         const BackupEngine &e = *engs[k];
         const TcState *tc = e.tc;
-        if (tc == nullptr || tc->last.topk == 0) {
+        if (tc == nullptr || tc->last.groups == 0) {
             NOVA_ERR(fn, "A solver of the batch has no prepared tensor-core launch.");
             return NOVA_ERROR_INVALID_DATA;
         }
         const TcState::Launch &L = tc->last;
-        if (L.topk != 8u && L.topk != 16u && L.topk != 32u) {
-            NOVA_ERR(fn, "Unsupported candidate-list length for a batched launch.");
-            return NOVA_ERROR_INVALID_DATA;
-        }
         size_t gi = 0;
-        while (gi < b->groups.size() && (b->groups[gi].topk != L.topk || b->groups[gi].fp16 != L.fp16)) gi++;
+        while (gi < b->groups.size() && b->groups[gi].fp16 != L.fp16) gi++;
         if (gi == b->groups.size()) {
             b->groups.emplace_back();
-            b->groups.back().topk = L.topk;
             b->groups.back().fp16 = L.fp16;
             host.emplace_back();
         }
@@ -1533,7 +1497,7 @@ int tc_batch_create(BackupEngine *const *engs, unsigned count, TcBatch **out, co
         m.kBlocks = (unsigned)(tc->nPad / BK);
         m.kSplit = L.kSplit;
         m.a1 = tc->a1; m.d1 = tc->d1; m.scal = tc->scal;
-        m.candV = tc->candV; m.candU = tc->candU; m.candX = tc->candX;
+        m.cand = tc->cand;
         const unsigned long long units = (unsigned long long)m.MZ * m.mTiles * m.groups;
         if ((unsigned long long)g.totalUnits + units >= (1ull << 31)) {
             NOVA_ERR(fn, "Too many work units for one batched launch.");
@@ -1563,9 +1527,7 @@ int tc_batch_gemm(TcBatch *b, cudaStream_t stream, const char *fn) {
         const unsigned grid = std::min<unsigned>(g.totalUnits, (unsigned)b->numSMs);
         CUtensorMap unused;
         memset(&unused, 0, sizeof(unused));
-        auto kern = g.topk == 32u ? tc_score_gemm_kernel<32, BatchUnits>
-                    : (g.topk == 16u ? tc_score_gemm_kernel<16, BatchUnits> : tc_score_gemm_kernel<8, BatchUnits>);
-        kern<<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(unused, unused, make_idesc(g.fp16 ? 0u : 1u), units);
+        tc_score_gemm_kernel<BatchUnits><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(unused, unused, make_idesc(g.fp16 ? 0u : 1u), units);
         int rc = check_launch(fn, "batched tensor-core scoring");
         if (rc != NOVA_SUCCESS) return rc;
     }

@@ -287,3 +287,19 @@ def test_exact_scan(n, r, rz, m, z, distinct):
     G, pi, stats, Go, po = backups(md, npp.SCORING_EXACT, 2)
     np.testing.assert_array_equal(bits(G), bits(Go))
     np.testing.assert_array_equal(pi, po)
+
+
+@pytest.mark.parametrize("mode", [npp.SCORING_FP16, npp.SCORING_BF16])
+@pytest.mark.parametrize("step,order", [(0.1, "rising"), (2e-3, "rising"), (2e-3, "falling"), (0.1, "shuffled")])
+def test_candidate_lists(step, order, mode):
+    """Lists that fill with scores the rising best leaves behind and are
+    trimmed (every 32 alphas hold a new best, alone or with near ones), lists
+    that run out of room, and lists whose first entry stays the best."""
+    r = 8300
+    md = synth.random_pomdp(n=16, m=1, z=1, ns=3, r=r, rz=2, gamma=0.9, horizon=1, seed=5)
+    rng = np.random.default_rng(7)
+    rank = {"rising": np.arange(r), "falling": np.arange(r)[::-1], "shuffled": rng.permutation(r)}[order]
+    md["GammaInitial"] = (step * rank[:, None] + step * rng.uniform(size=(r, 16))).astype(np.float32)
+    G, pi, stats, Go, po = backups(md, mode, 1)
+    np.testing.assert_array_equal(bits(G), bits(Go))
+    np.testing.assert_array_equal(pi, po)

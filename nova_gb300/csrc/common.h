@@ -31,6 +31,14 @@ int dev_free(void *p, const char *fn, const char *what);
 int h2d(void *dst, const void *src, size_t bytes, const char *fn, const char *what);
 int d2h(void *dst, const void *src, size_t bytes, const char *fn, const char *what);
 int check_launch(const char *fn, const char *what);  // call once after every kernel launch
+// Lets a kernel be launched with that much dynamic shared memory. The limit
+// belongs to the kernel, not to a launch or thread: it is only ever raised,
+// so that no thread takes it below what another is about to launch with.
+bool allow_dynamic_smem(const void *kernel, size_t bytes);
+template <typename... Args>
+bool allow_dynamic_smem(void (*kernel)(Args...), size_t bytes) {
+    return allow_dynamic_smem(reinterpret_cast<const void *>(kernel), bytes);
+}
 unsigned long long launch_count();
 void add_launches(long long delta);  // kernels run by a graph replay (negative: captured, not run)
 int sync_device(const char *fn);

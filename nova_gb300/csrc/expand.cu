@@ -705,11 +705,11 @@ int build_workspace(const POMDP *p, ExpWorkspace &ws, const char *fn) {
         return NOVA_ERROR_INVALID_DATA;
     }
     if (ws.smem > 40 * 1024) {
-        cudaFuncSetAttribute(distinct_mass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws.smem);
-        cudaFuncSetAttribute(distinct_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws.smem);
-        cudaFuncSetAttribute(random_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws.smem);
-        cudaFuncSetAttribute(pema_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws.smem);
-        cudaFuncSetAttribute(update_one_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws.smem);
+        allow_dynamic_smem(distinct_mass_kernel, ws.smem);
+        allow_dynamic_smem(distinct_select_kernel, ws.smem);
+        allow_dynamic_smem(random_kernel, ws.smem);
+        allow_dynamic_smem(pema_kernel, ws.smem);
+        allow_dynamic_smem(update_one_kernel, ws.smem);
     }
     return NOVA_SUCCESS;
 }
@@ -842,7 +842,7 @@ int run_distinct(const ExpWorkspace &ws, std::vector<float> &Bnew, const char *f
     auto bound = wide ? distinct_bound_kernel<64, true> : shared ? distinct_bound_kernel<32, true>
                                                                  : distinct_bound_kernel<32, false>;
     if (boundSmem > 48 * 1024 &&
-            cudaFuncSetAttribute(bound, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)boundSmem) != cudaSuccess) {
+            !allow_dynamic_smem(bound, boundSmem)) {
         cudaGetLastError();
         NOVA_ERR(fn, "Failed to configure the distance kernel.");
         return NOVA_ERROR_KERNEL_EXECUTION;

@@ -190,7 +190,7 @@ int vi_resident_sweeps(const MDP *mdp, const int *S, const float *T, const float
     const unsigned threads = (unsigned)std::min<unsigned long long>(kMaxThreads, std::max<unsigned long long>(128, pitch));
     const void *kernel = shared ? (const void *)vi_resident_kernel<true> : (const void *)vi_resident_kernel<false>;
     if (smem > 48 * 1024 &&
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+            !allow_dynamic_smem(kernel, smem)) {
         cudaGetLastError();
         return NOVA_SUCCESS;
     }

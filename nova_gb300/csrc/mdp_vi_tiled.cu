@@ -952,8 +952,7 @@ int vi_plan_build(ViTilePlan *plan, const MDP *mdp, const int *S, const float *T
     const unsigned blocks = ceil_div(n, Sb);
     const size_t smemBytes = round_up((size_t)kStages * Vt * 4 + (size_t)Sb * m * 4, 16) + kBarrierBytes;
 
-    if (cudaFuncSetAttribute(bellman_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemBytes) !=
-            cudaSuccess) {
+    if (!allow_dynamic_smem(bellman_tiled_kernel, smemBytes)) {
         cudaGetLastError();
         return NOVA_SUCCESS;
     }
@@ -1011,8 +1010,7 @@ int vi_plan_build(ViTilePlan *plan, const MDP *mdp, const int *S, const float *T
     const bool vec = ns % 4u == 0u && (uintptr_t)S % 16u == 0u;
     auto countKernel = vec ? vi_plan_count_kernel<true> : vi_plan_count_kernel<false>;
     auto fillKernel = vec ? vi_plan_fill_kernel<true> : vi_plan_fill_kernel<false>;
-    if (fillBytes > 48 * 1024)
-        cudaFuncSetAttribute(fillKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fillBytes);
+    allow_dynamic_smem(fillKernel, fillBytes);
     const unsigned ctas = blocks * kRowWarps;
     countKernel<<<ctas, kPlanThreads, (size_t)perPass * L * 4, stream>>>(g, S, perPass, plan->levelCnt, sliceSize);
     rc = check_launch(fn, "sweep plan (count)");

@@ -1118,7 +1118,7 @@ template <int ZC>
 static void launch_exact(BackupEngine &e, const unsigned *items, unsigned nItems, unsigned nU, unsigned splits,
                          unsigned splitLen, unsigned grid) {
     const size_t smem = (size_t)e.md.ns * ZC * sizeof(float) + (size_t)e.md.ns * sizeof(int);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(exact_score_kernel<ZC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_dynamic_smem(exact_score_kernel<ZC>, smem);
     exact_score_kernel<ZC><<<dim3(grid, splits), 128, smem, e.stream>>>(e.md, e.succLen, e.suppLen, e.C1, e.Gt,
             e.gtCols, nU, items, nItems, splits, splitLen, e.partV, e.partU);
 }
@@ -1312,7 +1312,7 @@ int BackupEngine::scan_all(unsigned nU, const char *fn) {
     }
     auto kernel = uc == 64 ? scan_all_kernel<64> : uc == 32 ? scan_all_kernel<32> : uc == 16 ? scan_all_kernel<16>
                   : uc == 8 ? scan_all_kernel<8> : scan_all_kernel<4>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_dynamic_smem(kernel, smem);
     kernel<<<dim3(tiles, ceil_div(md.r, share)), threads, smem, stream>>>(md, suppLen, proj_view(), nU, chunks, share,
                                                                         scanKeys, 1.0f);
     if ((rc = check_launch(fn, "exact scan")) != NOVA_SUCCESS) return rc;

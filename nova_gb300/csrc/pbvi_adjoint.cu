@@ -421,8 +421,7 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
         return NOVA_ERROR_INVALID_DATA;
     }
     if (stepSmem > 48 * 1024 &&
-            cudaFuncSetAttribute(adjoint_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stepSmem) !=
-                cudaSuccess) {
+            !allow_dynamic_smem(adjoint_step_kernel, stepSmem)) {
         cudaGetLastError();
         NOVA_ERR(fn, "Failed to configure the reverse step kernel.");
         return NOVA_ERROR_KERNEL_EXECUTION;
@@ -461,8 +460,7 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
     const size_t rowsSmem = 2 * (size_t)kGroup * round_up(n, 4) * sizeof(float);
     const bool rowsShared = rowsSmem + 1024 <= (size_t)optin;
     if (rowsShared && rowsSmem > 48 * 1024 &&
-            cudaFuncSetAttribute(replay_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rowsSmem) !=
-                cudaSuccess) {
+            !allow_dynamic_smem(replay_kernel<true>, rowsSmem)) {
         cudaGetLastError();
         NOVA_ERR(fn, "Failed to configure the replay kernel.");
         return NOVA_ERROR_KERNEL_EXECUTION;

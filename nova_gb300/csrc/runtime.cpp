@@ -9,6 +9,7 @@
 
 #include <cmath>
 #include <atomic>
+#include <mutex>
 
 #include <nova/constants.h>
 #include <nova/pomdp/pomdp.h>
@@ -96,6 +97,18 @@ static std::atomic<unsigned long long> g_launches{0};
 unsigned long long launch_count() { return g_launches.load(); }
 
 void add_launches(long long delta) { g_launches.fetch_add((unsigned long long)delta); }
+
+bool allow_dynamic_smem(const void *kernel, size_t bytes) {
+    static std::mutex mutex;
+    if (bytes <= 48 * 1024) return true;
+    std::lock_guard<std::mutex> lock(mutex);
+    cudaFuncAttributes now;
+    if (cudaFuncGetAttributes(&now, kernel) == cudaSuccess && now.maxDynamicSharedSizeBytes >= (int)bytes) return true;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
+        return true;
+    cudaGetLastError();
+    return false;
+}
 
 int check_launch(const char *fn, const char *what) {
     g_launches.fetch_add(1);

@@ -371,7 +371,7 @@ static int value_batched(const float *dG, const unsigned *dPi, unsigned r, unsig
         const unsigned share = (unsigned)round_up(ceil_div(count, shares), 2 * TB);
         auto kernel = staged ? (H == 2 ? value_sparse_kernel<2, true> : value_sparse_kernel<1, true>)
                              : (H == 2 ? value_sparse_kernel<2, false> : value_sparse_kernel<1, false>);
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_dynamic_smem(kernel, smem);
         kernel<<<dim3(aTiles, ceil_div(count, share)), threads, smem>>>(dG, r, n, dB, count, share, cap, count, list,
                                                                          nnz, keys, 1.0f);
         rc = check_launch(fn, "belief values");

@@ -303,3 +303,32 @@ def test_candidate_lists(step, order, mode):
     G, pi, stats, Go, po = backups(md, mode, 1)
     np.testing.assert_array_equal(bits(G), bits(Go))
     np.testing.assert_array_equal(pi, po)
+
+
+@pytest.mark.parametrize("n,r,rz", [(2050, 2049, 17), (4200, 1001, 33)])
+def test_merge_in_order(n, r, rz):
+    """Projection slabs large enough for rows to be merged in their own order
+    (odd row counts, supports past half a warp and past a warp)."""
+    md = synth.random_pomdp(n=n, m=1, z=3, ns=4, r=r, rz=rz, gamma=0.9, horizon=1, seed=n)
+    rng = np.random.default_rng(r)
+    md["GammaInitial"] = (rng.normal(-3.0, 1.0, size=(1, n)) + 1e-2 * rng.normal(size=(r, n))).astype(np.float32)
+    G, pi, stats, Go, po = backups(md, npp.SCORING_FP16, 1)
+    assert stats[-1]["rowsMultiCand"] > 0
+    np.testing.assert_array_equal(bits(G), bits(Go))
+    np.testing.assert_array_equal(pi, po)
+
+
+def test_shared_memory_limits_across_threads():
+    """Solvers on several threads launch the same kernels with different
+    amounts of shared memory: none takes the limit from under another."""
+    from nova_gb300.pomdp_pbvi import solve_batched
+    models = [synth.random_pomdp(n=n, m=2, z=2, ns=3, r=40, rz=min(n, 9), gamma=0.9, horizon=40, seed=n)
+              for n in (700, 820, 640, 900, 760, 850, 670, 880, 720, 810, 650, 910, 770, 840, 680, 890)]
+    ps = [POMDP.from_arrays(md) for md in models]
+    for p in ps:
+        p.initialize_gpu()
+    alone = [POMDPPBVIGPU(p).solve() for p in ps]
+    for _ in range(4):
+        for got, want in zip(solve_batched(ps, scoring=npp.SCORING_EXACT), alone):
+            np.testing.assert_array_equal(bits(got.gamma_array()), bits(want.gamma_array()))
+            np.testing.assert_array_equal(got.pi_array(), want.pi_array())

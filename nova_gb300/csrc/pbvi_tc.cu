@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) tc_score_gemm_kernel(
 #pragma unroll
                     for (int q = 0; q < 4; q++) m8[q] = max8(v + 8 * q);
                     const float mx = max3(max3(m8[0], m8[1], m8[2]), m8[3], m8[3]);
-                    if (mx >= lim) {
+                    if (mx >= lim && real) {
                         // The chunk's maximum raises the running best first,
                         // so only its scores within thr of the new best are
                         // listed.
@@ -831,36 +831,113 @@ struct DirectScorer {
     }
 };
 
-// One warp per row; returns (in every lane) the number of candidates it
-// re-scored exactly, 0 when the row was settled without re-scoring or sent to
-// the exact scan (*flagged). Slot e of the warp's view is slot e / nLists of
-// list e % nLists, so the lists' headers (slot 0) come first, in lanes
-// 0 .. nLists - 1; NE slots per lane are loaded before the lists' lengths are
-// known, what is beyond them (rare: lists of more than 7 entries, 15 of two)
-// after that.
-//
-// Bound by the latency of dependent loads (lists, then the candidates' table
-// entries), so what a row needs before its candidates are known is loaded at
-// once, the candidates are scored together (each lane gathers one support
-// state's entry of up to kMergeBatch candidates before any is used, and lane
-// t adds candidate t's products in support order from shared memory), and
-// few entries are held per lane, which lets 40 warps share an SM: n = 512 (131,072 rows, 1.4 candidates each) 204 to 90 us,
-// n = 4,096 (2.1 M rows, 6.2 each) 6.2 to 5.3 ms, the latter near the DRAM
-// time of its 32-byte sectors.
-constexpr unsigned kMergeBatch = 8;    // candidates gathered together
+// The merge, in two launches. Most rows have one candidate, which a thread
+// can see: one thread per row looks through the row's lists (their header and
+// first three entries are one sector) and settles it, or queues it. The queued
+// rows are re-scored by half a warp each: half warps fit rows of two to four
+// candidates and 16 to 32 support states, of which each lane gathers two
+// states' entries of up to kMergeBatch candidates before any is used; lane t
+// then adds candidate t's products in support order from shared memory. Every
+// block draws its rows from the queue, so both kinds spread over the device
+// whatever their share.
+// Bound by the table's random 32-byte sectors where rows have many candidates
+// (n = 700: 12 candidates of 40 states, 1.3 GB of sectors, at 6 TB/s) and by
+// latency and instructions elsewhere. With one warp per row from the lists to
+// the argmax against this, looking and re-scoring: n = 150 (400,000 rows, 1.4
+// candidates re-scored each) 285 and 145 us, n = 200 (512,000) 350 and 167,
+// n = 512 (131,072) 103 and 75, n = 700 (84,000, 12 each) 239 and 210.
+// The queue is in no order (the looking blocks append to it as they run). Where
+// the table's slab of one (action, observation) is a good part of L2, rows are
+// instead taken in their own order, a block per 16 rows as the device gets to
+// them, so that the rows in flight share one slab or two: n = 4,096 with 4,096
+// alphas (64 MB) 12.7 ms from the queue, 12.0 in order but dealt to resident
+// blocks (which drift apart), 4.6 so (5.8 with a warp per row). n = 1,500 with
+// 3,500 (21 MB): updates of 12.29 and 12.22 ms; n = 2,000 with 800 (6 MB): 245
+// and 253 us of scoring; n = 512 with 1,024 (2 MB) 177 and 198.
+constexpr size_t kMergeOrderedSlab = 16u << 20;
+// Few rows (up to two rounds of resident blocks) are settled in one launch, 16
+// of them looked at and re-scored per block: n = 64 (8,192 rows) 41 and 37 us
+// of scoring with two launches and one; at four rounds n = 300 (37,800) 68 and
+// 76 us, n = 100 (32,000) 93 and 99.
+constexpr unsigned kMergeWholeRounds = 2;
+constexpr unsigned kMergeBlocks = 4;   // resident blocks per SM (64 registers a thread)
+constexpr unsigned kMergeBatch = 4;    // candidates gathered together
 constexpr unsigned kMergePitch = 33;   // shared-memory row of one candidate's products
 
-template <bool kDirect, int NE>
+// A row's flag: kRowExact is what the compaction lists (0 and 1 once merged).
+enum RowOutcome : unsigned { kRowSettled, kRowExact, kRowSeveral };
+
+// Looks through one row's lists (per thread): the row is left to the exact
+// scan, settled by its only candidate, or has several (from *cutOut on).
+__device__ __forceinline__ RowOutcome merge_look(unsigned row, const DevModel &md,
+                                                 const unsigned *__restrict__ uniqJ, unsigned nLists, size_t rPad,
+                                                 const float *__restrict__ a1, const float *__restrict__ d1,
+                                                 const float *__restrict__ a1raw,
+                                                 const unsigned *__restrict__ scal,
+                                                 const uint2 *__restrict__ cand,
+                                                 const unsigned *__restrict__ badModel,
+                                                 unsigned *__restrict__ ustar, unsigned *__restrict__ jstar,
+                                                 unsigned *__restrict__ rowFlag, unsigned *__restrict__ rowCand,
+                                                 float *cutOut) {
+    const unsigned ao = row / md.r, i = row % md.r;
+    const uint4 *lists = reinterpret_cast<const uint4 *>(cand + (size_t)row * (MAX_LISTS * LIST_SLOTS));
+    const float thr = row_margin(a1, d1, (size_t)ao * rPad + i, __uint_as_float(scal[2]), __uint_as_float(scal[7]));
+    const float rawBound = a1raw[(size_t)ao * rPad + i] * __uint_as_float(scal[1]);
+    float best = -INFINITY, second = -INFINITY, x = -INFINITY;
+    unsigned bestU = kNoneU;
+    auto take = [&](unsigned score, unsigned u) {
+        const float f = __uint_as_float(score);
+        second = fmaxf(second, fminf(best, f));
+        if (f > best) { best = f; bestU = u; }
+    };
+#pragma unroll 2
+    for (unsigned q = 0; q < nLists; q++) {
+        // The header and three entries are one sector.
+        const uint4 *l = lists + (size_t)q * (LIST_SLOTS / 2);
+        const uint4 w0 = __ldg(l), w1 = __ldg(l + 1);
+        const unsigned len = min(w0.y, LIST_CAP);
+        x = fmaxf(x, __uint_as_float(w0.x));
+        if (len >= 1u) take(w0.z, w0.w);
+        if (len >= 2u) take(w1.x, w1.y);
+        if (len >= 3u) take(w1.z, w1.w);
+        for (unsigned k = 4; k <= len; k += 4) {
+            const uint4 w2 = __ldg(l + k / 2), w3 = __ldg(l + k / 2 + 1);
+            take(w2.x, w2.y);
+            if (k + 1u <= len) take(w2.z, w2.w);
+            if (k + 2u <= len) take(w3.x, w3.y);
+            if (k + 3u <= len) take(w3.z, w3.w);
+        }
+    }
+    // Usable only with lists that the GEMM has finished, a finite margin,
+    // non-negative probabilities, and scores far from the reference's -1e10
+    // sentinel.
+    const bool usable = (thr < 1e30f) && (best > -INFINITY) && *badModel == 0u && (rawBound < 1e9f) &&
+                        g_device_error == 0u;
+    const float cut = best - thr;
+    const RowOutcome res = !usable || x >= cut ? kRowExact : second >= cut ? kRowSeveral : kRowSettled;
+    rowFlag[row] = res;
+    rowCand[row] = 0u;
+    if (res == kRowSettled) {
+        const size_t js = ((size_t)i * md.m + ao / md.z) * md.z + ao % md.z;
+        ustar[js] = bestU;
+        jstar[js] = uniqJ[bestU];
+    }
+    *cutOut = cut;
+    return res;
+}
+
+// One warp re-scores a row's candidates (listed scores at or above the cut);
+// returns (in every lane) how many there are. Slot e of the warp's view is
+// slot e / nLists of list e % nLists, so the lists' headers (slot 0) come
+// first, in lanes 0 .. nLists - 1; NE slots per lane are loaded before the
+// lists' lengths are known, what lies beyond (rare: lists of more than 7
+// entries, 15 of two) after that.
+template <int NE>
 __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const DevModel &md,
-                                              const unsigned *__restrict__ suppLen, const ProjView &pv,
-                                              const DirectScorer &ds, float *scratch, unsigned *list,
+                                              const unsigned *__restrict__ suppLen, const DirectScorer &ds, float *scratch, unsigned *list,
                                               const unsigned *__restrict__ uniqJ, unsigned nLists,
-                                              size_t rPad, const float *__restrict__ a1,
-                                              const float *__restrict__ d1,
-                                              const float *__restrict__ a1raw, const unsigned *__restrict__ scal,
                                               const uint2 *__restrict__ cand, unsigned *__restrict__ ustar,
-                                              unsigned *__restrict__ jstar, bool *flagged,
-                                              const unsigned *__restrict__ badModel) {
+                                              unsigned *__restrict__ jstar, bool *flagged) {
     const unsigned ao = row / md.r, i = row % md.r;
     const unsigned a = ao / md.z, o = ao % md.z;
     const uint2 *lists = cand + (size_t)row * (MAX_LISTS * LIST_SLOTS);
@@ -872,73 +949,31 @@ __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const
         const unsigned e = lane + 32u * j;
         ent[j] = e < nEnt ? __ldg(slot_of(e)) : make_uint2(0u, 0u);
     }
-    const float thr = row_margin(a1, d1, (size_t)ao * rPad + i, __uint_as_float(scal[2]), __uint_as_float(scal[7]));
-    const float rawBound = a1raw[(size_t)ao * rPad + i] * __uint_as_float(scal[1]);
     const unsigned Li = suppLen[i];
     const int *sk = md.Z + (size_t)i * md.rz;
     const float *bk = md.B + (size_t)i * md.rz;
-    const unsigned s0 = lane < Li ? (unsigned)__ldg(sk + lane) : 0u;
-    const float b0 = lane < Li ? __ldg(bk + lane) : 0.0f;
-    // Lane l < nLists holds list l's header.
+    // Lane l < nLists holds list l's header; list 0's has the cut.
+    const float cut = __uint_as_float(__shfl_sync(0xffffffffu, ent[0].x, 0));
     const unsigned held = lane < nLists ? min(ent[0].y, LIST_CAP) : 0u;
-    float x = lane < nLists ? __uint_as_float(ent[0].x) : -INFINITY;
     const unsigned steps = (__reduce_max_sync(0xffffffffu, held) + 1u) * nLists;  // e beyond these is in no list
-    // The score of the warp's entry e (-inf where e's list is shorter).
-    auto score_of = [&](unsigned e, uint2 en) {
-        const unsigned len = __shfl_sync(0xffffffffu, held, e % nLists), k = e / nLists;
-        return k != 0u && k <= len ? __uint_as_float(en.x) : -INFINITY;
-    };
-    float v[NE];
-    float tmax = -INFINITY;
-#pragma unroll
-    for (int j = 0; j < NE; j++) {
-        v[j] = score_of(lane + 32u * j, ent[j]);
-        tmax = fmaxf(tmax, v[j]);
-    }
-    for (unsigned e0 = 32u * NE; e0 < steps; e0 += 32u) {
-        const unsigned e = e0 + lane;
-        tmax = fmaxf(tmax, score_of(e, e < nEnt ? __ldg(slot_of(e)) : make_uint2(0u, 0u)));
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-        tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, off));
-        x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, off));
-    }
-    // Usable only with lists that the GEMM has finished, a finite margin,
-    // non-negative probabilities, and scores far from the reference's -1e10
-    // sentinel.
-    const bool usable = (thr < 1e30f) && (tmax > -INFINITY) && *badModel == 0u && (rawBound < 1e9f) &&
-                        g_device_error == 0u;
-    const float cut = tmax - thr;
-    if (!usable || x >= cut) {
-        *flagged = true;
-        return 0u;
-    }
     // The candidates, listed in shared memory.
     unsigned count = 0;
-    auto keep = [&](float score, unsigned u) {
-        const bool c = score >= cut;
+    auto keep = [&](unsigned e, uint2 en) {
+        const unsigned len = __shfl_sync(0xffffffffu, held, e % nLists), k = e / nLists;
+        const bool c = k != 0u && k <= len && __uint_as_float(en.x) >= cut;
         const unsigned msk = __ballot_sync(0xffffffffu, c);
-        if (c) list[count + __popc(msk & ((1u << lane) - 1u))] = u;
+        if (c) list[count + __popc(msk & ((1u << lane) - 1u))] = en.y;
         count += __popc(msk);
     };
 #pragma unroll
-    for (int j = 0; j < NE; j++) keep(v[j], ent[j].y);
+    for (int j = 0; j < NE; j++) keep(lane + 32u * j, ent[j]);
     for (unsigned e0 = 32u * NE; e0 < steps; e0 += 32u) {
         const unsigned e = e0 + lane;
-        const uint2 en = e < nEnt ? __ldg(slot_of(e)) : make_uint2(0u, 0u);
-        keep(score_of(e, en), en.y);
+        keep(e, e < nEnt ? __ldg(slot_of(e)) : make_uint2(0u, 0u));
     }
     __syncwarp();
     const size_t js = ((size_t)i * md.m + a) * md.z + o;
-    if (count == 1) {
-        if (lane == 0) {
-            const unsigned uu = list[0];
-            ustar[js] = uu;
-            jstar[js] = uniqJ[uu];
-        }
-        return 0u;
-    }
-    // Several candidates: re-scored in the exact order, up to 32 at a time
+    // Re-scored in the exact order, up to 32 at a time
     // (candidate t of the batch in lane t).
     float best = -INFINITY;
     unsigned bu = kNoneU;
@@ -947,104 +982,72 @@ __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const
         if (lane < nb && (bu == kNoneU || total > best || (total == best && myU < bu))) { best = total; bu = myU; }
     };
     auto score_batch = [&]() {
-        if constexpr (!kDirect) {
-            const float *P = pv.slab(ao);
-            float total = 0.0f;
-            for (unsigned t0 = 0; t0 < nb; t0 += kMergeBatch) {
-                const unsigned nt = min(kMergeBatch, nb - t0);
-                for (unsigned k0 = 0; k0 < Li; k0 += 32u) {
-                    const unsigned k = k0 + lane;
-                    const bool kv = k < Li;
-                    const unsigned s = k0 == 0 ? s0 : (kv ? (unsigned)__ldg(sk + k) : 0u);
-                    const float b = k0 == 0 ? b0 : (kv ? __ldg(bk + k) : 0.0f);
-                    float pq[kMergeBatch];
+        // The gathers of one candidate stay within one alpha row: lane k
+        // computes support state k's term of every candidate of the
+        // batch into the warp's scratch, then lane t adds candidate t's
+        // terms in support order.
+        float total = 0.0f;
+        for (unsigned k0 = 0; k0 < Li; k0 += 32u) {
+            const unsigned k = k0 + lane;
+            const bool kv = k < Li;
+            const unsigned s = kv ? (unsigned)sk[k] : 0u;
+            const float b = kv ? bk[k] : 0.0f;
+            if (md.ns <= kDirectNs) {
+                // The state's coefficients and successors, loaded once for
+                // the whole batch.
+                const unsigned Ls = kv ? __ldg(ds.succLen + (size_t)s * md.m + a) : 0u;
+                const float *cp = ds.C3 + (((size_t)a * md.z + o) * md.n + s) * md.ns;
+                const int *spp = md.S + ((size_t)s * md.m + a) * md.ns;
+                float cc[kDirectNs];
+                int ss[kDirectNs];
 #pragma unroll
-                    for (unsigned t = 0; t < kMergeBatch; t++) {
-                        const unsigned uu = __shfl_sync(0xffffffffu, myU, t0 + t);
-                        pq[t] = t < nt && kv ? __ldg(P + pv.at(s, uu)) : 0.0f;
-                    }
-#pragma unroll
-                    for (unsigned t = 0; t < kMergeBatch; t++)
-                        if (t < nt) scratch[t * kMergePitch + lane] = fmul(pq[t], b);
-                    __syncwarp();
-                    if (lane >= t0 && lane < t0 + nt) {
-                        const float *mine = scratch + (lane - t0) * kMergePitch;
-                        const unsigned cnt = min(32u, Li - k0);
-#pragma unroll 8
-                        for (unsigned q = 0; q < cnt; q++) total = fadd(total, mine[q]);
-                    }
-                    __syncwarp();
+                for (unsigned l = 0; l < kDirectNs; l++) {
+                    cc[l] = l < Ls ? __ldg(cp + l) : 0.0f;
+                    ss[l] = l < Ls ? __ldg(spp + l) : 0;
                 }
-            }
-            settle(total);
-        } else {
-            // The gathers of one candidate stay within one alpha row: lane k
-            // computes support state k's term of every candidate of the
-            // batch into the warp's scratch, then lane t adds candidate t's
-            // terms in support order.
-            float total = 0.0f;
-            for (unsigned k0 = 0; k0 < Li; k0 += 32u) {
-                const unsigned k = k0 + lane;
-                const bool kv = k < Li;
-                const unsigned s = kv ? (unsigned)sk[k] : 0u;
-                const float b = kv ? bk[k] : 0.0f;
-                if (md.ns <= kDirectNs) {
-                    // The state's coefficients and successors, loaded once for
-                    // the whole batch.
-                    const unsigned Ls = kv ? __ldg(ds.succLen + (size_t)s * md.m + a) : 0u;
-                    const float *cp = ds.C3 + (((size_t)a * md.z + o) * md.n + s) * md.ns;
-                    const int *spp = md.S + ((size_t)s * md.m + a) * md.ns;
-                    float cc[kDirectNs];
-                    int ss[kDirectNs];
+                // Two candidates at a time: their gathers are issued
+                // together, their sums are two independent chains.
+                for (unsigned t = 0; t < nb; t += 2) {
+                    const unsigned t1 = t + 1 < nb ? t + 1 : t;
+                    const unsigned u0 = __shfl_sync(0xffffffffu, myU, t);
+                    const unsigned u1 = __shfl_sync(0xffffffffu, myU, t1);
+                    const float *G0 = ds.G + (size_t)__ldg(uniqJ + u0) * md.n;
+                    const float *G1 = ds.G + (size_t)__ldg(uniqJ + u1) * md.n;
+                    float g0[kDirectNs], g1[kDirectNs];
 #pragma unroll
                     for (unsigned l = 0; l < kDirectNs; l++) {
-                        cc[l] = l < Ls ? __ldg(cp + l) : 0.0f;
-                        ss[l] = l < Ls ? __ldg(spp + l) : 0;
-                    }
-                    // Two candidates at a time: their gathers are issued
-                    // together, their sums are two independent chains.
-                    for (unsigned t = 0; t < nb; t += 2) {
-                        const unsigned t1 = t + 1 < nb ? t + 1 : t;
-                        const unsigned u0 = __shfl_sync(0xffffffffu, myU, t);
-                        const unsigned u1 = __shfl_sync(0xffffffffu, myU, t1);
-                        const float *G0 = ds.G + (size_t)__ldg(uniqJ + u0) * md.n;
-                        const float *G1 = ds.G + (size_t)__ldg(uniqJ + u1) * md.n;
-                        float g0[kDirectNs], g1[kDirectNs];
-#pragma unroll
-                        for (unsigned l = 0; l < kDirectNs; l++) {
-                            if (l < Ls) {
-                                g0[l] = __ldg(G0 + ss[l]);
-                                g1[l] = __ldg(G1 + ss[l]);
-                            }
+                        if (l < Ls) {
+                            g0[l] = __ldg(G0 + ss[l]);
+                            g1[l] = __ldg(G1 + ss[l]);
                         }
-                        float v0 = 0.0f, v1 = 0.0f;
+                    }
+                    float v0 = 0.0f, v1 = 0.0f;
 #pragma unroll
-                        for (unsigned l = 0; l < kDirectNs; l++) {
-                            if (l < Ls) {
-                                v0 = fadd(v0, fmul(cc[l], g0[l]));
-                                v1 = fadd(v1, fmul(cc[l], g1[l]));
-                            }
+                    for (unsigned l = 0; l < kDirectNs; l++) {
+                        if (l < Ls) {
+                            v0 = fadd(v0, fmul(cc[l], g0[l]));
+                            v1 = fadd(v1, fmul(cc[l], g1[l]));
                         }
-                        scratch[t * 32u + lane] = kv ? fmul(fmul(v0, md.gamma), b) : 0.0f;
-                        if (t1 != t) scratch[t1 * 32u + lane] = kv ? fmul(fmul(v1, md.gamma), b) : 0.0f;
                     }
-                } else {
-                    for (unsigned t = 0; t < nb; t++) {
-                        const unsigned uu = __shfl_sync(0xffffffffu, myU, t);
-                        float p = 0.0f;
-                        if (kv) p = fmul(fmul(ds.vt(md, a, o, s, ds.G + (size_t)__ldg(uniqJ + uu) * md.n), md.gamma), b);
-                        scratch[t * 32u + lane] = p;
-                    }
+                    scratch[t * 32u + lane] = kv ? fmul(fmul(v0, md.gamma), b) : 0.0f;
+                    if (t1 != t) scratch[t1 * 32u + lane] = kv ? fmul(fmul(v1, md.gamma), b) : 0.0f;
                 }
-                __syncwarp();
-                if (lane < nb) {
-                    const unsigned cnt = min(32u, Li - k0);
-                    for (unsigned q = 0; q < cnt; q++) total = fadd(total, scratch[lane * 32u + q]);
+            } else {
+                for (unsigned t = 0; t < nb; t++) {
+                    const unsigned uu = __shfl_sync(0xffffffffu, myU, t);
+                    float p = 0.0f;
+                    if (kv) p = fmul(fmul(ds.vt(md, a, o, s, ds.G + (size_t)__ldg(uniqJ + uu) * md.n), md.gamma), b);
+                    scratch[t * 32u + lane] = p;
                 }
-                __syncwarp();
             }
-            settle(total);
+            __syncwarp();
+            if (lane < nb) {
+                const unsigned cnt = min(32u, Li - k0);
+                for (unsigned q = 0; q < cnt; q++) total = fadd(total, scratch[lane * 32u + q]);
+            }
+            __syncwarp();
         }
+        settle(total);
     };
     for (unsigned f = 0; f < count; f += 32u) {
         nb = min(32u, count - f);
@@ -1065,53 +1068,242 @@ __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const
     return count;
 }
 
-// Rows re-scored and candidates re-scored are counted per block in shared
-// memory, then added to the global counters once per block; rows left to the
-// exact scan are flagged and counted per compaction chunk.
+// First half of the merge: settles the rows that one thread can and queues
+// the others in rowList (their number in counters[0]), each with its cut in
+// place of its first list's dropped score. Rows left to the exact scan are
+// flagged and counted per compaction chunk, which the block lies in.
 constexpr unsigned kCompactChunk = 4096;  // rows per block of the compaction (4 per thread)
+constexpr unsigned kLookRows = 128;       // rows per block
 
-template <bool kDirect, int NE>
-__global__ void __launch_bounds__(256, kDirect ? 1 : 5) tc_merge_kernel(
-                                DevModel md, const unsigned *__restrict__ suppLen,
-                                const ProjView pv, const DirectScorer ds, const unsigned *__restrict__ uniqJ,
-                                unsigned nLists,
-                                size_t rPad, const float *__restrict__ a1, const float *__restrict__ d1,
+__global__ void __launch_bounds__(kLookRows) tc_merge_look_kernel(
+                                DevModel md, const unsigned *__restrict__ uniqJ, unsigned nLists, size_t rPad,
+                                const float *__restrict__ a1, const float *__restrict__ d1,
                                 const float *__restrict__ a1raw, const unsigned *__restrict__ scal,
-                                const uint2 *__restrict__ cand, unsigned *__restrict__ ustar,
-                                unsigned *__restrict__ jstar, unsigned *__restrict__ rowFlag,
-                                unsigned *__restrict__ rowCand, unsigned *__restrict__ counters,
+                                uint2 *cand, unsigned *__restrict__ ustar, unsigned *__restrict__ jstar,
+                                unsigned *__restrict__ rowFlag, unsigned *__restrict__ rowCand,
+                                unsigned *__restrict__ rowList, unsigned *__restrict__ counters,
                                 unsigned *__restrict__ chunkCount, const unsigned *__restrict__ badModel) {
-    __shared__ unsigned blockCount[2];
-    // Direct form: [warps][32 candidates][32 states]; otherwise [warps][kMergeBatch][kMergePitch].
+    const unsigned rows = md.m * md.z * md.r;  // fewer than 2^31 (tc_supported)
+    const unsigned row = blockIdx.x * kLookRows + threadIdx.x, lane = threadIdx.x & 31;
+    RowOutcome res = kRowSettled;
+    if (row < rows) {
+        float cut = 0.0f;
+        res = merge_look(row, md, uniqJ, nLists, rPad, a1, d1, a1raw, scal, cand, badModel, ustar, jstar, rowFlag,
+                         rowCand, &cut);
+        if (res == kRowSeveral) cand[(size_t)row * (MAX_LISTS * LIST_SLOTS)].x = __float_as_uint(cut);
+    }
+    const unsigned msk = __ballot_sync(0xffffffffu, res == kRowSeveral);
+    unsigned at = 0;
+    if (lane == 0 && msk) at = atomicAdd(&counters[0], __popc(msk));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (res == kRowSeveral) rowList[at + __popc(msk & ((1u << lane) - 1u))] = row;
+    const unsigned exact = __popc(__ballot_sync(0xffffffffu, res == kRowExact));
+    if (lane == 0 && exact) atomicAdd(chunkCount + row / kCompactChunk, exact);
+}
+
+// Second half: the rows with several candidates, re-scored from the projection
+// table by half a warp each: queued rows; or all rows in order, of which those
+// flagged kRowSeveral are meant; or all 16 rows of a block, which has not been
+// looked at before (both halves of the merge in one launch). Slot e of a half
+// warp's view is slot e / nLists of list e % nLists; NE slots per lane are
+// loaded before the lists' lengths are known.
+enum class MergeRows { kQueued, kInOrder, kWhole };
+
+template <int NE, MergeRows kRows>
+__global__ void __launch_bounds__(256, kMergeBlocks) tc_merge_kernel(
+                                DevModel md, const unsigned *__restrict__ suppLen,
+                                const ProjView pv, const unsigned *__restrict__ uniqJ,
+                                unsigned nLists, size_t rPad, const float *__restrict__ a1,
+                                const float *__restrict__ d1, const float *__restrict__ a1raw,
+                                const unsigned *__restrict__ scal, const uint2 *__restrict__ cand,
+                                unsigned *__restrict__ ustar, unsigned *__restrict__ jstar,
+                                unsigned *__restrict__ rowFlag, unsigned *__restrict__ rowCand,
+                                const unsigned *__restrict__ rowList, unsigned *__restrict__ counters,
+                                unsigned *__restrict__ chunkCount, const unsigned *__restrict__ badModel) {
+    __shared__ float scratch[8][2][kMergeBatch * kMergePitch];
+    extern __shared__ unsigned mergeLists[];   // [16 halves][nLists * LIST_SLOTS]
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, hl = lane & 15u;
+    unsigned *list = mergeLists + (size_t)(threadIdx.x >> 4) * (nLists * LIST_SLOTS);
+    float *prod = scratch[warp][half];
+    const unsigned nEnt = nLists * LIST_SLOTS;
+    unsigned sum = 0, queued = md.m * md.z * md.r, first = (blockIdx.x * 8u + warp) * 2u;
+    __shared__ unsigned severalRow[16];
+    __shared__ float severalCut[16];
+    if constexpr (kRows == MergeRows::kQueued) queued = counters[0];
+    if constexpr (kRows == MergeRows::kWhole) {
+        if (warp == 0) {
+            const unsigned row = blockIdx.x * 16u + lane;
+            RowOutcome res = kRowSettled;
+            float cut = 0.0f;
+            if (lane < 16u && row < queued)
+                res = merge_look(row, md, uniqJ, nLists, rPad, a1, d1, a1raw, scal, cand, badModel, ustar, jstar,
+                                 rowFlag, rowCand, &cut);
+            const unsigned msk = __ballot_sync(0xffffffffu, res == kRowSeveral);
+            const unsigned exact = __popc(__ballot_sync(0xffffffffu, res == kRowExact));
+            if (res == kRowSeveral) {
+                const unsigned k = __popc(msk & ((1u << lane) - 1u));
+                severalRow[k] = row;
+                severalCut[k] = cut;
+            }
+            if (lane == 0) {
+                const unsigned several = __popc(msk);
+                for (unsigned k = several; k < 16u; k++) severalRow[k] = kNoneU;
+                if (several) atomicAdd(&counters[0], several);
+                if (exact) atomicAdd(chunkCount + row / kCompactChunk, exact);
+            }
+        }
+        __syncthreads();
+        first = warp * 2u;
+        queued = 16u;
+    }
+    for (unsigned k0 = first; k0 < queued; k0 += gridDim.x * 16u) {
+        // With an odd row at the end both halves look at it, one writes.
+        bool mine = k0 + half < queued;
+        unsigned row = mine ? k0 + half : k0;
+        if constexpr (kRows == MergeRows::kInOrder) {
+            mine = mine && rowFlag[row] == kRowSeveral;
+            if (__ballot_sync(0xffffffffu, mine) == 0u) continue;
+            if (!mine) row = k0 + (half ^ 1u);
+        } else if constexpr (kRows == MergeRows::kWhole) {
+            mine = severalRow[k0 + half] != kNoneU;
+            if (severalRow[k0] == kNoneU) break;
+            row = severalRow[mine ? k0 + half : k0];
+        } else {
+            row = __ldg(rowList + row);
+        }
+        const unsigned ao = row / md.r, i = row % md.r;
+        const uint2 *lists = cand + (size_t)row * (MAX_LISTS * LIST_SLOTS);
+        auto slot_of = [&](unsigned e) { return lists + (e % nLists) * LIST_SLOTS + e / nLists; };
+        uint2 ent[NE];
+#pragma unroll
+        for (int j = 0; j < NE; j++) {
+            const unsigned e = hl + 16u * j;
+            ent[j] = e < nEnt ? __ldg(slot_of(e)) : make_uint2(0u, 0u);
+        }
+        const unsigned Li = suppLen[i];
+        const int *sk = md.Z + (size_t)i * md.rz;
+        const float *bk = md.B + (size_t)i * md.rz;
+        unsigned s0 = 0, s1 = 0;
+        float b0 = 0.0f, b1 = 0.0f;
+        if (hl < md.rz) { s0 = (unsigned)__ldg(sk + hl); b0 = __ldg(bk + hl); }
+        if (hl + 16u < md.rz) { s1 = (unsigned)__ldg(sk + hl + 16u); b1 = __ldg(bk + hl + 16u); }
+        // Lane l < nLists of a half holds list l's header; list 0's has the cut.
+        float cut = __uint_as_float(__shfl_sync(0xffffffffu, ent[0].x, 0, 16));
+        if constexpr (kRows == MergeRows::kWhole) cut = severalCut[mine ? k0 + half : k0];
+        const unsigned held = hl < nLists ? min(ent[0].y, LIST_CAP) : 0u;
+        const unsigned steps = (__reduce_max_sync(0xffffffffu, held) + 1u) * nLists;
+        unsigned count = 0;
+        auto keep = [&](unsigned e, uint2 en) {
+            const unsigned len = __shfl_sync(0xffffffffu, held, e % nLists, 16), k = e / nLists;
+            const bool c = k != 0u && k <= len && __uint_as_float(en.x) >= cut;
+            const unsigned msk = (__ballot_sync(0xffffffffu, c) >> (16u * half)) & 0xffffu;
+            if (c) list[count + __popc(msk & ((1u << hl) - 1u))] = en.y;
+            count += __popc(msk);
+        };
+#pragma unroll
+        for (int j = 0; j < NE; j++) keep(hl + 16u * j, ent[j]);
+        for (unsigned e0 = 16u * NE; e0 < steps; e0 += 16u) {
+            const unsigned e = e0 + hl;
+            keep(e, e < nEnt ? __ldg(slot_of(e)) : make_uint2(0u, 0u));
+        }
+        __syncwarp();
+        const float *P = pv.slab(ao);
+        const unsigned most = max(count, __shfl_xor_sync(0xffffffffu, count, 16));
+        const unsigned longest = max(Li, __shfl_xor_sync(0xffffffffu, Li, 16));
+        float best = -INFINITY;
+        unsigned bu = kNoneU;
+        for (unsigned f = 0; f < most; f += kMergeBatch) {
+            const unsigned nt = f < count ? min(kMergeBatch, count - f) : 0u;
+            unsigned uu[kMergeBatch];
+#pragma unroll
+            for (unsigned t = 0; t < kMergeBatch; t++) uu[t] = t < nt ? list[f + t] : 0u;
+            float total = 0.0f;
+            for (unsigned q0 = 0; q0 < longest; q0 += 32u) {
+                if (q0 != 0u || f != 0u) {
+                    const unsigned q = q0 + hl;
+                    if (q < md.rz) { s0 = (unsigned)__ldg(sk + q); b0 = __ldg(bk + q); }
+                    if (q + 16u < md.rz) { s1 = (unsigned)__ldg(sk + q + 16u); b1 = __ldg(bk + q + 16u); }
+                }
+                const bool v0 = q0 + hl < Li, v1 = q0 + 16u + hl < Li;
+                float p0[kMergeBatch], p1[kMergeBatch];
+#pragma unroll
+                for (unsigned t = 0; t < kMergeBatch; t++) {
+                    p0[t] = t < nt && v0 ? __ldg(P + pv.at(s0, uu[t])) : 0.0f;
+                    p1[t] = t < nt && v1 ? __ldg(P + pv.at(s1, uu[t])) : 0.0f;
+                }
+#pragma unroll
+                for (unsigned t = 0; t < kMergeBatch; t++) {
+                    if (t < nt) {
+                        prod[t * kMergePitch + hl] = fmul(p0[t], b0);
+                        prod[t * kMergePitch + hl + 16u] = fmul(p1[t], b1);
+                    }
+                }
+                __syncwarp();
+                if (hl < nt && q0 < Li) {
+                    const float *row0 = prod + hl * kMergePitch;
+                    const unsigned cnt = min(32u, Li - q0);
+#pragma unroll 8
+                    for (unsigned q = 0; q < cnt; q++) total = fadd(total, row0[q]);
+                }
+                __syncwarp();
+            }
+            if (hl < nt) {
+                const unsigned u = list[f + hl];
+                if (bu == kNoneU || total > best || (total == best && u < bu)) { best = total; bu = u; }
+            }
+        }
+#pragma unroll
+        for (int off = kMergeBatch / 2; off > 0; off >>= 1) {
+            const float b2 = __shfl_xor_sync(0xffffffffu, best, off);
+            const unsigned u2 = __shfl_xor_sync(0xffffffffu, bu, off);
+            if (u2 != kNoneU && (bu == kNoneU || b2 > best || (b2 == best && u2 < bu))) { best = b2; bu = u2; }
+        }
+        if (hl == 0 && mine) {
+            const bool exact = !(best > -1e10f);  // sentinel case: the exact scan applies the reference's rule
+            rowCand[row] = count;
+            rowFlag[row] = exact ? 1u : 0u;
+            if (exact) {
+                atomicAdd(chunkCount + row / kCompactChunk, 1u);
+            } else {
+                const size_t js = ((size_t)i * md.m + ao / md.z) * md.z + ao % md.z;
+                ustar[js] = bu;
+                jstar[js] = uniqJ[bu];
+            }
+            sum += count;
+        }
+        __syncwarp();
+    }
+    if (sum) atomicAdd(&counters[1], sum);
+}
+
+// The same without a table: one warp per queued row.
+__global__ void __launch_bounds__(256, 1) tc_merge_direct_kernel(
+                                DevModel md, const unsigned *__restrict__ suppLen,
+                                const DirectScorer ds, const unsigned *__restrict__ uniqJ,
+                                unsigned nLists, const uint2 *__restrict__ cand, unsigned *__restrict__ ustar,
+                                unsigned *__restrict__ jstar, unsigned *__restrict__ rowFlag,
+                                unsigned *__restrict__ rowCand, const unsigned *__restrict__ rowList,
+                                unsigned *__restrict__ counters, unsigned *__restrict__ chunkCount) {
+    // [warps][32 candidates][32 states], then each warp's candidate list.
     extern __shared__ float mergeScratch[];
-    // Then each warp's candidate list.
-    constexpr unsigned kWarpScratch = kDirect ? 1024u : kMergeBatch * kMergePitch;
-    if (threadIdx.x == 0) { blockCount[0] = 0u; blockCount[1] = 0u; }
-    __syncthreads();
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned row = blockIdx.x * 8u + warp;  // fewer than 2^31 rows (tc_supported)
-    if (row < md.m * md.z * md.r) {
+    const unsigned queued = counters[0];
+    unsigned *list = reinterpret_cast<unsigned *>(mergeScratch + 8u * 1024u) + warp * (nLists * LIST_SLOTS);
+    unsigned sum = 0;
+    for (unsigned k = blockIdx.x * 8u + warp; k < queued; k += gridDim.x * 8u) {
+        const unsigned row = __ldg(rowList + k);
         bool flagged = false;
-        unsigned *list = reinterpret_cast<unsigned *>(mergeScratch + 8u * kWarpScratch) + warp * (nLists * LIST_SLOTS);
-        const unsigned rescored =
-            merge_row<kDirect, NE>(row, lane, md, suppLen, pv, ds, mergeScratch + warp * kWarpScratch, list, uniqJ,
-                                   nLists, rPad, a1, d1, a1raw, scal, cand, ustar, jstar,
-                                   &flagged, badModel);
+        const unsigned rescored = merge_row<2>(row, lane, md, suppLen, ds, mergeScratch + warp * 1024u, list, uniqJ,
+                                               nLists, cand, ustar, jstar, &flagged);
         if (lane == 0) {
             rowCand[row] = rescored;
             rowFlag[row] = flagged ? 1u : 0u;
             if (flagged) atomicAdd(chunkCount + row / kCompactChunk, 1u);
-            if (rescored) {
-                atomicAdd(&blockCount[0], 1u);
-                atomicAdd(&blockCount[1], rescored);
-            }
         }
+        sum += rescored;
+        __syncwarp();
     }
-    __syncthreads();
-    if (threadIdx.x == 0 && blockCount[0]) {
-        atomicAdd(&counters[0], blockCount[0]);
-        atomicAdd(&counters[1], blockCount[1]);
-    }
+    if (lane == 0 && sum) atomicAdd(&counters[1], sum);
 }
 
 // Indices of the flagged rows in increasing order, from the flagged rows per
@@ -1392,13 +1584,31 @@ int tc_finish(BackupEngine &eng, const char *fn) {
     const unsigned nChunks = ceil_div(rows, kCompactChunk);
     const DirectScorer ds{eng.succLen, eng.C3, tc->src};
     const bool table = eng.useProjNow;
-    const size_t mergeSmem =
-        8 * ((table ? kMergeBatch * kMergePitch : 1024u) + L.lists * LIST_SLOTS) * sizeof(float);
-    auto merge = !table ? tc_merge_kernel<true, 2> : L.lists <= 2u ? tc_merge_kernel<false, 1> : tc_merge_kernel<false, 2>;
-    merge<<<(unsigned)ceil_div(rows * 32, 256), 256, mergeSmem, eng.stream>>>(
-        md, eng.suppLen, table ? eng.proj_view() : ProjView{}, ds, eng.uniqMap, L.lists, tc->rPad,
-        tc->a1, tc->d1, tc->a1raw, tc->scal, tc->cand, eng.ustar, eng.jstar, tc->rowFlag,
-        tc->rowCand, tc->scal + 3, tc->chunkCount, tc->badModel);
+    const unsigned blocks = (unsigned)ceil_div(rows, 16);
+    const bool whole = table && blocks <= kMergeWholeRounds * kMergeBlocks * (unsigned)tc->numSMs;
+    if (!whole) {
+        tc_merge_look_kernel<<<(unsigned)ceil_div(rows, kLookRows), kLookRows, 0, eng.stream>>>(
+            md, eng.uniqMap, L.lists, tc->rPad, tc->a1, tc->d1, tc->a1raw, tc->scal, tc->cand, eng.ustar, eng.jstar,
+            tc->rowFlag, tc->rowCand, tc->rowList, tc->scal + 3, tc->chunkCount, tc->badModel);
+        if ((rc = check_launch(fn, "candidate lists")) != NOVA_SUCCESS) return rc;
+    }
+    if (table) {
+        const bool inOrder = eng.proj_view().slice * sizeof(float) >= kMergeOrderedSlab;
+        const bool two = L.lists <= 2u;
+        auto merge = whole     ? (two ? tc_merge_kernel<2, MergeRows::kWhole> : tc_merge_kernel<4, MergeRows::kWhole>)
+                     : inOrder ? (two ? tc_merge_kernel<2, MergeRows::kInOrder> : tc_merge_kernel<4, MergeRows::kInOrder>)
+                               : (two ? tc_merge_kernel<2, MergeRows::kQueued> : tc_merge_kernel<4, MergeRows::kQueued>);
+        const unsigned grid = whole || inOrder ? blocks : std::min(blocks, kMergeBlocks * (unsigned)tc->numSMs);
+        merge<<<grid, 256, 16 * L.lists * LIST_SLOTS * sizeof(unsigned), eng.stream>>>(
+            md, eng.suppLen, eng.proj_view(), eng.uniqMap, L.lists, tc->rPad, tc->a1, tc->d1, tc->a1raw, tc->scal,
+            tc->cand, eng.ustar, eng.jstar, tc->rowFlag, tc->rowCand, tc->rowList, tc->scal + 3, tc->chunkCount,
+            tc->badModel);
+    } else {
+        const unsigned grid = std::min((unsigned)ceil_div(rows, 8), (unsigned)tc->numSMs);
+        tc_merge_direct_kernel<<<grid, 256, 8 * (1024u + L.lists * LIST_SLOTS) * sizeof(float), eng.stream>>>(
+            md, eng.suppLen, ds, eng.uniqMap, L.lists, tc->cand, eng.ustar, eng.jstar, tc->rowFlag, tc->rowCand,
+            tc->rowList, tc->scal + 3, tc->chunkCount);
+    }
     if ((rc = check_launch(fn, "candidate merge")) != NOVA_SUCCESS) return rc;
     tc_compact_write_kernel<<<nChunks, 1024, 0, eng.stream>>>(tc->rowFlag, (unsigned)rows, tc->chunkCount,
                                                               tc->rowList, eng.itemCount, tc->scal);

@@ -625,32 +625,33 @@ constexpr size_t kProjSmemMax = 200 * 1024;
 // registers. Successor lists are staged successor-major ([l][8 states]), so
 // the 8 states' l-th successors sit in 8 banks, and each lane's vector
 // gathers of the transposed alphas run two successors ahead of the
-// arithmetic. Bound by FP32 issue (f32x2: 38 T operations/s measured) and by
-// the load/store unit's wavefronts (at z = 24 both over 50 % busy): one
-// vector gather per lane, guard-free stores for whole tiles and about eight
-// rounds of blocks took n = 512 (z = 16, r = 1,024) from 192 to 136 us, n =
-// 1,000 (z = 11, r = 1,500) from 332 to 188 us and n = 4,096 (z = 32, m = 16,
-// r = 4,096) from 29.6 to 23.2 ms.
-template <int UPL>
-__device__ __forceinline__ void load_alphas(const float *__restrict__ p, float (&g)[UPL]) {
-    if constexpr (UPL == 4) {
-        const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
-        g[0] = v.x; g[1] = v.y; g[2] = v.z; g[3] = v.w;
-    } else {
-        const float2 v = __ldg(reinterpret_cast<const float2 *>(p));
-        g[0] = v.x; g[1] = v.y;
-    }
-}
+// arithmetic, from one tile of alphas into the next.
+// Bound by FP32 issue (f32x2: 38 T operations/s measured; its pipe is 70 %
+// busy at n = 512) and by the load/store unit's wavefronts (53 %), so what
+// else those pipes do counts: row offsets are kept in units of 16 bytes (a
+// gather's address is one multiply-add), coefficients are staged without
+// divisions, and three or four successors per loop step leave no moves
+// between the gathers' registers. n = 512 (z = 16, r = 1,024): 192 us at
+// first, 134 with one vector gather per lane, guard-free stores for whole
+// tiles and about eight rounds of blocks, 98 with the above and a block more
+// per SM; n = 1,000 (z = 11, r = 1,500): 332, 188, 147; n = 4,096 (z = 32, m =
+// 16, r = 4,096): 29.6, 24.3 and 19.1 ms.
+constexpr int kProjUPL = 4;
+constexpr int kProjThreads = 128;
+// Blocks per SM that the sums' registers allow.
+constexpr int proj_blocks(int ZC) { return ZC <= 8 ? 6 : ZC <= 12 ? 5 : ZC <= 16 ? 4 : 3; }
 
-template <int ZC, int UPL, int THREADS, int BLOCKS>
-__global__ void __launch_bounds__(THREADS, BLOCKS) proj_state_lanes_kernel(
+template <int ZC>
+__global__ void __launch_bounds__(kProjThreads, proj_blocks(ZC)) proj_state_lanes_kernel(
         DevModel md, const unsigned *__restrict__ succLen, const float *__restrict__ C1,
         const float *__restrict__ Gt, size_t gtCols, unsigned nU, float *__restrict__ Proj, size_t uRows,
         size_t sCols, unsigned uRange, float one) {
+    constexpr int UPL = kProjUPL, THREADS = kProjThreads;
+    constexpr int STEPS = ZC <= 12 ? 3 : 4;   // successors per loop step
     extern __shared__ float smem[];
     const unsigned cStride = md.ns * ZC + 4;
     float *Cs = smem;                                                   // [8][cStride]
-    int *Ss = reinterpret_cast<int *>(Cs + (size_t)kProjTileS * cStride);  // [ns + 2][8]
+    unsigned *Ss = reinterpret_cast<unsigned *>(Cs + (size_t)kProjTileS * cStride);  // [ns + 2][8] rows of Gt, in float4
     __shared__ unsigned Ls[kProjTileS];
     const unsigned long long one2 = pack_f32x2(one, one);
     const unsigned tilesS = (md.n + kProjTileS - 1) / kProjTileS;
@@ -661,45 +662,53 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) proj_state_lanes_kernel(
     const float gamma = md.gamma;
     if (threadIdx.x < kProjTileS)
         Ls[threadIdx.x] = s0 + threadIdx.x < md.n ? succLen[(size_t)(s0 + threadIdx.x) * md.m + a] : 0u;
-    for (unsigned e = threadIdx.x; e < kProjTileS * (md.ns + 2); e += blockDim.x) {
-        const unsigned st = e / (md.ns + 2), l = e % (md.ns + 2);
+    for (unsigned e = threadIdx.x; e < kProjTileS * (md.ns + 2); e += THREADS) {
+        const unsigned st = e % kProjTileS, l = e / kProjTileS;
         int succ = 0;
         if (s0 + st < md.n && l < md.ns) succ = md.S[((size_t)(s0 + st) * md.m + a) * md.ns + l];
-        Ss[l * kProjTileS + st] = max(succ, 0);  // past a row's end: state 0, gathered and not used
+        Ss[e] = (unsigned)max(succ, 0) * (unsigned)(gtCols / 4);  // past a row's end: state 0, gathered and not used
     }
     for (unsigned o0 = 0; o0 < md.z; o0 += ZC) {
         __syncthreads();
-        for (unsigned e = threadIdx.x; e < kProjTileS * md.ns * ZC; e += blockDim.x) {
-            const unsigned st = e / (md.ns * ZC), rem = e % (md.ns * ZC), l = rem / ZC, q = rem % ZC;
-            Cs[st * cStride + rem] = (s0 + st < md.n && l < Ls[st] && o0 + q < md.z)
-                ? C1[(((size_t)a * md.n + s0 + st) * md.ns + l) * md.z + o0 + q] : 0.0f;
+        for (unsigned st = warp; st < kProjTileS; st += THREADS / 32) {
+            const float *crow = C1 + ((size_t)a * md.n + s0 + st) * md.ns * md.z + o0;
+            const unsigned used = Ls[st] * ZC;
+#pragma unroll 4
+            for (unsigned e = lane; e < used; e += 32) {
+                const unsigned l = e / ZC, q = e % ZC;
+                Cs[st * cStride + e] = o0 + q < md.z ? __ldg(crow + l * md.z + q) : 0.0f;
+            }
         }
         __syncthreads();
         const unsigned zc = min((unsigned)ZC, md.z - o0);
         const unsigned L = Ls[sl];
         const float *cw = Cs + (size_t)sl * cStride;
-        const int *sw = Ss + sl;
+        const unsigned *sw = Ss + sl;
         const unsigned uBegin = blockIdx.y * uRange, uEnd = min(nU, uBegin + uRange);
-        for (unsigned u0 = uBegin + (warp * 4u + ul) * UPL; u0 < uEnd; u0 += (THREADS / 8) * UPL) {
-            // Gt's columns are padded to 32, so a lane's UPL alphas are always readable.
-            const float *gcol = Gt + u0;
+        constexpr unsigned STEP = (THREADS / 8) * UPL;
+        // Gt's columns are padded to 32, so a lane's UPL alphas are always readable.
+        float4 gn, gn2;
+        bool fetched = false;   // gn, gn2 hold the next tile's first two gathers
+        for (unsigned u0 = uBegin + (warp * 4u + ul) * UPL; u0 < uEnd; u0 += STEP) {
+            const float4 *gcol = reinterpret_cast<const float4 *>(Gt + u0);
             unsigned long long acc[UPL][ZC / 2];
 #pragma unroll
             for (int j = 0; j < UPL; j++)
 #pragma unroll
                 for (int q = 0; q < ZC / 2; q++) acc[j][q] = 0ull;
-            float gn[UPL], gn2[UPL];
-            load_alphas<UPL>(gcol + (size_t)sw[0] * gtCols, gn);
-            load_alphas<UPL>(gcol + (size_t)sw[kProjTileS] * gtCols, gn2);
-#pragma unroll 2
+            if (!fetched) {
+                gn = __ldg(gcol + sw[0]);
+                gn2 = __ldg(gcol + sw[kProjTileS]);
+            }
+            fetched = L >= 2u && u0 + STEP < uEnd;
+            const unsigned wrap = fetched ? L : md.ns + 2u;
+#pragma unroll STEPS
             for (unsigned l = 0; l < L; l++) {
-                unsigned long long gg[UPL];
-#pragma unroll
-                for (int j = 0; j < UPL; j++) {
-                    gg[j] = pack_f32x2(gn[j], gn[j]);
-                    gn[j] = gn2[j];
-                }
-                load_alphas<UPL>(gcol + (size_t)sw[(l + 2) * kProjTileS] * gtCols, gn2);
+                const unsigned long long gg[UPL] = {pack_f32x2(gn.x, gn.x), pack_f32x2(gn.y, gn.y),
+                                                    pack_f32x2(gn.z, gn.z), pack_f32x2(gn.w, gn.w)};
+                gn = gn2;
+                const bool ahead = l + 2u >= wrap;
+                gn2 = __ldg(gcol + (ahead ? STEP / 4u : 0u) + sw[(ahead ? l + 2u - wrap : l + 2u) * kProjTileS]);
                 const ulonglong2 *c2 = reinterpret_cast<const ulonglong2 *>(cw + l * ZC);
 #pragma unroll
                 for (int q4 = 0; q4 < ZC / 4; q4++) {
@@ -1185,13 +1194,16 @@ bool BackupEngine::ensure_proj(unsigned nU) {
 }
 
 // Observations a projection thread keeps in registers: the z observations in
-// ceil(z / 32) equal chunks, rounded up to 4 (one 16-byte coefficient read).
-// Both kernels are bound by FP32 issue, so lanes of padding cost their full
-// share: with chunks of 32 for z >= 16 and of 8 below, z = 16 computed twice
-// and z = 11 half again what it needed (alpha-contiguous, n = 512, z = 16:
-// 201 against 117 us).
-static int proj_chunk(unsigned z) {
-    const unsigned chunks = ceil_div(z, 32);
+// equal chunks of at most `limit`, rounded up to 4 (one 16-byte coefficient
+// read). Both kernels are bound by FP32 issue, so lanes of padding cost their
+// full share: with chunks of 32 for z >= 16 and of 8 below, z = 16 computed
+// twice and z = 11 half again what it needed (alpha-contiguous, n = 512, z =
+// 16: 201 against 117 us). State-contiguous, more than 24 leave registers for
+// two alphas a lane only, and two chunks are faster (z = 32, n = 4,096 with
+// 2,048 alphas: 11.9 and 11.5 ms; z = 30, n = 1,500: 3.3 and 3.25).
+constexpr unsigned kProjStateChunk = 24;
+static int proj_chunk(unsigned z, unsigned limit) {
+    const unsigned chunks = ceil_div(z, limit);
     return (int)round_up(ceil_div(z, chunks), 4);
 }
 
@@ -1219,8 +1231,8 @@ static void with_chunk(int zc, F f) {
 }
 
 int BackupEngine::project(unsigned nU, const char *fn) {
-    int zc = proj_chunk(md.z);
     if (projStateMajor) {
+        const int zc = proj_chunk(md.z, kProjStateChunk);
         const size_t smem = proj_state_smem(md, zc);
         // Column ranges of at most 32 MB of the transposed alphas, and enough
         // of them for about eight rounds of blocks (multiples of 128).
@@ -1230,19 +1242,16 @@ int BackupEngine::project(unsigned nU, const char *fn) {
         const unsigned uRange = (unsigned)std::max<size_t>(128, std::min(byL2, byRounds));
         const dim3 blocks(tiles, ceil_div(std::max(nU, 1u), uRange));
         with_chunk(zc, [&](auto c) {
-            // Up to 24 observations' sums of four alphas fit in registers, which
-            // halves the coefficient reads per product; above, two alphas a
-            // lane are faster (z = 30, n = 1,500: 3.2 against 3.7 ms).
-            constexpr int ZC = decltype(c)::value;
-            constexpr int UPL = ZC <= 24 ? 4 : 2, THREADS = ZC <= 24 ? 128 : 256, BLOCKS = ZC <= 24 ? 3 : 2;
-            auto kernel = proj_state_lanes_kernel<ZC, UPL, THREADS, BLOCKS>;
+            constexpr int ZC = std::min(decltype(c)::value, (int)kProjStateChunk);
+            auto kernel = proj_state_lanes_kernel<ZC>;
             if (!projAttrDone) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjSmemMax);
-            kernel<<<blocks, THREADS, smem, stream>>>(md, succLen, C1, Gt, gtCols, nU, Proj, projCols, projSCols, uRange,
-                                                  1.0f);
+            kernel<<<blocks, kProjThreads, smem, stream>>>(md, succLen, C1, Gt, gtCols, nU, Proj, projCols, projSCols,
+                                                           uRange, 1.0f);
         });
         projAttrDone = true;
         return check_launch(fn, "projection table");
     }
+    int zc = proj_chunk(md.z, 32);
     if (proj_rows_smem(md, zc) > kProjSmemMax) zc = std::min(zc, 8);  // long successor lists
     const size_t smem = proj_rows_smem(md, zc);
     with_chunk(zc, [&](auto c) {
@@ -1515,7 +1524,11 @@ int BackupEngine::backup_all(const float *src, unsigned rGamma, float *dst, unsi
 }
 
 bool BackupEngine::state_major_wanted(bool tensor) const {
-    if (proj_state_smem(md, proj_chunk(md.z)) > kProjSmemMax) return false;
+    if (proj_state_smem(md, proj_chunk(md.z, kProjStateChunk)) > kProjSmemMax) return false;
+    // The kernel's row offsets into the transposed alphas are 32 bits, in
+    // units of 16 bytes (64 GB).
+    if (md.n * (gtCols / 4) >= 1ull << 32)
+        return false;
     return tensor ? lastScanFrac <= 0.01f : scan_all_shape(md).alphas != 0;
 }
 

@@ -80,6 +80,7 @@ constexpr int STAGES = 4;
 constexpr int MAX_LISTS = 8;       // candidate lists per row: two per alpha group
 constexpr unsigned LIST_SLOTS = 32;            // a list's header and entries: 256 bytes
 constexpr unsigned LIST_CAP = LIST_SLOTS - 1;  // entries per list
+constexpr size_t kRowListBytes = MAX_LISTS * LIST_SLOTS * 8;  // a row's lists
 constexpr unsigned kNoneU = 0xffffffffu;
 constexpr int A_STAGE_BYTES = BM * BK * 2;   // 16 KB
 constexpr int B_STAGE_BYTES = BN * BK * 2;   // 32 KB
@@ -151,10 +152,12 @@ void tc_release(TcState *tc) {
 }
 
 bool tc_supported(const DevModel &md) {
-    // The dense row of W_a must fit in shared memory while A is built, and
-    // the row index must stay in TMA's 32-bit coordinate range.
+    // While A is built, the dense row of W_a must fit in shared memory and the
+    // transposed O where the candidate lists will be; the row index must stay
+    // in TMA's 32-bit coordinate range.
     const size_t nPad = round_up(md.n, BK), rPad = round_up(md.r, BM);
-    return md.n <= 40000 && (size_t)md.m * md.z * rPad < (1ull << 31) && nPad < (1ull << 31) && md.r >= 1;
+    return md.n <= 40000 && nPad * sizeof(float) <= md.r * kRowListBytes &&
+           (size_t)md.m * md.z * rPad < (1ull << 31) && nPad < (1ull << 31) && md.r >= 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -608,79 +611,113 @@ __device__ __forceinline__ float from_half_bits(uint16_t b, bool fp16) {
     return __bfloat162float(__ushort_as_bfloat16(b));
 }
 
-__global__ void tc_build_a_kernel(DevModel md, const unsigned *__restrict__ succLen,
-                                  const unsigned *__restrict__ suppLen, size_t rPad, size_t nPad, int fp16,
-                                  uint16_t *__restrict__ A, float *__restrict__ a1, float *__restrict__ a1raw,
-                                  float *__restrict__ d1, float a1Slack, float d1Slack,
-                                  unsigned *__restrict__ badModel) {
-    extern __shared__ float W[];  // [n]
-    const unsigned i = blockIdx.x / md.m, a = blockIdx.x % md.m;
-    for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) W[s] = 0.0f;
+// O with the states innermost, [m][z][nPad] (0 past n): 32 x 32 tiles.
+__global__ void tc_transpose_o_kernel(DevModel md, size_t nPad, float *__restrict__ Ot,
+                                      unsigned *__restrict__ badModel) {
+    __shared__ float tile[32][33];
+    const unsigned a = blockIdx.z, s0 = blockIdx.x * 32u, o0 = blockIdx.y * 32u;
+    for (unsigned k = threadIdx.y; k < 32u; k += 8u) {
+        float v = 0.0f;
+        if (s0 + k < md.n && o0 + threadIdx.x < md.z) {
+            v = md.O[((size_t)a * md.n + s0 + k) * md.z + o0 + threadIdx.x];
+            if (!(v >= 0.0f)) atomicOr(badModel, 1u);  // the bound assumes non-negative B, T, O
+        }
+        tile[k][threadIdx.x] = v;
+    }
     __syncthreads();
-    const unsigned Li = suppLen[i];
-    for (unsigned e = threadIdx.x; e < Li * md.ns; e += blockDim.x) {
-        const unsigned k = e / md.ns, l = e % md.ns;
-        const int s = md.Z[(size_t)i * md.rz + k];
-        if (l < succLen[(size_t)s * md.m + a]) {
-            const size_t row = ((size_t)s * md.m + a) * md.ns + l;
-            const float w = md.B[(size_t)i * md.rz + k] * md.T[row];
-            if (!(w >= 0.0f)) atomicOr(badModel, 1u);  // the bound assumes non-negative B, T, O
-            atomicAdd(&W[md.S[row]], w);
+    for (unsigned k = threadIdx.y; k < 32u; k += 8u)
+        if (o0 + k < md.z) Ot[((size_t)a * md.z + o0 + k) * nPad + s0 + threadIdx.x] = tile[threadIdx.x][k];
+}
+
+// One block per action and NB beliefs: their successor distributions W in
+// shared memory, then one warp per observation reads O's row once for all NB
+// beliefs, twice over (the rows' maxima set their scales). Bound by its FP32
+// work and by writing A: n = 1,024 (r = 1,024, m z = 128, 268 MB: 40 us at
+// memory speed) 105 us; with one belief per block, all its warps on one
+// observation and O as the model holds it (64-byte strides) 650 us.
+template <int NB>
+__global__ void __launch_bounds__(256) tc_build_a_kernel(
+                                  DevModel md, const unsigned *__restrict__ succLen,
+                                  const unsigned *__restrict__ suppLen, size_t rPad, size_t nPad, int fp16,
+                                  const float *__restrict__ Ot, uint16_t *__restrict__ A, float *__restrict__ a1,
+                                  float *__restrict__ a1raw, float *__restrict__ d1, float a1Slack, float d1Slack,
+                                  unsigned *__restrict__ badModel) {
+    extern __shared__ __align__(16) float W[];  // [NB][nPad]
+    const unsigned i0 = blockIdx.x / md.m * NB, a = blockIdx.x % md.m;
+    for (unsigned s = threadIdx.x; s < NB * nPad; s += blockDim.x) W[s] = 0.0f;
+    __syncthreads();
+    for (unsigned b = 0; b < NB && i0 + b < md.r; b++) {
+        const unsigned i = i0 + b, Li = suppLen[i];
+        for (unsigned e = threadIdx.x; e < Li * md.ns; e += blockDim.x) {
+            const unsigned k = e / md.ns, l = e % md.ns;
+            const int s = md.Z[(size_t)i * md.rz + k];
+            if (l < succLen[(size_t)s * md.m + a]) {
+                const size_t row = ((size_t)s * md.m + a) * md.ns + l;
+                const float w = md.B[(size_t)i * md.rz + k] * md.T[row];
+                if (!(w >= 0.0f)) atomicOr(badModel, 1u);
+                atomicAdd(&W[b * nPad + md.S[row]], w);
+            }
         }
     }
     __syncthreads();
-    __shared__ float red[32], redD[32];
-    __shared__ float rowScale;
-    for (unsigned o = 0; o < md.z; o++) {
+    const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (unsigned o = warp; o < md.z; o += 8u) {
         const size_t ao = (size_t)a * md.z + o;
-        uint16_t *row = A + (ao * rPad + i) * nPad;
-        float mx = 0.0f, sum = 0.0f;
-        for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) {
-            const float ob = md.O[((size_t)a * md.n + s) * md.z + o];
-            if (!(ob >= 0.0f)) atomicOr(badModel, 1u);
-            const float v = md.gamma * W[s] * ob;
-            mx = fmaxf(mx, v);
-            sum += v;
+        const float4 *orow = reinterpret_cast<const float4 *>(Ot + ao * nPad);
+        auto values = [&](unsigned b, unsigned s4, const float4 &ob) {
+            const float4 w = reinterpret_cast<const float4 *>(W + b * nPad)[s4];
+            return make_float4(md.gamma * w.x * ob.x, md.gamma * w.y * ob.y, md.gamma * w.z * ob.z,
+                               md.gamma * w.w * ob.w);
+        };
+        float mx[NB], sum[NB], dsum[NB], scale[NB];
+#pragma unroll
+        for (int b = 0; b < NB; b++) mx[b] = sum[b] = dsum[b] = 0.0f;
+        for (unsigned s4 = lane; s4 < nPad / 4; s4 += 32) {
+            const float4 ob = __ldg(orow + s4);
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                const float4 v = values(b, s4, ob);
+                mx[b] = fmaxf(mx[b], fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+                sum[b] += (v.x + v.y) + (v.z + v.w);
+            }
         }
-        for (int off = 16; off > 0; off >>= 1) {
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-            sum += __shfl_xor_sync(0xffffffffu, sum, off);
-        }
-        __syncthreads();
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (unsigned w = 0; w < blockDim.x / 32; w++) mx = fmaxf(mx, red[w]);
+#pragma unroll
+        for (int b = 0; b < NB; b++) {
+            for (int off = 16; off > 0; off >>= 1) {
+                mx[b] = fmaxf(mx[b], __shfl_xor_sync(0xffffffffu, mx[b], off));
+                sum[b] += __shfl_xor_sync(0xffffffffu, sum[b], off);
+            }
             int e = 0;
-            if (mx > 0.0f) frexpf(mx, &e);          // mx in [2^(e-1), 2^e)
-            rowScale = mx > 0.0f ? ldexpf(1.0f, 14 - e) : 1.0f;
+            if (mx[b] > 0.0f) frexpf(mx[b], &e);          // mx in [2^(e-1), 2^e)
+            scale[b] = mx[b] > 0.0f ? ldexpf(1.0f, 14 - e) : 1.0f;
         }
-        __syncthreads();
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
-        __syncthreads();
-        const float scale = rowScale;
         // d1 = sum_s |A - half(A)| in the row's scaled units: the actual
         // rounding of this row's operand (each term is exact in FP32).
-        float dsum = 0.0f;
-        for (unsigned s = threadIdx.x; s < nPad; s += blockDim.x) {
-            float v = 0.0f;
-            if (s < md.n) v = md.gamma * W[s] * md.O[((size_t)a * md.n + s) * md.z + o];
-            const float x = v * scale;
-            const uint16_t hb = to_half_bits(x, fp16 != 0);
-            row[s] = hb;
-            dsum += fabsf(x - from_half_bits(hb, fp16 != 0));
+        for (unsigned s4 = lane; s4 < nPad / 4; s4 += 32) {
+            const float4 ob = __ldg(orow + s4);
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                const float4 v = values(b, s4, ob);
+                const float x[4] = {v.x * scale[b], v.y * scale[b], v.z * scale[b], v.w * scale[b]};
+                ushort4 h;
+                h.x = to_half_bits(x[0], fp16 != 0);
+                h.y = to_half_bits(x[1], fp16 != 0);
+                h.z = to_half_bits(x[2], fp16 != 0);
+                h.w = to_half_bits(x[3], fp16 != 0);
+                dsum[b] += (fabsf(x[0] - from_half_bits(h.x, fp16 != 0)) + fabsf(x[1] - from_half_bits(h.y, fp16 != 0))) +
+                           (fabsf(x[2] - from_half_bits(h.z, fp16 != 0)) + fabsf(x[3] - from_half_bits(h.w, fp16 != 0)));
+                if (i0 + b < md.r) reinterpret_cast<ushort4 *>(A + (ao * rPad + i0 + b) * nPad)[s4] = h;
+            }
         }
-        for (int off = 16; off > 0; off >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, off);
-        if ((threadIdx.x & 31) == 0) redD[threadIdx.x >> 5] = dsum;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float t = 0.0f, d = 0.0f;
-            for (unsigned w = 0; w < blockDim.x / 32; w++) { t += red[w]; d += redD[w]; }
-            a1[ao * rPad + i] = t * scale * a1Slack;
-            a1raw[ao * rPad + i] = t * a1Slack;
-            d1[ao * rPad + i] = d * d1Slack;
+#pragma unroll
+        for (int b = 0; b < NB; b++) {
+            for (int off = 16; off > 0; off >>= 1) dsum[b] += __shfl_xor_sync(0xffffffffu, dsum[b], off);
+            if (lane == 0 && i0 + b < md.r) {
+                a1[ao * rPad + i0 + b] = sum[b] * scale[b] * a1Slack;
+                a1raw[ao * rPad + i0 + b] = sum[b] * a1Slack;
+                d1[ao * rPad + i0 + b] = dsum[b] * d1Slack;
+            }
         }
-        __syncthreads();
     }
 }
 
@@ -1393,6 +1430,9 @@ static int encode_map(TcState *tc, CUtensorMap *map, const void *base, size_t ro
     return NOVA_SUCCESS;
 }
 
+// Shared memory of an operand-building block (four blocks fit on an SM).
+constexpr size_t kBuildSmem = 56 * 1024;
+
 // (Re)builds A in the element type of the engine's scoring mode.
 static int tc_build_operand(BackupEngine &eng, TcState *tc, const char *fn) {
     const DevModel &md = eng.md;
@@ -1404,8 +1444,10 @@ static int tc_build_operand(BackupEngine &eng, TcState *tc, const char *fn) {
         tc->tuneWarm = false;
     }
     tc->mode = eng.scoring;
-    const size_t aElems = (size_t)tc->MZ * tc->rPad * tc->nPad;
-    cudaMemsetAsync(tc->A, 0, aElems * sizeof(uint16_t), eng.stream);
+    // The build writes every column of the beliefs' rows; the padding's are 0.
+    if (tc->rPad > md.r)
+        cudaMemset2DAsync(tc->A + (size_t)md.r * tc->nPad, tc->rPad * tc->nPad * sizeof(uint16_t), 0,
+                          (tc->rPad - md.r) * tc->nPad * sizeof(uint16_t), tc->MZ, eng.stream);
     cudaMemsetAsync(tc->a1, 0, (size_t)tc->MZ * tc->rPad * sizeof(float), eng.stream);
     cudaMemsetAsync(tc->a1raw, 0, (size_t)tc->MZ * tc->rPad * sizeof(float), eng.stream);
     cudaMemsetAsync(tc->d1, 0, (size_t)tc->MZ * tc->rPad * sizeof(float), eng.stream);
@@ -1415,10 +1457,19 @@ static int tc_build_operand(BackupEngine &eng, TcState *tc, const char *fn) {
     const float slack = 1.0f + (float)(md.n + md.rz * md.ns + 8) * 1.2e-7f;
     // d1 is an FP32 sum of nPad exact non-negative terms.
     const float dslack = 1.0f + (float)(tc->nPad + 8) * 1.2e-7f;
-    tc_build_a_kernel<<<md.r * md.m, 256, md.n * sizeof(float), eng.stream>>>(
-        md, eng.succLen, eng.suppLen, tc->rPad, tc->nPad, tc->mode == NOVA_SCORING_FP16 ? 1 : 0, tc->A, tc->a1,
+    float *Ot = reinterpret_cast<float *>(tc->cand);   // as the lists are written after A is built (tc_supported)
+    int rc;
+    tc_transpose_o_kernel<<<dim3((unsigned)(tc->nPad / 32), ceil_div(md.z, 32), md.m), dim3(32, 8), 0, eng.stream>>>(
+        md, tc->nPad, Ot, tc->badModel);
+    if ((rc = check_launch(fn, "observation transpose")) != NOVA_SUCCESS) return rc;
+    const size_t wBytes = tc->nPad * sizeof(float);
+    const unsigned nb = 4 * wBytes <= kBuildSmem ? 4u : 2 * wBytes <= kBuildSmem ? 2u : 1u;
+    auto build = nb == 4 ? tc_build_a_kernel<4> : nb == 2 ? tc_build_a_kernel<2> : tc_build_a_kernel<1>;
+    allow_dynamic_smem(build, nb * wBytes);
+    build<<<ceil_div(md.r, nb) * md.m, 256, nb * wBytes, eng.stream>>>(
+        md, eng.succLen, eng.suppLen, tc->rPad, tc->nPad, tc->mode == NOVA_SCORING_FP16 ? 1 : 0, Ot, tc->A, tc->a1,
         tc->a1raw, tc->d1, slack, dslack, tc->badModel);
-    int rc = check_launch(fn, "scoring operand build");
+    rc = check_launch(fn, "scoring operand build");
     if (rc != NOVA_SUCCESS) return rc;
     return encode_map(tc, &tc->tmA, tc->A, (size_t)tc->MZ * tc->rPad, tc->nPad, BM, fn);
 }

@@ -332,3 +332,18 @@ def test_shared_memory_limits_across_threads():
         for got, want in zip(solve_batched(ps, scoring=npp.SCORING_EXACT), alone):
             np.testing.assert_array_equal(bits(got.gamma_array()), bits(want.gamma_array()))
             np.testing.assert_array_equal(got.pi_array(), want.pi_array())
+
+
+@pytest.mark.parametrize("n,r,m,z", [(5, 33, 2, 9), (64, 130, 1, 1), (1000, 37, 3, 33), (3585, 41, 1, 2), (7200, 65, 1, 3),
+                                     (12300, 40, 1, 2), (16384, 64, 2, 1)])
+@pytest.mark.parametrize("mode", [npp.SCORING_FP16, npp.SCORING_BF16])
+def test_scoring_operand(n, r, m, z, mode):
+    """Four, two and one belief per building block with remainders, more
+    observations than warps, states past a whole number of vectors; scored on
+    the tensor cores throughout."""
+    md = synth.random_pomdp(n=n, m=m, z=z, ns=min(3, n), r=r, rz=min(5, n), gamma=0.9, horizon=1, seed=n)
+    md["GammaInitial"] = np.random.default_rng(r).normal(-3.0, 1.0, size=(r, n)).astype(np.float32)
+    G, pi, stats, Go, po = backups(md, mode, 1)
+    assert stats[-1]["scoring"] == mode and stats[-1]["rowsOverflow"] == 0
+    np.testing.assert_array_equal(bits(G), bits(Go))
+    np.testing.assert_array_equal(pi, po)

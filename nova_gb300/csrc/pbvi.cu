@@ -828,21 +828,6 @@ __global__ void __launch_bounds__(1024) scan_all_kernel(DevModel md, const unsig
     }
 }
 
-// The choices of scan_all_kernel (kNone where nothing beat the sentinel).
-__global__ void scan_all_finish_kernel(DevModel md, const unsigned long long *__restrict__ keys,
-                                       const unsigned *__restrict__ uniqJ, unsigned *__restrict__ ustar,
-                                       unsigned *__restrict__ jstar) {
-    const unsigned rows = md.m * md.z * md.r;
-    for (unsigned row = blockIdx.x * blockDim.x + threadIdx.x; row < rows; row += gridDim.x * blockDim.x) {
-        const unsigned ao = row / md.r, i = row % md.r;
-        const size_t js = ((size_t)i * md.m + ao / md.z) * md.z + ao % md.z;
-        const unsigned long long k = keys[row];
-        const unsigned bu = k == 0ull ? kNone : ~(unsigned)k;
-        ustar[js] = bu;
-        jstar[js] = bu == kNone ? kNone : uniqJ[bu];
-    }
-}
-
 // The same for listed rows (those a tensor-core update leaves open), or for
 // all of them where a state column of four alphas does not fit in shared
 // memory. One block per row. The alphas are scanned in
@@ -855,7 +840,8 @@ __global__ void __launch_bounds__(256) scan_rows_kernel(DevModel md, const unsig
                                                         unsigned u1, const unsigned *__restrict__ rowList,
                                                         unsigned nRows, const unsigned *__restrict__ nRowsDev,
                                                         float *__restrict__ runV,
-                                                        unsigned *__restrict__ runU, int first) {
+                                                        unsigned *__restrict__ runU, int first,
+                                                        unsigned *__restrict__ ustar) {
     extern __shared__ float sh[];
     float *bk = sh;                                              // [rz]
     unsigned *sk = reinterpret_cast<unsigned *>(sh + md.rz);     // [rz]
@@ -897,72 +883,75 @@ __global__ void __launch_bounds__(256) scan_rows_kernel(DevModel md, const unsig
                 const unsigned pu = runU[w];
                 if (pu != kNone && (bu == kNone || !(best > runV[w]))) { best = runV[w]; bu = pu; }
             }
-            runV[w] = best;
-            runU[w] = bu;
+            if (ustar == nullptr) {
+                runV[w] = best;
+                runU[w] = bu;
+            } else {   // the last column chunk
+                ustar[((size_t)i * md.m + ao / md.z) * md.z + ao % md.z] = bu;
+            }
         }
-    }
-}
-
-// Final choice of each scanned row (kNone where nothing beat the sentinel).
-__global__ void scan_finish_kernel(DevModel md, const unsigned *__restrict__ rowList, unsigned nRows,
-                                   const unsigned *__restrict__ nRowsDev,
-                                   const unsigned *__restrict__ runU, const unsigned *__restrict__ uniqJ,
-                                   unsigned *__restrict__ ustar, unsigned *__restrict__ jstar) {
-    if (nRowsDev) nRows = min(nRows, *nRowsDev);
-    for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < nRows; w += gridDim.x * blockDim.x) {
-        const unsigned row = rowList ? rowList[w] : w;
-        const unsigned ao = row / md.r, i = row % md.r;
-        const size_t js = ((size_t)i * md.m + ao / md.z) * md.z + ao % md.z;
-        const unsigned bu = runU[w];
-        ustar[js] = bu;
-        jstar[js] = bu == kNone ? kNone : uniqJ[bu];
-    }
-}
-
-// Rows with no alpha above the -1e10 sentinel take the previous
-// observation's choice (0 for the first), as the reference's bestj does.
-// Only scanned rows can be such (nRowsDev: how many there are).
-__global__ void sentinel_fixup_kernel(DevModel md, const unsigned *__restrict__ nRowsDev, unsigned *__restrict__ ustar,
-                                      unsigned *__restrict__ jstar) {
-    const unsigned ia = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ia >= md.r * md.m || (nRowsDev && *nRowsDev == 0u)) return;
-    unsigned prevU = 0, prevJ = 0;
-    for (unsigned o = 0; o < md.z; o++) {
-        const size_t js = (size_t)ia * md.z + o;
-        if (jstar[js] == kNone) {
-            // Alpha 0 has unique index 0: the first row is its own representative.
-            jstar[js] = prevJ;
-            ustar[js] = prevU;
-        }
-        prevJ = jstar[js];
-        prevU = ustar[js];
     }
 }
 
 // Action values from the projection table (one warp per (belief, action)):
 // alpha_a(s_k) = R(s_k,a) + sum_o Proj[a][o][s_k][u*], value = sum_k alpha * b_k.
+// The choices come from ustar or, after scan_all, as its keys, and are left in
+// ustar. Rows with no alpha above the -1e10 sentinel (kNone, a key of 0) take
+// the previous observation's choice (0 for the first, whose row is its own
+// representative), as the reference's bestj does. Done here, where every choice
+// is read anyway, this and the decoding need no launches of their own (two of
+// an update's 15, three of an exact one's 10; n = 64: 11 of 115 us).
+// Bound by the gathers' random sectors (n = 512: 134 MB in 14 us); more than
+// two of them in flight per lane are slower (16 and 20 us with two and four).
 __global__ void action_value_proj_kernel(DevModel md, const unsigned *__restrict__ suppLen,
-                                         const ProjView pv,
-                                         const unsigned *__restrict__ ustar, float *__restrict__ actVal) {
+                                         const ProjView pv, const unsigned long long *__restrict__ keys,
+                                         unsigned *ustar, float *__restrict__ actVal) {
     const unsigned warpGlobal = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned lane = threadIdx.x & 31;
     if (warpGlobal >= md.r * md.m) return;
     const unsigned ia = warpGlobal;
     const unsigned i = ia / md.m, a = ia % md.m;
     const unsigned Li = suppLen[i];
+    unsigned *choice = ustar + (size_t)ia * md.z;
+    unsigned uo = 0, prev = 0;   // lane's choice of the present 32 observations, the last one of those before
+    for (unsigned o0 = 0; o0 < md.z; o0 += 32) {
+        const unsigned o = o0 + lane;
+        uo = 0;
+        if (o < md.z) {
+            if (keys == nullptr) {
+                uo = choice[o];
+            } else {
+                const unsigned long long key = __ldg(keys + ((size_t)a * md.z + o) * md.r + i);
+                uo = key == 0ull ? kNone : ~(unsigned)key;
+            }
+        }
+        const unsigned none = __ballot_sync(0xffffffffu, uo == kNone);
+        if (none != 0u) {
+            const unsigned chosen = ~none & (0xffffffffu >> (31u - lane));
+            const unsigned last = __shfl_sync(0xffffffffu, uo, chosen ? 31u - __clz(chosen) : 0u);
+            if (uo == kNone) uo = chosen ? last : prev;
+        }
+        if (o < md.z && (none != 0u || keys != nullptr)) choice[o] = uo;
+        prev = __shfl_sync(0xffffffffu, uo, min(31u, md.z - 1u - o0));
+    }
+    __syncwarp();
     float value = 0.0f;
     for (unsigned k0 = 0; k0 < Li; k0 += 32) {
         const unsigned k = k0 + lane;
-        float p = 0.0f;
-        if (k < Li) {
-            const int s = md.Z[(size_t)i * md.rz + k];
-            float alpha = md.R[(size_t)s * md.m + a];
-            for (unsigned o = 0; o < md.z; o++) {
-                const unsigned u = ustar[(size_t)ia * md.z + o];
-                alpha = fadd(alpha, pv.slab(a * md.z + o)[pv.at(s, u)]);
+        const unsigned s = k < Li ? (unsigned)md.Z[(size_t)i * md.rz + k] : 0u;
+        float alpha = k < Li ? md.R[(size_t)s * md.m + a] : 0.0f;
+        for (unsigned o0 = 0; o0 < md.z; o0 += 32) {
+            if (md.z > 32u) uo = o0 + lane < md.z ? choice[o0 + lane] : 0u;
+            const unsigned cnt = min(32u, md.z - o0);
+            const float *P = pv.slab(a * md.z + o0);
+#pragma unroll 2
+            for (unsigned t = 0; t < cnt; t++) {
+                const unsigned u = __shfl_sync(0xffffffffu, uo, t);
+                if (k < Li) alpha = fadd(alpha, __ldg(P + pv.at(s, u)));
+                P += pv.slice;
             }
-            p = fmul(alpha, md.B[(size_t)i * md.rz + k]);
         }
+        const float p = k < Li ? fmul(alpha, md.B[(size_t)i * md.rz + k]) : 0.0f;
         const unsigned cnt = min(32u, Li - k0);
         for (unsigned t = 0; t < cnt; t++) value = fadd(value, __shfl_sync(0xffffffffu, p, t));
     }
@@ -1325,15 +1314,13 @@ int BackupEngine::scan_all(unsigned nU, const char *fn) {
     kernel<<<dim3(tiles, ceil_div(md.r, share)), threads, smem, stream>>>(md, suppLen, proj_view(), nU, chunks, share,
                                                                         scanKeys, 1.0f);
     if ((rc = check_launch(fn, "exact scan")) != NOVA_SUCCESS) return rc;
-    scan_all_finish_kernel<<<std::min(ceil_div(rows, 256), 152u * 8u), 256, 0, stream>>>(md, scanKeys, uniqMap, ustar,
-                                                                                        jstar);
-    if ((rc = check_launch(fn, "exact scan (finish)")) != NOVA_SUCCESS) return rc;
-    sentinel_fixup_kernel<<<ceil_div((size_t)md.r * md.m, 256), 256, 0, stream>>>(md, nullptr, ustar, jstar);
-    return check_launch(fn, "sentinel fixup");
+    choicesAsKeys = true;
+    return NOVA_SUCCESS;
 }
 
 int BackupEngine::scan_rows(const unsigned *rowList, unsigned nRows, unsigned nU, const char *fn,
                             const unsigned *nRowsDev) {
+    choicesAsKeys = false;
     if (nRows == 0) return NOVA_SUCCESS;
     int rc;
     if (rowList == nullptr && projStateMajor) return scan_all(nU, fn);
@@ -1346,14 +1333,10 @@ int BackupEngine::scan_rows(const unsigned *rowList, unsigned nRows, unsigned nU
         const unsigned u1 = (unsigned)std::min<size_t>(nU, u0 + chunk);
         scan_rows_kernel<<<grid, 256, 2 * md.rz * sizeof(float), stream>>>(md, suppLen, proj_view(), (unsigned)u0,
                                                                           u1, rowList, nRows, nRowsDev, scanV,
-                                                                          scanU, u0 == 0 ? 1 : 0);
+                                                                          scanU, u0 == 0 ? 1 : 0, u0 + chunk >= nU ? ustar : nullptr);
         if ((rc = check_launch(fn, "exact row scan")) != NOVA_SUCCESS) return rc;
     }
-    scan_finish_kernel<<<std::min(ceil_div(nRows, 256), 152u * 8u), 256, 0, stream>>>(md, rowList, nRows, nRowsDev,
-                                                                                     scanU, uniqMap, ustar, jstar);
-    if ((rc = check_launch(fn, "exact row scan (finish)")) != NOVA_SUCCESS) return rc;
-    sentinel_fixup_kernel<<<ceil_div((size_t)md.r * md.m, 256), 256, 0, stream>>>(md, nRowsDev, ustar, jstar);
-    return check_launch(fn, "sentinel fixup");
+    return NOVA_SUCCESS;
 }
 
 int BackupEngine::scan_rows_direct(const unsigned *rowList, unsigned nRows, unsigned nU, const char *fn) {
@@ -1385,8 +1368,8 @@ int BackupEngine::assemble(const float *src, float *dst, unsigned *pi, const cha
     int rc;
     const unsigned nItems = md.r * md.m;
     if (useProjNow)
-        action_value_proj_kernel<<<ceil_div((size_t)nItems * 32, 256), 256, 0, stream>>>(md, suppLen, proj_view(),
-                                                                                         ustar, actVal);
+        action_value_proj_kernel<<<ceil_div((size_t)nItems * 32, 256), 256, 0, stream>>>(
+            md, suppLen, proj_view(), choicesAsKeys ? scanKeys : nullptr, ustar, actVal);
     else
         action_value_kernel<<<ceil_div((size_t)nItems * 32, 256), 256, 0, stream>>>(md, succLen, suppLen, C3, src,
                                                                                     jstar, nItems, actVal);

@@ -71,8 +71,8 @@ struct BackupEngine {
     unsigned *nUniqueDev = nullptr;      // report[0]
     float *Gt = nullptr;                 // [n][gtCols] transposed unique alphas
     size_t gtCols = 0;
-    unsigned *jstar = nullptr;           // [r][m][z] chosen alpha per (belief, action, observation)
-    unsigned *ustar = nullptr;           // [r][m][z] the same choice as a unique-alpha index
+    unsigned *jstar = nullptr;           // [r][m][z] chosen alpha per (belief, action, observation), without a table
+    unsigned *ustar = nullptr;           // [r][m][z] the choice as a unique-alpha index, with a table
     float *Proj = nullptr;               // exact projections of the unique alphas (layout: ProjView)
     size_t projCap = 0, projCols = 0;    // projCols: alpha columns (rows in the state-contiguous layout)
     bool projStateMajor = false;         // this update's table is state-contiguous
@@ -83,6 +83,7 @@ struct BackupEngine {
     // running values and indices, or scan_all's keys, in the same memory (from
     // the arena for up to kDeferredRows rows, else scanLate).
     unsigned long long *scanKeys = nullptr, *scanLate = nullptr;
+    bool choicesAsKeys = false;          // the last scan's choices are scanKeys, ustar is behind
     float *scanV = nullptr;
     unsigned *scanU = nullptr;
     size_t scanCap = 0;
@@ -196,7 +197,7 @@ bool tc_supported(const DevModel &md);
 // Builds the BF16 operand tables once; returns NOVA_SUCCESS or an error.
 int tc_build(BackupEngine &eng, const char *fn);
 // Scores every (belief, action, observation) row against the nU unique rows
-// of src (gathered through eng.uniqMap), writes eng.jstar for rows whose argmax
+// of src (gathered through eng.uniqMap), writes the choice of rows whose argmax
 // is proven, and appends the (belief, action) items that need the exact full
 // scan to *rowList / *nRows as (a*z+o)*r + i row indices (a device list
 // owned by the tensor-core state, sized for every row).

@@ -905,7 +905,8 @@ constexpr unsigned kMergePitch = 33;   // shared-memory row of one candidate's p
 enum RowOutcome : unsigned { kRowSettled, kRowExact, kRowSeveral };
 
 // Looks through one row's lists (per thread): the row is left to the exact
-// scan, settled by its only candidate, or has several (from *cutOut on).
+// scan, settled by its only candidate (choice: its index among the unique
+// alphas, or with uniqJ among all), or has several (from *cutOut on).
 __device__ __forceinline__ RowOutcome merge_look(unsigned row, const DevModel &md,
                                                  const unsigned *__restrict__ uniqJ, unsigned nLists, size_t rPad,
                                                  const float *__restrict__ a1, const float *__restrict__ d1,
@@ -913,8 +914,8 @@ __device__ __forceinline__ RowOutcome merge_look(unsigned row, const DevModel &m
                                                  const unsigned *__restrict__ scal,
                                                  const uint2 *__restrict__ cand,
                                                  const unsigned *__restrict__ badModel,
-                                                 unsigned *__restrict__ ustar, unsigned *__restrict__ jstar,
-                                                 unsigned *__restrict__ rowFlag, unsigned *__restrict__ rowCand,
+                                                 unsigned *__restrict__ choice, unsigned *__restrict__ rowFlag,
+                                                 unsigned *__restrict__ rowCand,
                                                  float *cutOut) {
     const unsigned ao = row / md.r, i = row % md.r;
     const uint4 *lists = reinterpret_cast<const uint4 *>(cand + (size_t)row * (MAX_LISTS * LIST_SLOTS));
@@ -956,8 +957,7 @@ __device__ __forceinline__ RowOutcome merge_look(unsigned row, const DevModel &m
     rowCand[row] = 0u;
     if (res == kRowSettled) {
         const size_t js = ((size_t)i * md.m + ao / md.z) * md.z + ao % md.z;
-        ustar[js] = bestU;
-        jstar[js] = uniqJ[bestU];
+        choice[js] = uniqJ == nullptr ? bestU : uniqJ[bestU];
     }
     *cutOut = cut;
     return res;
@@ -973,8 +973,8 @@ template <int NE>
 __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const DevModel &md,
                                               const unsigned *__restrict__ suppLen, const DirectScorer &ds, float *scratch, unsigned *list,
                                               const unsigned *__restrict__ uniqJ, unsigned nLists,
-                                              const uint2 *__restrict__ cand, unsigned *__restrict__ ustar,
-                                              unsigned *__restrict__ jstar, bool *flagged) {
+                                              const uint2 *__restrict__ cand, unsigned *__restrict__ jstar,
+                                              bool *flagged) {
     const unsigned ao = row / md.r, i = row % md.r;
     const unsigned a = ao / md.z, o = ao % md.z;
     const uint2 *lists = cand + (size_t)row * (MAX_LISTS * LIST_SLOTS);
@@ -1099,7 +1099,6 @@ __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const
     if (!(best > -1e10f)) {
         *flagged = true;  // sentinel case: the exact scan applies the reference's rule
     } else if (lane == 0) {
-        ustar[js] = bu;
         jstar[js] = uniqJ[bu];
     }
     return count;
@@ -1116,8 +1115,7 @@ __global__ void __launch_bounds__(kLookRows) tc_merge_look_kernel(
                                 DevModel md, const unsigned *__restrict__ uniqJ, unsigned nLists, size_t rPad,
                                 const float *__restrict__ a1, const float *__restrict__ d1,
                                 const float *__restrict__ a1raw, const unsigned *__restrict__ scal,
-                                uint2 *cand, unsigned *__restrict__ ustar, unsigned *__restrict__ jstar,
-                                unsigned *__restrict__ rowFlag, unsigned *__restrict__ rowCand,
+                                uint2 *cand, unsigned *__restrict__ choice, unsigned *__restrict__ rowFlag, unsigned *__restrict__ rowCand,
                                 unsigned *__restrict__ rowList, unsigned *__restrict__ counters,
                                 unsigned *__restrict__ chunkCount, const unsigned *__restrict__ badModel) {
     const unsigned rows = md.m * md.z * md.r;  // fewer than 2^31 (tc_supported)
@@ -1125,8 +1123,8 @@ __global__ void __launch_bounds__(kLookRows) tc_merge_look_kernel(
     RowOutcome res = kRowSettled;
     if (row < rows) {
         float cut = 0.0f;
-        res = merge_look(row, md, uniqJ, nLists, rPad, a1, d1, a1raw, scal, cand, badModel, ustar, jstar, rowFlag,
-                         rowCand, &cut);
+        res = merge_look(row, md, uniqJ, nLists, rPad, a1, d1, a1raw, scal, cand, badModel, choice, rowFlag, rowCand,
+                         &cut);
         if (res == kRowSeveral) cand[(size_t)row * (MAX_LISTS * LIST_SLOTS)].x = __float_as_uint(cut);
     }
     const unsigned msk = __ballot_sync(0xffffffffu, res == kRowSeveral);
@@ -1149,14 +1147,13 @@ enum class MergeRows { kQueued, kInOrder, kWhole };
 template <int NE, MergeRows kRows>
 __global__ void __launch_bounds__(256, kMergeBlocks) tc_merge_kernel(
                                 DevModel md, const unsigned *__restrict__ suppLen,
-                                const ProjView pv, const unsigned *__restrict__ uniqJ,
-                                unsigned nLists, size_t rPad, const float *__restrict__ a1,
+                                const ProjView pv, unsigned nLists, size_t rPad, const float *__restrict__ a1,
                                 const float *__restrict__ d1, const float *__restrict__ a1raw,
                                 const unsigned *__restrict__ scal, const uint2 *__restrict__ cand,
-                                unsigned *__restrict__ ustar, unsigned *__restrict__ jstar,
-                                unsigned *__restrict__ rowFlag, unsigned *__restrict__ rowCand,
-                                const unsigned *__restrict__ rowList, unsigned *__restrict__ counters,
-                                unsigned *__restrict__ chunkCount, const unsigned *__restrict__ badModel) {
+                                unsigned *__restrict__ ustar, unsigned *__restrict__ rowFlag,
+                                unsigned *__restrict__ rowCand, const unsigned *__restrict__ rowList,
+                                unsigned *__restrict__ counters, unsigned *__restrict__ chunkCount,
+                                const unsigned *__restrict__ badModel) {
     __shared__ float scratch[8][2][kMergeBatch * kMergePitch];
     extern __shared__ unsigned mergeLists[];   // [16 halves][nLists * LIST_SLOTS]
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, hl = lane & 15u;
@@ -1173,8 +1170,8 @@ __global__ void __launch_bounds__(256, kMergeBlocks) tc_merge_kernel(
             RowOutcome res = kRowSettled;
             float cut = 0.0f;
             if (lane < 16u && row < queued)
-                res = merge_look(row, md, uniqJ, nLists, rPad, a1, d1, a1raw, scal, cand, badModel, ustar, jstar,
-                                 rowFlag, rowCand, &cut);
+                res = merge_look(row, md, nullptr, nLists, rPad, a1, d1, a1raw, scal, cand, badModel, ustar, rowFlag,
+                                 rowCand, &cut);
             const unsigned msk = __ballot_sync(0xffffffffu, res == kRowSeveral);
             const unsigned exact = __popc(__ballot_sync(0xffffffffu, res == kRowExact));
             if (res == kRowSeveral) {
@@ -1304,7 +1301,6 @@ __global__ void __launch_bounds__(256, kMergeBlocks) tc_merge_kernel(
             } else {
                 const size_t js = ((size_t)i * md.m + ao / md.z) * md.z + ao % md.z;
                 ustar[js] = bu;
-                jstar[js] = uniqJ[bu];
             }
             sum += count;
         }
@@ -1317,7 +1313,7 @@ __global__ void __launch_bounds__(256, kMergeBlocks) tc_merge_kernel(
 __global__ void __launch_bounds__(256, 1) tc_merge_direct_kernel(
                                 DevModel md, const unsigned *__restrict__ suppLen,
                                 const DirectScorer ds, const unsigned *__restrict__ uniqJ,
-                                unsigned nLists, const uint2 *__restrict__ cand, unsigned *__restrict__ ustar,
+                                unsigned nLists, const uint2 *__restrict__ cand,
                                 unsigned *__restrict__ jstar, unsigned *__restrict__ rowFlag,
                                 unsigned *__restrict__ rowCand, const unsigned *__restrict__ rowList,
                                 unsigned *__restrict__ counters, unsigned *__restrict__ chunkCount) {
@@ -1331,7 +1327,7 @@ __global__ void __launch_bounds__(256, 1) tc_merge_direct_kernel(
         const unsigned row = __ldg(rowList + k);
         bool flagged = false;
         const unsigned rescored = merge_row<2>(row, lane, md, suppLen, ds, mergeScratch + warp * 1024u, list, uniqJ,
-                                               nLists, cand, ustar, jstar, &flagged);
+                                               nLists, cand, jstar, &flagged);
         if (lane == 0) {
             rowCand[row] = rescored;
             rowFlag[row] = flagged ? 1u : 0u;
@@ -1639,8 +1635,9 @@ int tc_finish(BackupEngine &eng, const char *fn) {
     const bool whole = table && blocks <= kMergeWholeRounds * kMergeBlocks * (unsigned)tc->numSMs;
     if (!whole) {
         tc_merge_look_kernel<<<(unsigned)ceil_div(rows, kLookRows), kLookRows, 0, eng.stream>>>(
-            md, eng.uniqMap, L.lists, tc->rPad, tc->a1, tc->d1, tc->a1raw, tc->scal, tc->cand, eng.ustar, eng.jstar,
-            tc->rowFlag, tc->rowCand, tc->rowList, tc->scal + 3, tc->chunkCount, tc->badModel);
+            md, table ? nullptr : eng.uniqMap, L.lists, tc->rPad, tc->a1, tc->d1, tc->a1raw, tc->scal, tc->cand,
+            table ? eng.ustar : eng.jstar, tc->rowFlag, tc->rowCand, tc->rowList, tc->scal + 3, tc->chunkCount,
+            tc->badModel);
         if ((rc = check_launch(fn, "candidate lists")) != NOVA_SUCCESS) return rc;
     }
     if (table) {
@@ -1651,13 +1648,12 @@ int tc_finish(BackupEngine &eng, const char *fn) {
                                : (two ? tc_merge_kernel<2, MergeRows::kQueued> : tc_merge_kernel<4, MergeRows::kQueued>);
         const unsigned grid = whole || inOrder ? blocks : std::min(blocks, kMergeBlocks * (unsigned)tc->numSMs);
         merge<<<grid, 256, 16 * L.lists * LIST_SLOTS * sizeof(unsigned), eng.stream>>>(
-            md, eng.suppLen, eng.proj_view(), eng.uniqMap, L.lists, tc->rPad, tc->a1, tc->d1, tc->a1raw, tc->scal,
-            tc->cand, eng.ustar, eng.jstar, tc->rowFlag, tc->rowCand, tc->rowList, tc->scal + 3, tc->chunkCount,
-            tc->badModel);
+            md, eng.suppLen, eng.proj_view(), L.lists, tc->rPad, tc->a1, tc->d1, tc->a1raw, tc->scal, tc->cand,
+            eng.ustar, tc->rowFlag, tc->rowCand, tc->rowList, tc->scal + 3, tc->chunkCount, tc->badModel);
     } else {
         const unsigned grid = std::min((unsigned)ceil_div(rows, 8), (unsigned)tc->numSMs);
         tc_merge_direct_kernel<<<grid, 256, 8 * (1024u + L.lists * LIST_SLOTS) * sizeof(float), eng.stream>>>(
-            md, eng.suppLen, ds, eng.uniqMap, L.lists, tc->cand, eng.ustar, eng.jstar, tc->rowFlag, tc->rowCand,
+            md, eng.suppLen, ds, eng.uniqMap, L.lists, tc->cand, eng.jstar, tc->rowFlag, tc->rowCand,
             tc->rowList, tc->scal + 3, tc->chunkCount);
     }
     if ((rc = check_launch(fn, "candidate merge")) != NOVA_SUCCESS) return rc;

@@ -347,3 +347,20 @@ def test_scoring_operand(n, r, m, z, mode):
     assert stats[-1]["scoring"] == mode and stats[-1]["rowsOverflow"] == 0
     np.testing.assert_array_equal(bits(G), bits(Go))
     np.testing.assert_array_equal(pi, po)
+
+
+@pytest.mark.parametrize("mode", [npp.SCORING_EXACT, npp.SCORING_FP16])
+@pytest.mark.parametrize("n,z,r,rz", [(12, 1, 40, 3), (30, 32, 50, 5), (40, 33, 70, 40), (25, 71, 35, 25), (9000, 3, 33, 4)])
+def test_choices_below_the_sentinel(n, z, r, rz, mode):
+    """(Belief, action, observation) rows without an alpha above -1e10, alone
+    and in runs, first and later, past 32 observations: the previous
+    observation's choice stands."""
+    md = synth.random_pomdp(n=n, m=2, z=z, ns=2, r=r, rz=rz, gamma=0.9, horizon=2, seed=n + z)
+    rng = np.random.default_rng(z)
+    md["O"] = np.where(rng.uniform(size=md["O"].shape) < 0.5, md["O"], 0).astype(np.float32)
+    G = rng.normal(-3.0, 1.0, size=(r, n))
+    G[:, n // 3:] -= 1e13 * rng.uniform(0.5, 1, size=(r, n - n // 3))
+    md["GammaInitial"] = G.astype(np.float32)
+    got, pi, stats, want, po = backups(md, mode, 2)
+    np.testing.assert_array_equal(bits(got), bits(want))
+    np.testing.assert_array_equal(pi, po)

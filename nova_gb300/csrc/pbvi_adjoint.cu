@@ -282,54 +282,185 @@ __global__ void value_argmax_kernel(unsigned r, unsigned n, const double *__rest
     for (unsigned s = threadIdx.x; s < n; s += blockDim.x) lam[(size_t)istar * n + s] = (double)b[s];
 }
 
-// One reverse step for belief i = blockIdx.x. Shared memory: c_i and w_i
-// (n doubles each) and the z selections.
-__global__ void adjoint_step_kernel(AdjModel md, const unsigned *__restrict__ len, const float *__restrict__ Gprev,
-                                    const unsigned *__restrict__ act, const unsigned *__restrict__ sel,
-                                    const double *__restrict__ lam, double *__restrict__ lamPrev,
-                                    double *__restrict__ dR, double *__restrict__ dT, double *__restrict__ dO) {
+// Threads and shared memory of a reverse-step block.
+constexpr unsigned kStepThreads = 128;
+constexpr size_t kStepSmem = 56 * 1024;
+
+// The predecessors of every (a, s'): the (s, T(s,a,l)) with S(s,a,l) = s', one
+// entry per l. Counted, given places (in no particular order of the lists) and
+// filled.
+__global__ void adj_pred_count_kernel(AdjModel md, const unsigned *__restrict__ len, unsigned *__restrict__ count) {
+    const size_t all = (size_t)md.n * md.m * md.ns, stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < all; e += stride) {
+        const size_t row = e / md.ns;
+        if (e % md.ns < len[row]) atomicAdd(count + (row % md.m) * md.n + md.S[e], 1u);
+    }
+}
+__global__ void adj_pred_place_kernel(size_t rows, const unsigned *__restrict__ count, unsigned long long *next,
+                                      unsigned long long *__restrict__ start, unsigned *__restrict__ filled) {
+    const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned lane = threadIdx.x & 31, c = k < rows ? count[k] : 0u;
+    unsigned v = c;
+    for (int off = 1; off < 32; off <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, v, off);
+        if (lane >= (unsigned)off) v += y;
+    }
+    unsigned long long base = 0;
+    if (lane == 31) base = atomicAdd(next, (unsigned long long)v);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    if (k < rows) {
+        start[k] = base + (v - c);
+        filled[k] = 0u;
+    }
+}
+__global__ void adj_pred_fill_kernel(AdjModel md, const unsigned *__restrict__ len,
+                                     const unsigned long long *__restrict__ start, unsigned *__restrict__ filled,
+                                     uint2 *__restrict__ pred, unsigned *__restrict__ predK) {
+    const size_t all = (size_t)md.n * md.m * md.ns, stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < all; e += stride) {
+        const size_t row = e / md.ns;
+        if (e % md.ns >= len[row]) continue;
+        const size_t k = (row % md.m) * md.n + md.S[e];
+        const unsigned long long at = start[k] + atomicAdd(filled + k, 1u);
+        pred[at] = make_uint2((unsigned)(row / md.m), __float_as_uint(md.T[e]));
+        predK[at] = (unsigned)(e % md.ns);
+    }
+}
+
+// x in FP64: the conversion instruction runs at the FP64 rate (1/64 of FP32),
+// the shifts of a normal number's bits do not.
+__device__ __forceinline__ double widen(float x) {
+    const unsigned b = __float_as_uint(x);
+    if (((b >> 23) & 255u) - 1u < 254u)
+        return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
+    return (double)x;
+}
+
+__device__ __forceinline__ bool nonzero(double x) {   // by its bits: compares run at the FP64 rate too
+    return (((unsigned)__double2hiint(x) & 0x7fffffffu) | (unsigned)__double2loint(x)) != 0u;
+}
+
+// One reverse step for up to NB beliefs of one action (of a group made for the
+// replay; those with a zero adjoint drop out) at kStepThreads successors s',
+// one per thread: c and w of the beliefs stay in registers, the s' terms of dT
+// are those of its predecessors. Shared memory: the beliefs' lambda (n doubles
+// each), their selections, and with kStaged a tile per warp through which dO's
+// terms, computed for consecutive states, reach consecutive observations.
+// Bound by FP64 arithmetic (1/64 of the FP32 rate), so factors are widened and
+// tested by integer operations, and what does not depend on the belief is
+// shared by the group; blocks of a part of the states even out the groups'
+// unequal numbers of beliefs. n = 1,024 (m = 8, z = 16, ns = 16, 600 beliefs
+// with an adjoint): 430 us a step with a block per belief and w by atomics in
+// shared memory, 225 so (the FP64 pipe 70 % busy; 240 with two beliefs per
+// block, 250 with one).
+template <int NB, bool kStaged>
+__global__ void __launch_bounds__(kStepThreads) adjoint_step_kernel(
+        AdjModel md, const unsigned *__restrict__ predCount, const unsigned long long *__restrict__ predStart,
+        const uint2 *__restrict__ pred, const unsigned *__restrict__ predK, const float *__restrict__ Gprev,
+        const unsigned *__restrict__ acts, const unsigned *__restrict__ ids, const unsigned *__restrict__ sel,
+        const double *__restrict__ lam, double *__restrict__ lamPrev, double *__restrict__ dR,
+        double *__restrict__ dT, double *__restrict__ dO) {
     extern __shared__ __align__(16) unsigned char smem[];
-    double *csh = reinterpret_cast<double *>(smem);
-    double *wsh = csh + md.n;
-    unsigned *jsh = reinterpret_cast<unsigned *>(wsh + md.n);
-    const unsigned i = blockIdx.x;
-    const double *lrow = lam + (size_t)i * md.n;
-    bool nz = false;
-    for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) nz |= lrow[s] != 0.0;
-    if (!__syncthreads_or(nz)) return;
-    const unsigned a = min(act[i], md.m - 1);
-    for (unsigned o = threadIdx.x; o < md.z; o += blockDim.x) jsh[o] = min(sel[(size_t)i * md.z + o], md.r - 1);
+    double *lsh = reinterpret_cast<double *>(smem);          // [NB][n]
+    double *tiles = lsh + (size_t)NB * md.n;                 // [warps][32][9] with kStaged
+    unsigned *jsh = reinterpret_cast<unsigned *>(tiles + (kStaged ? kStepThreads * 9 : 0));  // [NB][z]
+    constexpr unsigned kParts = kGroup / NB;
+    const unsigned a = acts[blockIdx.x / kParts];
+    if (a == kNoRow) return;
+    ids += (size_t)blockIdx.x * NB;
+    unsigned nb = 0;
+    for (unsigned q = 0; q < NB; q++) {
+        const unsigned i = ids[q];
+        bool nz = false;
+        if (i != kNoRow)
+            for (unsigned s = threadIdx.x; s < md.n; s += kStepThreads) {
+                const double l = lam[(size_t)i * md.n + s];
+                lsh[(size_t)nb * md.n + s] = l;
+                nz |= nonzero(l);
+            }
+        if (!__syncthreads_or(nz)) continue;   // its place is taken by the next
+        for (unsigned o = threadIdx.x; o < md.z; o += kStepThreads)
+            jsh[nb * md.z + o] = min(sel[(size_t)i * md.z + o], md.r - 1);
+        nb++;
+    }
+    if (nb == 0) return;
     __syncthreads();
     const double g = (double)md.gamma;
-    for (unsigned sp = threadIdx.x; sp < md.n; sp += blockDim.x) {
-        const float *Orow = md.O + ((size_t)a * md.n + sp) * md.z;
-        double c = 0.0;
-        for (unsigned o = 0; o < md.z; o++) c += (double)Orow[o] * (double)Gprev[(size_t)jsh[o] * md.n + sp];
-        csh[sp] = c;
-        wsh[sp] = 0.0;
-    }
-    __syncthreads();
-    for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) {
-        const double l = lrow[s];
-        if (l == 0.0) continue;
-        atomicAdd(dR + (size_t)s * md.m + a, l);
-        const size_t row = ((size_t)s * md.m + a) * md.ns;
-        const unsigned L = len[(size_t)s * md.m + a];
-        for (unsigned k = 0; k < L; k++) {
-            const unsigned sp = (unsigned)md.S[row + k];
-            atomicAdd(wsh + sp, (double)md.T[row + k] * l);
-            atomicAdd(dT + row + k, g * l * csh[sp]);
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned sp = blockIdx.y * kStepThreads + threadIdx.x, sp0 = sp - lane;
+    if (sp0 >= md.n) return;
+    const bool in = sp < md.n;
+    const size_t ob = ((size_t)a * md.n + sp) * md.z;
+    double c[NB], w[NB];
+#pragma unroll
+    for (int b = 0; b < NB; b++) c[b] = w[b] = 0.0;
+    if (in) {
+        double l = 0.0;
+        for (unsigned b = 0; b < nb; b++) l += lsh[(size_t)b * md.n + sp];
+        if (nonzero(l)) atomicAdd(dR + (size_t)sp * md.m + a, l);
+#pragma unroll 2
+        for (unsigned o = 0; o < md.z; o++) {
+            const double po = widen(__ldg(md.O + ob + o));
+#pragma unroll
+            for (int b = 0; b < NB; b++)
+                if (b < nb) c[b] += po * widen(__ldg(Gprev + (size_t)jsh[b * md.z + o] * md.n + sp));
+        }
+        const size_t first = predStart[(size_t)a * md.n + sp];
+        const unsigned cnt = predCount[(size_t)a * md.n + sp];
+#pragma unroll 2
+        for (unsigned k = 0; k < cnt; k++) {
+            const uint2 e = __ldg(pred + first + k);
+            const size_t row = ((size_t)e.x * md.m + a) * md.ns + __ldg(predK + first + k);
+            const double t = widen(__uint_as_float(e.y));
+            double u = 0.0;
+            bool nz = false;
+#pragma unroll
+            for (int b = 0; b < NB; b++)
+                if (b < nb) {
+                    const double lb = lsh[(size_t)b * md.n + e.x];
+                    if (nonzero(lb)) {
+                        w[b] += t * lb;
+                        u += lb * c[b];
+                        nz = true;
+                    }
+                }
+            if (nz) atomicAdd(dT + row, g * u);
         }
     }
-    __syncthreads();
-    for (unsigned sp = threadIdx.x; sp < md.n; sp += blockDim.x) {
-        const double w = wsh[sp];
-        if (w == 0.0) continue;
-        const size_t ob = ((size_t)a * md.n + sp) * md.z;
-        for (unsigned o = 0; o < md.z; o++) {
-            const size_t gj = (size_t)jsh[o] * md.n + sp;
-            atomicAdd(dO + ob + o, g * w * (double)Gprev[gj]);
-            atomicAdd(lamPrev + gj, g * (double)md.O[ob + o] * w);
+    bool nzb[NB], nz = false;
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+        nzb[b] = nonzero(w[b]);
+        nz |= nzb[b];
+        w[b] *= g;
+    }
+    if (!__any_sync(0xffffffffu, nz)) return;
+    double *tile = tiles + (size_t)(threadIdx.x >> 5) * 32 * 9;
+    for (unsigned o0 = 0; o0 < md.z; o0 += 8) {
+        const unsigned oEnd = min(8u, md.z - o0);
+        for (unsigned q = 0; q < oEnd; q++) {
+            const unsigned o = o0 + q;
+            const double po = nz ? widen(__ldg(md.O + ob + o)) : 0.0;
+            double d = 0.0;
+#pragma unroll
+            for (int b = 0; b < NB; b++)
+                if (nzb[b]) {
+                    const size_t gj = (size_t)jsh[b * md.z + o] * md.n + sp;
+                    d += w[b] * widen(__ldg(Gprev + gj));
+                    atomicAdd(lamPrev + gj, po * w[b]);
+                }
+            if constexpr (kStaged) tile[lane * 9 + q] = d;
+            else if (nz) atomicAdd(dO + ob + o, d);
+        }
+        if constexpr (kStaged) {
+            __syncwarp();
+            const size_t ob0 = ((size_t)a * md.n + sp0) * md.z + o0;
+            for (unsigned t = lane; t < 32u * 8u; t += 32u) {
+                const unsigned k = t >> 3, q = t & 7u;
+                const double d = q < oEnd ? tile[k * 9 + q] : 0.0;
+                if (nonzero(d)) atomicAdd(dO + ob0 + (size_t)k * md.z + q, d);
+            }
+            __syncwarp();
         }
     }
 }
@@ -340,6 +471,9 @@ struct AdjBuffers {
     float *CT = nullptr, *seg = nullptr;
     double *lamA = nullptr, *lamB = nullptr, *vals = nullptr, *V = nullptr;
     unsigned *istar = nullptr;
+    unsigned *predCount = nullptr, *predFilled = nullptr, *predK = nullptr;
+    unsigned long long *predStart = nullptr, *predNext = nullptr;
+    uint2 *pred = nullptr;
 };
 
 // Gamma_t from Gamma_{t-1} in FP64 with recorded selections:
@@ -411,17 +545,24 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
     }
     AdjModel md{pomdp->n, pomdp->ns, pomdp->m, pomdp->z, pomdp->r, pomdp->gamma,
                 pomdp->d_S, pomdp->d_T, pomdp->d_O, pomdp->d_R};
-    const size_t stepSmem = 2 * (size_t)md.n * sizeof(double) + (size_t)md.z * sizeof(unsigned);
+    // Four beliefs per block, or two, where four blocks fit on an SM.
+    auto step_smem = [&](size_t nb) {
+        return nb * ((size_t)md.n * sizeof(double) + md.z * sizeof(unsigned)) +
+               (nb > 1 ? kStepThreads * 9 * sizeof(double) : 0);
+    };
+    const unsigned nb = step_smem(4) <= kStepSmem ? 4u : step_smem(2) <= kStepSmem ? 2u : 1u;
+    const size_t stepSmem = step_smem(nb);
+    auto step = nb == 4 ? adjoint_step_kernel<4, true> : nb == 2 ? adjoint_step_kernel<2, true>
+                                                                 : adjoint_step_kernel<1, false>;
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-            stepSmem > (size_t)optin) {
+            2 * (size_t)md.n * sizeof(double) + md.z * sizeof(unsigned) > (size_t)optin) {
         cudaGetLastError();
         NOVA_ERR(fn, "Too many states for the reverse step's shared-memory buffers.");
         return NOVA_ERROR_INVALID_DATA;
     }
-    if (stepSmem > 48 * 1024 &&
-            !allow_dynamic_smem(adjoint_step_kernel, stepSmem)) {
+    if (!allow_dynamic_smem(step, stepSmem)) {
         cudaGetLastError();
         NOVA_ERR(fn, "Failed to configure the reverse step kernel.");
         return NOVA_ERROR_KERNEL_EXECUTION;
@@ -442,6 +583,12 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
     bf.arena.add(&bf.vals, r);
     bf.arena.add(&bf.V, 1);
     bf.arena.add(&bf.istar, 1);
+    bf.arena.add(&bf.predCount, (size_t)m * n);
+    bf.arena.add(&bf.predFilled, (size_t)m * n);
+    bf.arena.add(&bf.predStart, (size_t)m * n);
+    bf.arena.add(&bf.predNext, 1);
+    bf.arena.add(&bf.pred, (size_t)m * n * ns);
+    bf.arena.add(&bf.predK, (size_t)m * n * ns);
     const bool manyActions = m > 8192;
     if (manyActions) bf.arena.add(&bf.cursor, (size_t)horizon * m);
     if ((rc = bf.arena.commit(fn, "the adjoint")) != NOVA_SUCCESS) return rc;
@@ -471,11 +618,23 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
     if (cudaMemset(d_dR, 0, (size_t)n * m * sizeof(double)) != cudaSuccess ||
             cudaMemset(d_dT, 0, (size_t)n * m * ns * sizeof(double)) != cudaSuccess ||
             cudaMemset(d_dO, 0, (size_t)m * n * z * sizeof(double)) != cudaSuccess ||
-            cudaMemset(bf.lamA, 0, rn * sizeof(double)) != cudaSuccess) {
+            cudaMemset(bf.lamA, 0, rn * sizeof(double)) != cudaSuccess ||
+            cudaMemset(bf.predCount, 0, (size_t)m * n * sizeof(unsigned)) != cudaSuccess ||
+            cudaMemset(bf.predNext, 0, sizeof(unsigned long long)) != cudaSuccess) {
         cudaGetLastError();
         NOVA_ERR(fn, "Failed to clear the gradients.");
         return NOVA_ERROR_KERNEL_EXECUTION;
     }
+
+    const unsigned predBlocks = (unsigned)std::min<size_t>(ceil_div((size_t)m * n * ns, 256), 65535u * 8u);
+    adj_pred_count_kernel<<<predBlocks, 256>>>(md, bf.len, bf.predCount);
+    if ((rc = check_launch(fn, "predecessor counts")) != NOVA_SUCCESS) return rc;
+    adj_pred_place_kernel<<<ceil_div((size_t)m * n, 256), 256>>>((size_t)m * n, bf.predCount, bf.predNext,
+                                                                 bf.predStart, bf.predFilled);
+    if ((rc = check_launch(fn, "predecessor places")) != NOVA_SUCCESS) return rc;
+    adj_pred_fill_kernel<<<predBlocks, 256>>>(md, bf.len, bf.predStart, bf.predFilled, bf.pred,
+                                              bf.predK);
+    if ((rc = check_launch(fn, "predecessor lists")) != NOVA_SUCCESS) return rc;
 
     // Recompute the segment of checkpoint c: seg[q] = Gamma_{ck + q} for
     // q = 0 .. last (last = k - 1, or horizon - ck for the final segment,
@@ -523,9 +682,10 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
             NOVA_ERR(fn, "Failed to clear the adjoint.");
             return NOVA_ERROR_KERNEL_EXECUTION;
         }
-        adjoint_step_kernel<<<r, 256, stepSmem>>>(md, bf.len, bf.seg + (size_t)(p - segStart) * rn,
-                                                  d_actions + (size_t)p * r, d_selects + (size_t)p * r * z, bf.lamA,
-                                                  bf.lamB, d_dR, d_dT, d_dO);
+        step<<<dim3(groups * (kGroup / nb), ceil_div(n, kStepThreads)), kStepThreads, stepSmem>>>(
+            md, bf.predCount, bf.predStart, bf.pred, bf.predK, bf.seg + (size_t)(p - segStart) * rn,
+            bf.acts + (size_t)p * groups, bf.ids + (size_t)p * groups * kGroup, d_selects + (size_t)p * r * z, bf.lamA,
+            bf.lamB, d_dR, d_dT, d_dO);
         if ((rc = check_launch(fn, "reverse step")) != NOVA_SUCCESS) return rc;
         std::swap(bf.lamA, bf.lamB);
     }

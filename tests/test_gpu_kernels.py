@@ -364,3 +364,24 @@ def test_choices_below_the_sentinel(n, z, r, rz, mode):
     got, pi, stats, want, po = backups(md, mode, 2)
     np.testing.assert_array_equal(bits(got), bits(want))
     np.testing.assert_array_equal(pi, po)
+
+
+@pytest.mark.parametrize("n,m,z,ns,r", [(3, 2, 1, 2, 5), (31, 1, 9, 4, 70), (97, 3, 17, 5, 33), (1430, 2, 8, 6, 20),
+                                        (1500, 2, 3, 7, 19), (3100, 2, 5, 3, 9)])
+def test_reverse_steps(n, m, z, ns, r):
+    """Four, two and one belief per block, beliefs without an adjoint among
+    them, observations and states that are no multiple of a tile, ragged
+    successor rows: against the FP64 reverse mode with the same selections
+    (which differs by the FP32 rounding of the alphas)."""
+    from nova_gb300.pomdp_adjoint import pbvi_record_and_adjoint
+    md = synth.random_pomdp(n=n, m=m, z=z, ns=ns, r=r, rz=min(5, n), gamma=0.9, horizon=4, seed=n + r)
+    rng = np.random.default_rng(n)
+    length = rng.integers(1, ns + 1, size=(n, m, 1))
+    md["S"] = np.where(np.arange(ns) < length, md["S"], -1).astype(np.int32)
+    md["GammaInitial"] = rng.normal(-3.0, 1.0, size=(r, n)).astype(np.float32)
+    b0 = np.full(n, 1.0 / n, np.float32)
+    V, istar, dR, dT, dO, dG, acts, sels = pbvi_record_and_adjoint(md, b0, 4, 2)
+    want = orc.pbvi_fixed_reverse_f64(md, md["GammaInitial"], acts, sels, b0, istar=istar)
+    assert abs(V - want[0]) <= 1e-4
+    for x, y in zip((dR, dT, dO, dG), want[1:]):
+        assert np.abs(x - y).max() <= 1e-5 * np.abs(y).max()

@@ -15,13 +15,16 @@
 //                       C = fl(O(a,S,o) * T(s,a,l)) in two layouts
 //   * dedup_*           bitwise-identical alpha rows collapse to the lowest
 //                       index (they score identically, and lowest j wins)
-//   * exact_score       per (i,a): all observations x all unique alphas, lanes
-//                       over alphas reading the transposed alpha table
-//                       (coalesced), coefficients broadcast from shared memory
-//   * action_value      per (i,a): alpha_a on the belief support and its value
-//   * assemble          per belief: action argmax, full alpha_{a*} over n states
-// The tensor-core scoring (pbvi_tc.cu) replaces exact_score for rows whose
-// argmax it can prove and hands the rest back to exact_score.
+//   * proj_*            projection table of every (a, o, state, unique alpha),
+//                       in one of two layouts
+//   * scan_all, scan_rows  exact argmax over the table, of all rows or of the
+//                       (a, o, i) rows that the tensor cores leave open
+//   * action_value_proj, assemble_proj  per (i,a) the value of alpha_a, per
+//                       belief the action argmax and alpha_{a*}, from the table
+//   * exact_score, action_value, assemble  the same without a table, from the
+//                       model and the alphas
+// The tensor-core scoring (pbvi_tc.cu) replaces the scan for rows whose argmax
+// it can prove and hands the rest back to it.
 
 #include "pbvi.h"
 
@@ -847,6 +850,7 @@ __global__ void __launch_bounds__(256) scan_rows_kernel(DevModel md, const unsig
     unsigned *sk = reinterpret_cast<unsigned *>(sh + md.rz);     // [rz]
     __shared__ float redV[8];
     __shared__ unsigned redU[8];
+    __shared__ size_t place;
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (nRowsDev) nRows = min(nRows, *nRowsDev);
     for (unsigned w = blockIdx.x; w < nRows; w += gridDim.x) {
@@ -858,6 +862,8 @@ __global__ void __launch_bounds__(256) scan_rows_kernel(DevModel md, const unsig
             bk[k] = md.B[(size_t)i * md.rz + k];
             sk[k] = (unsigned)md.Z[(size_t)i * md.rz + k];
         }
+        // Worked out beside the loads: at the end the block waits for thread 0.
+        if (threadIdx.x == blockDim.x - 1) place = ((size_t)i * md.m + ao / md.z) * md.z + ao % md.z;
         __syncthreads();
         const float *P = pv.slab(ao);
         float best = NOVA_FLT_MIN;
@@ -887,7 +893,7 @@ __global__ void __launch_bounds__(256) scan_rows_kernel(DevModel md, const unsig
                 runV[w] = best;
                 runU[w] = bu;
             } else {   // the last column chunk
-                ustar[((size_t)i * md.m + ao / md.z) * md.z + ao % md.z] = bu;
+                ustar[place] = bu;
             }
         }
     }
@@ -1277,11 +1283,20 @@ struct ScanShape {
     unsigned alphas, threads;
 };
 static ScanShape scan_all_shape(const DevModel &md) {
-    for (unsigned alphas = 64; alphas >= 4; alphas /= 2)
-        for (unsigned threads = 1024; threads >= 256; threads /= 2)
-            if (scan_all_smem(md, alphas, threads) <= kScanSmemMax && scan_all_smem(md, 4, 128) <= kScanSmemMax)
-                return ScanShape{alphas, threads};
+    for (unsigned alphas = 64; alphas >= 16; alphas /= 2)
+        for (unsigned threads = 1024; threads >= 512; threads /= 2)
+            if (scan_all_smem(md, alphas, threads) <= kScanSmemMax) return ScanShape{alphas, threads};
     return ScanShape{0, 0};
+}
+// Blocks of 32 and 64 alphas score 4.2 to 5.6e12 terms a second (n = 512 to
+// 1,100), blocks of 16 1.6e12 (n = 2,048) with half as many alphas to a read of
+// a belief's list and more bank conflicts. Scanning row by row over the
+// alpha-contiguous table is 2.3e12 while a (a, o) slab stays in L2 beside
+// others (n = 1,500 and 2,048 with 2,048 alphas: 12 and 16 MB), 1.3e12 above
+// (n = 1,500 with 4,096 alphas, 24 MB: 38 ms in blocks, 57 by rows).
+static bool scan_all_wanted(const DevModel &md) {
+    const unsigned alphas = scan_all_shape(md).alphas;
+    return alphas >= 32 || (alphas == 16 && (size_t)md.n * md.r * sizeof(float) > (16u << 20));
 }
 
 int BackupEngine::scan_all(unsigned nU, const char *fn) {
@@ -1323,7 +1338,7 @@ int BackupEngine::scan_rows(const unsigned *rowList, unsigned nRows, unsigned nU
     choicesAsKeys = false;
     if (nRows == 0) return NOVA_SUCCESS;
     int rc;
-    if (rowList == nullptr && projStateMajor) return scan_all(nU, fn);
+    if (rowList == nullptr && projStateMajor && scan_all_wanted(md)) return scan_all(nU, fn);
     if ((rc = scan_capacity(nRows, fn)) != NOVA_SUCCESS) return rc;
     // Column chunk: one (a, o) slice of at most ~48 MB stays L2-resident.
     size_t chunk = ((48ull << 20) / ((size_t)md.n * sizeof(float))) / 256 * 256;
@@ -1512,7 +1527,7 @@ bool BackupEngine::state_major_wanted(bool tensor) const {
     // units of 16 bytes (64 GB).
     if (md.n * (gtCols / 4) >= 1ull << 32)
         return false;
-    return tensor ? lastScanFrac <= 0.01f : scan_all_shape(md).alphas != 0;
+    return tensor ? lastScanFrac <= 0.01f : scan_all_wanted(md);
 }
 
 bool BackupEngine::fixed_ready() const {

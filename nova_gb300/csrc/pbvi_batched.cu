@@ -231,7 +231,7 @@ double solver_footprint(const POMDP *p) {
     const double rPad = (double)((p->r + 127) / 128 * 128), nPad = (double)((p->n + 63) / 64 * 64);
     const double operand = mz * rPad * nPad * 2.0;
     const double table = mz * nPad * (double)((p->r + 31) / 32 * 32) * 4.0;
-    const double lists = mz * r * 8.0 * (32.0 * 8.0) + mz * r * 16.0;
+    const double lists = mz * r * (nPad <= 2048.0 ? 4.0 : 8.0) * (32.0 * 8.0) + mz * r * 16.0;
     const double coef = 2.0 * n * p->m * p->ns * p->z * 4.0;
     const double alphas = 5.0 * r * n * 4.0 + mz * r * 16.0;
     return operand + table + lists + coef + alphas;

@@ -77,10 +77,13 @@ constexpr int BM = 128;            // rows (beliefs) per tile
 constexpr int BN = 256;            // alphas per tile
 constexpr int BK = 64;             // K (states) per stage: 128 bytes of BF16
 constexpr int STAGES = 4;
-constexpr int MAX_LISTS = 8;       // candidate lists per row: two per alpha group
 constexpr unsigned LIST_SLOTS = 32;            // a list's header and entries: 256 bytes
 constexpr unsigned LIST_CAP = LIST_SLOTS - 1;  // entries per list
-constexpr size_t kRowListBytes = MAX_LISTS * LIST_SLOTS * 8;  // a row's lists
+// Models of at most this many (padded) states choose between one and two alpha
+// groups, larger ones take four; a group leaves two candidate lists per row.
+constexpr size_t kTuneMaxNPad = 2048;
+constexpr size_t max_lists(size_t nPad) { return nPad <= kTuneMaxNPad ? 4 : 8; }
+constexpr size_t row_list_bytes(size_t nPad) { return max_lists(nPad) * LIST_SLOTS * 8; }
 constexpr unsigned kNoneU = 0xffffffffu;
 constexpr int A_STAGE_BYTES = BM * BK * 2;   // 16 KB
 constexpr int B_STAGE_BYTES = BN * BK * 2;   // 32 KB
@@ -105,8 +108,8 @@ struct TcState {
     // packing blocks; what is accumulated is 0 again after an update (scalClean).
     unsigned *scal = nullptr;
     bool scalClean = false;
-    // [MZ][r][MAX_LISTS][LIST_SLOTS]: slot 0 of a list is {best score that found no room, entries}, then
-    // {score, unique alpha} in the order of the alphas.
+    // [MZ][r][lists of the launch][LIST_SLOTS]: slot 0 of a list is {best score that found no room, entries}, then
+    // {score, unique alpha}.
     uint2 *cand = nullptr;
     unsigned *rowFlag = nullptr;    // [MZ*r] rows needing the exact scan
     unsigned *rowCand = nullptr;    // [MZ*r] alphas each row re-scored exactly in the merge
@@ -127,7 +130,7 @@ struct TcState {
     unsigned tuneNext = 0;          // next trial
     bool tuneWarm = false;          // the first tensor-core update (lazy set-up) is not timed
     unsigned groupsUsed = 0;        // groups of the last launch
-    float tuneCost[3] = {0, 0, 0};  // one per tuned schedule
+    float tuneCost[2] = {0, 0};  // one per tuned schedule
     // The launch prepared by tc_prepare for tc_gemm / tc_finish.
     struct Launch {
         unsigned nU = 0, nTiles = 0, groups = 0, lists = 0, kSplit = 1;
@@ -136,13 +139,13 @@ struct TcState {
     } last;
 };
 
-// Alpha groups per row tile that small models time.
-constexpr unsigned kSchedules[3] = {4u, 2u, 1u};
-constexpr int kTunedSchedules = 3;
-// Deep contractions keep the epilogue hidden behind the MMAs and take the most
-// groups (the evenest split) without tuning.
-constexpr int kDeepSchedule = 0;
-constexpr size_t kTuneMaxNPad = 2048;
+// Alpha groups per row tile: the first two are timed on small models. Deep
+// contractions keep the epilogue hidden behind the MMAs and take the third (the
+// evenest split) without tuning. Four groups on small models were never the
+// fastest by more than the timing's noise, and their lists would double the
+// memory that a solver of many rows allocates.
+constexpr unsigned kSchedules[3] = {2u, 1u, 4u};
+constexpr int kTunedSchedules = 2, kDeepSchedule = 2;
 
 void tc_release(TcState *tc) {
     if (!tc) return;
@@ -156,7 +159,7 @@ bool tc_supported(const DevModel &md) {
     // transposed O where the candidate lists will be; the row index must stay
     // in TMA's 32-bit coordinate range.
     const size_t nPad = round_up(md.n, BK), rPad = round_up(md.r, BM);
-    return md.n <= 40000 && nPad * sizeof(float) <= md.r * kRowListBytes &&
+    return md.n <= 40000 && nPad * sizeof(float) <= md.r * row_list_bytes(nPad) &&
            (size_t)md.m * md.z * rPad < (1ull << 31) && nPad < (1ull << 31) && md.r >= 1;
 }
 
@@ -296,6 +299,68 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 __device__ __forceinline__ float max8(const float *v) {
     return max3(max3(max3(v[0], v[1], v[2]), v[3], v[4]), max3(v[5], v[6], v[7]), v[7]);
 }
+// Sorted top-K of (score, alpha) in registers; `excl` is the best score
+// that fell off (or never entered) the list.
+template <int K>
+struct TopList {
+    float v[K];
+    unsigned u[K];
+    float excl;
+    __device__ __forceinline__ void reset() {
+#pragma unroll
+        for (int k = 0; k < K; k++) { v[k] = -INFINITY; u[k] = kNoneU; }
+        excl = -INFINITY;
+    }
+    __device__ __forceinline__ void push(float x, unsigned idx) {
+        if (!(x > v[K - 1])) {   // also drops NaN
+            excl = fmaxf(excl, x);
+            return;
+        }
+        excl = fmaxf(excl, v[K - 1]);
+        // insertion from the bottom; equal scores keep the earlier (lower) index first
+#pragma unroll
+        for (int k = K - 1; k > 0; k--) {
+            const bool shift = x > v[k - 1];
+            const bool place = !shift && x > v[k];
+            if (shift) { v[k] = v[k - 1]; u[k] = u[k - 1]; }
+            else if (place) { v[k] = x; u[k] = idx; }
+        }
+        if (x > v[0]) { v[0] = x; u[0] = idx; }
+    }
+};
+
+// Branch-free helpers over one 32-column chunk of a row's scores.
+__device__ __forceinline__ unsigned chunk_mask(const float (&v)[32], float lim) {
+    unsigned t[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++)
+        t[k] = (v[2 * k] >= lim ? 1u << (2 * k) : 0u) | (v[2 * k + 1] >= lim ? 1u << (2 * k + 1) : 0u);
+#pragma unroll
+    for (int w = 8; w > 0; w >>= 1)
+#pragma unroll
+        for (int k = 0; k < w; k++) t[k] = t[2 * k] | t[2 * k + 1];
+    return t[0];
+}
+// The smallest float above a finite or -inf f (+0 and -0 step to the
+// smallest subnormal): x > f is x >= next_up(f) for every non-NaN x.
+__device__ __forceinline__ float next_up(float f) {
+    const unsigned b = __float_as_uint(f);
+    if ((b & 0x7fffffffu) == 0u) return __uint_as_float(1u);
+    return __uint_as_float((b & 0x80000000u) ? b - 1u : b + 1u);
+}
+// v[c] for a run-time c without indexing the register array.
+__device__ __forceinline__ float chunk_select(const float (&v)[32], unsigned c) {
+    float t[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) t[k] = (c & 1u) ? v[2 * k + 1] : v[2 * k];
+    unsigned bit = 2u;
+#pragma unroll
+    for (int w = 8; w > 0; w >>= 1, bit <<= 1)
+#pragma unroll
+        for (int k = 0; k < w; k++) t[k] = (c & bit) ? t[2 * k + 1] : t[2 * k];
+    return t[0];
+}
+
 // Drops a list's entries below the limit; returns how many are left.
 __device__ __forceinline__ unsigned list_trim(uint2 *list, unsigned count, float lim) {
     unsigned kept = 0;
@@ -321,7 +386,7 @@ __device__ __forceinline__ float row_margin(const float *__restrict__ a1, const 
 struct UnitParams {
     const CUtensorMap *tmA, *tmB;
     unsigned ao, mt, g, nt0, nt1;
-    unsigned rPad, r, nU, kBlocks, kSplit;
+    unsigned rPad, r, nU, kBlocks, kSplit, lists;
     const float *a1, *d1;
     const unsigned *scal;
     uint2 *cand;
@@ -336,7 +401,7 @@ struct SingleUnits {
     __device__ __forceinline__ unsigned total() const { return MZ * mTiles * groups; }
     __device__ __forceinline__ void get(unsigned unit, UnitParams &p) const {
         decode_unit(unit, groups, mTiles, nTiles, p.ao, p.mt, p.g, p.nt0, p.nt1);
-        p.rPad = rPad; p.r = r; p.nU = nU; p.kBlocks = kBlocks; p.kSplit = kSplit;
+        p.rPad = rPad; p.r = r; p.nU = nU; p.kBlocks = kBlocks; p.kSplit = kSplit; p.lists = 2u * groups;
         p.a1 = a1; p.d1 = d1; p.scal = scal; p.cand = cand;
     }
 };
@@ -370,11 +435,12 @@ struct BatchUnits {
         decode_unit(unit - b.unitStart, b.groups, b.mTiles, b.nTiles, p.ao, p.mt, p.g, p.nt0, p.nt1);
         p.tmA = &b.tmA; p.tmB = &b.tmB;
         p.rPad = b.rPad; p.r = b.r; p.nU = b.nU; p.kBlocks = b.kBlocks; p.kSplit = b.kSplit;
+        p.lists = 2u * b.groups;
         p.a1 = b.a1; p.d1 = b.d1; p.scal = b.scal; p.cand = b.cand;
     }
 };
 
-template <class Units>
+template <bool kSorted, class Units>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) tc_score_gemm_kernel(
         const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, uint32_t idesc,
         const Units units) {
@@ -490,11 +556,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) tc_score_gemm_kernel(
         // 400,000 rows): 591 us with a sorted list in registers, 348 so; 200
         // states: 692 to 395; 512: 135 to 101 (its MMAs need 71); 700 with
         // 12 candidates a row: 354 to 225.
+        // Behind a deep contraction's MMAs the epilogue costs nothing, and its
+        // lists are kept sorted in registers (kSorted), so that a full one
+        // loses its least entry: in BF16 at n = 4,096, whose wide margin lists
+        // 24 candidates a row, 91 rows are left to the exact scan instead of
+        // 17,855 (113 ms of an update of 499).
         const unsigned quarter = warp & 3u;   // TMEM lanes this warp may access
         const unsigned half = (warp - 2u) >> 2;
         const unsigned rowInTile = quarter * 32u + lane;
         const float qnan = __uint_as_float(0x7fc00000u);
         unsigned acc = 0, accPhase = 0;
+        TopList<kSorted ? (int)LIST_CAP : 1> top;
         for (unsigned unit = blockIdx.x; unit < totalUnits && !*abortFlag; unit += gridDim.x) {
             UnitParams p;
             unit_params(unit, p);
@@ -509,9 +581,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) tc_score_gemm_kernel(
             // tile's padding skip everything.
             const float thr = real ? row_margin(p.a1, p.d1, (size_t)ao * p.rPad + iRow, escale, dscale) : 0.0f;
             float best = real ? -INFINITY : INFINITY, lim = best;
-            uint2 *list = p.cand + (((size_t)ao * p.r + (real ? iRow : 0u)) * MAX_LISTS + 2u * p.g + half) * LIST_SLOTS;
+            uint2 *list = p.cand + (((size_t)ao * p.r + (real ? iRow : 0u)) * p.lists + 2u * p.g + half) * LIST_SLOTS;
             unsigned count = 0;
             float excl = -INFINITY, limTrim = -INFINITY;
+            if constexpr (kSorted) top.reset();
             volatile unsigned long long *myBest = &bar->best[half][rowInTile];
             volatile unsigned long long *otherBest = &bar->best[half ^ 1u][rowInTile];
             const unsigned long long tag = (unsigned long long)(unit + 1u) << 32;
@@ -548,6 +621,22 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) tc_score_gemm_kernel(
                         // listed.
                         best = fmaxf(best, mx);
                         lim = best - thr;
+                        if constexpr (kSorted) {
+                            // Scores at or below the list's last entry f would
+                            // only raise the dropped maximum (push's first
+                            // branch). If any score of the chunk is above f,
+                            // its insertion drops f itself, which bounds them
+                            // all; otherwise the chunk's maximum is the
+                            // largest of them.
+                            unsigned mask = chunk_mask(v, fmaxf(lim, next_up(top.v[LIST_CAP - 1])));
+                            if (mask == 0u) top.excl = fmaxf(top.excl, mx);
+                            while (mask) {
+                                const unsigned c = __ffs(mask) - 1;
+                                mask &= mask - 1;
+                                top.push(chunk_select(v, c), u0 + c);
+                            }
+                            continue;
+                        }
 #pragma unroll
                         for (int q = 0; q < 4; q++) {
                             if (!(m8[q] >= lim)) continue;
@@ -585,6 +674,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) tc_score_gemm_kernel(
                 if (acc == 0) accPhase ^= 1u;
             }
             if (!ok) break;
+            if constexpr (kSorted) {
+                excl = top.excl;
+#pragma unroll
+                for (int k = 0; k < (int)LIST_CAP; k++)
+                    if (real && top.u[k] != kNoneU) list[++count] = make_uint2(__float_as_uint(top.v[k]), top.u[k]);
+            }
             if (real) list[0] = make_uint2(__float_as_uint(excl), count);
         }
     }
@@ -918,7 +1013,7 @@ __device__ __forceinline__ RowOutcome merge_look(unsigned row, const DevModel &m
                                                  unsigned *__restrict__ rowCand,
                                                  float *cutOut) {
     const unsigned ao = row / md.r, i = row % md.r;
-    const uint4 *lists = reinterpret_cast<const uint4 *>(cand + (size_t)row * (MAX_LISTS * LIST_SLOTS));
+    const uint4 *lists = reinterpret_cast<const uint4 *>(cand + (size_t)row * (nLists * LIST_SLOTS));
     const float thr = row_margin(a1, d1, (size_t)ao * rPad + i, __uint_as_float(scal[2]), __uint_as_float(scal[7]));
     const float rawBound = a1raw[(size_t)ao * rPad + i] * __uint_as_float(scal[1]);
     float best = -INFINITY, second = -INFINITY, x = -INFINITY;
@@ -977,7 +1072,7 @@ __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const
                                               bool *flagged) {
     const unsigned ao = row / md.r, i = row % md.r;
     const unsigned a = ao / md.z, o = ao % md.z;
-    const uint2 *lists = cand + (size_t)row * (MAX_LISTS * LIST_SLOTS);
+    const uint2 *lists = cand + (size_t)row * (nLists * LIST_SLOTS);
     const unsigned nEnt = nLists * LIST_SLOTS;
     auto slot_of = [&](unsigned e) { return lists + (size_t)(e % nLists) * LIST_SLOTS + e / nLists; };
     uint2 ent[NE];
@@ -1125,7 +1220,7 @@ __global__ void __launch_bounds__(kLookRows) tc_merge_look_kernel(
         float cut = 0.0f;
         res = merge_look(row, md, uniqJ, nLists, rPad, a1, d1, a1raw, scal, cand, badModel, choice, rowFlag, rowCand,
                          &cut);
-        if (res == kRowSeveral) cand[(size_t)row * (MAX_LISTS * LIST_SLOTS)].x = __float_as_uint(cut);
+        if (res == kRowSeveral) cand[(size_t)row * (nLists * LIST_SLOTS)].x = __float_as_uint(cut);
     }
     const unsigned msk = __ballot_sync(0xffffffffu, res == kRowSeveral);
     unsigned at = 0;
@@ -1206,7 +1301,7 @@ __global__ void __launch_bounds__(256, kMergeBlocks) tc_merge_kernel(
             row = __ldg(rowList + row);
         }
         const unsigned ao = row / md.r, i = row % md.r;
-        const uint2 *lists = cand + (size_t)row * (MAX_LISTS * LIST_SLOTS);
+        const uint2 *lists = cand + (size_t)row * (nLists * LIST_SLOTS);
         auto slot_of = [&](unsigned e) { return lists + (e % nLists) * LIST_SLOTS + e / nLists; };
         uint2 ent[NE];
 #pragma unroll
@@ -1477,8 +1572,10 @@ static bool gemm_attributes_set() {
     std::call_once(once, [] {
         const int b = (int)GEMM_SMEM;
         const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        ok = cudaFuncSetAttribute(tc_score_gemm_kernel<SingleUnits>, attr, b) == cudaSuccess &&
-             cudaFuncSetAttribute(tc_score_gemm_kernel<BatchUnits>, attr, b) == cudaSuccess;
+        ok = cudaFuncSetAttribute(tc_score_gemm_kernel<false, SingleUnits>, attr, b) == cudaSuccess &&
+             cudaFuncSetAttribute(tc_score_gemm_kernel<true, SingleUnits>, attr, b) == cudaSuccess &&
+             cudaFuncSetAttribute(tc_score_gemm_kernel<false, BatchUnits>, attr, b) == cudaSuccess &&
+             cudaFuncSetAttribute(tc_score_gemm_kernel<true, BatchUnits>, attr, b) == cudaSuccess;
         if (!ok) cudaGetLastError();
     });
     return ok;
@@ -1496,7 +1593,7 @@ int tc_build(BackupEngine &eng, const char *fn) {
     const size_t aElems = (size_t)tc->MZ * tc->rPad * tc->nPad;
     size_t freeB = 0, totalB = 0;
     cudaMemGetInfo(&freeB, &totalB);
-    const size_t slots = (size_t)tc->MZ * md.r * MAX_LISTS;
+    const size_t slots = (size_t)tc->MZ * md.r * max_lists(tc->nPad);
     const size_t need = aElems * 2 + tc->capN * tc->nPad * 4 + slots * LIST_SLOTS * 8 + (size_t)tc->MZ * md.r * 12;
     if (need + (256ull << 20) > freeB) {
         NOVA_ERR(fn, "Not enough device memory for the tensor-core operands; using exact scoring.");
@@ -1612,7 +1709,8 @@ int tc_gemm(BackupEngine &eng, bool timed, const char *fn) {
     if (timed) cudaEventRecord(tc->g0, eng.stream);
     const SingleUnits units{tc->MZ, (unsigned)tc->rPad, eng.md.r, tc->mTiles, L.nTiles, L.groups, L.nU,
                             (unsigned)(tc->nPad / BK), L.kSplit, tc->a1, tc->d1, tc->scal, tc->cand};
-    tc_score_gemm_kernel<SingleUnits><<<grid, GEMM_THREADS, GEMM_SMEM, eng.stream>>>(tc->tmA, L.tmB, make_idesc(L.fp16 ? 0u : 1u), units);
+    auto gemm = tc->nPad > kTuneMaxNPad ? tc_score_gemm_kernel<true, SingleUnits> : tc_score_gemm_kernel<false, SingleUnits>;
+    gemm<<<grid, GEMM_THREADS, GEMM_SMEM, eng.stream>>>(tc->tmA, L.tmB, make_idesc(L.fp16 ? 0u : 1u), units);
     int rc = check_launch(fn, "tensor-core scoring");
     if (rc != NOVA_SUCCESS) return rc;
     if (timed) cudaEventRecord(tc->g1, eng.stream);
@@ -1710,10 +1808,10 @@ int tc_score_launch(BackupEngine &eng, const float *src, unsigned nU, bool timed
 struct TcBatch {
     struct Group {
         unsigned totalUnits = 0, nModels = 0;
-        bool fp16 = true;
+        bool fp16 = true, sorted = false;
         BatchModel *models = nullptr;   // device work table
     };
-    std::vector<Group> groups;   // one per operand form
+    std::vector<Group> groups;   // one per operand form and kind of list
     int numSMs = 0;
     ~TcBatch() {
         for (auto &g : groups) cudaFree(g.models);
@@ -1731,11 +1829,13 @@ int tc_batch_create(BackupEngine *const *engs, unsigned count, TcBatch **out, co
             return NOVA_ERROR_INVALID_DATA;
         }
         const TcState::Launch &L = tc->last;
+        const bool sorted = tc->nPad > kTuneMaxNPad;
         size_t gi = 0;
-        while (gi < b->groups.size() && b->groups[gi].fp16 != L.fp16) gi++;
+        while (gi < b->groups.size() && (b->groups[gi].fp16 != L.fp16 || b->groups[gi].sorted != sorted)) gi++;
         if (gi == b->groups.size()) {
             b->groups.emplace_back();
             b->groups.back().fp16 = L.fp16;
+            b->groups.back().sorted = sorted;
             host.emplace_back();
         }
         TcBatch::Group &g = b->groups[gi];
@@ -1784,7 +1884,8 @@ int tc_batch_gemm(TcBatch *b, cudaStream_t stream, const char *fn) {
         const unsigned grid = std::min<unsigned>(g.totalUnits, (unsigned)b->numSMs);
         CUtensorMap unused;
         memset(&unused, 0, sizeof(unused));
-        tc_score_gemm_kernel<BatchUnits><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(unused, unused, make_idesc(g.fp16 ? 0u : 1u), units);
+        auto gemm = g.sorted ? tc_score_gemm_kernel<true, BatchUnits> : tc_score_gemm_kernel<false, BatchUnits>;
+        gemm<<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(unused, unused, make_idesc(g.fp16 ? 0u : 1u), units);
         int rc = check_launch(fn, "batched tensor-core scoring");
         if (rc != NOVA_SUCCESS) return rc;
     }

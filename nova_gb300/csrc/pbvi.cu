@@ -629,8 +629,8 @@ constexpr size_t kProjSmemMax = 200 * 1024;
 // the 8 states' l-th successors sit in 8 banks, and each lane's vector
 // gathers of the transposed alphas run two successors ahead of the
 // arithmetic, from one tile of alphas into the next.
-// Bound by FP32 issue (f32x2: 38 T operations/s measured; its pipe is 70 %
-// busy at n = 512) and by the load/store unit's wavefronts (53 %), so what
+// Bound by FP32 issue (f32x2: 38 T operations/s measured; its pipe is 63 %
+// busy at n = 512) and by the load/store unit's wavefronts (61 %), so what
 // else those pipes do counts: row offsets are kept in units of 16 bytes (a
 // gather's address is one multiply-add), coefficients are staged without
 // divisions, and three or four successors per loop step leave no moves

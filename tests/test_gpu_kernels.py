@@ -385,3 +385,17 @@ def test_reverse_steps(n, m, z, ns, r):
     assert abs(V - want[0]) <= 1e-4
     for x, y in zip((dR, dT, dO, dG), want[1:]):
         assert np.abs(x - y).max() <= 1e-5 * np.abs(y).max()
+
+
+@pytest.mark.parametrize("mode", [npp.SCORING_FP16, npp.SCORING_BF16])
+@pytest.mark.parametrize("r,spread", [(33, 1.0), (290, 1e-2), (1030, 1e-3), (1030, 1e-7)])
+def test_sorted_lists(r, spread, mode):
+    """Deep contractions: lists with room, full ones that lose their least
+    entries, and rows with more candidates than lists hold."""
+    md = synth.random_pomdp(n=2100, m=1, z=2, ns=4, r=r, rz=9, gamma=0.9, horizon=1, seed=r)
+    rng = np.random.default_rng(r)
+    md["GammaInitial"] = (rng.normal(-3.0, 1.0, size=(1, 2100)) + spread * rng.normal(size=(r, 2100))).astype(np.float32)
+    G, pi, stats, Go, po = backups(md, mode, 1)
+    assert stats[-1]["scoring"] == mode
+    np.testing.assert_array_equal(bits(G), bits(Go))
+    np.testing.assert_array_equal(pi, po)

@@ -832,8 +832,7 @@ __global__ void __launch_bounds__(1024) scan_all_kernel(DevModel md, const unsig
 }
 
 // The same for listed rows (those a tensor-core update leaves open), or for
-// all of them where a state column of four alphas does not fit in shared
-// memory. One block per row. The alphas are scanned in
+// all of them where scan_all_wanted says so. One block per row. The alphas are scanned in
 // column chunks [u0, u1) so that the (a, o) slice being read stays in L2
 // while the rows of that (a, o) (consecutive in the list) use it; a chunk
 // after the first merges with the running best of the earlier ones, which
@@ -1270,9 +1269,10 @@ int BackupEngine::scan_capacity(size_t rows, const char *fn) {
     return NOVA_SUCCESS;
 }
 
-// Shared memory of scan_all_kernel with `threads` threads, and its shape: as
-// many alphas per block as fit beside the belief lists of at least 256
-// threads' groups (alphas 0: not even four do).
+// Shared memory of scan_all_kernel with `threads` threads (rz, the beliefs'
+// width, counts as much as n: every LANES lanes hold a belief's list), and its
+// shape: 64, 32 or 16 alphas per block, as many as fit with 1,024 or 512
+// threads (alphas 0: not even 16 do).
 constexpr size_t kScanSmemMax = 222 * 1024;
 
 static size_t scan_all_smem(const DevModel &md, unsigned alphas, unsigned threads) {
@@ -1303,10 +1303,13 @@ int BackupEngine::scan_all(unsigned nU, const char *fn) {
     int rc;
     const size_t rows = (size_t)md.m * md.z * md.r;
     if ((rc = scan_capacity(rows, fn)) != NOVA_SUCCESS) return rc;
-    // No more alphas than there are, no more warps than the beliefs keep
-    // busy; 512 threads where two blocks then share an SM.
+    // No more alphas than there are (but fewer alphas share a belief's lanes
+    // among more lists: only while these still fit with 128 threads), no more
+    // warps than the beliefs keep busy; 512 threads where two blocks then
+    // share an SM.
     ScanShape shape = scan_all_shape(md);
-    while (shape.alphas > 4 && shape.alphas / 2 >= nU) shape.alphas /= 2;
+    while (shape.alphas > 4 && shape.alphas / 2 >= nU && scan_all_smem(md, shape.alphas / 2, 128) <= kScanSmemMax)
+        shape.alphas /= 2;
     const unsigned uc = shape.alphas, lanes = uc / 4;
     unsigned threads = 2 * scan_all_smem(md, uc, 512) <= kScanSmemMax ? 512u : shape.threads;
     while (threads > 128 && (threads / lanes > md.r || scan_all_smem(md, uc, threads) > kScanSmemMax)) threads /= 2;
@@ -1325,7 +1328,10 @@ int BackupEngine::scan_all(unsigned nU, const char *fn) {
     }
     auto kernel = uc == 64 ? scan_all_kernel<64> : uc == 32 ? scan_all_kernel<32> : uc == 16 ? scan_all_kernel<16>
                   : uc == 8 ? scan_all_kernel<8> : scan_all_kernel<4>;
-    allow_dynamic_smem(kernel, smem);
+    if (!allow_dynamic_smem(kernel, smem)) {
+        NOVA_ERR(fn, "Failed to configure the exact scan's shared memory.");
+        return NOVA_ERROR_KERNEL_EXECUTION;
+    }
     kernel<<<dim3(tiles, ceil_div(md.r, share)), threads, smem, stream>>>(md, suppLen, proj_view(), nU, chunks, share,
                                                                         scanKeys, 1.0f);
     if ((rc = check_launch(fn, "exact scan")) != NOVA_SUCCESS) return rc;

@@ -399,3 +399,39 @@ def test_sorted_lists(r, spread, mode):
     assert stats[-1]["scoring"] == mode
     np.testing.assert_array_equal(bits(G), bits(Go))
     np.testing.assert_array_equal(pi, po)
+
+
+@pytest.mark.parametrize("mode", [npp.SCORING_EXACT, npp.SCORING_FP16, npp.SCORING_BF16])
+@pytest.mark.parametrize("n,r,rz,distinct", [(256, 40, 256, 1), (300, 64, 300, 2), (400, 40, 400, 1), (430, 33, 430, 5),
+                                             (512, 40, 300, 1), (640, 33, 263, 4), (230, 50, 220, 3), (400, 3, 400, 3),
+                                             (1024, 40, 150, 2)])
+def test_exact_scan_wide_beliefs(n, r, rz, distinct, mode):
+    """Few distinct alphas (the default initial set has one) and beliefs of
+    hundreds of states, whose lists leave no room for four alphas to a block
+    of 128 threads, beside narrow beliefs."""
+    md = synth.random_pomdp(n=n, m=2, z=2, ns=4, r=r, rz=rz, gamma=0.9, horizon=2, seed=n + r)
+    if distinct > 1:
+        pool = np.random.default_rng(n).normal(-3.0, 1.0, size=(distinct, n)).astype(np.float32)
+        md["GammaInitial"] = pool[np.arange(r) % distinct]
+    md["Z"][1:r // 2, 7:], md["B"][1:r // 2, 7:] = -1, 0.0
+    G, pi, stats, Go, po = backups(md, mode, 2)
+    np.testing.assert_array_equal(bits(G), bits(Go))
+    np.testing.assert_array_equal(pi, po)
+
+
+def test_expand_then_solve():
+    """A distinct expansion widens the beliefs to hundreds of states; solves
+    from the default initial alphas, on device and host arrays and batched."""
+    from nova_gb300.pomdp_pbvi import POMDPPBVICPU, solve_batched
+    md = synth.random_pomdp(n=512, m=3, z=4, ns=12, r=40, rz=32, gamma=0.9, horizon=3, seed=4)
+    p = POMDP.from_arrays(md)
+    p.expand(method="distinct_beliefs")
+    md.update({k: v for k, v in p.arrays().items() if k in ("Z", "B")}, r=int(p.r), rz=int(p.rz))
+    assert md["r"] > 40 and 212 <= md["rz"] <= 343
+    G, pi = orc.pbvi_solve(md, GammaInitial=np.full((md["r"], 512), md["GammaInitial"][0, 0], np.float32))
+    p = POMDP.from_arrays(md)
+    p.initialize_gpu()
+    for pol in [POMDPPBVIGPU(p).solve(), POMDPPBVICPU(p).solve(), solve_batched([p])[0],
+                solve_batched([p], persistent=True)[0]]:
+        np.testing.assert_array_equal(bits(pol.gamma_array()), bits(G))
+        np.testing.assert_array_equal(pol.pi_array(), pi)

@@ -1339,6 +1339,9 @@ int BackupEngine::scan_all(unsigned nU, const char *fn) {
     return NOVA_SUCCESS;
 }
 
+// A block holds the states and values of its row's belief.
+static size_t scan_rows_smem(const DevModel &md) { return 2 * (size_t)md.rz * sizeof(float); }
+
 int BackupEngine::scan_rows(const unsigned *rowList, unsigned nRows, unsigned nU, const char *fn,
                             const unsigned *nRowsDev) {
     choicesAsKeys = false;
@@ -1350,9 +1353,13 @@ int BackupEngine::scan_rows(const unsigned *rowList, unsigned nRows, unsigned nU
     size_t chunk = ((48ull << 20) / ((size_t)md.n * sizeof(float))) / 256 * 256;
     if (chunk < 256) chunk = 256;
     const unsigned grid = std::min(nRows, 152u * 16u);
+    if (!allow_dynamic_smem(scan_rows_kernel, scan_rows_smem(md))) {
+        NOVA_ERR(fn, "Too many states per belief for the exact row scan.");
+        return NOVA_ERROR_KERNEL_EXECUTION;
+    }
     for (size_t u0 = 0; u0 < std::max(nU, 1u); u0 += chunk) {
         const unsigned u1 = (unsigned)std::min<size_t>(nU, u0 + chunk);
-        scan_rows_kernel<<<grid, 256, 2 * md.rz * sizeof(float), stream>>>(md, suppLen, proj_view(), (unsigned)u0,
+        scan_rows_kernel<<<grid, 256, scan_rows_smem(md), stream>>>(md, suppLen, proj_view(), (unsigned)u0,
                                                                           u1, rowList, nRows, nRowsDev, scanV,
                                                                           scanU, u0 == 0 ? 1 : 0, u0 + chunk >= nU ? ustar : nullptr);
         if ((rc = check_launch(fn, "exact row scan")) != NOVA_SUCCESS) return rc;
@@ -1472,8 +1479,10 @@ int BackupEngine::backup_all(const float *src, unsigned rGamma, float *dst, unsi
     // With the table, and with few rows expected to be left open, the exact
     // scan reads their number on the device, and nothing is waited for before
     // the update's end (n = 64, r = 256: a read-back and its gap cost 15 us of
-    // an update of 85).
-    const bool deferred = scored && useProjNow && allRows <= kDeferredRows && lastScanFrac <= 0.01f;
+    // an update of 85). Beliefs too wide for the row scan have none launched
+    // unless a row is open.
+    const bool deferred = scored && useProjNow && allRows <= kDeferredRows && lastScanFrac <= 0.01f &&
+                          scan_rows_smem(md) <= kScanSmemMax;
     if (scored) {
         stats.scoring = scoring;
         if (deferred) {

@@ -435,3 +435,20 @@ def test_expand_then_solve():
                 solve_batched([p], persistent=True)[0]]:
         np.testing.assert_array_equal(bits(pol.gamma_array()), bits(G))
         np.testing.assert_array_equal(pol.pi_array(), pi)
+
+
+@pytest.mark.parametrize("n,rz,mode", [(7000, 6150, npp.SCORING_FP16), (7000, 6150, npp.SCORING_EXACT),
+                                       (8192, 7000, npp.SCORING_BF16), (12200, 12200, npp.SCORING_FP16),
+                                       (30000, 29900, npp.SCORING_FP16), (30000, 29900, npp.SCORING_BF16)])
+def test_wide_beliefs_without_open_rows(n, rz, mode):
+    """Beliefs of more states than a block of the row scan holds without
+    raising its limit, or at all, and alphas far enough apart that no row is
+    left to it."""
+    r = 64
+    md = synth.random_pomdp(n=n, m=1, z=2, ns=2, r=r, rz=rz, gamma=0.9, horizon=1, seed=n)
+    rng = np.random.default_rng(n)
+    md["GammaInitial"] = (rng.normal(0.0, 0.1, size=(r, n)) + rng.permutation(r)[:, None]).astype(np.float32)
+    G, pi, stats, Go, po = backups(md, mode, 1)
+    assert stats[-1]["scoring"] == mode and stats[-1]["rowsOverflow"] == 0
+    np.testing.assert_array_equal(bits(G), bits(Go))
+    np.testing.assert_array_equal(pi, po)

@@ -1912,6 +1912,11 @@ static int graph_replay(BackupEngine &e, const float *src, bool *done, const cha
         NOVA_ERR(fn, "A device-side wait timed out; results of this update are invalid.");
         return NOVA_ERROR_KERNEL_EXECUTION;
     }
+    // As the captured update left them: an ordinary one since may have chosen
+    // otherwise, and the selections are recorded through these.
+    e.uniqMap = e.uniqIota;
+    e.useProjNow = true;
+    e.choicesAsKeys = false;
     e.stats.scoring = e.scoring;
     e.stats.uniqueAlphas = e.md.r;
     e.stats.launches = e.graphLaunches[dir];

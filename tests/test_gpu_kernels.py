@@ -452,3 +452,27 @@ def test_wide_beliefs_without_open_rows(n, rz, mode):
     assert stats[-1]["scoring"] == mode and stats[-1]["rowsOverflow"] == 0
     np.testing.assert_array_equal(bits(G), bits(Go))
     np.testing.assert_array_equal(pi, po)
+
+
+def test_recorded_graph_updates_after_ordinary_ones():
+    """Graph mode switched off for an update whose alphas repeat, and on
+    again: the replayed update's recorded selections are alpha indices."""
+    import torch
+    md = synth.random_pomdp(n=40, m=3, z=4, ns=5, r=200, rz=6, gamma=0.95, horizon=14, seed=8)
+    md["Z"], md["B"] = np.repeat(md["Z"][:100], 2, axis=0), np.repeat(md["B"][:100], 2, axis=0)
+    p = POMDP.from_arrays(md)
+    p.initialize_gpu()
+    s = POMDPPBVIGPU(p)
+    s.set_scoring(npp.SCORING_FP16)
+    acts = torch.empty((14, 200), dtype=torch.int32, device="cuda")
+    sels = torch.empty((14, 200, 4), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    replayed = []
+    for t in range(14):
+        s.set_graph(t != 11)
+        assert npp._nova.pomdp_pbvi_update_record_gpu(s.pomdpPtr, s, acts[t].data_ptr(), sels[t].data_ptr()) == 0
+        replayed.append(s.stats()["msTotal"] == 0.0)
+    assert replayed[10] and not replayed[11] and replayed[12] and replayed[13]
+    G, acts_o, sels_o = orc.pbvi_record(md, 14)
+    np.testing.assert_array_equal(acts.cpu().numpy(), acts_o)
+    np.testing.assert_array_equal(sels.cpu().numpy(), sels_o)

@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kThreads) value_tiles_kernel(const float *__re
     __shared__ __align__(16) float sG[2][TK][TA + 4];
     const unsigned tid = threadIdx.x;
     const unsigned b0 = blockIdx.y * TB, a0 = blockIdx.x * TA;
-    if (tile_listed(nnz, b0, count, cap, tid & 31)) return;
+    if (cap != 0u && tile_listed(nnz, b0, count, cap, tid & 31)) return;   // cap 0: no lists, no other kernel
     const unsigned tx = tid % 16, ty = tid / 16;   // alpha group, belief group
     const unsigned long long one2 = pack_f32x2(one, one);
     unsigned long long acc[NB][NA / 2];

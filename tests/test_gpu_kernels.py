@@ -476,3 +476,24 @@ def test_recorded_graph_updates_after_ordinary_ones():
     G, acts_o, sels_o = orc.pbvi_record(md, 14)
     np.testing.assert_array_equal(acts.cpu().numpy(), acts_o)
     np.testing.assert_array_equal(sels.cpu().numpy(), sels_o)
+
+
+@pytest.mark.parametrize("n,r", [(15000, 3), (15000, 700)])
+def test_zero_beliefs_of_many_states(n, r):
+    """Beliefs without a nonzero, alone in a tile of beliefs, where the states
+    are too many for alphas in shared memory: V = 0 with alpha 0's action."""
+    import torch
+    from nova_gb300 import nova_pomdp_alpha_vectors as npav
+    rng = np.random.default_rng(n)
+    G = rng.uniform(-5, 5, size=(r, n)).astype(np.float32)
+    pi = rng.integers(1, 9, size=r).astype(np.int32)
+    B = np.zeros((130, n), np.float32)
+    B[128, 7], B[129, n - 1] = 0.5, 1.0
+    dG, dB, dPi = (torch.as_tensor(x, device="cuda") for x in (G, B, pi))
+    dV, dA = torch.empty(130, device="cuda"), torch.empty(130, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert npav._nova.pomdp_alpha_vectors_value_batched_gpu(dG.data_ptr(), dPi.data_ptr(), r, n, dB.data_ptr(), 130,
+                                                            dV.data_ptr(), dA.data_ptr()) == 0
+    for i in (0, 127, 128, 129):
+        V, a = orc.alpha_value(G, pi.astype(np.uint32), B[i])
+        assert bits(dV[i].cpu().numpy()) == bits(np.float32(V)) and int(dA[i]) == a, i

@@ -70,7 +70,10 @@ public:
         *p = nullptr;
         items.push_back(Item{reinterpret_cast<void **>(p), count * sizeof(T)});
     }
+    // An earlier commit's arrays are given back first (a build that failed and is tried again).
     int commit(const char *fn, const char *what) {
+        cudaFree(base);
+        base = nullptr;
         size_t total = 0;
         for (const Item &i : items) total += (i.bytes + 255) / 256 * 256;
         const int rc = dev_malloc(&base, total, fn, what);

@@ -497,3 +497,23 @@ def test_zero_beliefs_of_many_states(n, r):
     for i in (0, 127, 128, 129):
         V, a = orc.alpha_value(G, pi.astype(np.uint32), B[i])
         assert bits(dV[i].cpu().numpy()) == bits(np.float32(V)) and int(dA[i]) == a, i
+
+
+def test_failed_builds_leak_nothing():
+    """An update that fails while its tables are built, tried again: the
+    device memory in use does not grow."""
+    from nova_gb300._lib import load as lib
+    import torch
+    md = synth.random_pomdp(n=3000, m=8, z=16, ns=16, r=64, rz=8, gamma=0.9, horizon=3, seed=1)
+    p = POMDP.from_arrays(md)
+    p.initialize_gpu()
+    s = POMDPPBVIGPU(p)
+    free = []
+    for _ in range(6):
+        lib().nova_gb300_inject_fault(4, 2)
+        with pytest.raises(RuntimeError):
+            s.update()
+        lib().nova_gb300_inject_fault(0, 0)
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[-1] < 32 << 20
+    s.update()

@@ -706,22 +706,28 @@ __device__ __forceinline__ float from_half_bits(uint16_t b, bool fp16) {
     return __bfloat162float(__ushort_as_bfloat16(b));
 }
 
-// O with the states innermost, [m][z][nPad] (0 past n): 32 x 32 tiles.
+// O with the states innermost, [m][z][nPad] (0 past n): 32 x 32 tiles, the
+// actions over the grid's third dimension (which ends at kMaxGridZ).
+constexpr unsigned kMaxGridZ = 65535;
+
 __global__ void tc_transpose_o_kernel(DevModel md, size_t nPad, float *__restrict__ Ot,
                                       unsigned *__restrict__ badModel) {
     __shared__ float tile[32][33];
-    const unsigned a = blockIdx.z, s0 = blockIdx.x * 32u, o0 = blockIdx.y * 32u;
-    for (unsigned k = threadIdx.y; k < 32u; k += 8u) {
-        float v = 0.0f;
-        if (s0 + k < md.n && o0 + threadIdx.x < md.z) {
-            v = md.O[((size_t)a * md.n + s0 + k) * md.z + o0 + threadIdx.x];
-            if (!(v >= 0.0f)) atomicOr(badModel, 1u);  // the bound assumes non-negative B, T, O
+    const unsigned s0 = blockIdx.x * 32u, o0 = blockIdx.y * 32u;
+    for (unsigned a = blockIdx.z; a < md.m; a += gridDim.z) {
+        for (unsigned k = threadIdx.y; k < 32u; k += 8u) {
+            float v = 0.0f;
+            if (s0 + k < md.n && o0 + threadIdx.x < md.z) {
+                v = md.O[((size_t)a * md.n + s0 + k) * md.z + o0 + threadIdx.x];
+                if (!(v >= 0.0f)) atomicOr(badModel, 1u);  // the bound assumes non-negative B, T, O
+            }
+            tile[k][threadIdx.x] = v;
         }
-        tile[k][threadIdx.x] = v;
+        __syncthreads();
+        for (unsigned k = threadIdx.y; k < 32u; k += 8u)
+            if (o0 + k < md.z) Ot[((size_t)a * md.z + o0 + k) * nPad + s0 + threadIdx.x] = tile[threadIdx.x][k];
+        __syncthreads();
     }
-    __syncthreads();
-    for (unsigned k = threadIdx.y; k < 32u; k += 8u)
-        if (o0 + k < md.z) Ot[((size_t)a * md.z + o0 + k) * nPad + s0 + threadIdx.x] = tile[threadIdx.x][k];
 }
 
 // One block per action and NB beliefs: their successor distributions W in
@@ -1550,8 +1556,8 @@ static int tc_build_operand(BackupEngine &eng, TcState *tc, const char *fn) {
     const float dslack = 1.0f + (float)(tc->nPad + 8) * 1.2e-7f;
     float *Ot = reinterpret_cast<float *>(tc->cand);   // as the lists are written after A is built (tc_supported)
     int rc;
-    tc_transpose_o_kernel<<<dim3((unsigned)(tc->nPad / 32), ceil_div(md.z, 32), md.m), dim3(32, 8), 0, eng.stream>>>(
-        md, tc->nPad, Ot, tc->badModel);
+    const dim3 tiles((unsigned)(tc->nPad / 32), ceil_div(md.z, 32), std::min(md.m, kMaxGridZ));
+    tc_transpose_o_kernel<<<tiles, dim3(32, 8), 0, eng.stream>>>(md, tc->nPad, Ot, tc->badModel);
     if ((rc = check_launch(fn, "observation transpose")) != NOVA_SUCCESS) return rc;
     const size_t wBytes = tc->nPad * sizeof(float);
     const unsigned nb = 4 * wBytes <= kBuildSmem ? 4u : 2 * wBytes <= kBuildSmem ? 2u : 1u;

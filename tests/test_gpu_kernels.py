@@ -517,3 +517,13 @@ def test_failed_builds_leak_nothing():
         free.append(torch.cuda.mem_get_info()[0])
     assert free[0] - free[-1] < 32 << 20
     s.update()
+
+
+def test_scoring_operand_of_many_actions():
+    """More actions than a grid's third dimension holds."""
+    md = synth.random_pomdp(n=20, m=66000, z=1, ns=1, r=33, rz=2, gamma=0.9, horizon=1, seed=3)
+    md["GammaInitial"] = np.random.default_rng(3).normal(-3.0, 1.0, size=(33, 20)).astype(np.float32)
+    G, pi, stats, Go, po = backups(md, npp.SCORING_FP16, 1)
+    assert stats[-1]["scoring"] == npp.SCORING_FP16
+    np.testing.assert_array_equal(bits(G), bits(Go))
+    np.testing.assert_array_equal(pi, po)

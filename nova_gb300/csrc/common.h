@@ -27,6 +27,8 @@ enum FaultKind : unsigned { kFaultNone = 0, kFaultMalloc = 1, kFaultH2D = 2, kFa
 bool fault_fires(FaultKind kind);
 
 int dev_malloc(void **p, size_t bytes, const char *fn, const char *what);
+bool try_malloc(void **p, size_t bytes);                 // false, without a message, where there is no room
+int malloc_failed(const char *fn, const char *what);     // the message, and NOVA_ERROR_DEVICE_MALLOC
 int dev_free(void *p, const char *fn, const char *what);
 int h2d(void *dst, const void *src, size_t bytes, const char *fn, const char *what);
 int d2h(void *dst, const void *src, size_t bytes, const char *fn, const char *what);
@@ -71,13 +73,14 @@ public:
         items.push_back(Item{reinterpret_cast<void **>(p), count * sizeof(T)});
     }
     // An earlier commit's arrays are given back first (a build that failed and is tried again).
-    int commit(const char *fn, const char *what) {
+    // False, without a message, where there is no room.
+    bool try_commit() {
         cudaFree(base);
         base = nullptr;
         size_t total = 0;
         for (const Item &i : items) total += (i.bytes + 255) / 256 * 256;
-        const int rc = dev_malloc(&base, total, fn, what);
-        if (rc == NOVA_SUCCESS) {
+        const bool ok = try_malloc(&base, total);
+        if (ok) {
             size_t at = 0;
             for (const Item &i : items) {
                 *i.p = static_cast<unsigned char *>(base) + at;
@@ -85,8 +88,9 @@ public:
             }
         }
         items.clear();
-        return rc;
+        return ok;
     }
+    int commit(const char *fn, const char *what) { return try_commit() ? NOVA_SUCCESS : malloc_failed(fn, what); }
 };
 
 // Device-side error word: bounded waits write a code here instead of hanging.

@@ -807,22 +807,29 @@ int run_distinct(const ExpWorkspace &ws, std::vector<float> &Bnew, const char *f
     }
     Distinct d{};
     d.cap = std::min(md.n, md.rz);
-    // Beliefs whose successors are held at once: about 512 MB of them.
+    // Beliefs whose successors are held at once: about 512 MB of them, fewer
+    // where these cannot be had.
     const size_t perBelief = (n * mz + md.m * n + 2 * mz) * sizeof(float);
     d.chunk = (unsigned)std::min<size_t>(md.r, std::max<size_t>(1, (512ull << 20) / perBelief));
     float *dB = nullptr;
     Arena arena;
     int rc;
-    arena.add(&dB, rn);
-    arena.add(&d.W, (size_t)d.chunk * md.m * n);
-    arena.add(&d.bp, (size_t)d.chunk * n * mz);
-    arena.add(&d.mass, (size_t)d.chunk * mz);
-    arena.add(&d.bound, (size_t)d.chunk * mz);
-    arena.add(&d.list, (size_t)md.r * d.cap);
-    arena.add(&d.nnz, md.r);
-    arena.add(&d.total, md.r);
-    arena.add(&d.odd, 2);
-    if ((rc = arena.commit(fn, "the successor beliefs")) != NOVA_SUCCESS) return rc;
+    auto allocate = [&]() {
+        arena.add(&dB, rn);
+        arena.add(&d.W, (size_t)d.chunk * md.m * n);
+        arena.add(&d.bp, (size_t)d.chunk * n * mz);
+        arena.add(&d.mass, (size_t)d.chunk * mz);
+        arena.add(&d.bound, (size_t)d.chunk * mz);
+        arena.add(&d.list, (size_t)md.r * d.cap);
+        arena.add(&d.nnz, md.r);
+        arena.add(&d.total, md.r);
+        arena.add(&d.odd, 2);
+        return arena.try_commit();
+    };
+    while (!allocate()) {
+        if (d.chunk == 1) return malloc_failed(fn, "the successor beliefs");
+        d.chunk = (d.chunk + 1) / 2;
+    }
     if (cudaMemsetAsync(d.odd, 0, 2 * sizeof(unsigned)) != cudaSuccess) {
         cudaGetLastError();
         NOVA_ERR(fn, "Failed to clear the belief check.");

@@ -43,17 +43,25 @@ bool fault_fires(FaultKind kind) {
     return false;
 }
 
-int dev_malloc(void **p, size_t bytes, const char *fn, const char *what) {
+bool try_malloc(void **p, size_t bytes) {
     *p = nullptr;
     if (fault_fires(kFaultMalloc) || cudaMalloc(p, bytes == 0 ? 4 : bytes) != cudaSuccess) {
         cudaGetLastError();
         *p = nullptr;
-        char msg[256];
-        snprintf(msg, sizeof(msg), "Failed to allocate device-side memory for %s.", what);
-        NOVA_ERR(fn, msg);
-        return NOVA_ERROR_DEVICE_MALLOC;
+        return false;
     }
-    return NOVA_SUCCESS;
+    return true;
+}
+
+int malloc_failed(const char *fn, const char *what) {
+    char msg[256];
+    snprintf(msg, sizeof(msg), "Failed to allocate device-side memory for %s.", what);
+    NOVA_ERR(fn, msg);
+    return NOVA_ERROR_DEVICE_MALLOC;
+}
+
+int dev_malloc(void **p, size_t bytes, const char *fn, const char *what) {
+    return try_malloc(p, bytes) ? NOVA_SUCCESS : malloc_failed(fn, what);
 }
 
 int dev_free(void *p, const char *fn, const char *what) {

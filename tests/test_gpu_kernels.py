@@ -527,3 +527,19 @@ def test_scoring_operand_of_many_actions():
     assert stats[-1]["scoring"] == npp.SCORING_FP16
     np.testing.assert_array_equal(bits(G), bits(Go))
     np.testing.assert_array_equal(pi, po)
+
+
+def test_distinct_expansion_with_little_memory():
+    """The successors' buffer is made smaller where it cannot be allocated."""
+    from nova_gb300._lib import load as lib
+    md = synth.random_pomdp(n=60, m=2, z=5, ns=4, r=23, rz=6, gamma=0.9, horizon=2, seed=9)
+    p = POMDP.from_arrays(md)
+    want = orc.merge_raw_beliefs(md["Z"], md["B"], orc.expand_distinct(md))
+    lib().nova_gb300_inject_fault(1, 2)
+    try:
+        p.expand(method="distinct_beliefs")
+    finally:
+        lib().nova_gb300_inject_fault(0, 0)
+    out = p.arrays()
+    np.testing.assert_array_equal(out["Z"], want[0])
+    np.testing.assert_array_equal(bits(out["B"]), bits(want[1]))

@@ -363,11 +363,9 @@ struct PerseusCore {
     unsigned *done = nullptr;     // [1] finished blocks of perseus_commit_kernel
     float *partV = nullptr, *proj = nullptr;   // the scoring's partial maxima and projections
     unsigned *partU = nullptr;
-    size_t partCap = 0;
+    Arena parts;
+    unsigned maxSplits = 0;       // that these hold
     std::vector<unsigned> btHost;
-    ~PerseusCore() {
-        cudaFree(partV); cudaFree(partU); cudaFree(proj);
-    }
 
     int build(const DevModel &md, const char *fn) {
         int rc = eng.build(md, fn);
@@ -440,21 +438,21 @@ struct PerseusCore {
         // alpha, and every observation takes row 0 (the reference's best-alpha
         // index is never assigned there, pomdp_perseus_cpu.cpp:78-84).
         const unsigned mz = md.m * md.z;
-        const unsigned splits = std::max(1u, std::min(rGamma, 8192u / mz));
+        if (partV == nullptr) {
+            // Room for every step's splits, allocated once; fewer splits where
+            // the projections (8 rz bytes a warp) cannot be had.
+            for (maxSplits = std::max(1u, std::min(md.r, 8192u / mz));; maxSplits = (maxSplits + 1) / 2) {
+                const size_t most = (size_t)mz * maxSplits;
+                parts.add(&partV, most);
+                parts.add(&partU, most);
+                parts.add(&proj, most * 2 * md.rz);
+                if (parts.try_commit()) break;
+                if (maxSplits == 1) return malloc_failed(fn, "the projections");
+            }
+        }
+        const unsigned splits = std::max(1u, std::min(rGamma, maxSplits));
         const unsigned share = ceil_div(rGamma, splits);
         const size_t need = (size_t)mz * splits;
-        if (need > partCap) {
-            // Room for every later step's splits, allocated once.
-            const size_t most = (size_t)mz * std::max(1u, std::min(md.r, 8192u / mz));
-            cudaFree(partV); cudaFree(partU); cudaFree(proj);
-            partV = proj = nullptr;
-            partU = nullptr;
-            partCap = 0;
-            if ((rc = dev_alloc(&partV, most, fn, "the partial maxima")) != NOVA_SUCCESS) return rc;
-            if ((rc = dev_alloc(&partU, most, fn, "the partial arg-maxima")) != NOVA_SUCCESS) return rc;
-            if ((rc = dev_alloc(&proj, most * 2 * md.rz, fn, "the projections")) != NOVA_SUCCESS) return rc;
-            partCap = most;
-        }
         perseus_score_kernel<<<ceil_div(need, 4), 128, 0, eng.stream>>>(md, eng.succLen, eng.suppLen, eng.C3, G, rGamma,
                                                                         bIndex, splits, share, partV, partU, proj);
         if ((rc = check_launch(fn, "belief scoring")) != NOVA_SUCCESS) return rc;

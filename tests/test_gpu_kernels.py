@@ -543,3 +543,23 @@ def test_distinct_expansion_with_little_memory():
     out = p.arrays()
     np.testing.assert_array_equal(out["Z"], want[0])
     np.testing.assert_array_equal(bits(out["B"]), bits(want[1]))
+
+
+def test_perseus_with_little_memory():
+    """Fewer splits of the alphas where the buffer for all of them cannot be
+    allocated (the solve's fourth allocation)."""
+    from nova_gb300._lib import load as lib
+    from nova_gb300.pomdp_perseus import POMDPPerseusGPU
+    md = synth.random_pomdp(n=40, m=2, z=3, ns=4, r=90, rz=9, gamma=0.9, horizon=4, seed=6)
+    Go, po = orc.perseus_solve(md, seed=3)
+    p = POMDP.from_arrays(md)
+    p.initialize_gpu()
+    alg = POMDPPerseusGPU(p, GammaInitial=md["GammaInitial"])
+    orc.lib().oracle_srand(3)
+    lib().nova_gb300_inject_fault(1, 4)
+    try:
+        pol = alg.solve()
+    finally:
+        lib().nova_gb300_inject_fault(0, 0)
+    np.testing.assert_array_equal(bits(pol.gamma_array()), bits(Go))
+    np.testing.assert_array_equal(pol.pi_array(), po)

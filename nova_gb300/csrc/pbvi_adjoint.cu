@@ -64,7 +64,7 @@ __global__ void adj_len_kernel(unsigned rows, unsigned ns, const int *__restrict
 // CT[a][o][l][s] = fl(O(a,S(s,a,l),o) * T(s,a,l)), the reference's first
 // product (0 past the row end).
 __global__ void adj_coef_kernel(AdjModel md, const unsigned *__restrict__ len, unsigned *__restrict__ ST,
-                                float *__restrict__ CT) {
+                                float *__restrict__ CT, unsigned *__restrict__ predCount) {
     const size_t total = (size_t)md.m * md.ns * md.n;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
         const unsigned s = (unsigned)(e % md.n);
@@ -76,6 +76,7 @@ __global__ void adj_coef_kernel(AdjModel md, const unsigned *__restrict__ len, u
         const unsigned sp = live ? (unsigned)md.S[row] : 0u;
         const float T = live ? md.T[row] : 0.0f;
         ST[e] = sp;
+        if (live) atomicAdd(predCount + (size_t)a * md.n + sp, 1u);
         for (unsigned o = 0; o < md.z; o++)
             CT[(((size_t)a * md.z + o) * md.ns + l) * md.n + s] =
                 live ? fmul(md.O[((size_t)a * md.n + sp) * md.z + o], T) : 0.0f;
@@ -140,7 +141,7 @@ __device__ __forceinline__ void copy_async(float *dst, const float *src, bool wi
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
-template <bool kShared>
+template <int NB, bool kShared>
 __global__ void __launch_bounds__(kReplayThreads) replay_kernel(AdjModel md, const unsigned *__restrict__ len,
                                                                 const unsigned *__restrict__ ST,
                                                                 const float *__restrict__ CT,
@@ -149,60 +150,61 @@ __global__ void __launch_bounds__(kReplayThreads) replay_kernel(AdjModel md, con
                                                                 const unsigned *__restrict__ ids,
                                                                 const unsigned *__restrict__ sel, int wide,
                                                                 float *__restrict__ Gout) {
-    extern __shared__ __align__(16) float rows[];  // [2][kGroup][pitch]
-    const unsigned a = acts[blockIdx.x];
+    extern __shared__ __align__(16) float rows[];  // [2][NB][pitch]
+    const unsigned a = acts[blockIdx.x / (kGroup / NB)];
     if (a == kNoRow) return;
     const unsigned pitch = (md.n + 3u) & ~3u;
-    unsigned id[kGroup];
+    unsigned id[NB];
 #pragma unroll
-    for (unsigned b = 0; b < kGroup; b++) id[b] = ids[blockIdx.x * kGroup + b];
+    for (unsigned b = 0; b < NB; b++) id[b] = ids[blockIdx.x * NB + b];
+    if (NB == 1 && id[0] == kNoRow) return;
     auto chosen = [&](unsigned b, unsigned o) { return Gin + (size_t)min(sel[(size_t)id[b] * md.z + o], md.r - 1) * md.n; };
     auto stage = [&](unsigned o) {
         if constexpr (kShared) {
 #pragma unroll
-            for (unsigned b = 0; b < kGroup; b++) {
+            for (unsigned b = 0; b < NB; b++) {
                 if (id[b] == kNoRow) continue;
                 const float *src = chosen(b, o);
-                float *dst = rows + ((o & 1u) * kGroup + b) * pitch;
+                float *dst = rows + ((o & 1u) * NB + b) * pitch;
                 const unsigned w = wide ? 4u : 1u;
-                for (unsigned s = threadIdx.x * w; s < md.n; s += kReplayThreads * w) copy_async(dst + s, src + s, wide != 0);
+                for (unsigned s = threadIdx.x * w; s < md.n; s += blockDim.x * w) copy_async(dst + s, src + s, wide != 0);
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
     };
-    const unsigned s0 = blockIdx.y * (kReplayThreads * kReplayStates) + threadIdx.x;
-    float alpha[kReplayStates][kGroup];
+    const unsigned s0 = blockIdx.y * (blockDim.x * kReplayStates) + threadIdx.x;
+    float alpha[kReplayStates][NB];
     unsigned L[kReplayStates];
 #pragma unroll
     for (unsigned q = 0; q < kReplayStates; q++) {
-        const unsigned s = s0 + q * kReplayThreads;
+        const unsigned s = s0 + q * blockDim.x;
         const bool live = s < md.n;
         L[q] = live ? len[(size_t)s * md.m + a] : 0u;
         const float R = live ? md.R[(size_t)s * md.m + a] : 0.0f;
 #pragma unroll
-        for (unsigned b = 0; b < kGroup; b++) alpha[q][b] = R;
+        for (unsigned b = 0; b < NB; b++) alpha[q][b] = R;
     }
     stage(0);
     for (unsigned o = 0; o < md.z; o++) {
-        const float *g[kGroup];
+        const float *g[NB];
         if constexpr (kShared) {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();  // observation o's rows are in, observation o - 1's free
             if (o + 1 < md.z) stage(o + 1);
 #pragma unroll
-            for (unsigned b = 0; b < kGroup; b++) g[b] = rows + ((o & 1u) * kGroup + b) * pitch;
+            for (unsigned b = 0; b < NB; b++) g[b] = rows + ((o & 1u) * NB + b) * pitch;
         } else {
 #pragma unroll
-            for (unsigned b = 0; b < kGroup; b++) g[b] = id[b] == kNoRow ? Gin : chosen(b, o);
+            for (unsigned b = 0; b < NB; b++) g[b] = id[b] == kNoRow ? Gin : chosen(b, o);
         }
         const float *C = CT + ((size_t)a * md.z + o) * md.ns * md.n;
         const unsigned *Sa = ST + (size_t)a * md.ns * md.n;
 #pragma unroll
         for (unsigned q = 0; q < kReplayStates; q++) {
-            const unsigned s = s0 + q * kReplayThreads;
-            float vt[kGroup];
+            const unsigned s = s0 + q * blockDim.x;
+            float vt[NB];
 #pragma unroll
-            for (unsigned b = 0; b < kGroup; b++) vt[b] = 0.0f;
+            for (unsigned b = 0; b < NB; b++) vt[b] = 0.0f;
             for (unsigned l0 = 0; l0 < L[q]; l0 += 4) {
                 float c[4];
                 unsigned sp[4];
@@ -216,21 +218,21 @@ __global__ void __launch_bounds__(kReplayThreads) replay_kernel(AdjModel md, con
                 for (unsigned k = 0; k < 4; k++) {
                     if (l0 + k < L[q]) {
 #pragma unroll
-                        for (unsigned b = 0; b < kGroup; b++)
+                        for (unsigned b = 0; b < NB; b++)
                             if (kShared || id[b] != kNoRow) vt[b] = fadd(vt[b], fmul(c[k], g[b][sp[k]]));
                     }
                 }
             }
 #pragma unroll
-            for (unsigned b = 0; b < kGroup; b++) alpha[q][b] = fadd(alpha[q][b], fmul(vt[b], md.gamma));
+            for (unsigned b = 0; b < NB; b++) alpha[q][b] = fadd(alpha[q][b], fmul(vt[b], md.gamma));
         }
     }
 #pragma unroll
     for (unsigned q = 0; q < kReplayStates; q++) {
-        const unsigned s = s0 + q * kReplayThreads;
+        const unsigned s = s0 + q * blockDim.x;
         if (s < md.n) {
 #pragma unroll
-            for (unsigned b = 0; b < kGroup; b++)
+            for (unsigned b = 0; b < NB; b++)
                 if (id[b] != kNoRow) Gout[(size_t)id[b] * md.n + s] = alpha[q][b];
         }
     }
@@ -257,28 +259,31 @@ __global__ void value_rows_kernel(const float *__restrict__ G, unsigned n, const
 // lambda_H[i*] = b.
 __global__ void value_argmax_kernel(unsigned r, unsigned n, const double *__restrict__ vals,
                                     const float *__restrict__ b, double *__restrict__ Vout,
-                                    unsigned *__restrict__ iout, double *__restrict__ lam) {
-    __shared__ double sv[256];
-    __shared__ unsigned si[256];
+                                    unsigned *__restrict__ iout, double *__restrict__ lam,
+                                    unsigned *__restrict__ live) {
+    __shared__ double sv[8];
+    __shared__ unsigned si[8];
     double best = (double)NOVA_FLT_MIN;
     unsigned bi = kNoRow;
-    for (unsigned j = threadIdx.x; j < r; j += blockDim.x)
+    for (unsigned j = threadIdx.x; j < r; j += 256)
         if (vals[j] > best) { best = vals[j]; bi = j; }
-    sv[threadIdx.x] = best;
-    si[threadIdx.x] = bi;
-    __syncthreads();
-    __shared__ unsigned istar;
-    if (threadIdx.x == 0) {
-        for (unsigned t = 1; t < blockDim.x; t++) {
-            if (si[t] == kNoRow) continue;
-            if (si[0] == kNoRow || sv[t] > sv[0] || (sv[t] == sv[0] && si[t] < si[0])) { sv[0] = sv[t]; si[0] = si[t]; }
-        }
-        *Vout = sv[0];
-        *iout = si[0];
-        istar = si[0];
+    auto take = [&](double v, unsigned j) {
+        if (j != kNoRow && (bi == kNoRow || v > best || (v == best && j < bi))) { best = v; bi = j; }
+    };
+    for (int off = 16; off > 0; off >>= 1) {
+        const double v = __shfl_xor_sync(0xffffffffu, best, off);
+        take(v, __shfl_xor_sync(0xffffffffu, bi, off));
     }
+    if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = best; si[threadIdx.x >> 5] = bi; }
     __syncthreads();
+    for (unsigned w = 0; w < 8; w++) take(sv[w], si[w]);
+    const unsigned istar = bi;   // the same in every thread
+    if (threadIdx.x == 0) {
+        *Vout = best;
+        *iout = bi;
+    }
     if (istar == kNoRow) return;
+    if (threadIdx.x == 0) live[istar] = 1u;
     for (unsigned s = threadIdx.x; s < n; s += blockDim.x) lam[(size_t)istar * n + s] = (double)b[s];
 }
 
@@ -289,13 +294,6 @@ constexpr size_t kStepSmem = 56 * 1024;
 // The predecessors of every (a, s'): the (s, T(s,a,l)) with S(s,a,l) = s', one
 // entry per l. Counted, given places (in no particular order of the lists) and
 // filled.
-__global__ void adj_pred_count_kernel(AdjModel md, const unsigned *__restrict__ len, unsigned *__restrict__ count) {
-    const size_t all = (size_t)md.n * md.m * md.ns, stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < all; e += stride) {
-        const size_t row = e / md.ns;
-        if (e % md.ns < len[row]) atomicAdd(count + (row % md.m) * md.n + md.S[e], 1u);
-    }
-}
 __global__ void adj_pred_place_kernel(size_t rows, const unsigned *__restrict__ count, unsigned long long *next,
                                       unsigned long long *__restrict__ start, unsigned *__restrict__ filled) {
     const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -341,44 +339,55 @@ __device__ __forceinline__ bool nonzero(double x) {   // by its bits: compares r
 }
 
 // One reverse step for up to NB beliefs of one action (of a group made for the
-// replay; those with a zero adjoint drop out) at kStepThreads successors s',
-// one per thread: c and w of the beliefs stay in registers, the s' terms of dT
-// are those of its predecessors. Shared memory: the beliefs' lambda (n doubles
-// each), their selections, and with kStaged a tile per warp through which dO's
-// terms, computed for consecutive states, reach consecutive observations.
+// replay; those without an adjoint, live 0, drop out) at kStepThreads successors
+// s', one per thread: c and w of the beliefs stay in registers, the s' terms of
+// dT are those of its predecessors, whose lambda are gathered from L2. Shared
+// memory: the beliefs' selections, and with NB > 1 a tile per warp through which
+// dO's terms, computed for consecutive states, reach consecutive observations.
+// Marks the rows of lamPrev that it adds to in livePrev.
 // Bound by FP64 arithmetic (1/64 of the FP32 rate), so factors are widened and
 // tested by integer operations, and what does not depend on the belief is
 // shared by the group; blocks of a part of the states even out the groups'
-// unequal numbers of beliefs. n = 1,024 (m = 8, z = 16, ns = 16, 600 beliefs
+// unequal numbers of beliefs. n = 1,024 (m = 8, z = ns = 16, up to 600 beliefs
 // with an adjoint): 430 us a step with a block per belief and w by atomics in
-// shared memory, 225 so (the FP64 pipe 70 % busy; 240 with two beliefs per
-// block, 250 with one).
-template <int NB, bool kStaged>
+// shared memory, 200 so (the FP64 pipe 70 % busy; with two beliefs per block 240,
+// one 250). Copying each belief's lambda into every block's shared memory instead
+// gained nothing there and cost r n ceil(n / 128) reads where few beliefs have an
+// adjoint: 5.7 ms a step at n = 14,000, r = 1,000, z = 1, ns = 2, against 0.1 so.
+template <int NB>
 __global__ void __launch_bounds__(kStepThreads) adjoint_step_kernel(
         AdjModel md, const unsigned *__restrict__ predCount, const unsigned long long *__restrict__ predStart,
         const uint2 *__restrict__ pred, const unsigned *__restrict__ predK, const float *__restrict__ Gprev,
         const unsigned *__restrict__ acts, const unsigned *__restrict__ ids, const unsigned *__restrict__ sel,
-        const double *__restrict__ lam, double *__restrict__ lamPrev, double *__restrict__ dR,
-        double *__restrict__ dT, double *__restrict__ dO) {
+        const double *__restrict__ lam, const unsigned *__restrict__ live, double *__restrict__ lamPrev,
+        unsigned *__restrict__ livePrev, double *__restrict__ dR, double *__restrict__ dT, double *__restrict__ dO) {
+    constexpr bool kStaged = NB > 1;
     extern __shared__ __align__(16) unsigned char smem[];
-    double *lsh = reinterpret_cast<double *>(smem);          // [NB][n]
-    double *tiles = lsh + (size_t)NB * md.n;                 // [warps][32][9] with kStaged
+    double *tiles = reinterpret_cast<double *>(smem);        // [warps][32][9] with kStaged
     unsigned *jsh = reinterpret_cast<unsigned *>(tiles + (kStaged ? kStepThreads * 9 : 0));  // [NB][z]
     constexpr unsigned kParts = kGroup / NB;
+    ids += (size_t)blockIdx.x * NB;
+    unsigned id[NB];
+#pragma unroll
+    for (int q = 0; q < NB; q++) id[q] = ids[q];
     const unsigned a = acts[blockIdx.x / kParts];
     if (a == kNoRow) return;
-    ids += (size_t)blockIdx.x * NB;
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned sp = blockIdx.y * kStepThreads + threadIdx.x, sp0 = sp - lane;
+    const bool in = sp < md.n;
+    const unsigned cnt = in ? predCount[(size_t)a * md.n + sp] : 0u;
+    const size_t first = in ? predStart[(size_t)a * md.n + sp] : 0u;
     unsigned nb = 0;
-    for (unsigned q = 0; q < NB; q++) {
-        const unsigned i = ids[q];
-        bool nz = false;
-        if (i != kNoRow)
-            for (unsigned s = threadIdx.x; s < md.n; s += kStepThreads) {
-                const double l = lam[(size_t)i * md.n + s];
-                lsh[(size_t)nb * md.n + s] = l;
-                nz |= nonzero(l);
-            }
-        if (!__syncthreads_or(nz)) continue;   // its place is taken by the next
+    const double *lambda[NB];   // lambda of the beliefs taken
+#pragma unroll
+    for (int q = 0; q < NB; q++) lambda[q] = lam;
+#pragma unroll
+    for (int q = 0; q < NB; q++) {
+        const unsigned i = id[q];
+        if (i == kNoRow || live[i] == 0u) continue;   // its place is taken by the next
+#pragma unroll
+        for (int b = 0; b < NB; b++)
+            if (b == nb) lambda[b] = lam + (size_t)i * md.n;
         for (unsigned o = threadIdx.x; o < md.z; o += kStepThreads)
             jsh[nb * md.z + o] = min(sel[(size_t)i * md.z + o], md.r - 1);
         nb++;
@@ -386,17 +395,16 @@ __global__ void __launch_bounds__(kStepThreads) adjoint_step_kernel(
     if (nb == 0) return;
     __syncthreads();
     const double g = (double)md.gamma;
-    const unsigned lane = threadIdx.x & 31;
-    const unsigned sp = blockIdx.y * kStepThreads + threadIdx.x, sp0 = sp - lane;
     if (sp0 >= md.n) return;
-    const bool in = sp < md.n;
     const size_t ob = ((size_t)a * md.n + sp) * md.z;
     double c[NB], w[NB];
 #pragma unroll
     for (int b = 0; b < NB; b++) c[b] = w[b] = 0.0;
     if (in) {
         double l = 0.0;
-        for (unsigned b = 0; b < nb; b++) l += lsh[(size_t)b * md.n + sp];
+#pragma unroll
+        for (int b = 0; b < NB; b++)
+            if (b < nb) l += __ldg(lambda[b] + sp);
         if (nonzero(l)) atomicAdd(dR + (size_t)sp * md.m + a, l);
 #pragma unroll 2
         for (unsigned o = 0; o < md.z; o++) {
@@ -405,9 +413,7 @@ __global__ void __launch_bounds__(kStepThreads) adjoint_step_kernel(
             for (int b = 0; b < NB; b++)
                 if (b < nb) c[b] += po * widen(__ldg(Gprev + (size_t)jsh[b * md.z + o] * md.n + sp));
         }
-        const size_t first = predStart[(size_t)a * md.n + sp];
-        const unsigned cnt = predCount[(size_t)a * md.n + sp];
-#pragma unroll 2
+#pragma unroll (NB == 1 ? 4 : 2)
         for (unsigned k = 0; k < cnt; k++) {
             const uint2 e = __ldg(pred + first + k);
             const size_t row = ((size_t)e.x * md.m + a) * md.ns + __ldg(predK + first + k);
@@ -417,7 +423,7 @@ __global__ void __launch_bounds__(kStepThreads) adjoint_step_kernel(
 #pragma unroll
             for (int b = 0; b < NB; b++)
                 if (b < nb) {
-                    const double lb = lsh[(size_t)b * md.n + e.x];
+                    const double lb = __ldg(lambda[b] + e.x);
                     if (nonzero(lb)) {
                         w[b] += t * lb;
                         u += lb * c[b];
@@ -435,6 +441,10 @@ __global__ void __launch_bounds__(kStepThreads) adjoint_step_kernel(
         w[b] *= g;
     }
     if (!__any_sync(0xffffffffu, nz)) return;
+#pragma unroll
+    for (int b = 0; b < NB; b++)
+        if (__any_sync(0xffffffffu, nzb[b]))
+            for (unsigned o = lane; o < md.z; o += 32u) livePrev[jsh[b * md.z + o]] = 1u;
     double *tile = tiles + (size_t)(threadIdx.x >> 5) * 32 * 9;
     for (unsigned o0 = 0; o0 < md.z; o0 += 8) {
         const unsigned oEnd = min(8u, md.z - o0);
@@ -469,7 +479,7 @@ struct AdjBuffers {
     Arena arena;
     unsigned *len = nullptr, *ST = nullptr, *acts = nullptr, *ids = nullptr, *cursor = nullptr;
     float *CT = nullptr, *seg = nullptr;
-    double *lamA = nullptr, *lamB = nullptr, *vals = nullptr, *V = nullptr;
+    double *lamA = nullptr, *lamB = nullptr, *vals = nullptr, *V = nullptr;  // lambda: [r][n], then [r] marks of its rows
     unsigned *istar = nullptr;
     unsigned *predCount = nullptr, *predFilled = nullptr, *predK = nullptr;
     unsigned long long *predStart = nullptr, *predNext = nullptr;
@@ -545,15 +555,20 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
     }
     AdjModel md{pomdp->n, pomdp->ns, pomdp->m, pomdp->z, pomdp->r, pomdp->gamma,
                 pomdp->d_S, pomdp->d_T, pomdp->d_O, pomdp->d_R};
-    // Four beliefs per block, or two, where four blocks fit on an SM.
+    // Four beliefs per block, which share what does not depend on them; one
+    // where that leaves fewer blocks than a wave (four an SM; n = 100, r = 200, m
+    // = 4: 18.4 and 12.0 us a step, n = 60, r = 1,200: 10.6 and 7.8; at n = 500,
+    // r = 1,500, 1,500 blocks, either way 34). With very many observations (more
+    // than 2,900 or 5,900), whose selections would leave room for few blocks on
+    // an SM, two or one.
+    const unsigned groups = ceil_div(md.r, kGroup) + md.m;
+    const bool fewSteps = (size_t)groups * ceil_div(md.n, kStepThreads) <= 4u * 152u;
     auto step_smem = [&](size_t nb) {
-        return nb * ((size_t)md.n * sizeof(double) + md.z * sizeof(unsigned)) +
-               (nb > 1 ? kStepThreads * 9 * sizeof(double) : 0);
+        return nb * md.z * sizeof(unsigned) + (nb > 1 ? kStepThreads * 9 * sizeof(double) : 0);
     };
-    const unsigned nb = step_smem(4) <= kStepSmem ? 4u : step_smem(2) <= kStepSmem ? 2u : 1u;
+    const unsigned nb = fewSteps ? 1u : step_smem(4) <= kStepSmem ? 4u : step_smem(2) <= kStepSmem ? 2u : 1u;
     const size_t stepSmem = step_smem(nb);
-    auto step = nb == 4 ? adjoint_step_kernel<4, true> : nb == 2 ? adjoint_step_kernel<2, true>
-                                                                 : adjoint_step_kernel<1, false>;
+    auto step = nb == 4 ? adjoint_step_kernel<4> : nb == 2 ? adjoint_step_kernel<2> : adjoint_step_kernel<1>;
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
@@ -574,30 +589,40 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
     bf.arena.add(&bf.len, (size_t)n * m);
     bf.arena.add(&bf.ST, (size_t)m * n * ns);
     bf.arena.add(&bf.CT, (size_t)m * z * n * ns);
-    const unsigned groups = ceil_div(r, kGroup) + m;
     bf.arena.add(&bf.acts, (size_t)horizon * groups);
     bf.arena.add(&bf.ids, (size_t)horizon * groups * kGroup);
     bf.arena.add(&bf.seg, (size_t)(k + 1) * rn);
-    bf.arena.add(&bf.lamA, rn);
-    bf.arena.add(&bf.lamB, rn);
+    const size_t lamDoubles = rn + ceil_div(r, 2);   // one piece, cleared at once
+    bf.arena.add(&bf.lamA, lamDoubles);
+    bf.arena.add(&bf.lamB, lamDoubles);
     bf.arena.add(&bf.vals, r);
-    bf.arena.add(&bf.V, 1);
-    bf.arena.add(&bf.istar, 1);
-    bf.arena.add(&bf.predCount, (size_t)m * n);
+    bf.arena.add(&bf.V, 2);          // the value, and istar beside it
+    const size_t predRows = round_up((size_t)m * n, 2);
+    bf.arena.add(&bf.predCount, predRows + 2);   // and predNext behind it
     bf.arena.add(&bf.predFilled, (size_t)m * n);
     bf.arena.add(&bf.predStart, (size_t)m * n);
-    bf.arena.add(&bf.predNext, 1);
     bf.arena.add(&bf.pred, (size_t)m * n * ns);
     bf.arena.add(&bf.predK, (size_t)m * n * ns);
     const bool manyActions = m > 8192;
     if (manyActions) bf.arena.add(&bf.cursor, (size_t)horizon * m);
     if ((rc = bf.arena.commit(fn, "the adjoint")) != NOVA_SUCCESS) return rc;
+    bf.istar = reinterpret_cast<unsigned *>(bf.V + 1);
+    bf.predNext = reinterpret_cast<unsigned long long *>(bf.predCount + predRows);
     if ((rc = sync_device(fn)) != NOVA_SUCCESS) return rc;
 
+    if (cudaMemset(d_dR, 0, (size_t)n * m * sizeof(double)) != cudaSuccess ||
+            cudaMemset(d_dT, 0, (size_t)n * m * ns * sizeof(double)) != cudaSuccess ||
+            cudaMemset(d_dO, 0, (size_t)m * n * z * sizeof(double)) != cudaSuccess ||
+            cudaMemset(bf.lamA, 0, lamDoubles * sizeof(double)) != cudaSuccess ||
+            cudaMemset(bf.predCount, 0, (predRows + 2) * sizeof(unsigned)) != cudaSuccess) {
+        cudaGetLastError();
+        NOVA_ERR(fn, "Failed to clear the gradients.");
+        return NOVA_ERROR_KERNEL_EXECUTION;
+    }
     adj_len_kernel<<<ceil_div((size_t)n * m, 256), 256>>>(n * m, ns, md.S, bf.len);
     if ((rc = check_launch(fn, "successor lengths")) != NOVA_SUCCESS) return rc;
-    adj_coef_kernel<<<std::min<size_t>(ceil_div((size_t)m * n * ns, 256), 65535u * 8u), 256>>>(md, bf.len, bf.ST,
-                                                                                              bf.CT);
+    adj_coef_kernel<<<std::min<size_t>(ceil_div((size_t)m * n * ns, 256), 65535u * 8u), 256>>>(
+        md, bf.len, bf.ST, bf.CT, bf.predCount);
     if ((rc = check_launch(fn, "projection coefficients")) != NOVA_SUCCESS) return rc;
     replay_groups_kernel<<<horizon, 1024, manyActions ? 0 : m * sizeof(unsigned)>>>(r, m, groups, d_actions, bf.acts,
                                                                                   bf.ids, bf.cursor);
@@ -606,8 +631,15 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
     // larger models gather from the alpha rows themselves.
     const size_t rowsSmem = 2 * (size_t)kGroup * round_up(n, 4) * sizeof(float);
     const bool rowsShared = rowsSmem + 1024 <= (size_t)optin;
-    if (rowsShared && rowsSmem > 48 * 1024 &&
-            !allow_dynamic_smem(replay_kernel<true>, rowsSmem)) {
+    // One belief per block, unstaged, where the groups would leave half the SMs
+    // idle (m z = 512, ns = 32: n = 100, 41 groups, 145 and 116 us a step; n =
+    // 1,000, 91 groups, 480 and 690).
+    const bool fewReplays = (size_t)groups * ceil_div(n, kReplayThreads * kReplayStates) <= 76u;
+    auto replay = fewReplays ? replay_kernel<1, false> : rowsShared ? replay_kernel<4, true> : replay_kernel<4, false>;
+    const size_t replaySmem = !fewReplays && rowsShared ? rowsSmem : 0;
+    const unsigned replayThreads = (unsigned)std::min<size_t>(kReplayThreads, round_up(n, 32));
+    const dim3 replayBlocks(groups * (fewReplays ? kGroup : 1u), ceil_div(n, replayThreads * kReplayStates));
+    if (!allow_dynamic_smem(replay, replaySmem)) {
         cudaGetLastError();
         NOVA_ERR(fn, "Failed to configure the replay kernel.");
         return NOVA_ERROR_KERNEL_EXECUTION;
@@ -615,20 +647,7 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
     // 16-byte copies where every alpha row starts on a 16-byte boundary (the
     // segment buffer itself does).
     const int wide = n % 4u == 0u ? 1 : 0;
-    if (cudaMemset(d_dR, 0, (size_t)n * m * sizeof(double)) != cudaSuccess ||
-            cudaMemset(d_dT, 0, (size_t)n * m * ns * sizeof(double)) != cudaSuccess ||
-            cudaMemset(d_dO, 0, (size_t)m * n * z * sizeof(double)) != cudaSuccess ||
-            cudaMemset(bf.lamA, 0, rn * sizeof(double)) != cudaSuccess ||
-            cudaMemset(bf.predCount, 0, (size_t)m * n * sizeof(unsigned)) != cudaSuccess ||
-            cudaMemset(bf.predNext, 0, sizeof(unsigned long long)) != cudaSuccess) {
-        cudaGetLastError();
-        NOVA_ERR(fn, "Failed to clear the gradients.");
-        return NOVA_ERROR_KERNEL_EXECUTION;
-    }
-
     const unsigned predBlocks = (unsigned)std::min<size_t>(ceil_div((size_t)m * n * ns, 256), 65535u * 8u);
-    adj_pred_count_kernel<<<predBlocks, 256>>>(md, bf.len, bf.predCount);
-    if ((rc = check_launch(fn, "predecessor counts")) != NOVA_SUCCESS) return rc;
     adj_pred_place_kernel<<<ceil_div((size_t)m * n, 256), 256>>>((size_t)m * n, bf.predCount, bf.predNext,
                                                                  bf.predStart, bf.predFilled);
     if ((rc = check_launch(fn, "predecessor places")) != NOVA_SUCCESS) return rc;
@@ -649,11 +668,9 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
         }
         for (unsigned q = 1; q <= last; q++) {
             const size_t step = base + q - 1;
-            auto kernel = rowsShared ? replay_kernel<true> : replay_kernel<false>;
-            kernel<<<dim3(groups, ceil_div(n, kReplayThreads * kReplayStates)), kReplayThreads,
-                     rowsShared ? rowsSmem : 0>>>(md, bf.len, bf.ST, bf.CT, bf.seg + (size_t)(q - 1) * rn,
-                                                  bf.acts + step * groups, bf.ids + step * groups * kGroup,
-                                                  d_selects + step * r * z, wide, bf.seg + (size_t)q * rn);
+            replay<<<replayBlocks, replayThreads, replaySmem>>>(
+                md, bf.len, bf.ST, bf.CT, bf.seg + (size_t)(q - 1) * rn, bf.acts + step * groups,
+                bf.ids + step * groups * kGroup, d_selects + step * r * z, wide, bf.seg + (size_t)q * rn);
             int e = check_launch(fn, "alpha recomputation");
             if (e != NOVA_SUCCESS) return e;
         }
@@ -667,7 +684,8 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
     const float *GH = bf.seg + (size_t)(horizon - segStart) * rn;
     value_rows_kernel<<<r, 256>>>(GH, n, d_b, bf.vals);
     if ((rc = check_launch(fn, "FP64 values")) != NOVA_SUCCESS) return rc;
-    value_argmax_kernel<<<1, 256>>>(r, n, bf.vals, d_b, bf.V, bf.istar, bf.lamA);
+    auto marks = [&](double *lam) { return reinterpret_cast<unsigned *>(lam + rn); };
+    value_argmax_kernel<<<1, 256>>>(r, n, bf.vals, d_b, bf.V, bf.istar, bf.lamA, marks(bf.lamA));
     if ((rc = check_launch(fn, "FP64 argmax")) != NOVA_SUCCESS) return rc;
 
     for (unsigned t = horizon; t >= 1; t--) {
@@ -677,7 +695,7 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
             segStart = segC * k;
             if ((rc = recompute(segC, k - 1)) != NOVA_SUCCESS) return rc;
         }
-        if (cudaMemsetAsync(bf.lamB, 0, rn * sizeof(double)) != cudaSuccess) {
+        if (cudaMemsetAsync(bf.lamB, 0, lamDoubles * sizeof(double)) != cudaSuccess) {
             cudaGetLastError();
             NOVA_ERR(fn, "Failed to clear the adjoint.");
             return NOVA_ERROR_KERNEL_EXECUTION;
@@ -685,7 +703,7 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
         step<<<dim3(groups * (kGroup / nb), ceil_div(n, kStepThreads)), kStepThreads, stepSmem>>>(
             md, bf.predCount, bf.predStart, bf.pred, bf.predK, bf.seg + (size_t)(p - segStart) * rn,
             bf.acts + (size_t)p * groups, bf.ids + (size_t)p * groups * kGroup, d_selects + (size_t)p * r * z, bf.lamA,
-            bf.lamB, d_dR, d_dT, d_dO);
+            marks(bf.lamA), bf.lamB, marks(bf.lamB), d_dR, d_dT, d_dO);
         if ((rc = check_launch(fn, "reverse step")) != NOVA_SUCCESS) return rc;
         std::swap(bf.lamA, bf.lamB);
     }
@@ -696,10 +714,12 @@ extern "C" int pomdp_pbvi_adjoint_gpu(const POMDP *pomdp, unsigned int horizon, 
         return NOVA_ERROR_KERNEL_EXECUTION;
     }
     if ((rc = sync_device(fn)) != NOVA_SUCCESS) return rc;
-    if (Vb != nullptr && (rc = d2h(Vb, bf.V, sizeof(double), fn, "the value")) != NOVA_SUCCESS) return rc;
-    if (bestAlpha != nullptr && (rc = d2h(bestAlpha, bf.istar, sizeof(unsigned), fn, "the maximising alpha")) !=
-            NOVA_SUCCESS)
-        return rc;
+    struct { double V; unsigned istar; } h;
+    if (Vb != nullptr || bestAlpha != nullptr) {
+        if ((rc = d2h(&h, bf.V, sizeof(h), fn, "the value and the maximising alpha")) != NOVA_SUCCESS) return rc;
+        if (Vb != nullptr) *Vb = h.V;
+        if (bestAlpha != nullptr) *bestAlpha = h.istar;
+    }
     return NOVA_SUCCESS;
 }
 

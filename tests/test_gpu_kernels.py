@@ -563,3 +563,19 @@ def test_perseus_with_little_memory():
         lib().nova_gb300_inject_fault(0, 0)
     np.testing.assert_array_equal(bits(pol.gamma_array()), bits(Go))
     np.testing.assert_array_equal(pol.pi_array(), po)
+
+
+@pytest.mark.parametrize("n,m,z,ns,r", [(30, 1, 2, 3, 300), (5, 1, 1, 2, 310), (33, 3, 2, 5, 300), (1026, 2, 3, 9, 150),
+                                        (70, 2, 17, 31, 401), (7300, 2, 2, 4, 30)])
+def test_replayed_groups(n, m, z, ns, r):
+    """The most beliefs that are replayed one per block, and more: four of one
+    action, their alphas in and out of shared memory."""
+    test_replayed_backups(n, m, z, ns, r)
+
+
+@pytest.mark.parametrize("n,m,z,ns,r", [(20, 2, 3, 3, 2424), (20, 2, 3, 3, 2428), (129, 3, 9, 4, 1211), (2000, 1, 2, 3, 161),
+                                        (3, 1, 3100, 2, 2450), (14500, 1, 2, 2, 30)])
+def test_reverse_groups(n, m, z, ns, r):
+    """One belief per block up to a wave of blocks, four beyond it, two with
+    thousands of observations, and the most states that are accepted."""
+    test_reverse_steps(n, m, z, ns, r)

@@ -944,8 +944,8 @@ __global__ void tc_pack_kernel(const float *__restrict__ G, unsigned n, size_t n
 
 // ---------------------------------------------------------------------------
 // Merge the per-group lists, apply the proven margin, re-score near ties
-// exactly from the projection table. One warp per (a*z+o, belief) row; rows
-// whose candidate set may be incomplete go to the exact row scan.
+// exactly from the projection table; rows whose candidate set may be
+// incomplete go to the exact row scan.
 // ---------------------------------------------------------------------------
 
 // Without the projection table: the same exact scores straight from the
@@ -993,6 +993,8 @@ struct DirectScorer {
 // 3,500 (21 MB): updates of 12.29 and 12.22 ms; n = 2,000 with 800 (6 MB): 245
 // and 253 us of scoring; n = 512 with 1,024 (2 MB) 177 and 198.
 constexpr size_t kMergeOrderedSlab = 16u << 20;
+// (All this with the state-contiguous table; tc_merge_warps_kernel below has the
+// other one.)
 // Few rows (up to two rounds of resident blocks) are settled in one launch, 16
 // of them looked at and re-scored per block: n = 64 (8,192 rows) 41 and 37 us
 // of scoring with two launches and one; at four rounds n = 300 (37,800) 68 and
@@ -1069,12 +1071,16 @@ __device__ __forceinline__ RowOutcome merge_look(unsigned row, const DevModel &m
 // slot e / nLists of list e % nLists, so the lists' headers (slot 0) come
 // first, in lanes 0 .. nLists - 1; NE slots per lane are loaded before the
 // lists' lengths are known, what lies beyond (rare: lists of more than 7
-// entries, 15 of two) after that.
-template <int NE>
+// entries, 15 of two) after that. With kTable the scores come from the
+// alpha-contiguous projection table: entries of one state lie side by side
+// there, so every lane takes a candidate and reads eight states' entries ahead
+// of its sum. Without, from the model and the alphas.
+template <int NE, bool kTable>
 __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const DevModel &md,
-                                              const unsigned *__restrict__ suppLen, const DirectScorer &ds, float *scratch, unsigned *list,
+                                              const unsigned *__restrict__ suppLen, const ProjView &pv,
+                                              const DirectScorer &ds, float *scratch, unsigned *list,
                                               const unsigned *__restrict__ uniqJ, unsigned nLists,
-                                              const uint2 *__restrict__ cand, unsigned *__restrict__ jstar,
+                                              const uint2 *__restrict__ cand, unsigned *__restrict__ choice,
                                               bool *flagged) {
     const unsigned ao = row / md.r, i = row % md.r;
     const unsigned a = ao / md.z, o = ao % md.z;
@@ -1118,6 +1124,21 @@ __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const
     unsigned myU = kNoneU, nb = 0;
     auto settle = [&](float total) {
         if (lane < nb && (bu == kNoneU || total > best || (total == best && myU < bu))) { best = total; bu = myU; }
+    };
+    auto score_columns = [&]() {
+        const float *P = pv.slab(ao) + (lane < nb ? myU : 0u) * pv.uStride;
+        float total = 0.0f;
+        unsigned k = 0;
+        for (; k + 8u <= Li; k += 8u) {
+            float p[8];
+#pragma unroll
+            for (unsigned q = 0; q < 8u; q++) p[q] = lane < nb ? __ldg(P + (unsigned)__ldg(sk + k + q) * pv.sStride) : 0.0f;
+#pragma unroll
+            for (unsigned q = 0; q < 8u; q++) total = fadd(total, fmul(p[q], __ldg(bk + k + q)));
+        }
+        for (; k < Li; k++)
+            if (lane < nb) total = fadd(total, fmul(__ldg(P + (unsigned)__ldg(sk + k) * pv.sStride), __ldg(bk + k)));
+        settle(total);
     };
     auto score_batch = [&]() {
         // The gathers of one candidate stay within one alpha row: lane k
@@ -1190,7 +1211,8 @@ __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const
     for (unsigned f = 0; f < count; f += 32u) {
         nb = min(32u, count - f);
         myU = lane < nb ? list[f + lane] : kNoneU;
-        score_batch();
+        if constexpr (kTable) score_columns();
+        else score_batch();
     }
     for (int off = 16; off > 0; off >>= 1) {
         const float b2 = __shfl_xor_sync(0xffffffffu, best, off);
@@ -1200,7 +1222,7 @@ __device__ __forceinline__ unsigned merge_row(unsigned row, unsigned lane, const
     if (!(best > -1e10f)) {
         *flagged = true;  // sentinel case: the exact scan applies the reference's rule
     } else if (lane == 0) {
-        jstar[js] = uniqJ[bu];
+        choice[js] = kTable ? bu : uniqJ[bu];
     }
     return count;
 }
@@ -1410,25 +1432,33 @@ __global__ void __launch_bounds__(256, kMergeBlocks) tc_merge_kernel(
     if (sum) atomicAdd(&counters[1], sum);
 }
 
-// The same without a table: one warp per queued row.
-__global__ void __launch_bounds__(256, 1) tc_merge_direct_kernel(
-                                DevModel md, const unsigned *__restrict__ suppLen,
+// Rows with several candidates, one warp each: with the alpha-contiguous table
+// (which an update keeps after one that left more than 1 % of its rows open:
+// many candidates per row, often wide beliefs) all rows in their own order, of
+// which those flagged kRowSeveral are meant; without a table the queued rows.
+// BF16, n = 4,096, m z = 32, 4,096 near-tied alphas (87 candidates a row): 3.5
+// ms, 6.3 by half warps that gather four candidates at a time.
+template <bool kTable>
+__global__ void __launch_bounds__(256, kTable ? 3 : 1) tc_merge_warps_kernel(
+                                DevModel md, const unsigned *__restrict__ suppLen, const ProjView pv,
                                 const DirectScorer ds, const unsigned *__restrict__ uniqJ,
                                 unsigned nLists, const uint2 *__restrict__ cand,
-                                unsigned *__restrict__ jstar, unsigned *__restrict__ rowFlag,
+                                unsigned *__restrict__ choice, unsigned *__restrict__ rowFlag,
                                 unsigned *__restrict__ rowCand, const unsigned *__restrict__ rowList,
                                 unsigned *__restrict__ counters, unsigned *__restrict__ chunkCount) {
-    // [warps][32 candidates][32 states], then each warp's candidate list.
+    // Each warp's candidate list; before them, without a table, [warps][32
+    // candidates][32 states].
     extern __shared__ float mergeScratch[];
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned queued = counters[0];
-    unsigned *list = reinterpret_cast<unsigned *>(mergeScratch + 8u * 1024u) + warp * (nLists * LIST_SLOTS);
+    const unsigned queued = kTable ? md.m * md.z * md.r : counters[0];
+    unsigned *list = reinterpret_cast<unsigned *>(mergeScratch + (kTable ? 0u : 8u * 1024u)) + warp * (nLists * LIST_SLOTS);
     unsigned sum = 0;
     for (unsigned k = blockIdx.x * 8u + warp; k < queued; k += gridDim.x * 8u) {
-        const unsigned row = __ldg(rowList + k);
+        const unsigned row = kTable ? k : __ldg(rowList + k);
+        if (kTable && rowFlag[row] != kRowSeveral) continue;
         bool flagged = false;
-        const unsigned rescored = merge_row<2>(row, lane, md, suppLen, ds, mergeScratch + warp * 1024u, list, uniqJ,
-                                               nLists, cand, jstar, &flagged);
+        const unsigned rescored = merge_row<2, kTable>(row, lane, md, suppLen, pv, ds, mergeScratch + warp * 1024u, list,
+                                                       uniqJ, nLists, cand, choice, &flagged);
         if (lane == 0) {
             rowCand[row] = rescored;
             rowFlag[row] = flagged ? 1u : 0u;
@@ -1736,7 +1766,7 @@ int tc_finish(BackupEngine &eng, const char *fn) {
     const DirectScorer ds{eng.succLen, eng.C3, tc->src};
     const bool table = eng.useProjNow;
     const unsigned blocks = (unsigned)ceil_div(rows, 16);
-    const bool whole = table && blocks <= kMergeWholeRounds * kMergeBlocks * (unsigned)tc->numSMs;
+    const bool whole = table && eng.projStateMajor && blocks <= kMergeWholeRounds * kMergeBlocks * (unsigned)tc->numSMs;
     if (!whole) {
         tc_merge_look_kernel<<<(unsigned)ceil_div(rows, kLookRows), kLookRows, 0, eng.stream>>>(
             md, table ? nullptr : eng.uniqMap, L.lists, tc->rPad, tc->a1, tc->d1, tc->a1raw, tc->scal, tc->cand,
@@ -1744,7 +1774,7 @@ int tc_finish(BackupEngine &eng, const char *fn) {
             tc->badModel);
         if ((rc = check_launch(fn, "candidate lists")) != NOVA_SUCCESS) return rc;
     }
-    if (table) {
+    if (table && eng.projStateMajor) {
         const bool inOrder = eng.proj_view().slice * sizeof(float) >= kMergeOrderedSlab;
         const bool two = L.lists <= 2u;
         auto merge = whole     ? (two ? tc_merge_kernel<2, MergeRows::kWhole> : tc_merge_kernel<4, MergeRows::kWhole>)
@@ -1755,10 +1785,12 @@ int tc_finish(BackupEngine &eng, const char *fn) {
             md, eng.suppLen, eng.proj_view(), L.lists, tc->rPad, tc->a1, tc->d1, tc->a1raw, tc->scal, tc->cand,
             eng.ustar, tc->rowFlag, tc->rowCand, tc->rowList, tc->scal + 3, tc->chunkCount, tc->badModel);
     } else {
-        const unsigned grid = std::min((unsigned)ceil_div(rows, 8), (unsigned)tc->numSMs);
-        tc_merge_direct_kernel<<<grid, 256, 8 * (1024u + L.lists * LIST_SLOTS) * sizeof(float), eng.stream>>>(
-            md, eng.suppLen, ds, eng.uniqMap, L.lists, tc->cand, eng.jstar, tc->rowFlag, tc->rowCand,
-            tc->rowList, tc->scal + 3, tc->chunkCount);
+        const unsigned warpBlocks = (unsigned)ceil_div(rows, 8);
+        const unsigned grid = table ? warpBlocks : std::min(warpBlocks, (unsigned)tc->numSMs);
+        const size_t smem = 8 * ((table ? 0u : 1024u) + L.lists * LIST_SLOTS) * sizeof(float);
+        (table ? tc_merge_warps_kernel<true> : tc_merge_warps_kernel<false>)<<<grid, 256, smem, eng.stream>>>(
+            md, eng.suppLen, table ? eng.proj_view() : ProjView{}, ds, eng.uniqMap, L.lists, tc->cand,
+            table ? eng.ustar : eng.jstar, tc->rowFlag, tc->rowCand, tc->rowList, tc->scal + 3, tc->chunkCount);
     }
     if ((rc = check_launch(fn, "candidate merge")) != NOVA_SUCCESS) return rc;
     tc_compact_write_kernel<<<nChunks, 1024, 0, eng.stream>>>(tc->rowFlag, (unsigned)rows, tc->chunkCount,

@@ -579,3 +579,19 @@ def test_reverse_groups(n, m, z, ns, r):
     """One belief per block up to a wave of blocks, four beyond it, two with
     thousands of observations, and the most states that are accepted."""
     test_reverse_steps(n, m, z, ns, r)
+
+
+@pytest.mark.parametrize("n,r,rz,mode", [(130, 300, 97, npp.SCORING_FP16), (130, 300, 97, npp.SCORING_BF16),
+                                         (300, 200, 290, npp.SCORING_FP16), (300, 200, 290, npp.SCORING_BF16),
+                                         (70, 1100, 33, npp.SCORING_BF16), (2100, 300, 300, npp.SCORING_BF16)])
+def test_merge_after_open_rows(n, r, rz, mode):
+    """Updates after one that left more than 1 % of its rows open keep the
+    alpha-contiguous table: rows with up to and more than 32 candidates, over
+    supports around multiples of 8, narrow and wide."""
+    md = synth.random_pomdp(n=n, m=2, z=3, ns=12, r=r, rz=rz, gamma=0.9, horizon=6, seed=r)
+    md["Z"][r // 3:r // 2, 5:], md["B"][r // 3:r // 2, 5:] = -1, 0.0
+    md["GammaInitial"] = np.random.default_rng(2).normal(-3.0, 1.0, size=(r, n)).astype(np.float32)
+    G, pi, stats, Go, po = backups(md, mode, 6)
+    assert any(s["rowsOverflow"] > 0.01 * 6 * r and t["rowsMultiCand"] > 0 for s, t in zip(stats, stats[1:]))
+    np.testing.assert_array_equal(bits(G), bits(Go))
+    np.testing.assert_array_equal(pi, po)

@@ -202,29 +202,30 @@ __global__ void __launch_bounds__(1024) value_sparse_kernel(const float *__restr
     }
 }
 
-// Dense tiles: TB beliefs x TA alphas, 8 x TA/16 sums a thread; the next
+// Dense tiles: 16 NB beliefs x TA alphas, NB x TA/16 sums a thread; the next
 // TK states of both operands are loaded into registers while this stage's
 // products are added. Bound by FP32 issue: 2 n operations per (belief,
-// alpha).
-template <int TA>
+// alpha); with few tiles by the chain of a tile's stages, so tiles are small
+// then.
+template <int TA, int NB>
 __global__ void __launch_bounds__(kThreads) value_tiles_kernel(const float *__restrict__ G, unsigned r, unsigned n,
                                                                const float *__restrict__ Bd, unsigned count,
                                                                unsigned cap, const unsigned *__restrict__ nnz,
                                                                unsigned long long *__restrict__ keys, float one) {
-    constexpr unsigned NA = TA / 16, NB = 8;       // sums per thread: NB beliefs x NA alphas
-    constexpr unsigned LB = TB * TK / kThreads, LA = TA * TK / kThreads;  // staged values per thread
+    constexpr unsigned NA = TA / 16, TBD = 16 * NB;
+    constexpr unsigned LB = TBD * TK / kThreads, LA = TA * TK / kThreads;  // staged values per thread
     // State-major tiles; rows padded by 4 floats so the staging stores spread
     // over the banks and rows stay 16-byte aligned.
-    __shared__ __align__(16) float sB[2][TK][TB + 4];
+    __shared__ __align__(16) float sB[2][TK][TBD + 4];
     __shared__ __align__(16) float sG[2][TK][TA + 4];
     const unsigned tid = threadIdx.x;
-    const unsigned b0 = blockIdx.y * TB, a0 = blockIdx.x * TA;
+    const unsigned b0 = blockIdx.y * TBD, a0 = blockIdx.x * TA;
     if (cap != 0u && tile_listed(nnz, b0, count, cap, tid & 31)) return;   // cap 0: no lists, no other kernel
     const unsigned tx = tid % 16, ty = tid / 16;   // alpha group, belief group
     const unsigned long long one2 = pack_f32x2(one, one);
     unsigned long long acc[NB][NA / 2];
 #pragma unroll
-    for (unsigned i = 0; i < NB; i++)
+    for (unsigned i = 0; i < (unsigned)NB; i++)
 #pragma unroll
         for (unsigned j = 0; j < NA / 2; j++) acc[i][j] = 0ull;
     // Thread tid stages states (tid % TK) of rows tid / TK + (kThreads / TK) q:
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(kThreads) value_tiles_kernel(const float *__re
         auto step = [&](unsigned k) {
             float bq[NB];
 #pragma unroll
-            for (unsigned i = 0; i < NB; i += 4) {
+            for (unsigned i = 0; i < (unsigned)NB; i += 4) {
                 const float4 v = *reinterpret_cast<const float4 *>(&sB[buf][k][NB * ty + i]);
                 bq[i] = v.x; bq[i + 1] = v.y; bq[i + 2] = v.z; bq[i + 3] = v.w;
             }
@@ -272,7 +273,7 @@ __global__ void __launch_bounds__(kThreads) value_tiles_kernel(const float *__re
                 gq[2 * j] = v.x; gq[2 * j + 1] = v.y;
             }
 #pragma unroll
-            for (unsigned i = 0; i < NB; i++) {
+            for (unsigned i = 0; i < (unsigned)NB; i++) {
                 const unsigned long long bb = pack_f32x2(bq[i], bq[i]);
 #pragma unroll
                 for (unsigned j = 0; j < NA / 2; j++) acc[i][j] = fma_f32x2(mul_f32x2(gq[j], bb), one2, acc[i][j]);
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(kThreads) value_tiles_kernel(const float *__re
     // Best alpha of this tile per belief: the 16 threads of a belief group
     // hold NA alphas each; reduce with shuffles (max value, then lowest index).
 #pragma unroll
-    for (unsigned i = 0; i < NB; i++) {
+    for (unsigned i = 0; i < (unsigned)NB; i++) {
         float best = NOVA_FLT_MIN;
         unsigned bi = 0xffffffffu;
 #pragma unroll
@@ -377,14 +378,16 @@ static int value_batched(const float *dG, const unsigned *dPi, unsigned r, unsig
         rc = check_launch(fn, "belief values");
     }
     if (rc == NOVA_SUCCESS && cap < n) {
-        // Wide tiles once they fill the device twice over.
-        const unsigned bTiles = ceil_div(count, TB);
-        if ((size_t)ceil_div(r, 128) * bTiles >= 2ull * sms)
-            value_tiles_kernel<128><<<dim3(ceil_div(r, 128), bTiles), kThreads>>>(dG, r, n, dB, count, cap, nnz, keys,
-                                                                                  1.0f);
-        else
-            value_tiles_kernel<64><<<dim3(ceil_div(r, 64), bTiles), kThreads>>>(dG, r, n, dB, count, cap, nnz, keys,
-                                                                                1.0f);
+        // Wide tiles once they fill the device twice over, smaller ones while
+        // larger would not fill it (200 alphas of 20,000 states, 50 beliefs:
+        // 2.1 ms with tiles of 128 x 64, 1.3 with 64 x 64).
+        const unsigned bTiles = ceil_div(count, TB), aTiles = ceil_div(r, 64);
+        auto dense = [&](auto kernel, unsigned ta, unsigned tb) {
+            kernel<<<dim3(ceil_div(r, ta), ceil_div(count, tb)), kThreads>>>(dG, r, n, dB, count, cap, nnz, keys, 1.0f);
+        };
+        if ((size_t)ceil_div(r, 128) * bTiles >= 2ull * sms) dense(value_tiles_kernel<128, 8>, 128, 128);
+        else if ((size_t)aTiles * bTiles >= 2ull * sms) dense(value_tiles_kernel<64, 8>, 64, 128);
+        else dense(value_tiles_kernel<64, 4>, 64, 64);
         rc = check_launch(fn, "belief values (dense)");
     }
     if (rc == NOVA_SUCCESS) {

@@ -595,3 +595,11 @@ def test_merge_after_open_rows(n, r, rz, mode):
     assert any(s["rowsOverflow"] > 0.01 * 6 * r and t["rowsMultiCand"] > 0 for s, t in zip(stats, stats[1:]))
     np.testing.assert_array_equal(bits(G), bits(Go))
     np.testing.assert_array_equal(pi, po)
+
+
+@pytest.mark.parametrize("r,n,count,nz", [(65, 14500, 63, 14500), (64, 14500, 65, 0), (129, 14470, 129, 9), (3000, 50, 900, 50)])
+@pytest.mark.parametrize("odd", [False, True])
+def test_dense_belief_tiles(r, n, count, nz, odd):
+    """Tiles of 64 and 128 beliefs around their edges, where states are too
+    many for the lists' kernel or beliefs have too many nonzeros."""
+    test_belief_values(r, n, count, nz, odd)

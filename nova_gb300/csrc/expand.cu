@@ -704,13 +704,11 @@ int build_workspace(const POMDP *p, ExpWorkspace &ws, const char *fn) {
         NOVA_ERR(fn, "Too many states for the expansion's shared-memory buffers.");
         return NOVA_ERROR_INVALID_DATA;
     }
-    if (ws.smem > 40 * 1024) {
-        allow_dynamic_smem(distinct_mass_kernel, ws.smem);
-        allow_dynamic_smem(distinct_select_kernel, ws.smem);
-        allow_dynamic_smem(random_kernel, ws.smem);
-        allow_dynamic_smem(pema_kernel, ws.smem);
-        allow_dynamic_smem(update_one_kernel, ws.smem);
-    }
+    allow_dynamic_smem(distinct_mass_kernel, ws.smem);
+    allow_dynamic_smem(distinct_select_kernel, ws.smem);
+    allow_dynamic_smem(random_kernel, ws.smem);
+    allow_dynamic_smem(pema_kernel, ws.smem);
+    allow_dynamic_smem(update_one_kernel, ws.smem);
     return NOVA_SUCCESS;
 }
 
@@ -848,9 +846,7 @@ int run_distinct(const ExpWorkspace &ws, std::vector<float> &Bnew, const char *f
     const size_t boundSmem = wide ? tile64 : shared ? tile32 : 32 * 32 * sizeof(float);
     auto bound = wide ? distinct_bound_kernel<64, true> : shared ? distinct_bound_kernel<32, true>
                                                                  : distinct_bound_kernel<32, false>;
-    if (boundSmem > 48 * 1024 &&
-            !allow_dynamic_smem(bound, boundSmem)) {
-        cudaGetLastError();
+    if (!allow_dynamic_smem(bound, boundSmem)) {
         NOVA_ERR(fn, "Failed to configure the distance kernel.");
         return NOVA_ERROR_KERNEL_EXECUTION;
     }

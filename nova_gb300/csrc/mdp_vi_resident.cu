@@ -189,11 +189,7 @@ int vi_resident_sweeps(const MDP *mdp, const int *S, const float *T, const float
     const size_t smem = (size_t)(base + (shared ? n * sizeof(float) : 0));
     const unsigned threads = (unsigned)std::min<unsigned long long>(kMaxThreads, std::max<unsigned long long>(128, pitch));
     const void *kernel = shared ? (const void *)vi_resident_kernel<true> : (const void *)vi_resident_kernel<false>;
-    if (smem > 48 * 1024 &&
-            !allow_dynamic_smem(kernel, smem)) {
-        cudaGetLastError();
-        return NOVA_SUCCESS;
-    }
+    if (!allow_dynamic_smem(kernel, smem)) return NOVA_SUCCESS;
     unsigned un = n, um = m, uns = ns, usp = statesPerBlock, upitch = (unsigned)pitch;
     float gamma = mdp->gamma;
     for (unsigned k = 0; k < sweeps;) {

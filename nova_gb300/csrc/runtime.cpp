@@ -7,6 +7,7 @@
 
 #include "common.h"
 
+#include <algorithm>
 #include <cmath>
 #include <atomic>
 #include <mutex>
@@ -108,12 +109,16 @@ void add_launches(long long delta) { g_launches.fetch_add((unsigned long long)de
 
 bool allow_dynamic_smem(const void *kernel, size_t bytes) {
     static std::mutex mutex;
-    if (bytes <= 48 * 1024) return true;
+    constexpr int kDefault = 48 * 1024;          // the kernel's own (static) shared memory counts against it
+    if (bytes <= 32 * 1024) return true;         // no kernel here has 16 KB of its own
     std::lock_guard<std::mutex> lock(mutex);
     cudaFuncAttributes now;
-    if (cudaFuncGetAttributes(&now, kernel) == cudaSuccess && now.maxDynamicSharedSizeBytes >= (int)bytes) return true;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
+    if (cudaFuncGetAttributes(&now, kernel) == cudaSuccess &&
+            (now.sharedSizeBytes + bytes <= (size_t)kDefault ||
+             (now.maxDynamicSharedSizeBytes > kDefault && now.maxDynamicSharedSizeBytes >= (int)bytes)))
         return true;
+    const int limit = std::max((int)bytes, kDefault + 4);   // above the default, to be told from it
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) == cudaSuccess) return true;
     cudaGetLastError();
     return false;
 }

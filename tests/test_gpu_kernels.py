@@ -603,3 +603,32 @@ def test_dense_belief_tiles(r, n, count, nz, odd):
     """Tiles of 64 and 128 beliefs around their edges, where states are too
     many for the lists' kernel or beliefs have too many nonzeros."""
     test_belief_values(r, n, count, nz, odd)
+
+
+@pytest.mark.parametrize("what", ["pema", "random", "exact"])
+def test_shared_memory_just_below_the_default_limit(what):
+    """Launches whose dynamic shared memory stays below 48 KB while the kernel's
+    own takes the sum above it, first in a process (the limit, once raised,
+    stays raised)."""
+    import subprocess, sys
+    from conftest import ROOT
+    code = {"pema": "import ctypes as ct\n"
+                    "from nova_gb300 import nova_pomdp as npm, nova_pomdp_alpha_vectors as npav\n"
+                    "md = synth.random_pomdp(n=3000, m=1, z=2, ns=2, r=5, rz=3, gamma=0.9, horizon=2, seed=1)\n"
+                    "G, pi = np.zeros((5, 3000), np.float32), np.zeros(5, np.uint32)\n"
+                    "pol = npav.NovaPOMDPAlphaVectors()\n"
+                    "pol.n, pol.m, pol.r = 3000, 1, 5\n"
+                    "pol.Gamma, pol.pi = G.ctypes.data_as(ct.POINTER(ct.c_float)), pi.ctypes.data_as(ct.POINTER(ct.c_uint))\n"
+                    "assert npm._nova.pomdp_expand_pema_cpu(POMDP.from_arrays(md), ct.byref(pol)) == 0\n",
+            "random": "md = synth.random_pomdp(n=3071, m=1, z=2, ns=2, r=5, rz=3, gamma=0.9, horizon=2, seed=1)\n"
+                      "POMDP.from_arrays(md).expand(method='random', numBeliefsToAdd=4)\n",
+            "exact": "md = synth.random_pomdp(n=400, m=1, z=16, ns=365, r=9, rz=3, gamma=0.9, horizon=1, seed=1)\n"
+                     "p = POMDP.from_arrays(md)\n"
+                     "p.initialize_gpu()\n"
+                     "alg = POMDPPBVIGPU(p)\n"
+                     "alg.set_scoring(npp.SCORING_EXACT)\n"
+                     "alg.set_table(npp.TABLE_NEVER)\n"
+                     "alg.update()\n"}[what]
+    code = ("import numpy as np\nfrom nova_gb300 import synth, nova_pomdp_pbvi as npp\nfrom nova_gb300.pomdp import POMDP\n"
+            "from nova_gb300.pomdp_pbvi import POMDPPBVIGPU\n" + code)
+    assert subprocess.run([sys.executable, "-c", code], cwd=ROOT, timeout=120).returncode == 0

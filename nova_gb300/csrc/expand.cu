@@ -96,6 +96,38 @@ __device__ float seq_sum(const float *v, unsigned n, float *slot) {
     return *slot;
 }
 
+// The sum of term(0) .. term(n - 1) in that order, by a whole warp: the lanes
+// form 128 terms (the next ones' loads under way meanwhile), lane 0 adds them.
+// buf: 128 floats of the warp's.
+template <typename F>
+__device__ __forceinline__ float warp_ordered_sum(unsigned n, float *buf, unsigned lane, F term) {
+    float acc = 0.0f, t[4];
+    auto fetch = [&](unsigned s0) {
+#pragma unroll
+        for (unsigned q = 0; q < 4; q++) t[q] = s0 + 32 * q + lane < n ? term(s0 + 32 * q + lane) : 0.0f;
+    };
+    fetch(0);
+    for (unsigned s0 = 0; s0 < n; s0 += 128) {
+#pragma unroll
+        for (unsigned q = 0; q < 4; q++) buf[32 * q + lane] = t[q];
+        __syncwarp();
+        if (s0 + 128 < n) fetch(s0 + 128);
+        if (lane == 0) {
+            if (s0 + 128 <= n) {
+#pragma unroll
+                for (unsigned q = 0; q < 128; q += 4) {
+                    const float4 v = *reinterpret_cast<const float4 *>(buf + q);
+                    acc = fadd(fadd(fadd(fadd(acc, v.x), v.y), v.z), v.w);
+                }
+            } else {
+                for (unsigned q = 0; q < n - s0; q++) acc = fadd(acc, buf[q]);
+            }
+        }
+        __syncwarp();
+    }
+    return __shfl_sync(0xffffffffu, acc, 0);
+}
+
 // PO[a][s][o]: the belief-independent part of
 // pomdp_expand_probability_observation_cpu (pomdp_expand_cpu.cpp:56-78).
 __global__ void prob_table_kernel(unsigned n, unsigned ns, unsigned m, unsigned z, const int *__restrict__ S,
@@ -296,6 +328,56 @@ __global__ void __launch_bounds__(kThreads) distinct_rows_kernel(ExpModel md, Di
     d.mass[t] = mass;
 }
 
+// The same with a warp per row, for rows too few to fill the device with
+// threads whose chains take n steps each: n = 500, 9,600 rows 175 and 53 us, n =
+// 4,000, 6,400 rows 1,540 and 255, n = 2,000, 38,400 rows 752 and 701, n = 1,000,
+// 64,000 rows 395 and 825.
+constexpr size_t kFewRows = 32768;
+
+__global__ void __launch_bounds__(kThreads) distinct_few_rows_kernel(ExpModel md, Distinct d) {
+    __shared__ __align__(16) float terms[kThreads / 32][128];
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, mz = md.m * md.z;
+    const size_t t = (size_t)blockIdx.x * (kThreads / 32) + warp;
+    if (t >= (size_t)d.chunk * mz) return;
+    const unsigned i = (unsigned)(t / mz), ao = (unsigned)(t % mz), a = ao / md.z, o = ao % md.z;
+    const float *po = md.PO + (size_t)a * md.n * md.z + o;
+    float pr;
+    if (d.odd[0] == 0u) {
+        const unsigned j = d.first + i;
+        const uint2 *list = d.list + (size_t)j * d.cap;
+        pr = warp_ordered_sum(d.nnz[j], terms[warp], lane, [&](unsigned k) {
+            const uint2 e = list[k];
+            return fmul(po[(size_t)e.x * md.z], __uint_as_float(e.y));
+        });
+    } else {
+        pr = warp_ordered_sum(md.n, terms[warp], lane, [&](unsigned s) {
+            return fmul(po[(size_t)s * md.z], md.BT[(size_t)s * md.r + d.first + i]);
+        });
+    }
+    float mass = -1.0f;
+    if (!(pr == 0.0f)) {
+        const float *W = d.W + ((size_t)i * md.m + a) * md.n;
+        const float *Oa = md.O + (size_t)a * md.n * md.z + o;
+        const float norm = warp_ordered_sum(md.n, terms[warp], lane,
+                                            [&](unsigned s) { return fmul(__ldg(W + s), __ldg(Oa + (size_t)s * md.z)); });
+        if (!(fabs((double)fabsf(norm)) < NOVA_FLT_ERR_TOL)) {
+            float *out = d.bp + (size_t)i * md.n * mz + ao;
+            mass = 0.0f;
+            bool odd = false;
+#pragma unroll 4
+            for (unsigned s = lane; s < md.n; s += 32) {
+                const float v = __fdiv_rn(fmul(__ldg(W + s), __ldg(Oa + (size_t)s * md.z)), norm);
+                out[(size_t)s * mz] = v;
+                odd |= !(v >= 0.0f && v <= NOVA_FLT_MAX);
+                mass += fabsf(v);
+            }
+            for (int off = 16; off > 0; off >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, off);
+            if (__any_sync(0xffffffffu, odd) && lane == 0) atomicOr(d.odd, 1u);
+        }
+    }
+    if (lane == 0) d.mass[t] = mass;
+}
+
 // Half-width of the interval around an approximate distance in which the
 // reference's FP32 sum lies. With both beliefs non-negative,
 //     sum_s |b_j - b'| = mass - total_j + 2 sum_{s in supp j} max(b_j - b', 0).
@@ -373,15 +455,19 @@ __global__ void __launch_bounds__(1024) distinct_bound_kernel(ExpModel md, Disti
 
 // Per belief: the successors whose bound lies within the error of the largest,
 // in (a, o) order; for each, the reference's sums to the beliefs within the
-// error of its smallest, one warp per belief: the lanes form 32 terms, lane 0
-// adds them in state order. The first successor with the strictly largest
-// smallest distance becomes the new belief.
+// error of its smallest. The first successor with the strictly largest smallest
+// distance becomes the new belief. With many states the error is wide and
+// distances that are exactly equal (disjoint supports) are common: n = 12,000,
+// r = 50 took 37 ms with every sum over all states, 0.23 so.
 __global__ void __launch_bounds__(kThreads) distinct_select_kernel(ExpModel md, Distinct d, float *__restrict__ Bnew) {
     extern __shared__ __align__(16) float smem[];
-    __shared__ float red[kThreads / 32], terms[kThreads / 32][32];
+    __shared__ float red[kThreads / 32];
+    __shared__ __align__(16) float terms[kThreads / 32][128];
+    __shared__ unsigned found[kThreads / 32];
     const unsigned mz = md.m * md.z, i = blockIdx.x;
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float *row = smem, *star = smem + md.n;
+    unsigned *states = reinterpret_cast<unsigned *>(star + md.n);   // the successor's nonzero states, in order
     const float *bound = d.bound + (size_t)i * mz, *mass = d.mass + (size_t)i * mz;
     float top = -INFINITY, heaviest = 0.0f;
     for (unsigned ao = threadIdx.x; ao < mz; ao += blockDim.x) {
@@ -408,6 +494,21 @@ __global__ void __launch_bounds__(kThreads) distinct_select_kernel(ExpModel md, 
         __syncthreads();
         for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) row[s] = d.bp[((size_t)i * md.n + s) * mz + ao];
         __syncthreads();
+        unsigned support = 0;
+        for (unsigned s0 = 0; s0 < md.n; s0 += kThreads) {
+            const unsigned s = s0 + threadIdx.x;
+            const bool some = s < md.n && !(row[s] == 0.0f);
+            const unsigned bits = __ballot_sync(0xffffffffu, some);
+            if (lane == 0) found[warp] = __popc(bits);
+            __syncthreads();
+            unsigned place = support;
+            for (unsigned w = 0; w < kThreads / 32; w++) {
+                if (w < warp) place += found[w];
+                support += found[w];
+            }
+            if (some) states[place + __popc(bits & ((1u << lane) - 1u))] = s;
+            __syncthreads();
+        }
         const float cut = bound[ao] + 2.0f * err;
         float low = NOVA_FLT_MAX;
         for (unsigned j0 = warp * 32; j0 < md.r; j0 += kThreads) {
@@ -423,23 +524,39 @@ __global__ void __launch_bounds__(kThreads) distinct_select_kernel(ExpModel md, 
                 }
                 near = !(mass[ao] + (2.0f * acc - d.total[j]) > cut);
             }
-            for (unsigned msk = __ballot_sync(0xffffffffu, near); msk != 0; msk &= msk - 1) {
-                const unsigned jj = j0 + __ffs(msk) - 1;
-                float dist = 0.0f;
-                for (unsigned s0 = 0; s0 < md.n; s0 += 32) {
-                    const unsigned s = s0 + lane;
-                    terms[warp][lane] = s < md.n ? fabsf(__fsub_rn(md.BT[(size_t)s * md.r + jj], row[s])) : 0.0f;
-                    __syncwarp();
-                    const unsigned cnt = min(32u, md.n - s0);
-                    if (lane == 0)
-#pragma unroll 8
-                        for (unsigned q = 0; q < cnt; q++) dist = fadd(dist, terms[warp][q]);
-                    __syncwarp();
+            // Zeros of both add nothing to the sum, so a lane can walk the
+            // nonzeros of its belief and of the successor side by side (about
+            // 100 cycles each, 32 beliefs at once), or the warp one belief after
+            // the other over all states (700 cycles per 128).
+            const unsigned msk = __ballot_sync(0xffffffffu, near);
+            const unsigned mine = near ? d.nnz[j] : 0u;
+            const unsigned steps = support + __reduce_max_sync(0xffffffffu, mine);
+            if (__popc(msk) * ((md.n + 127u) / 128u) * 7u > steps) {
+                if (near) {
+                    const uint2 *list = d.list + (size_t)j * d.cap;
+                    uint2 e = mine != 0 ? list[0] : make_uint2(kNoIndex, 0u);
+                    unsigned at = support != 0 ? states[0] : kNoIndex;
+                    float dist = 0.0f;
+                    for (unsigned k = 0, q = 0; k < mine || q < support;) {
+                        const unsigned s = min(e.x, at);
+                        const float b = e.x == s ? __uint_as_float(e.y) : 0.0f;
+                        dist = fadd(dist, fabsf(__fsub_rn(b, row[s])));
+                        if (at == s) at = ++q < support ? states[q] : kNoIndex;
+                        if (e.x == s) e = ++k < mine ? list[k] : make_uint2(kNoIndex, 0u);
+                    }
+                    if (dist < low) low = dist;
                 }
-                dist = __shfl_sync(0xffffffffu, dist, 0);
-                if (dist < low) low = dist;
+            } else {
+                for (unsigned left = msk; left != 0; left &= left - 1) {
+                    const unsigned jj = j0 + __ffs(left) - 1;
+                    const float dist = warp_ordered_sum(md.n, terms[warp], lane, [&](unsigned s) {
+                        return fabsf(__fsub_rn(__ldg(md.BT + (size_t)s * md.r + jj), row[s]));
+                    });
+                    if (dist < low) low = dist;
+                }
             }
         }
+        for (int off = 16; off > 0; off >>= 1) low = fminf(low, __shfl_xor_sync(0xffffffffu, low, off));
         __syncthreads();
         if (lane == 0) red[warp] = low;
         __syncthreads();
@@ -705,7 +822,7 @@ int build_workspace(const POMDP *p, ExpWorkspace &ws, const char *fn) {
         return NOVA_ERROR_INVALID_DATA;
     }
     allow_dynamic_smem(distinct_mass_kernel, ws.smem);
-    allow_dynamic_smem(distinct_select_kernel, ws.smem);
+    allow_dynamic_smem(distinct_select_kernel, 3 * (size_t)n * sizeof(float));
     allow_dynamic_smem(random_kernel, ws.smem);
     allow_dynamic_smem(pema_kernel, ws.smem);
     allow_dynamic_smem(update_one_kernel, ws.smem);
@@ -856,11 +973,14 @@ int run_distinct(const ExpWorkspace &ws, std::vector<float> &Bnew, const char *f
         part.chunk = count;
         distinct_mass_kernel<<<count * md.m, kThreads, n * sizeof(float)>>>(md, part);
         if ((rc = check_launch(fn, "successor masses")) != NOVA_SUCCESS) return rc;
-        distinct_rows_kernel<<<ceil_div((size_t)count * mz, kThreads), kThreads>>>(md, part);
+        if ((size_t)count * mz <= kFewRows)
+            distinct_few_rows_kernel<<<ceil_div((size_t)count * mz, kThreads / 32), kThreads>>>(md, part);
+        else
+            distinct_rows_kernel<<<ceil_div((size_t)count * mz, kThreads), kThreads>>>(md, part);
         if ((rc = check_launch(fn, "successor beliefs")) != NOVA_SUCCESS) return rc;
         bound<<<count * ceil_div(mz, rows), 1024, boundSmem>>>(md, part);
         if ((rc = check_launch(fn, "distance bounds")) != NOVA_SUCCESS) return rc;
-        distinct_select_kernel<<<count, kThreads, 2 * n * sizeof(float)>>>(md, part, dB);
+        distinct_select_kernel<<<count, kThreads, 3 * n * sizeof(float)>>>(md, part, dB);
         if ((rc = check_launch(fn, "distinct beliefs")) != NOVA_SUCCESS) return rc;
     }
     Bnew.assign(rn, 0.0f);

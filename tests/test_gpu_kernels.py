@@ -632,3 +632,12 @@ def test_shared_memory_just_below_the_default_limit(what):
     code = ("import numpy as np\nfrom nova_gb300 import synth, nova_pomdp_pbvi as npp\nfrom nova_gb300.pomdp import POMDP\n"
             "from nova_gb300.pomdp_pbvi import POMDPPBVIGPU\n" + code)
     assert subprocess.run([sys.executable, "-c", code], cwd=ROOT, timeout=120).returncode == 0
+
+
+@pytest.mark.parametrize("n,m,z,r,rz,odd", [(127, 2, 3, 5, 6, ""), (129, 1, 4, 40, 129, ""), (3000, 2, 2, 70, 4, ""),
+                                            (3000, 2, 2, 9, 2000, "same"), (2500, 1, 3, 70, 3, "infinite"),
+                                            (300, 8, 16, 257, 9, ""), (300, 8, 16, 255, 9, "same")])
+def test_distinct_expansion_forms(n, m, z, r, rz, odd):
+    """Rows by a warp and by a thread each, and exact sums over the nonzeros
+    (many beliefs equally far) and over all states."""
+    test_distinct_expansion(n, m, z, r, rz, odd)

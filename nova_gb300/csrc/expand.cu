@@ -589,15 +589,27 @@ __global__ void __launch_bounds__(kThreads) random_kernel(ExpModel md, const uns
     extern __shared__ __align__(16) float smem[];
     __shared__ float slot;
     __shared__ unsigned chosen;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     BlockBufs w = carve(smem, md.n);
+    float *terms = smem + (2 * md.n + 3) / 4 * 4 + warp * 128;   // where aux and tmp are not needed
     const unsigned k = blockIdx.x;
     volatile float *pr = probs + (size_t)k * md.z;
     load_belief(md, start[k], w.b);
     for (unsigned q = first[k]; q < first[k + 1]; q++) {
         const Step st = steps[q];
-        // Every observation's probability is a chain of n additions, one
-        // thread each side by side.
-        for (unsigned o = threadIdx.x; o < md.z; o += blockDim.x) pr[o] = prob_obs_dense(md, w.b, st.a, o);
+        // Every observation's probability is a chain of n additions, side by
+        // side: a warp each, or with more observations than eight rounds of
+        // the block's warps a thread each.
+        if (md.z <= kThreads / 4) {
+            for (unsigned o = warp; o < md.z; o += kThreads / 32) {
+                const float *po = md.PO + (size_t)st.a * md.n * md.z + o;
+                const float p = warp_ordered_sum(md.n, terms, lane,
+                                                 [&](unsigned s) { return fmul(__ldg(po + (size_t)s * md.z), w.b[s]); });
+                if (lane == 0) pr[o] = p;
+            }
+        } else {
+            for (unsigned o = threadIdx.x; o < md.z; o += blockDim.x) pr[o] = prob_obs_dense(md, w.b, st.a, o);
+        }
         __syncthreads();
         if (threadIdx.x == 0) {
             float cur = 0.0f;
@@ -892,7 +904,8 @@ int run_random(const POMDP *p, unsigned total, bool fromB0, std::vector<float> &
         if ((rc = h2d(dSteps, steps.data(), steps.size() * sizeof(Step), fn, "the trajectory steps")) != NOVA_SUCCESS)
             return rc;
         if ((rc = dev_alloc(&dProbs, s2.size() * p->z, fn, "the observation draws")) != NOVA_SUCCESS) return rc;
-        random_kernel<<<(unsigned)s2.size(), kThreads, ws.smem>>>(ws.md, dStart, dFirst, dSteps, fromB0 ? 0 : 1, dProbs,
+        const size_t smem = std::max(ws.smem, (round_up(2 * n, 4) + kThreads / 32 * 128) * sizeof(float));
+        random_kernel<<<(unsigned)s2.size(), kThreads, smem>>>(ws.md, dStart, dFirst, dSteps, fromB0 ? 0 : 1, dProbs,
                                                                   dB);
         if ((rc = check_launch(fn, "random trajectories")) != NOVA_SUCCESS) return rc;
     }

@@ -641,3 +641,21 @@ def test_distinct_expansion_forms(n, m, z, r, rz, odd):
     """Rows by a warp and by a thread each, and exact sums over the nonzeros
     (many beliefs equally far) and over all states."""
     test_distinct_expansion(n, m, z, r, rz, odd)
+
+
+@pytest.mark.parametrize("n,z", [(5, 2), (127, 3), (128, 9), (129, 64), (700, 65), (2051, 4), (14272, 2)])
+def test_random_expansion_sums(n, z):
+    """Observation probabilities by a warp and by a thread each, chunks of 128
+    states with remainders, and the most states that are accepted."""
+    from nova_gb300 import nova_pomdp as npm
+    md = synth.random_pomdp(n=n, m=2, z=z, ns=min(4, n), r=7, rz=min(5, n), gamma=0.9, horizon=9, seed=n)
+    npm._nova.nova_gb300_expand_seed(1, 77)
+    try:
+        p = POMDP.from_arrays(md)
+        p.expand(method="random", numBeliefsToAdd=30)
+    finally:
+        npm._nova.nova_gb300_expand_seed(0, 0)
+    Z, B = orc.merge_raw_beliefs(md["Z"], md["B"], orc.expand_random(md, 30, 77))
+    out = p.arrays()
+    np.testing.assert_array_equal(out["Z"], Z)
+    np.testing.assert_array_equal(bits(out["B"]), bits(B))

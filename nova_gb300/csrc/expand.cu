@@ -189,7 +189,8 @@ __device__ float min_distance(const ExpModel &md, const float *bp, unsigned *arg
     unsigned bj = kNoIndex;
     for (unsigned j = threadIdx.x; j < md.r; j += blockDim.x) {
         float d = 0.0f;
-        for (unsigned s = 0; s < md.n; s++) d = fadd(d, fabsf(__fsub_rn(md.BT[(size_t)s * md.r + j], bp[s])));
+#pragma unroll 8
+        for (unsigned s = 0; s < md.n; s++) d = fadd(d, fabsf(__fsub_rn(__ldg(md.BT + (size_t)s * md.r + j), bp[s])));
         if (d < best) { best = d; bj = j; }
     }
     sv[threadIdx.x] = best;
@@ -641,6 +642,7 @@ __global__ void __launch_bounds__(kThreads) pema_kernel(ExpModel md, unsigned pr
     __shared__ float slot, sv[kThreads];
     __shared__ unsigned si[kThreads];
     __shared__ unsigned alphaStar, closest;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     BlockBufs w = carve(smem, md.n);
     const unsigned i = blockIdx.x;
     load_belief(md, i, w.b);
@@ -694,10 +696,18 @@ __global__ void __launch_bounds__(kThreads) pema_kernel(ExpModel md, unsigned pr
             // Gamma_j(s) * bc(s) below -1e10 (its running value never moves).
             if (threadIdx.x == 0) alphaStar = 0;
             __syncthreads();
-            for (unsigned j = threadIdx.x; j < pr; j += blockDim.x) {
+            for (unsigned j = warp; j < pr; j += kThreads / 32) {
                 bool hit = false;
-                for (unsigned s = 0; s < md.n && !hit; s++) hit = fmul(Gamma[(size_t)j * md.n + s], bc[s]) < NOVA_FLT_MIN;
-                if (hit) atomicMax(&alphaStar, j);
+                for (unsigned s0 = 0; s0 < md.n && !hit; s0 += 128) {
+                    bool below = false;
+#pragma unroll
+                    for (unsigned q = 0; q < 4; q++) {
+                        const unsigned s = s0 + 32 * q + lane;
+                        if (s < md.n) below |= fmul(__ldg(Gamma + (size_t)j * md.n + s), bc[s]) < NOVA_FLT_MIN;
+                    }
+                    hit = __any_sync(0xffffffffu, below);
+                }
+                if (hit && lane == 0) atomicMax(&alphaStar, j);
             }
             __syncthreads();
             const float *g = Gamma + (size_t)alphaStar * md.n;

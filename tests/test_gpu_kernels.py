@@ -659,3 +659,25 @@ def test_random_expansion_sums(n, z):
     out = p.arrays()
     np.testing.assert_array_equal(out["Z"], Z)
     np.testing.assert_array_equal(bits(out["B"]), bits(B))
+
+
+@pytest.mark.parametrize("n,r,pr,low", [(31, 3, 9, 0), (128, 40, 40, 3), (129, 9, 300, 7), (700, 260, 65, 2)])
+def test_pema_alpha_search(n, r, pr, low):
+    """The last alpha with a product below -1e10 anywhere: none, few, in the
+    first and last states."""
+    import ctypes as ct
+    from nova_gb300 import nova_pomdp as npm, nova_pomdp_alpha_vectors as npav
+    md = synth.random_pomdp(n=n, m=2, z=3, ns=3, r=r, rz=4, gamma=0.9, horizon=3, seed=n)
+    G = np.random.default_rng(n).normal(size=(pr, n)).astype(np.float32)
+    for k in range(low):
+        G[(5 * k) % pr, (n - 1) * (k % 2)::17] = -1e13
+    pi = np.zeros(pr, np.uint32)
+    pol = npav.NovaPOMDPAlphaVectors()
+    pol.n, pol.m, pol.r = n, 2, pr
+    pol.Gamma, pol.pi = G.ctypes.data_as(ct.POINTER(ct.c_float)), pi.ctypes.data_as(ct.POINTER(ct.c_uint))
+    p = POMDP.from_arrays(md)
+    assert npm._nova.pomdp_expand_pema_cpu(p, ct.byref(pol)) == 0
+    Z, B = orc.merge_raw_beliefs(md["Z"], md["B"], orc.expand_pema(md, G)[None, :])
+    out = p.arrays()
+    np.testing.assert_array_equal(out["Z"], Z)
+    np.testing.assert_array_equal(bits(out["B"]), bits(B))

@@ -8,7 +8,8 @@
 // solve (152 SMs hold about 3.9 M entries), and a sweep is the gathers of V,
 // the action scan and one barrier across the grid: 300 rows take 2.2 us, 120,000
 // rows of ten 5.1 us. V is read past L1, which would keep the values of two
-// sweeps before, or copied into shared memory first where that moves less.
+// sweeps before, or copied into shared memory first where that moves less. Where
+// its gathers are the slower ones the ordinary sweeps run (vi_resident_sweeps).
 //
 // Order of operations as mdp_vi_cpu.cpp:36-63: Q = R(s,a), then Q += (gamma *
 // T) * V[s'] in list order up to the row's first negative entry, gamma * T
@@ -35,6 +36,9 @@ constexpr unsigned kMaxThreads = 1024;
 constexpr unsigned kBatch = 8;                    // successors whose values are in flight together
 constexpr unsigned kSweepsPerLaunch = 4096;
 constexpr long long kWaitCycles = 4000000000ll;   // ~2 s at 2 GHz
+// Models whose V does not fit beside their entries (vi_resident_sweeps).
+constexpr unsigned long long kGatherSmem = 196 * 1024, kL1Entries = 2000000;
+constexpr unsigned kL1States = 52000;
 
 // One arrival per block; returns once `target` blocks have arrived in this
 // launch, or false if a wait ran out here or elsewhere.
@@ -186,6 +190,12 @@ int vi_resident_sweeps(const MDP *mdp, const int *S, const float *T, const float
     // A gather moves a 32-byte sector, a copied value 4 bytes (n = 20,000, m =
     // 6, ns = 10, 7,900 gathers a block: 5.1 us a sweep copied, 10.2 gathered).
     const bool shared = base + n * sizeof(float) + reserve <= (unsigned long long)optin && n <= 4 * rows * ns;
+    // Gathering pays while the SM keeps 60 KB of L1 for the loads in flight (up to
+    // 196 KB of shared memory; us a sweep, resident and plain: 3.3 M entries 14 to
+    // 19 and 17 to 24, 3.8 M 26 and 22), and against plain sweeps whose gathers
+    // hit L1 only for fewer entries (n = 30,000 to 40,000: 1.3 M 9.5 and 13, 2.8 M
+    // 20 and 15; n = 58,000, 2.8 M 16 and 16).
+    if (!shared && (base + reserve > kGatherSmem || (n < kL1States && allRows * ns > kL1Entries))) return NOVA_SUCCESS;
     const size_t smem = (size_t)(base + (shared ? n * sizeof(float) : 0));
     const unsigned threads = (unsigned)std::min<unsigned long long>(kMaxThreads, std::max<unsigned long long>(128, pitch));
     const void *kernel = shared ? (const void *)vi_resident_kernel<true> : (const void *)vi_resident_kernel<false>;

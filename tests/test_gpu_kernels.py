@@ -681,3 +681,10 @@ def test_pema_alpha_search(n, r, pr, low):
     out = p.arrays()
     np.testing.assert_array_equal(out["Z"], Z)
     np.testing.assert_array_equal(bits(out["B"]), bits(B))
+
+
+@pytest.mark.parametrize("n,m,ns,horizon", [(30000, 16, 8, 3), (51999, 10, 4, 2), (51999, 7, 6, 3), (52000, 8, 6, 3),
+                                            (100000, 4, 9, 2), (250000, 2, 7, 4)])
+def test_resident_sweep_limits(n, m, ns, horizon):
+    """Models just within and beyond what the resident sweeps take."""
+    test_resident_sweeps(n, m, ns, horizon, "gpu")

@@ -1386,12 +1386,6 @@ int BackupEngine::scan_rows_direct(const unsigned *rowList, unsigned nRows, unsi
     return exact_score(items, nItems, nU, fn);
 }
 
-int BackupEngine::fill_items(unsigned first, unsigned count, const char *fn) {
-    if (count == 0) return NOVA_SUCCESS;
-    iota_items_kernel<<<ceil_div(count, 256), 256, 0, stream>>>(items, count, first);
-    return check_launch(fn, "work list");
-}
-
 int BackupEngine::assemble(const float *src, float *dst, unsigned *pi, const char *fn) {
     int rc;
     const unsigned nItems = md.r * md.m;

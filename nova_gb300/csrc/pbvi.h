@@ -171,8 +171,6 @@ struct BackupEngine {
     bool projRowsAttrDone = false; // and of the alpha-contiguous one
     float lastScanFrac = 0.0f;     // share of rows the last tensor-core update left to the exact scan
     bool state_major_wanted(bool tensor) const;
-    // Work list of `count` consecutive items starting at `first`.
-    int fill_items(unsigned first, unsigned count, const char *fn);
     // Write the last backup's selections (action per belief, alpha per
     // (belief, observation) under that action) to device arrays.
     int record(const unsigned *pi, unsigned *actOut, unsigned *selOut, const char *fn);

@@ -142,8 +142,8 @@ static int execute_batched(const POMDP *const *pomdps, POMDPPBVIGPU *const *solv
 //   2. Lock-step backups (one host thread, one stream per solver): every
 //      backup of every solver runs without host read-backs (the fixed update
 //      of graph mode); each solver's projection table and alpha packing are
-//      queued on its own stream, one persistent tcgen05 launch per list
-//      length scores the work units of all tensor-core solvers from a device
+//      queued on its own stream, one persistent tcgen05 launch per operand
+//      form scores the work units of all tensor-core solvers from a device
 //      table of their tensor maps and shapes, and each solver's merge, exact
 //      scan and assembly follow on its stream. The table is rebuilt only when
 //      the set of solvers still running changes.

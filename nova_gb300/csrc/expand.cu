@@ -460,6 +460,10 @@ __global__ void __launch_bounds__(1024) distinct_bound_kernel(ExpModel md, Disti
 // distance becomes the new belief. With many states the error is wide and
 // distances that are exactly equal (disjoint supports) are common: n = 12,000,
 // r = 50 took 37 ms with every sum over all states, 0.23 so.
+// Below kWalkStates the successor's list costs more than it saves (n = 512: 15 to
+// 35 of 240 us; n = 1,000: 124 us without, 87 with).
+constexpr unsigned kWalkStates = 768;
+
 __global__ void __launch_bounds__(kThreads) distinct_select_kernel(ExpModel md, Distinct d, float *__restrict__ Bnew) {
     extern __shared__ __align__(16) float smem[];
     __shared__ float red[kThreads / 32];
@@ -495,8 +499,9 @@ __global__ void __launch_bounds__(kThreads) distinct_select_kernel(ExpModel md, 
         __syncthreads();
         for (unsigned s = threadIdx.x; s < md.n; s += blockDim.x) row[s] = d.bp[((size_t)i * md.n + s) * mz + ao];
         __syncthreads();
+        const bool walks = md.n >= kWalkStates;
         unsigned support = 0;
-        for (unsigned s0 = 0; s0 < md.n; s0 += kThreads) {
+        for (unsigned s0 = 0; walks && s0 < md.n; s0 += kThreads) {
             const unsigned s = s0 + threadIdx.x;
             const bool some = s < md.n && !(row[s] == 0.0f);
             const unsigned bits = __ballot_sync(0xffffffffu, some);
@@ -532,7 +537,7 @@ __global__ void __launch_bounds__(kThreads) distinct_select_kernel(ExpModel md, 
             const unsigned msk = __ballot_sync(0xffffffffu, near);
             const unsigned mine = near ? d.nnz[j] : 0u;
             const unsigned steps = support + __reduce_max_sync(0xffffffffu, mine);
-            if (__popc(msk) * ((md.n + 127u) / 128u) * 7u > steps) {
+            if (walks && __popc(msk) * ((md.n + 127u) / 128u) * 7u > steps) {
                 if (near) {
                     const uint2 *list = d.list + (size_t)j * d.cap;
                     uint2 e = mine != 0 ? list[0] : make_uint2(kNoIndex, 0u);

@@ -180,7 +180,7 @@ NOVA_API int pomdp_pbvi_execute_batched_graph_gpu(const POMDP *const *pomdps, PO
  * cheaper also times one update with exact scoring and keeps it if it is);
  * from then on every backup of every solver is queued without host
  * read-backs on a stream of its own, and one persistent tcgen05 scoring
- * launch (per operand form) draws the work units of all
+ * launch (per operand form and kind of candidate list) draws the work units of all
  * tensor-core solvers from a device table of their tensor maps, shapes and
  * candidate arrays. The batch runs in waves whose solvers fit in device
  * memory together. Replaces the reference's one-solve-per-call structure

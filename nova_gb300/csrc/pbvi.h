@@ -212,8 +212,8 @@ int tc_finish(BackupEngine &eng, const char *fn);
 // The distinct (belief, action) items of the listed rows into eng.items
 // (count in eng.itemCount, on the device).
 int tc_rows_to_items(BackupEngine &eng, const unsigned *rowList, unsigned nRows, const char *fn);
-// One persistent scoring launch (per operand form) over the work
-// units of many prepared solvers, drawn from a device table of their
+// One persistent scoring launch (per operand form and kind of
+// candidate list) over the work units of many prepared solvers, drawn from a device table of their
 // tensor maps, shapes and candidate arrays; the table is built once from
 // the solvers' prepared launches and stays valid while their schedules,
 // operands and alpha counts do.
